@@ -1,6 +1,8 @@
-"""Python host-side mirror of the C ABI in ``include/gie_b200.h`` (ctypes; no torch types cross the boundary).
+"""Python host-side mirror of the C ABI in ``include/gie_b200.h`` (no torch types cross the boundary).  Plans, queries and
+status words go through ctypes; the calls a program makes once per layer go through the extension module ``_calls``
+(csrc/python_calls.cpp), which costs the host a fifth of a ctypes call.
 
-The native library ``libgie_b200.so`` is built in-tree by ``build.py``.  Importing this package never falls back to
+The native library ``libgie_b200.so`` and ``_calls.so`` are built in-tree by ``build.py``.  Importing this package never falls back to
 any other implementation: if the library is missing, loading raises.  Device memory and streams come from the caller
 (raw integer device pointers and a ``cudaStream_t`` value), exactly as in the reference's operator API.
 
@@ -10,6 +12,7 @@ Because the directory name contains a hyphen, load the package with ``importlib`
 from __future__ import annotations
 
 import ctypes as C
+import importlib
 import os
 from dataclasses import dataclass
 
@@ -56,11 +59,12 @@ class RmsNormDesc(C.Structure):
 
 
 _lib = None
+_calls = None  # the extension module, loaded with the library
 
 
 def lib() -> C.CDLL:
     """Loads the native library once; raises if it has not been built (there is no fallback path)."""
-    global _lib
+    global _lib, _calls
     if _lib is None:
         if not os.path.exists(LIB_PATH):
             raise ImportError(f"{LIB_PATH} is missing: run `python {os.path.join(HERE, 'build.py')}` (needs nvcc, no GPU)")
@@ -92,16 +96,24 @@ def lib() -> C.CDLL:
         L.gieb_maxpool2d_launch.argtypes = [i32] * 8 + [vp, vp, vp]
         L.gieb_maxpool2d_nhwc_launch.argtypes = [i32] * 8 + [vp, vp, vp]
         L.gieb_add_relu_launch.argtypes = [i32, i32, vp, vp, vp, i64, vp]
+        _calls = importlib.import_module("._calls", __name__)
         _lib = L
     return _lib
+
+
+def calls():
+    """The extension module of per-layer calls; raises like lib() if it has not been built."""
+    lib()
+    return _calls
 
 
 def last_error() -> str:
     return lib().gieb_last_error().decode("utf-8", "replace")
 
 
-def check(status: int) -> None:
-    if status != OK:
+def check(status: int | None) -> None:
+    """Raises the failure a call reported (0, or None from the extension module, is success)."""
+    if status:
         raise GieError(status, last_error())
 
 
@@ -169,6 +181,7 @@ class ConvPlan:
         self._h = C.c_void_p()
         check(lib().gieb_conv_plan_create(C.byref(problem.desc()), C.byref(cfg) if cfg is not None else None, device,
                                           C.byref(self._h)))
+        self._plan = self._h.value  # the handle as a number, for the extension module
         self.info = ConvInfo()
         check(lib().gieb_conv_plan_info(self._h, C.byref(self.info)))
 
@@ -178,7 +191,9 @@ class ConvPlan:
 
     def launch(self, x: int, w: int, bias: int | None, y: int, workspace: int | None, workspace_bytes: int, stream: int = 0) -> None:
         """execute_unchecked: raw device pointers, asynchronous on `stream`."""
-        check(lib().gieb_conv_launch(self._h, x, w, bias, y, workspace, workspace_bytes, stream))
+        status = _calls.conv_launch(self._plan, x, w, bias, y, workspace, workspace_bytes, stream)
+        if status:
+            check(status)
 
     @property
     def prepacked_weight_bytes(self) -> int:
@@ -194,7 +209,9 @@ class ConvPlan:
                      stream: int = 0) -> None:
         """launch() with a residual tensor (shape, layout and type of y) added before the activation; for plans whose
         problem carries FLAG_RESIDUAL."""
-        check(lib().gieb_conv_launch_fused(self._h, x, w, bias, residual, y, workspace, workspace_bytes, stream))
+        status = _calls.conv_launch_fused(self._plan, x, w, bias, residual, y, workspace, workspace_bytes, stream)
+        if status:
+            check(status)
 
     def launch_stages(self, stage_mask: int, x: int, w: int, bias: int | None, y: int, workspace: int | None, workspace_bytes: int,
                       stream: int = 0) -> None:
@@ -222,6 +239,7 @@ class ConvPlan:
         if self._h:
             lib().gieb_conv_plan_destroy(self._h)
             self._h = C.c_void_p()
+            self._plan = None
 
     def __del__(self):
         try:
@@ -257,24 +275,25 @@ def prepack_weights(src: int, dst: int, out_channels: int, channels: int, rs: in
 def rmsnorm_forward(rows: int, hidden: int, eps: float, dtype: int, x: int, gamma: int, y: int, residual_in: int | None = None,
                     residual_out: int | None = None, stream: int = 0, gamma_fp32: bool = False) -> None:
     """gie::rmsnorm_forward on raw device pointers; dtype uses gie::DataType order (0 fp32, 1 fp16, 2 bf16)."""
-    d = RmsNormDesc(rows, hidden, eps, dtype, 1 if gamma_fp32 else 0)
-    check(lib().gieb_rmsnorm_launch(C.byref(d), x, gamma, y, residual_in, residual_out, stream))
+    status = (_calls or calls()).rmsnorm_launch(rows, hidden, eps, dtype, 1 if gamma_fp32 else 0, x, gamma, y, residual_in, residual_out, stream)
+    if status:
+        check(status)
 
 
 def bias_act(precision: int, batch: int, channels: int, hw: int, bias: int | None, relu: bool, y: int, stream: int = 0) -> None:
-    check(lib().gieb_bias_act_launch(precision, batch, channels, hw, bias, int(relu), y, stream))
+    check(calls().bias_act_launch(precision, batch, channels, hw, bias, int(relu), y, stream))
 
 
 def maxpool2d(precision: int, batch: int, channels: int, h: int, w: int, kernel: int, stride: int, pad: int, x: int, y: int,
               stream: int = 0) -> None:
-    check(lib().gieb_maxpool2d_launch(precision, batch, channels, h, w, kernel, stride, pad, x, y, stream))
+    check(calls().maxpool2d_launch(precision, batch, channels, h, w, kernel, stride, pad, x, y, stream))
 
 
 def maxpool2d_nhwc(precision: int, batch: int, channels: int, h: int, w: int, kernel: int, stride: int, pad: int, x: int, y: int,
                    stream: int = 0) -> None:
     """maxpool2d on channel-contiguous [B][H][W][C] tensors (fp16 / bf16, C % 8 == 0)."""
-    check(lib().gieb_maxpool2d_nhwc_launch(precision, batch, channels, h, w, kernel, stride, pad, x, y, stream))
+    check(calls().maxpool2d_nhwc_launch(precision, batch, channels, h, w, kernel, stride, pad, x, y, stream))
 
 
 def add_relu(precision: int, relu: bool, a: int, b: int, y: int, n: int, stream: int = 0) -> None:
-    check(lib().gieb_add_relu_launch(precision, int(relu), a, b, y, n, stream))
+    check(calls().add_relu_launch(precision, int(relu), a, b, y, n, stream))

@@ -1,17 +1,21 @@
 """Builds the native library in-tree: every .cu under csrc/ is compiled for sm_100a with nvcc and linked into
-``libgie_b200.so`` beside this file.  No GPU is needed to build.  Usage: ``python build.py [--force] [--verbose]``."""
+``libgie_b200.so`` beside this file, and csrc/python_calls.cpp becomes the extension module ``_calls.so`` on top of it.
+No GPU is needed to build.  Usage: ``python build.py [--force] [--verbose]``."""
 from __future__ import annotations
 
 import concurrent.futures as cf
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libgie_b200.so")
+CALLS_SRC = os.path.join(CSRC, "python_calls.cpp")
+CALLS = os.path.join(HERE, "_calls.so")
 
 NVCC_FLAGS = ["-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
               "-Xcompiler", "-fPIC,-fvisibility=hidden,-Wall", "-I" + os.path.join(ROOT, "include"), "-I" + CSRC]
@@ -63,6 +67,13 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
+    if force or _stale(CALLS, [CALLS_SRC, os.path.join(ROOT, "include", "gie_b200.h")]):
+        cmd = ["g++", "-std=c++17", "-O2", "-Wall", "-fPIC", "-fvisibility=hidden", "-shared", "-I" + sysconfig.get_paths()["include"],
+               "-I" + os.path.join(ROOT, "include"), CALLS_SRC, LIB, "-Wl,-rpath,$ORIGIN", "-o", CALLS]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
+            raise RuntimeError("building _calls.so failed")
     return LIB
 
 

@@ -7,8 +7,8 @@ from __future__ import annotations
 
 import math
 
-from . import (ConvPlan, ConvProblem, GieError, add_relu, make_cfg, maxpool2d, maxpool2d_nhwc, FLAG_INPUT_NHWC, FLAG_OUTPUT_NHWC,
-               FLAG_RESIDUAL, FLAG_WEIGHTS_PREPACKED)
+from . import (ConvPlan, ConvProblem, GieError, calls, check, make_cfg, FLAG_INPUT_NHWC, FLAG_OUTPUT_NHWC, FLAG_RESIDUAL,
+               FLAG_WEIGHTS_PREPACKED)
 from .workloads import FP16, BF16, chain_flops, fuse_residuals, resnet50_chain
 
 
@@ -137,6 +137,7 @@ class ConvChain:
         self.ws_ptr = (self._ws.data_ptr() + 255) // 256 * 256
         self.ws_bytes = ws_bytes
         self.launches = sum(p.info.launches for _, p, _, _ in self.convs) + sum(1 for op in self.ops if op.kind != "conv")
+        self._steps = self._record()
         self.graph = None
 
     def _tuned_plan(self, problem: ConvProblem, op) -> ConvPlan:
@@ -192,27 +193,40 @@ class ConvChain:
     def output(self):
         return self.slots[len(self.slots) - 1]
 
-    def enqueue(self, stream: int) -> None:
-        """All launches of one forward pass on `stream` (capture-safe: no allocation, no synchronisation)."""
+    def _buffers(self):
+        """What a recording holds pointers into."""
+        return [t.data_ptr() for t in self.slots.values()] + [id(c) for c in self.convs] + [self.ws_ptr]
+
+    def _record(self):
+        """The launches of one pass with every pointer filled in, for ``enqueue`` to issue from native code: a pass of 107
+        launches spends ~1.7 us of Python per launch otherwise.  The chain's buffers stay where they are; should one have
+        been replaced, ``enqueue`` records again."""
+        self._recorded = self._buffers()
         ci = 0
+        steps = []
         for op in self.ops:
+            src, dst = self.slots[op.src].data_ptr(), self.slots[op.dst].data_ptr()
             if op.kind == "conv":
                 _, plan, w, b = self.convs[ci]
                 ci += 1
                 if op.other >= 0 and self.fused:
-                    plan.launch_fused(self.slots[op.src].data_ptr(), w.data_ptr(), b.data_ptr(), self.slots[op.other].data_ptr(),
-                                      self.slots[op.dst].data_ptr(), self.ws_ptr, self.ws_bytes, stream)
+                    steps.append(("conv_launch_fused", plan._plan, src, w.data_ptr(), b.data_ptr(), self.slots[op.other].data_ptr(), dst, self.ws_ptr,
+                                  self.ws_bytes))
                 else:
-                    plan.launch(self.slots[op.src].data_ptr(), w.data_ptr(), b.data_ptr(), self.slots[op.dst].data_ptr(), self.ws_ptr,
-                                self.ws_bytes, stream)
+                    steps.append(("conv_launch", plan._plan, src, w.data_ptr(), b.data_ptr(), dst, self.ws_ptr, self.ws_bytes))
             elif op.kind == "maxpool":
                 c, h, w, k, s, p = op.pool
-                pool = maxpool2d_nhwc if self.layout == "nhwc" else maxpool2d
-                pool(self.precision, self.batch, c, h, w, k, s, p, self.slots[op.src].data_ptr(), self.slots[op.dst].data_ptr(), stream)
+                steps.append(("maxpool2d_nhwc_launch" if self.layout == "nhwc" else "maxpool2d_launch", self.precision, self.batch, c, h, w, k, s, p,
+                              src, dst))
             else:
-                n = self.slots[op.dst].numel()
-                add_relu(self.precision, op.relu, self.slots[op.src].data_ptr(), self.slots[op.other].data_ptr(),
-                         self.slots[op.dst].data_ptr(), n, stream)
+                steps.append(("add_relu_launch", self.precision, int(op.relu), src, self.slots[op.other].data_ptr(), dst, self.slots[op.dst].numel()))
+        return calls().record(steps)
+
+    def enqueue(self, stream: int) -> None:
+        """All launches of one forward pass on `stream` (capture-safe: no allocation, no synchronisation)."""
+        if self._recorded != self._buffers():
+            self._steps = self._record()
+        check(calls().run_sequence(self._steps, stream))
 
     def capture(self, stream) -> None:
         """Runs the chain once eagerly on `stream` (a torch.cuda.Stream), then captures it as one CUDA graph."""
