@@ -319,7 +319,8 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
     if (d.flags & (GIEB_FLAG_WEIGHTS_PREPACKED | GIEB_FLAG_INPUT_NHWC | GIEB_FLAG_OUTPUT_NHWC | GIEB_FLAG_RESIDUAL))
       return no("prepacked weights, channel-contiguous tensors and the fused residual apply to the 16-bit tensor path only");
     r->variant = 3;
-    r->tile_m = r->tile_n = conv_fp32_tile(g.pixels, d.out_channels);
+    r->tile_m = conv_fp32_tile_pixels(d.out_channels);
+    r->tile_n = conv_fp32_tile_channels(d.out_channels);
     r->tile_k = 16;
     r->stages = 2;
     r->split_k = 1;
@@ -586,7 +587,7 @@ void fill_info(const gieb_conv_desc& d, const Resolved& r, gieb_conv_info* out) 
   out->padded_channels = d.precision == GIEB_TF32 ? r.c_padded / 2 : (d.precision == GIEB_FP8_E4M3 ? r.c_padded * 2 : r.c_padded);
   if (r.variant == 3) {
     out->dynamic_smem_bytes = 0;
-    out->threads_per_block = r.tile_n == 64 ? 256 : 64;
+    out->threads_per_block = 128;
     out->num_blocks = conv_fp32_num_blocks(g.pixels, d.out_channels);
     out->launches = 1;
   } else {

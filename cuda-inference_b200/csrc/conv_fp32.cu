@@ -2,22 +2,35 @@
 // the bias + ReLU epilogue fused.  Stands in for implicit_gemm_kernel (src/kernels/implicit_gemm.cu:47-189).
 //
 // GEMM view: rows = output pixels (b, oh, ow), columns = output channels, k = (c, r, s) in OIHW order so a weight
-// row is contiguous in k.  Per CTA: a TP x TO output tile, 4x4 outputs per thread, BK = 16 reduction slab staged in
-// shared memory by asynchronous copies (pixels contiguous in the X slab, so the gather from NCHW is coalesced along ow;
-// 128-bit copies of W along k), a ring of slabs in flight while one is consumed.  Accumulation is fmaf in k order.
+// row is contiguous in k.  Per CTA of 128 threads: a TP x TO output tile (64 x 64, or 128 x 32 for few channels), 8 pixels x
+// 4 channels per thread, BK = 16 reduction slabs in a ring of shared-memory buffers (pixels contiguous in the X slab, so the
+// gather from NCHW is coalesced along ow; 128-bit copies of W along k).  Accumulation is fmaf in k order.
+//
+// What bounds it: with enough CTAs per SM, ~1030 cycles per 64 x 64 x 16 slab against 512 of FMA issue -- a thread reads 12
+// words of shared memory per 32 FMAs, and the SM delivers 128 bytes per cycle (8 x 8 tiles read less but leave 12 warps per SM,
+// too few to hide their latencies: 1120).  The packed FMA (fma.rn.f32x2, two adjacent pixels against a duplicated weight; each
+// half rounds as fmaf does) halves the FMA instructions.  Gathered elements pass through registers: a 4-byte asynchronous
+// copy per element keeps the load/store unit busy several times as long.  Problems with few tiles split the reduction over
+// the CTAs of a thread-block cluster, which exchange their partial tiles through distributed shared memory and add them in
+// slice order, so that results are run-to-run identical.  Measured against scalar FMAs on 32 x 32 tiles: 11 x 212 -> 560
+// channels, 17 x 17, 5x5 1004 -> 540 us; 512 -> 512, 7 x 7, 3x3 137 -> 31 us; 64 -> 64, 56 x 56, 3x3 18.4 -> 15.6 us.
 #include <stdint.h>
 
+#include <cmath>
 #include <mutex>
 #include <set>
+#include <type_traits>
 #include <utility>
 
 #include "internal.h"
+#include "ptx.cuh"
 
 namespace gieb {
 namespace {
 
 constexpr int kBK = 16;
-constexpr int kLutMax = 2048;  // reduction length up to which the (c, r, s) decode of k is tabulated in shared memory
+constexpr int kLutMax = 4096;  // reduction length of a CTA up to which the (c, r, s) decode of k is tabulated in shared memory
+constexpr int kMaxSmem = 96 * 1024;
 
 struct Fp32Args {
   const float* x;
@@ -27,6 +40,8 @@ struct Fp32Args {
   int batch, c, h, wd, o, r, s, stride_h, stride_w, pad_h, pad_w, out_h, out_w, relu;
   int pixels;  // batch * out_h * out_w
   int k;       // c * r * s
+  int slices;  // CTAs of a cluster that share one output tile, each reducing slabs_per_slice slabs
+  int slabs_per_slice;
   FastDiv fd_rs, fd_s, fd_pq, fd_out_w;  // multiply-high reciprocals of r*s, s, out_h*out_w, out_w
 };
 
@@ -44,41 +59,58 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 constexpr int kWPitch = kBK + 4;  // floats per weight row in shared memory: 16-byte aligned rows, conflict-free 128-bit reads
+constexpr int kThreads = 128;
+constexpr int kRing = 4;          // slabs in shared memory
 
-// KG = number of thread groups that split the reduction inside one CTA (slab s goes to group s % KG); their partial
-// accumulators are summed in a fixed order at the end, so results are deterministic.  KG > 1 gives small problems
-// (few CTAs, long dependent slab chains) enough warps per SM to hide global-load latency.
-// Operands reach shared memory through asynchronous copies (cp.async) into a ring of NS slabs per group, so the loads of
-// the next NS - 1 slabs are in flight while one is consumed and no register or store instruction is spent on staging:
-//   X slab [kBK][TP]: one 4-byte copy per element, gathered from NCHW with zero-fill for padding (pixels contiguous);
-//   W slab [TO][kBK]: 128-bit copies along k (OIHW rows are contiguous in k) when W16, else 4-byte copies.
+// Two FP32 values in one 64-bit register: the operands of fma.rn.f32x2.
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
+
+// X slab [kBK][TP]: gathered from NCHW element by element with zeros for padding (pixels contiguous), or, for unpadded 1x1
+//   kernels of stride 1 whose planes are multiples of 4 pixels (XVEC), 16-byte asynchronous copies along the pixels;
+// W slab [TO][kBK]: asynchronous copies, 16 bytes along k (OIHW rows are contiguous in k) when W16, else 4 bytes.
 // LUT: k -> (offset of (c, r, s) inside one image, r, s) comes from a table built once per CTA (the analogue of
 // build_conv_lut, src/kernels/conv_common.cu:25-37) instead of two divisions per gathered element.
-template <int TP, int TO, int KG, int NS, bool LUT, bool W16>
-__global__ void __launch_bounds__((TP / 4) * (TO / 4) * KG)
+// A cluster of `slices` CTAs (blockIdx.x = pixel tile * slices + slice) shares one output tile.
+template <int TP, int TO, bool LUT, bool W16, bool XVEC>
+__global__ void __launch_bounds__(kThreads)
 conv_fp32_kernel(const Fp32Args a) {
-  constexpr int NT = (TP / 4) * (TO / 4);  // threads per group
-  constexpr int XE = kBK * TP / NT;        // X-slab elements copied per thread
+  static_assert(TP / 8 * (TO / 4) == kThreads, "8 pixels x 4 channels per thread");
+  constexpr int GP = TP / 8, GO = TO / 4;          // thread grid over pixels and channels
+  constexpr int XE = kBK * TP / kThreads;          // X-slab elements loaded per thread
   constexpr int XS = kBK * TP, WS = TO * kWPitch;  // floats per X / W slab
-  extern __shared__ __align__(16) float tiles[];    // [KG][NS] X slabs, then [KG][NS] W slabs; reused for the group reduction
-  __shared__ int2 lut[LUT ? kLutMax : 1];
+  extern __shared__ __align__(16) float tiles[];    // [kRing] X slabs, [kRing] W slabs, the table; reused for the exchange of partial tiles
+  float* xs_base = tiles;
+  float* ws_base = tiles + kRing * XS;
+  int2* lut = reinterpret_cast<int2*>(tiles + kRing * (XS + WS));
 
-  const int grp = threadIdx.x / NT;
-  const int t = threadIdx.x - grp * NT;
-  const int tx = t % (TP / 4), ty = t / (TP / 4);
-  const int pix0 = blockIdx.x * TP, oc0 = blockIdx.y * TO;
+  const int t = threadIdx.x;
+  const int tx = t % GP, ty = t / GP;  // pixels tx*4 .. +3 and TP/2 + tx*4 .. +3; channels ty + GO*j
+  const int slice = a.slices > 1 ? int(blockIdx.x % unsigned(a.slices)) : 0;
+  const int pix0 = int(blockIdx.x / unsigned(a.slices)) * TP, oc0 = blockIdx.y * TO;
   const int rs = a.r * a.s;
   const int pq = a.out_h * a.out_w;
-  float* xs_base = tiles + size_t(grp) * NS * XS;
-  float* ws_base = tiles + size_t(KG) * NS * XS + size_t(grp) * NS * WS;
+  const int slabs_all = (a.k + kBK - 1) / kBK;
+  const int slab0 = slice * a.slabs_per_slice;
+  const int slabs = max(0, min(a.slabs_per_slice, slabs_all - slab0));
+  const int kbase = slab0 * kBK;
 
-  // Loader roles. X: thread owns pixel (t % TP) and slab rows (t / TP) + i * (NT / TP).
+  // Loader role for X: thread owns pixel (t % TP) and slab rows (t / TP) + i * (kThreads / TP).
   const int lp = t % TP;
   const int lpix = pix0 + lp;
   const bool lp_ok = lpix < a.pixels;
   int ih0 = 0, iw0 = 0;
   const float* xb = a.x;
-  if (lp_ok) {
+  if (!XVEC && lp_ok) {
     const int b = a.fd_pq.div(lpix), rem = lpix - b * pq;
     const int oh = a.fd_out_w.div(rem), ow = rem - oh * a.out_w;
     ih0 = oh * a.stride_h - a.pad_h;
@@ -86,60 +118,83 @@ conv_fp32_kernel(const Fp32Args a) {
     xb = a.x + size_t(b) * a.c * a.h * a.wd;
   }
   const int xoff0 = ih0 * a.wd + iw0;  // offset of tap (0, 0) of this pixel inside a channel plane (may be negative)
+  // XVEC: thread owns pixel group (t % (TP/4)) and slab rows (t / (TP/4)) + i * (kThreads / (TP/4)); a group of four pixels
+  // lies in one image because planes are multiples of four
+  const int vg = t % (TP / 4), vpix = pix0 + vg * 4;
+  const bool v_ok = XVEC && vpix < a.pixels;
+  if (v_ok) {
+    const int b = a.fd_pq.div(vpix);
+    xb = a.x + size_t(b) * a.c * pq + (vpix - b * pq);
+  }
+  ptx::grid_dep_wait();
   if (LUT) {
-    const int kend = (a.k + kBK * KG - 1) / (kBK * KG) * (kBK * KG);  // slabs beyond K read zeros
-    for (int k = threadIdx.x; k < kend; k += NT * KG) {
+    for (int i = t; i < slabs * kBK; i += kThreads) {
+      const int k = kbase + i;
       int2 e = make_int2(0, 0x7fff0000);  // r far outside every image: never loaded
       if (k < a.k) {
         const int c = a.fd_rs.div(k), q = k - c * rs;
         const int r = a.fd_s.div(q), sx = q - r * a.s;
         e = make_int2((c * a.h + r) * a.wd + sx, (r << 16) | sx);
       }
-      lut[k] = e;
+      lut[i] = e;
     }
     __syncthreads();
   }
 
-  // issue the copies of the slab that starts at reduction index k0 into ring slot `slot`
-  auto fetch = [&](int k0, int slot) {
-    float* xs = xs_base + slot * XS;
-    float* ws = ws_base + slot * WS;
+  // gathered elements of a slab: loaded into registers one slab ahead of their store into the ring
+  float xreg[XVEC ? 1 : XE];
+  auto load_x = [&](int sl) {
+    const int k0 = kbase + sl * kBK;
 #pragma unroll
     for (int i = 0; i < XE; ++i) {
-      const int kk = t / TP + i * (NT / TP);
+      const int kk = t / TP + i * (kThreads / TP);
       const int k = k0 + kk;
-      const float* src = a.x;
-      bool ok = false;
+      float v = 0.f;
       if (LUT) {
-        const int2 e = lut[k];
+        const int2 e = lut[sl * kBK + kk];
         const int ih = ih0 + (e.y >> 16), iw = iw0 + (e.y & 0xffff);
-        ok = lp_ok && unsigned(ih) < unsigned(a.h) && unsigned(iw) < unsigned(a.wd);
-        if (ok) src = xb + (e.x + xoff0);
+        if (lp_ok && unsigned(ih) < unsigned(a.h) && unsigned(iw) < unsigned(a.wd)) v = xb[e.x + xoff0];
       } else if (lp_ok && k < a.k) {
         const int c = a.fd_rs.div(k), q = k - c * rs;
         const int r = a.fd_s.div(q), sx = q - r * a.s;
         const int ih = ih0 + r, iw = iw0 + sx;
-        ok = ih >= 0 && ih < a.h && iw >= 0 && iw < a.wd;
-        if (ok) src = xb + (size_t(c) * a.h + ih) * a.wd + iw;
+        if (ih >= 0 && ih < a.h && iw >= 0 && iw < a.wd) v = xb[(size_t(c) * a.h + ih) * a.wd + iw];
       }
-      cp_async4(xs + kk * TP + lp, src, ok);
+      xreg[i] = v;
+    }
+  };
+  auto store_x = [&](int slot) {
+    float* xs = xs_base + slot * XS;
+#pragma unroll
+    for (int i = 0; i < XE; ++i) xs[(t / TP + i * (kThreads / TP)) * TP + lp] = xreg[i];
+  };
+  // issue the asynchronous copies of slab `sl` of this slice into ring slot `slot`
+  auto fetch = [&](int sl, int slot) {
+    float* xs = xs_base + slot * XS;
+    float* ws = ws_base + slot * WS;
+    const int k0 = kbase + sl * kBK;
+    if (XVEC) {
+#pragma unroll
+      for (int i = 0; i < kBK * TP / 4 / kThreads; ++i) {
+        const int kk = t / (TP / 4) + i * (kThreads / (TP / 4));
+        const bool ok = v_ok && k0 + kk < a.k;
+        cp_async16(xs + kk * TP + vg * 4, ok ? xb + size_t(k0 + kk) * pq : a.x, ok ? 16 : 0);
+      }
     }
     if (W16) {  // TO rows x 4 vectors of 4 k-values
 #pragma unroll
-      for (int i = 0; i < (TO * 4 + NT - 1) / NT; ++i) {
-        const int v = t + i * NT;
-        if (v < TO * 4) {
-          const int row = v >> 2, kq = (v & 3) * 4;
-          const int oc = oc0 + row, k = k0 + kq;
-          const int left = (oc < a.o && k < a.k) ? min(4, a.k - k) * 4 : 0;
-          cp_async16(ws + row * kWPitch + kq, left ? a.w + size_t(oc) * a.k + k : a.w, left);
-        }
+      for (int i = 0; i < TO * 4 / kThreads; ++i) {
+        const int v = t + i * kThreads;
+        const int row = v >> 2, kq = (v & 3) * 4;
+        const int oc = oc0 + row, k = k0 + kq;
+        const int left = (oc < a.o && k < a.k) ? min(4, a.k - k) * 4 : 0;
+        cp_async16(ws + row * kWPitch + kq, left ? a.w + size_t(oc) * a.k + k : a.w, left);
       }
     } else {
       const int wk = t % kBK;
 #pragma unroll
-      for (int i = 0; i < kBK * TO / NT; ++i) {
-        const int row = t / kBK + i * (NT / kBK);
+      for (int i = 0; i < kBK * TO / kThreads; ++i) {
+        const int row = t / kBK + i * (kThreads / kBK);
         const int oc = oc0 + row, k = k0 + wk;
         const bool ok = oc < a.o && k < a.k;
         cp_async4(ws + row * kWPitch + wk, ok ? a.w + size_t(oc) * a.k + k : a.w, ok);
@@ -147,116 +202,153 @@ conv_fp32_kernel(const Fp32Args a) {
     }
   };
 
-  float acc[4][4];
+  uint64_t acc[4][4];  // [pixel pair][channel]
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0;
 
-  // every group runs the same number of rounds (slabs beyond K copy zeros), so the barriers stay uniform
-  const int rounds = (a.k + kBK * KG - 1) / (kBK * KG);
 #pragma unroll
-  for (int s = 0; s < NS - 1; ++s) {  // prologue: NS - 1 slabs in flight
-    if (s < rounds) fetch((s * KG + grp) * kBK, s);
+  for (int s = 0; s < kRing - 1; ++s) {  // prologue: kRing - 1 slabs in flight
+    if (s < slabs) fetch(s, s);
     cp_async_commit();
   }
-  for (int rd = 0; rd < rounds; ++rd) {
-    cp_async_wait<NS - 2>();  // this thread's copies of slab rd have landed
-    __syncthreads();          // everyone's have; and everyone has finished reading the slot refilled below
-    if (rd + NS - 1 < rounds) fetch(((rd + NS - 1) * KG + grp) * kBK, (rd + NS - 1) % NS);
+  if (!XVEC && slabs > 0) {
+    load_x(0);
+    store_x(0);
+    if (slabs > 1) load_x(1);
+  }
+  for (int sl = 0; sl < slabs; ++sl) {
+    cp_async_wait<kRing - 2>();  // this thread's copies of slab sl have landed
+    __syncthreads();             // everyone's have; and everyone has finished reading the slots refilled below
+    if (sl + kRing - 1 < slabs) fetch(sl + kRing - 1, (sl + kRing - 1) % kRing);
     cp_async_commit();
-    const float* xs = xs_base + (rd % NS) * XS;
-    const float* ws = ws_base + (rd % NS) * WS;
-    // Operands of four k steps at a time (four 128-bit reads of W, four of X), the next four read from shared memory
-    // while the current ones are multiplied: with two or three warps per scheduler nothing else hides that latency.
-    float4 wv[2][4], xv[2][4];
-    auto read_operands = [&](int k4, int buf) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) wv[buf][j] = *reinterpret_cast<const float4*>(ws + (ty * 4 + j) * kWPitch + k4);
-#pragma unroll
-      for (int kk = 0; kk < 4; ++kk) xv[buf][kk] = *reinterpret_cast<const float4*>(xs + (k4 + kk) * TP + tx * 4);
-    };
-    read_operands(0, 0);
+    if (!XVEC && sl + 1 < slabs) {
+      store_x((sl + 1) % kRing);
+      if (sl + 2 < slabs) load_x(sl + 2);
+    }
+    const float* xs = xs_base + (sl % kRing) * XS + tx * 4;
+    const float* ws = ws_base + (sl % kRing) * WS + ty * kWPitch;
 #pragma unroll
     for (int q = 0; q < kBK / 4; ++q) {
-      const int cur = q & 1;
-      if (q + 1 < kBK / 4) read_operands((q + 1) * 4, cur ^ 1);
+      float4 wv[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) wv[j] = *reinterpret_cast<const float4*>(ws + j * GO * kWPitch + q * 4);
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) {  // k order: the accumulation order of the strict-FP32 contract
-        const float xa[4] = {xv[cur][kk].x, xv[cur][kk].y, xv[cur][kk].z, xv[cur][kk].w};
+        const ulonglong2 xl = *reinterpret_cast<const ulonglong2*>(xs + (q * 4 + kk) * TP);
+        const ulonglong2 xh = *reinterpret_cast<const ulonglong2*>(xs + (q * 4 + kk) * TP + TP / 2);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const float wk = kk == 0 ? wv[cur][j].x : (kk == 1 ? wv[cur][j].y : (kk == 2 ? wv[cur][j].z : wv[cur][j].w));
-#pragma unroll
-          for (int i = 0; i < 4; ++i) acc[i][j] = fmaf(xa[i], wk, acc[i][j]);
+          const float wk = kk == 0 ? wv[j].x : (kk == 1 ? wv[j].y : (kk == 2 ? wv[j].z : wv[j].w));
+          const uint64_t w2 = pack2(wk, wk);
+          fma2(acc[0][j], xl.x, w2);
+          fma2(acc[1][j], xl.y, w2);
+          fma2(acc[2][j], xh.x, w2);
+          fma2(acc[3][j], xh.y, w2);
         }
       }
     }
   }
   cp_async_wait<0>();
-  __syncthreads();  // all slabs consumed: the tiles may be reused
+  ptx::grid_dep_launch();  // late: CTAs of the next launch that became resident earlier would crowd onto the SMs of this one
 
-  if (KG > 1) {  // fold groups 1..KG-1 into group 0, in group order
-    float* red = tiles;
-    static_assert(KG == 1 || (KG - 1) * NT * 16 <= KG * NS * (XS + WS), "reduction scratch must fit the operand tiles");
-    if (grp > 0) {
+  float out[4][8];  // [channel][pixel]
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) red[((grp - 1) * 16 + i * 4 + j) * NT + t] = acc[i][j];
-    }
-    __syncthreads();
-    if (grp > 0) return;
-    for (int g = 0; g < KG - 1; ++g)
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] += red[(g * 16 + i * 4 + j) * NT + t];
-  }
-
-  // Epilogue (fused_epilogue.cuh:11-16 order): + bias, ReLU, store.  Pixels are the fast index of NCHW: a thread's four
-  // pixels leave as one 128-bit store when they lie in one image and the address is 16-byte aligned.
-  const int pixq = pix0 + tx * 4;
-  const int bq = pixq < a.pixels ? a.fd_pq.div(pixq) : 0, remq = pixq - bq * pq;
-  const bool quad_ok = pixq + 3 < a.pixels && remq + 3 < pq;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const int oc = oc0 + ty * 4 + j;
-    if (oc >= a.o) continue;
-    const float bv = a.bias ? __ldg(a.bias + oc) : 0.f;
-    float v[4];
+  for (int j = 0; j < 4; ++j)
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      v[i] = acc[i][j] + bv;
-      if (a.relu) v[i] = fmaxf(v[i], 0.f);
+      const float2 v = unpack2(acc[i][j]);
+      out[j][2 * i] = v.x;
+      out[j][2 * i + 1] = v.y;
     }
-    float* dst = a.y + (size_t(bq) * a.o + oc) * pq + remq;
-    if (quad_ok && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
-      *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
-    } else {
+
+  if (a.slices > 1) {
+    // Partial tiles meet through distributed shared memory: every CTA lays its own out as [vector][thread] (16-byte vector
+    // v = 2 j + half), then thread t of CTA s sums the vectors v with v % slices == s over all slices, in slice order.
+    __syncthreads();  // all slabs consumed: the tiles may be overwritten
+    float4* mine = reinterpret_cast<float4*>(tiles);
+#pragma unroll
+    for (int v = 0; v < 8; ++v) mine[v * kThreads + t] = make_float4(out[v >> 1][(v & 1) * 4], out[v >> 1][(v & 1) * 4 + 1], out[v >> 1][(v & 1) * 4 + 2], out[v >> 1][(v & 1) * 4 + 3]);
+    ptx::cluster_sync_all();
+    const uint32_t base = ptx::smem_u32(mine) + uint32_t(t) * 16u;
+#pragma unroll
+    for (int v = 0; v < 8; ++v) {
+      if (v % a.slices != slice) continue;
+      float4 part[8];
+#pragma unroll
+      for (int s = 0; s < 8; ++s)  // all loads in flight, then the adds
+        if (s < a.slices) part[s] = ptx::ld_cluster_v4(ptx::map_to_cta(base + uint32_t(v * kThreads) * 16u, uint32_t(s)));
+      float4 sum = part[0];
+#pragma unroll
+      for (int s = 1; s < 8; ++s)
+        if (s < a.slices) { sum.x += part[s].x; sum.y += part[s].y; sum.z += part[s].z; sum.w += part[s].w; }
+      out[v >> 1][(v & 1) * 4] = sum.x; out[v >> 1][(v & 1) * 4 + 1] = sum.y; out[v >> 1][(v & 1) * 4 + 2] = sum.z; out[v >> 1][(v & 1) * 4 + 3] = sum.w;
+    }
+    ptx::cluster_sync_all();  // nobody leaves while a peer still reads its tile
+  }
+
+  // Epilogue (fused_epilogue.cuh:11-16 order): + bias, ReLU, store.  Pixels are the fast index of NCHW: a run of four
+  // pixels leaves as one 128-bit store when it lies in one image and the address is 16-byte aligned.
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    const int pixq = pix0 + half * (TP / 2) + tx * 4;
+    const int bq = pixq < a.pixels ? a.fd_pq.div(pixq) : 0, remq = pixq - bq * pq;
+    const bool quad_ok = pixq + 3 < a.pixels && remq + 3 < pq;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int oc = oc0 + ty + j * GO;
+      if (oc >= a.o || (a.slices > 1 && (2 * j + half) % a.slices != slice)) continue;
+      const float bv = a.bias ? __ldg(a.bias + oc) : 0.f;
+      float v[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const int pix = pixq + i;
-        if (pix >= a.pixels) continue;
-        const int b = a.fd_pq.div(pix), rem = pix - b * pq;
-        a.y[(size_t(b) * a.o + oc) * pq + rem] = v[i];
+        v[i] = out[j][half * 4 + i] + bv;
+        if (a.relu) v[i] = fmaxf(v[i], 0.f);
+      }
+      float* dst = a.y + (size_t(bq) * a.o + oc) * pq + remq;
+      if (quad_ok && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
+        *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int pix = pixq + i;
+          if (pix >= a.pixels) continue;
+          const int b = a.fd_pq.div(pix), rem = pix - b * pq;
+          a.y[(size_t(b) * a.o + oc) * pq + rem] = v[i];
+        }
       }
     }
   }
 }
 
-bool use_small_tile(int64_t pixels, int o) {
-  const int64_t big = ((pixels + 63) / 64) * ((o + 63) / 64);
-  return big < 2 * kNumSms;
+// Tile shape: 64 channels wide unless at most 32 are there to be computed.
+int tile_o(int o) { return o <= 32 ? 32 : 64; }
+int tile_p(int o) { return o <= 32 ? 128 : 64; }
+
+// CTAs that share one output tile.  The CTAs that an SM holds together hide each other's latencies: a slab costs ~1600 cycles
+// of a CTA alone on its SM, ~1100 per CTA of two and ~1030 of more; a CTA's prologue and epilogue cost ~1500 cycles, a
+// cluster's exchange ~2000 more, and up to five CTAs share an SM.
+int pick_slices(int64_t tiles, int slabs) {
+  int best = 1;
+  double best_t = 1e300;
+  for (int s = 1; s <= 8 && s <= slabs; ++s) {
+    const int per = (slabs + s - 1) / s;
+    if ((slabs + per - 1) / per != s) continue;  // (an empty slice)
+    const double load = double((tiles * s + kNumSms - 1) / kNumSms);
+    const double slab = load <= 1 ? 1600.0 : (load <= 2 ? 1100.0 : 1030.0);
+    const double t = load * per * slab + std::ceil(load / 5.0) * (1500.0 + (s > 1 ? 2000.0 : 0.0));
+    if (t < best_t * 0.98) { best_t = t; best = s; }
+  }
+  return best;
 }
 
 }  // namespace
 
-int conv_fp32_tile(int64_t pixels, int o) { return use_small_tile(pixels, o) ? 32 : 64; }
+int conv_fp32_tile_pixels(int o) { return tile_p(o); }
+int conv_fp32_tile_channels(int o) { return tile_o(o); }
 
-int64_t conv_fp32_num_blocks(int64_t pixels, int o) {
-  return use_small_tile(pixels, o) ? ((pixels + 31) / 32) * ((o + 31) / 32) : ((pixels + 63) / 64) * ((o + 63) / 64);
-}
+int64_t conv_fp32_num_blocks(int64_t pixels, int o) { return ((pixels + tile_p(o) - 1) / tile_p(o)) * ((o + tile_o(o) - 1) / tile_o(o)); }
 
 cudaError_t conv_fp32_launch(const void* x, const void* w, const void* bias, void* y, int batch, int c, int h, int wd, int o,
                              int r, int s, int stride_h, int stride_w, int pad_h, int pad_w, int out_h, int out_w, int relu,
@@ -275,9 +367,18 @@ cudaError_t conv_fp32_launch(const void* x, const void* w, const void* bias, voi
   a.fd_s = FastDiv::make(s);
   a.fd_pq = FastDiv::make(out_h * out_w);
   a.fd_out_w = FastDiv::make(out_w);
-  const bool lut = (a.k + 63) / 64 * 64 <= kLutMax && int64_t(c) * h * wd < (int64_t(1) << 31) && r < 0x7fff && s <= 0xffff && h < 0x7fff;
+  const int tp = tile_p(o), to = tile_o(o);
+  const int64_t tiles_p = (int64_t(a.pixels) + tp - 1) / tp, tiles_o = (o + to - 1) / to;
+  const int slabs = (a.k + kBK - 1) / kBK;
+  a.slices = pick_slices(tiles_p * tiles_o, slabs);
+  a.slabs_per_slice = (slabs + a.slices - 1) / a.slices;
+  const bool xvec = r == 1 && s == 1 && stride_h == 1 && stride_w == 1 && pad_h == 0 && pad_w == 0 && (out_h * out_w) % 4 == 0 &&
+                    (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+  const bool lut = !xvec && a.slabs_per_slice * kBK <= kLutMax && int64_t(c) * h * wd < (int64_t(1) << 31) && r < 0x7fff && s <= 0xffff && h < 0x7fff;
   const bool w16 = a.k % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15u) == 0;  // 128-bit copies along k
-  auto go = [&](auto kernel, dim3 grid, int threads, size_t smem) -> cudaError_t {
+  const size_t smem = size_t(kRing) * (kBK * tp + to * kWPitch) * sizeof(float) + (lut ? size_t(a.slabs_per_slice) * kBK * sizeof(int2) : 0);
+  const dim3 grid(unsigned(tiles_p * a.slices), unsigned(tiles_o));
+  auto go = [&](auto kernel) -> cudaError_t {
     // the opt-in to more than 48 KiB of dynamic shared memory is per function and device: done once each, under a mutex
     // (set_max_dynamic_smem of the reference, src/kernels/conv_common.cu:9-21)
     if (smem > 48 * 1024) {
@@ -289,26 +390,21 @@ cudaError_t conv_fp32_launch(const void* x, const void* w, const void* bias, voi
       std::lock_guard<std::mutex> lock(mu);
       const auto key = std::make_pair(reinterpret_cast<const void*>(kernel), dev);
       if (done.find(key) == done.end()) {
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
         if (e != cudaSuccess) return e;
         done.insert(key);
       }
     }
-    kernel<<<grid, threads, smem, stream>>>(a);
-    return cudaGetLastError();
+    return launch_pdl_cluster(kernel, grid, dim3(kThreads), smem, stream, unsigned(a.slices), a);
   };
-  if (use_small_tile(a.pixels, o)) {
-    constexpr int TP = 32, TO = 32, KG = 4, NS = 4;
-    const size_t smem = size_t(KG) * NS * (kBK * TP + TO * kWPitch) * sizeof(float);
-    dim3 grid(unsigned((a.pixels + 31) / 32), unsigned((o + 31) / 32));
-    if (lut) return w16 ? go(conv_fp32_kernel<TP, TO, KG, NS, true, true>, grid, (TP / 4) * (TO / 4) * KG, smem) : go(conv_fp32_kernel<TP, TO, KG, NS, true, false>, grid, (TP / 4) * (TO / 4) * KG, smem);
-    return w16 ? go(conv_fp32_kernel<TP, TO, KG, NS, false, true>, grid, (TP / 4) * (TO / 4) * KG, smem) : go(conv_fp32_kernel<TP, TO, KG, NS, false, false>, grid, (TP / 4) * (TO / 4) * KG, smem);
-  }
-  constexpr int TP = 64, TO = 64, KG = 1, NS = 4;
-  const size_t smem = size_t(KG) * NS * (kBK * TP + TO * kWPitch) * sizeof(float);
-  dim3 grid(unsigned((a.pixels + 63) / 64), unsigned((o + 63) / 64));
-  if (lut) return w16 ? go(conv_fp32_kernel<TP, TO, KG, NS, true, true>, grid, (TP / 4) * (TO / 4) * KG, smem) : go(conv_fp32_kernel<TP, TO, KG, NS, true, false>, grid, (TP / 4) * (TO / 4) * KG, smem);
-  return w16 ? go(conv_fp32_kernel<TP, TO, KG, NS, false, true>, grid, (TP / 4) * (TO / 4) * KG, smem) : go(conv_fp32_kernel<TP, TO, KG, NS, false, false>, grid, (TP / 4) * (TO / 4) * KG, smem);
+  auto pick = [&](auto tpc, auto toc) {
+    constexpr int TP = decltype(tpc)::value, TO = decltype(toc)::value;
+    if (xvec) return w16 ? go(conv_fp32_kernel<TP, TO, false, true, true>) : go(conv_fp32_kernel<TP, TO, false, false, true>);
+    if (lut) return w16 ? go(conv_fp32_kernel<TP, TO, true, true, false>) : go(conv_fp32_kernel<TP, TO, true, false, false>);
+    return w16 ? go(conv_fp32_kernel<TP, TO, false, true, false>) : go(conv_fp32_kernel<TP, TO, false, false, false>);
+  };
+  return to == 32 ? pick(std::integral_constant<int, 128>{}, std::integral_constant<int, 32>{})
+                  : pick(std::integral_constant<int, 64>{}, std::integral_constant<int, 64>{});
 }
 
 }  // namespace gieb

@@ -208,8 +208,9 @@ cudaError_t gather_rows_launch(const void* x, void* x2, int batch, int channels,
 cudaError_t conv_fp32_launch(const void* x, const void* w, const void* bias, void* y, int batch, int c, int h, int wd,
                              int o, int r, int s, int stride_h, int stride_w, int pad_h, int pad_w, int out_h, int out_w,
                              int relu, cudaStream_t stream);
-int conv_fp32_tile(int64_t pixels, int o);          // 64 or 32: edge of the square output tile a CTA computes
-int64_t conv_fp32_num_blocks(int64_t pixels, int o);
+int conv_fp32_tile_pixels(int o);    // output pixels ..
+int conv_fp32_tile_channels(int o);  // .. and channels of the tile a CTA (or a cluster that splits the reduction) computes
+int64_t conv_fp32_num_blocks(int64_t pixels, int o);  // output tiles
 
 cudaError_t rmsnorm_launch(int rows, int hidden, float eps, int dtype, int gamma_fp32, const void* x, const void* gamma,
                            void* y, const void* res_in, void* res_out, cudaStream_t stream);
