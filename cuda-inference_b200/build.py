@@ -69,7 +69,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
             raise RuntimeError("link failed")
     if force or _stale(CALLS, [CALLS_SRC, os.path.join(ROOT, "include", "gie_b200.h")]):
         cmd = ["g++", "-std=c++17", "-O2", "-Wall", "-fPIC", "-fvisibility=hidden", "-shared", "-I" + sysconfig.get_paths()["include"],
-               "-I" + os.path.join(ROOT, "include"), CALLS_SRC, LIB, "-Wl,-rpath,$ORIGIN", "-o", CALLS]
+               "-I" + os.path.join(ROOT, "include"), CALLS_SRC, "-L" + HERE, "-l:" + os.path.basename(LIB), "-Wl,-rpath,$ORIGIN", "-o", CALLS]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
