@@ -124,12 +124,11 @@ struct Resolved {
   size_t ws_x, ws_w, ws_part, ws_total;  // workspace layout (bytes; offsets are cumulative in this order)
 };
 
-int pick_tile_k(int c) {
-  const int base = round_up(c, 16);
-  if (double(round_up(c, 64)) <= 1.15 * base) return 64;
-  if (double(round_up(c, 32)) <= 1.15 * base) return 32;
-  return 16;
-}
+// Slab width for a channel count in 2-byte units: the narrowest of 16, 32 and 64 that holds all of it, else 64.  Channels are
+// padded to multiples of 16 only: the last slab of a tap reads on into the next tap's columns and the MMA steps over them are
+// left out, so a layer of 144 channels takes 3 slabs per tap (of 4 + 4 + 1 steps) instead of 9 of one step each, every one
+// of which costs the producers and the issuer the same (6 x 35 x 45, 144 -> 200 channels, 3x3: 22.0 -> 12.8 us).
+int pick_tile_k(int units) { return units <= 16 ? 16 : (units <= 32 ? 32 : 64); }
 
 // Measured on B200: with every SM pulling, one SM receives about 74 B/clk of operands from L2 through TMA, well below
 // the 128 B/clk the tensor pipe of a 128x128 tile would need, so operand bytes per slab usually decide.  CTAs that fit
@@ -383,10 +382,7 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
     // and padding quantity is kept in 2-byte units (half the FP8 counts), as for TF32.
     if (c.variant == 2 || c.variant == 5) return no("FP8 runs on the im2col (1) and tiled (4) routes");
     int tk = c.tile_k;
-    if (tk == 0) {
-      const int base = round_up(d.in_channels, 32);
-      tk = double(round_up(d.in_channels, 128)) <= 1.15 * base ? 128 : (double(round_up(d.in_channels, 64)) <= 1.15 * base ? 64 : 32);
-    }
+    if (tk == 0) tk = 2 * pick_tile_k((d.in_channels + 1) / 2);
     if (tk != 32 && tk != 64 && tk != 128) return no("tile_k must be 32, 64 or 128 for FP8 (values per slab row)");
     r->tile_k = tk / 2;
   } else if (tf32) {
@@ -394,30 +390,24 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
     // tile and padding quantity is kept in 2-byte units (twice the FP32 counts) so that the byte layouts coincide.
     if (c.variant == 2 || c.variant == 5) return no("TF32 runs on the im2col (1) and tiled (4) routes");
     int tk = c.tile_k;
-    if (tk == 0) {
-      const int base = round_up(d.in_channels, 8);
-      tk = double(round_up(d.in_channels, 32)) <= 1.15 * base ? 32 : (double(round_up(d.in_channels, 16)) <= 1.15 * base ? 16 : 8);
-    }
+    if (tk == 0) tk = pick_tile_k(2 * d.in_channels) / 2;
     if (tk != 8 && tk != 16 && tk != 32) return no("tile_k must be 8, 16 or 32 for TF32 (FP32 values per slab row)");
     r->tile_k = 2 * tk;
   } else {
-    r->tile_k = c.tile_k ? c.tile_k : (in_nhwc ? (d.in_channels % 64 == 0 ? 64 : (d.in_channels % 32 == 0 ? 32 : 16)) : pick_tile_k(d.in_channels));
+    r->tile_k = c.tile_k ? c.tile_k : pick_tile_k(d.in_channels);
   }
   if (r->tile_k != 16 && r->tile_k != 32 && r->tile_k != 64) return no("tile_k must be 16, 32 or 64");
-  if (in_nhwc && d.in_channels % r->tile_k != 0) return no("tile_k must divide the channel count of a channel-contiguous input (it is read in place)");
+  if (in_nhwc && c.tile_k && d.in_channels % r->tile_k != 0) return no("tile_k must divide the channel count of a channel-contiguous input (it is read in place)");
   if (gather) {
     const int gc2 = r->gather_pairs ? r->gp_t * 8 : gather_c2;
     if (!c.tile_k) r->tile_k = gc2 % 64 == 0 ? 64 : (gc2 % 32 == 0 ? 32 : 16);
     if (gc2 % r->tile_k != 0) return no("tile_k must divide the gathered row length (padded kernel_w * channels)");
     r->c_padded = gc2;
-  } else if (fp8) {
-    r->c_padded = round_up(d.in_channels, 2 * r->tile_k) / 2;
-  } else if (tf32) {
-    r->c_padded = 2 * round_up(d.in_channels, r->tile_k / 2);
-  } else {
-    r->c_padded = round_up(d.in_channels, r->tile_k);
+  } else {  // (a slab width that was asked for pads to whole slabs)
+    const int units = fp8 ? (d.in_channels + 1) / 2 : (tf32 ? 2 * d.in_channels : d.in_channels);
+    r->c_padded = round_up(units, c.tile_k ? r->tile_k : 16);
   }
-  r->kb_per_tap = r->c_padded / r->tile_k;
+  r->kb_per_tap = ceil_div(r->c_padded, r->tile_k);
   r->total_kb = d.kernel_h * r->eff_kernel_w * r->kb_per_tap;
 
   if (c.tile_n) {
@@ -843,6 +833,7 @@ int launch_impl(const gieb_conv_plan* pl, const void* x, const void* w, const vo
   p.kernel_w = r.eff_kernel_w;
   p.c_padded = r.c_padded;
   p.kb_per_tap = r.kb_per_tap;
+  p.last_ksteps = (r.c_padded - (r.kb_per_tap - 1) * r.tile_k) / 16;
   p.total_kb = r.total_kb;
   p.kb_per_split = r.kb_per_split;
   p.stride_h = d.stride_h; p.stride_w = r.eff_stride_w; p.pad_h = d.pad_h; p.pad_w = r.eff_pad_w;

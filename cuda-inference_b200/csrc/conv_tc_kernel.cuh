@@ -521,12 +521,14 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
       if (!__all_sync(0xffffffffu, drained)) break;
       ptx::tc_fence_after_sync();
       const uint32_t acc = tmem_base + buf * ACC_COLS;
-      // The slab loop exists three times (16-bit K-major A, 16-bit pixel-major A, TF32): the operand form and the MMA
-      // kind are compile-time inside it, so the elected lane's issue sequence carries no branch per instruction.
-      auto slab_loop = [&](auto form_tag) {
+      // The slab loop exists several times: the operand form, the MMA kind and whether a tap's last slab is a partial one (TAIL:
+      // it holds last_ksteps steps of 32 bytes along K) are compile-time inside it, so that the elected lane's issue sequence
+      // carries no branch per instruction (one test of the step count per slab made every layer 8 % slower).
+      auto slab_loop = [&](auto form_tag, auto tail_tag) {
+        constexpr bool TAIL = decltype(tail_tag)::value;
         constexpr int FORM = decltype(form_tag)::value;  // 0: kind::f16, K-major A; 1: kind::f16, pixel-major A; 2: kind::tf32; 3: kind::f8f6f4 (E4M3); 4: kind::f16, A = overlapping windows of an unswizzled strip
         // one slab's MMAs and the commit that frees its ring slot (elected lane only)
-        auto issue_slab = [&](int slot, bool first) {
+        auto issue_slab = [&](int slot, bool first, int ksteps) {
           const uint32_t a_addr = ptx::smem_u32(stage_base + size_t(slot) * STAGE_BYTES);
           const uint32_t b_addr = a_addr + A_BYTES;
           if constexpr (SWAP) {
@@ -535,6 +537,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
             for (int hc = 0; hc < BN / 128; ++hc) {
 #pragma unroll
               for (int k = 0; k < MMAS_PER_SLAB; ++k) {
+                if (TAIL && k >= ksteps) break;
                 const uint64_t wdesc = ptx::smem_desc_kmajor<ROW_BYTES>(b_addr + hc * (128 * ROW_BYTES) + k * 32);
                 const uint64_t xdesc = FORM == 1 ? ptx::smem_desc_mnmajor_sw128(a_addr + k * 2048, A_HALF_BYTES / 2, 1024)
                                                  : ptx::smem_desc_kmajor<ROW_BYTES>(a_addr + k * 32);
@@ -547,6 +550,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
             if (h < halves) {
 #pragma unroll
               for (int k = 0; k < MMAS_PER_SLAB; ++k) {
+                if (TAIL && k >= ksteps) break;
                 // K-major A: one MMA's K extent (16 two-byte or 8 four-byte values) = 32 bytes along a row.
                 // Pixel-major A (form 1): 16 channels = 16 rows of 128 B.
                 const uint64_t adesc = FORM == 1   ? ptx::smem_desc_mnmajor_sw128(a_addr + h * A_HALF_BYTES + k * 2048, A_HALF_BYTES / 2, 1024)
@@ -566,6 +570,13 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
           if constexpr (PAIR) ptx::mma_commit_pair(&empty_bar[slot], 3);
           else ptx::mma_commit(&empty_bar[slot]);
         };
+        int to_last = !TAIL ? 0 : p.kb_per_tap - 1 - (kb_begin - p.fd_kb_per_tap.div(kb_begin) * p.kb_per_tap);  // slabs to the end of the current tap
+        auto steps_of_next = [&]() {
+          if (!TAIL) return MMAS_PER_SLAB;
+          const int steps = to_last == 0 ? p.last_ksteps : MMAS_PER_SLAB;
+          to_last = to_last == 0 ? p.kb_per_tap - 1 : to_last - 1;
+          return steps;
+        };
         for (int i = 0; i < num_kb;) {
           const bool ok = ptx::mbar_wait(&full_bar[s], phase, p.status, kStatusMmaTimeout, p.wait_limit);
           if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
@@ -575,9 +586,10 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
           const uint32_t phase2 = s + 1 == stages ? phase ^ 1u : phase;
           const bool two = PAIR_SLABS && i + 1 < num_kb && __all_sync(0xffffffffu, ptx::mbar_try_wait(&full_bar[s2], phase2));
           ptx::tc_fence_after_sync();
+          const int steps1 = steps_of_next(), steps2 = two ? steps_of_next() : 0;
           if (ptx::elect_one()) {
-            issue_slab(s, i == 0);
-            if (two) issue_slab(s2, false);
+            issue_slab(s, i == 0, steps1);
+            if (two) issue_slab(s2, false, steps2);
           }
           __syncwarp();
           const int adv = two ? 2 : 1;
@@ -586,11 +598,15 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
           if (s >= stages) { s -= stages; phase ^= 1u; }
         }
       };
-      if (!PAIR && !SWAP && p.is_tf32) slab_loop(std::integral_constant<int, 2>{});
-      else if (!SWAP && p.is_fp8) slab_loop(std::integral_constant<int, 3>{});
-      else if (p.a_mode == 2) slab_loop(std::integral_constant<int, 1>{});
-      else if (!PAIR && !SWAP && p.a_mode == 3) slab_loop(std::integral_constant<int, 4>{});
-      else slab_loop(std::integral_constant<int, 0>{});
+      auto with_tail = [&](auto form_tag) {
+        if (BK == 64 && p.last_ksteps != MMAS_PER_SLAB) slab_loop(form_tag, std::integral_constant<bool, BK == 64>{});
+        else slab_loop(form_tag, std::integral_constant<bool, false>{});
+      };
+      if (!PAIR && !SWAP && p.is_tf32) with_tail(std::integral_constant<int, 2>{});
+      else if (!SWAP && p.is_fp8) with_tail(std::integral_constant<int, 3>{});
+      else if (p.a_mode == 2) with_tail(std::integral_constant<int, 1>{});
+      else if (!PAIR && !SWAP && p.a_mode == 3) slab_loop(std::integral_constant<int, 4>{}, std::integral_constant<bool, false>{});
+      else with_tail(std::integral_constant<int, 0>{});
       // accumulator set complete (also reached after a time-out in the slab loop, so nobody hangs)
       if (ptx::elect_one()) {
         if constexpr (PAIR) ptx::mma_commit_pair(&acc_full[buf], 3);  // wakes the epilogue warps of both CTAs

@@ -103,7 +103,8 @@ struct ConvTcParams {
   int pq;             // P * Q
   int kernel_w;       // S (taps are enumerated r-major: tap = r * S + s)
   int c_padded;       // channels of the NHWC copy / prepacked weights
-  int kb_per_tap;     // c_padded / BK
+  int kb_per_tap;     // ceil(c_padded / BK)
+  int last_ksteps;    // 16-channel steps of a tap's last slab: its columns beyond c_padded (the next tap's) are not multiplied
   int total_kb;       // R * S * kb_per_tap reduction slabs
   int kb_per_split;   // slabs per split-K slice
   int tiles_m, tiles_n;  // tile grid over (pixels, output channels)
