@@ -115,6 +115,7 @@ struct Resolved {
   int strip;  // the pair layout read as one position strip per (output row, filter row): see resolve()
   double est_cycles;  // the cost model's estimate for the chosen configuration (SM cycles; 0 on the FP32 path)
   int tma_epilogue;  // channel-contiguous output staged in shared memory and written by TMA stores
+  int row_epilogue;  // the same staging for channel counts that TMA cannot address, written row by row
   int swap;          // transposed accumulator (lane = output channel): NCHW output staged per warp and written by TMA stores
   int reduce;  // 1 workspace partials + reduction launch, 2 cluster (distributed shared memory); 0 when split_k == 1
   int c_padded, kb_per_tap, total_kb, kb_per_split;
@@ -502,6 +503,7 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
   // Channel-contiguous output goes through shared-memory boxes and TMA stores when the rows of the [pixels][O] matrix
   // are 16-byte multiples, rows are numbered by pixel (not the direct-NCHW route) and each CTA finishes its tiles alone.
   r->tma_epilogue = (d.flags & GIEB_FLAG_OUTPUT_NHWC) && d.out_channels % 8 == 0 && r->variant != 2 && !r->strip && r->split_k == 1;
+  r->row_epilogue = (d.flags & GIEB_FLAG_OUTPUT_NHWC) && d.out_channels % 8 != 0 && r->split_k == 1;
   bool swap = best_swap != 0 && !r->pair && !r->strip && r->split_k == 1;  // 2 KiB of staging per epilogue warp
   const int64_t total_tiles = int64_t(r->tiles_m) * r->tiles_n * r->split_k;
   auto stages_for = [&](size_t epi_smem) {
@@ -526,7 +528,7 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
     const bool single_tile = total_tiles <= kNumSms;
     return (alone && (r->tile_n >= 256 || (r->tile_n >= 128 && single_tile && best_mode != 2))) ? 16 : 8;
   };
-  size_t epi_smem = r->tma_epilogue ? conv_tc_epilogue_staging_bytes(r->tile_n) : (swap ? size_t(8) * 2048 : 0);
+  size_t epi_smem = r->tma_epilogue || r->row_epilogue ? conv_tc_epilogue_staging_bytes(r->tile_n) : (swap ? size_t(8) * 2048 : 0);
   int stages = stages_for(epi_smem);
   if (stages < 2 || stages > kMaxStages) return no("stages must be in [2, 8]");
   r->smem = conv_tc_smem_bytes(r->tile_m, r->tile_n, r->tile_k, stages, epi_smem, r->pair != 0);
@@ -588,7 +590,7 @@ void fill_info(const gieb_conv_desc& d, const Resolved& r, gieb_conv_info* out) 
     const bool x_in_place = r.variant == 2 || (d.flags & GIEB_FLAG_INPUT_NHWC);
     const bool w_in_place = (d.flags & GIEB_FLAG_WEIGHTS_PREPACKED) != 0 ||
                             (x_in_place && d.precision != GIEB_TF32 && d.kernel_h * d.kernel_w == 1 && r.c_padded == d.in_channels);  // 16-byte aligned w assumed
-    out->launches = (x_in_place && w_in_place ? 0 : 1) + 1 + (r.reduce == 1 ? 1 : 0) + (d.precision == GIEB_TF32 ? 1 : 0);  // TF32: X and W repacked by two launches
+    out->launches = (x_in_place && w_in_place ? 0 : 1) + 1 + (r.reduce == 1 ? 1 : 0);
   }
 }
 
@@ -798,9 +800,9 @@ int launch_impl(const gieb_conv_plan* pl, const void* x, const void* w, const vo
   } else if (d.precision == GIEB_FP8_E4M3) {  // 1-byte tensors: their own transposing repack (one launch); c_padded is in 2-byte units
     GIEB_CUDA(repack_bytes_pair_launch(x, xn, d.batch, d.in_channels, d.in_h * d.in_w, r.c_padded * 2, w, const_cast<void*>(wk), d.out_channels,
                                        d.in_channels, d.kernel_h * d.kernel_w, r.c_padded * 2, st));
-  } else if (d.precision == GIEB_TF32) {  // FP32 tensors rounded to TF32 while they are repacked (two launches)
-    GIEB_CUDA(repack_tf32_launch(x, xn, d.batch, d.in_channels, d.in_h * d.in_w, r.c_padded / 2, st));
-    GIEB_CUDA(repack_tf32_launch(w, const_cast<void*>(wk), d.out_channels, d.in_channels, d.kernel_h * d.kernel_w, r.c_padded / 2, st));
+  } else if (d.precision == GIEB_TF32) {  // FP32 tensors rounded to TF32 while they are repacked
+    GIEB_CUDA(repack_tf32_pair_launch(x, xn, d.batch, d.in_channels, d.in_h * d.in_w, r.c_padded / 2, w, const_cast<void*>(wk), d.out_channels,
+                                      d.in_channels, d.kernel_h * d.kernel_w, r.c_padded / 2, st));
   } else if (r.variant == 5 && r.gather_pairs) {
     const bool with_w = !(d.flags & GIEB_FLAG_WEIGHTS_PREPACKED);
     GIEB_CUDA(gather_pairs_launch(x, xn, d.batch, d.in_channels, d.in_h, d.in_w, r.gp_positions, r.gp_left, r.gp_t, r.gp_shift,
@@ -888,6 +890,11 @@ int launch_impl(const gieb_conv_plan* pl, const void* x, const void* w, const vo
       if (sr != GIEB_OK) return sr;
       p.res_tma = 1;
     }
+  }
+  // (a tensor off its alignment takes the row stores as well: the staging is there)
+  if ((r.row_epilogue || r.tma_epilogue) && !p.out_tma) {
+    const uintptr_t both = reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(residual);
+    p.out_rows = (both % 4 == 0 && d.out_channels % 2 == 0) ? 2 : 1;
   }
   if (r.swap) {
     const uintptr_t ya = reinterpret_cast<uintptr_t>(y);

@@ -180,6 +180,47 @@ __device__ __forceinline__ void chunk_to_staging(const uint32_t (&v)[32], const 
   }
 }
 
+// Channel-contiguous output whose rows TMA cannot address (O % 8 != 0, or a tensor off its 16-byte alignment): written
+// straight from the accumulator's rows, every store instruction would touch 32 pixels, i.e. 32 sectors for 64 bytes.  The
+// chunk goes through the staging box instead (layout of chunk_to_staging) and leaves row by row, the lanes along the channels:
+// two rows per instruction when rows are 4-byte aligned (PAIRS), else one.  The residual enters the box the same way.
+// `base`: this lane's element offset (pixel of its accumulator row, first channel of the chunk); row_ok: it is an output pixel.
+template <bool PAIRS, bool LOAD, typename T>
+__device__ __forceinline__ void staging_rows(uint8_t* box, int lane, T* gmem, int64_t base, bool row_ok, int nvalid) {
+  constexpr int STEP = PAIRS ? 2 : 1;
+  const int sub = PAIRS ? lane >> 4 : 0, ch = PAIRS ? (lane & 15) * 2 : lane;  // row within the step, first channel of the lane
+#pragma unroll 4
+  for (int r0 = 0; r0 < 32; r0 += STEP) {
+    const int r = r0 + sub;
+    const int64_t b = __shfl_sync(0xffffffffu, base, r);
+    const bool ok = __shfl_sync(0xffffffffu, int(row_ok), r) != 0;
+    uint8_t* cell = box + r * 64 + (((ch >> 3) ^ ((r >> 1) & 3)) << 4) + (ch & 7) * 2;
+    if (!ok || ch >= nvalid) continue;  // (PAIRS: nvalid is even)
+    if (PAIRS) {
+      if (LOAD) *reinterpret_cast<uint32_t*>(cell) = *reinterpret_cast<const uint32_t*>(gmem + b + ch);
+      else *reinterpret_cast<uint32_t*>(gmem + b + ch) = *reinterpret_cast<const uint32_t*>(cell);
+    } else {
+      if (LOAD) *reinterpret_cast<uint16_t*>(cell) = *reinterpret_cast<const uint16_t*>(gmem + b + ch);
+      else *reinterpret_cast<uint16_t*>(gmem + b + ch) = *reinterpret_cast<const uint16_t*>(cell);
+    }
+  }
+}
+
+template <typename T>
+__device__ __forceinline__ void store_chunk_rows(const uint32_t (&v)[32], const float* bias, uint8_t* box, int lane, T* y, T* res, int64_t base,
+                                                 bool row_ok, int nvalid, bool pairs, int relu) {
+  __syncwarp();  // the box's previous content has been read
+  if (res != nullptr) {
+    if (pairs) staging_rows<true, true>(box, lane, res, base, row_ok, nvalid);
+    else staging_rows<false, true>(box, lane, res, base, row_ok, nvalid);
+    __syncwarp();
+  }
+  chunk_to_staging<T>(v, bias, box, lane, relu, res != nullptr);
+  __syncwarp();
+  if (pairs) staging_rows<true, false>(box, lane, y, base, row_ok, nvalid);
+  else staging_rows<false, false>(box, lane, y, base, row_ok, nvalid);
+}
+
 // Transposed accumulator: 32 consecutive pixels of ONE channel (this lane's) -> + bias (+ residual), ReLU on the rounded pair
 // (rounding is monotonic and keeps zero), packed as 64 bytes and written as the lane's row of the warp's staging box (32 rows of 64
 // bytes, 64-byte swizzled: 16-byte cell q of row r sits at cell q ^ ((r >> 1) & 3); conflict-free).
@@ -933,6 +974,17 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
                 ptx::bulk_commit_group();
               }
             }
+            continue;
+          }
+          if (p.out_rows) {
+            const int nvalid = min(32, p.out_channels - (n0 + chunk * 32));
+            const int64_t off = base + chunk * 32;
+            if (p.is_bf16)
+              store_chunk_rows(v, bias_t + chunk * 32, stage_box(0), lane, static_cast<__nv_bfloat16*>(p.y),
+                               const_cast<__nv_bfloat16*>(static_cast<const __nv_bfloat16*>(p.residual)), off, m_ok, nvalid, p.out_rows == 2, p.relu);
+            else
+              store_chunk_rows(v, bias_t + chunk * 32, stage_box(0), lane, static_cast<__half*>(p.y),
+                               const_cast<__half*>(static_cast<const __half*>(p.residual)), off, m_ok, nvalid, p.out_rows == 2, p.relu);
             continue;
           }
           if (m_ok) {

@@ -135,6 +135,7 @@ struct ConvTcParams {
   const void* bias;
   const void* residual;  // optional tensor of the output's shape, layout and type, added before the activation
   int out_nhwc;          // 0: y (and residual, partials) are NCHW; 1: channel-contiguous [B][P][Q][O]
+  int out_rows;          // channel-contiguous output goes through shared memory and leaves row by row: 2 = in channel pairs, 1 = singly
   int out_tma, res_tma;  // channel-contiguous output leaves through TMA stores / the residual arrives through TMA loads
   // Transposed-accumulator kernels: swap_tma = y may be written by TMA stores over its {P*Q, O, N} view (16-byte aligned y,
   // P*Q % 8 == 0); out_vec = pixels per store (4, 2 or 1) of the path that handles everything else (a unit that crosses
@@ -181,8 +182,10 @@ cudaError_t splitk_reduce_launch(const float* partial, int splits, int64_t total
 
 // 16-bit [B][C][HW] -> [B][HW][Cp] (zero-filled channel padding).
 cudaError_t repack_launch(const void* src, void* dst, int batch, int channels, int hw, int c_padded, cudaStream_t stream);
-// FP32 [B][C][HW] -> [B][HW][Cp] (Cp in FP32 elements) with every value rounded to TF32 (ties away).
-cudaError_t repack_tf32_launch(const void* src, void* dst, int batch, int channels, int hw, int c_padded, cudaStream_t stream);
+// FP32, two tensors in one launch: [batch][channels][hw] -> [batch][hw][c_padded], every value rounded to TF32 (ties away);
+// c_padded counts FP32 elements (a multiple of 8).
+cudaError_t repack_tf32_pair_launch(const void* src_a, void* dst_a, int batch_a, int ch_a, int hw_a, int cp_a, const void* src_b,
+                                    void* dst_b, int batch_b, int ch_b, int hw_b, int cp_b, cudaStream_t stream);
 // 1-byte elements (FP8), two tensors in one launch: [batch][channels][hw] -> [batch][hw][c_padded], zero-padded channels;
 // c_padded counts elements (a multiple of 32); destinations 16-byte aligned.
 cudaError_t repack_bytes_pair_launch(const void* src_a, void* dst_a, int batch_a, int ch_a, int hw_a, int cp_a, const void* src_b,

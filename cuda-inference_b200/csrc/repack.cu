@@ -572,28 +572,118 @@ cudaError_t gather_rows_launch(const void* x, void* x2, int batch, int channels,
 namespace {
 
 // FP32 [B][C][HW] -> [B][HW][Cp] with every value rounded to TF32 (round to nearest, ties away: cvt.rna, the rounding
-// of round_to_tf32 in the reference, src/runtime/reference.cu:95-104), channels zero-padded to Cp.  32 x 32 tiles.
-__global__ void __launch_bounds__(256) repack_tf32_kernel(const float* __restrict__ src, float* __restrict__ dst, int C, int HW, int Cp) {
-  __shared__ float tile[32][33];
+// of round_to_tf32 in the reference, src/runtime/reference.cu:95-104), channels zero-padded to Cp (a multiple of 8).  Two
+// tensors per launch (activations and weights) in the two shapes of work of repack_jobs_kernel:
+//   tile mode: one CTA transposes 32 channels x 64 pixels, 16-byte loads along the pixels where planes and pointer allow it;
+//   slab mode (planes of at most 64 elements: filter taps and small maps): one CTA takes `span` channels of one batch entry,
+//     a contiguous slab that is read linearly and written as [HW][span].
+// All stores are 16 bytes.  Bound by HBM / latency; as two launches of 32 x 32 tiles with 4-byte accesses it took 6.2 us a launch
+// on the weights of 96 -> 192 channels, 5x5.
+struct Tf32Job {
+  const float* src;
+  float* dst;
+  int C, HW, Cp, hw_tiles, c_tiles, span;  // span > 0: slab mode
+  unsigned blocks;
+};
+constexpr int kTf32Slab = 4096;  // floats of shared memory a slab may take
+constexpr int kTf32Pitch = 65;
+
+__device__ __forceinline__ float to_tf32(float v) {
+  uint32_t u;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(v));
+  return __uint_as_float(u);
+}
+
+__global__ void __launch_bounds__(256) repack_tf32_kernel(const Tf32Job a, const Tf32Job b, int prefetch) {
+  __shared__ __align__(16) float tile[kTf32Slab];
+  static_assert(32 * kTf32Pitch <= kTf32Slab, "the 32 x 64 tile must fit the slab buffer");
+  const bool first = blockIdx.x < a.blocks;
+  const Tf32Job& j = first ? a : b;
+  unsigned id = first ? blockIdx.x : blockIdx.x - a.blocks;
+  const int hw_tile = int(id % unsigned(j.hw_tiles));
+  id /= unsigned(j.hw_tiles);
+  const int c_tile = int(id % unsigned(j.c_tiles));
+  const int bi = int(id / unsigned(j.c_tiles));
+  const int t = threadIdx.x;
+  if (j.span > 0) {
+    const int c0 = c_tile * j.span;
+    const int nch = min(j.span, j.C - c0);  // may be <= 0 for pure padding tiles
+    const int n = nch > 0 ? nch * j.HW : 0;
+    const float* s = j.src + (size_t(bi) * j.C + c0) * j.HW;
+    if (prefetch && n > 0)
+      for (int o = t * 32; o < n + 31; o += 256 * 32) ptx::prefetch_l2(s + min(o, n - 1));
+    ptx::grid_dep_wait();
+    ptx::grid_dep_launch();
+    if ((reinterpret_cast<uintptr_t>(s) & 15u) == 0 && (n & 3) == 0) {
+      for (int i = t; i < (n >> 2); i += 256) reinterpret_cast<float4*>(tile)[i] = reinterpret_cast<const float4*>(s)[i];
+    } else {
+      for (int i = t; i < n; i += 256) tile[i] = s[i];
+    }
+    __syncthreads();
+    const int groups = min(j.span, j.Cp - c0) >> 2;  // 4-channel vectors in this tile
+    for (int v = t; v < j.HW * groups; v += 256) {
+      const int px = v / groups, cg = v - px * groups;
+      float o[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[e] = cg * 4 + e < nch ? to_tf32(tile[(cg * 4 + e) * j.HW + px]) : 0.f;
+      *reinterpret_cast<float4*>(j.dst + (size_t(bi) * j.HW + px) * j.Cp + c0 + cg * 4) = make_float4(o[0], o[1], o[2], o[3]);
+    }
+    return;
+  }
+  const int c0 = c_tile * 32, px0 = hw_tile * 64;
+  const float* s = j.src + (size_t(bi) * j.C + c0) * j.HW + px0;
+  if (prefetch && t < 96 && c0 + t / 3 < j.C) {  // 256 bytes: at most three lines per channel
+    const int n = min(64, j.HW - px0);
+    ptx::prefetch_l2(s + size_t(t / 3) * j.HW + min((t % 3) * 32, n - 1));
+  }
   ptx::grid_dep_wait();
   ptx::grid_dep_launch();
-  const int b = blockIdx.z, c0 = blockIdx.y * 32, p0 = blockIdx.x * 32;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 8 rows of 32 threads
-  for (int r = ty; r < 32; r += 8) {
-    const int c = c0 + r, px = p0 + tx;
-    float v = 0.f;
-    if (c < C && px < HW) {
-      uint32_t u;
-      asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(src[(size_t(b) * C + c) * HW + px]));
-      v = __uint_as_float(u);
+  const bool vec = (j.HW & 3) == 0 && (reinterpret_cast<uintptr_t>(j.src) & 15u) == 0;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int idx = t + i * 256, ch = idx >> 4, q = (idx & 15) * 4;
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    if (c0 + ch < j.C && px0 + q < j.HW) {
+      const float* p = s + size_t(ch) * j.HW + q;
+      if (vec) {  // a group of four never straddles the plane (HW % 4 == 0)
+        const float4 f = *reinterpret_cast<const float4*>(p);
+        v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (px0 + q + e < j.HW) v[e] = p[e];
+      }
     }
-    tile[r][tx] = v;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) tile[ch * kTf32Pitch + q + e] = to_tf32(v[e]);
   }
   __syncthreads();
-  for (int r = ty; r < 32; r += 8) {
-    const int px = p0 + r, c = c0 + tx;
-    if (px < HW && c < Cp) dst[(size_t(b) * HW + px) * Cp + c] = tile[tx][r];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int idx = t + i * 256, px = idx >> 3, cg = idx & 7;
+    if (px0 + px < j.HW && c0 + cg * 4 < j.Cp)
+      *reinterpret_cast<float4*>(j.dst + (size_t(bi) * j.HW + px0 + px) * j.Cp + c0 + cg * 4) =
+          make_float4(tile[(cg * 4) * kTf32Pitch + px], tile[(cg * 4 + 1) * kTf32Pitch + px], tile[(cg * 4 + 2) * kTf32Pitch + px], tile[(cg * 4 + 3) * kTf32Pitch + px]);
   }
+}
+
+Tf32Job make_tf32_job(const void* src, void* dst, int batch, int channels, int hw, int c_padded) {
+  Tf32Job j;
+  j.src = static_cast<const float*>(src);
+  j.dst = static_cast<float*>(dst);
+  j.C = channels; j.HW = hw; j.Cp = c_padded;
+  if (hw <= 64) {
+    j.span = (kTf32Slab / hw) / 32 * 32;
+    if (j.span > (c_padded + 31) / 32 * 32) j.span = (c_padded + 31) / 32 * 32;
+    j.hw_tiles = 1;
+    j.c_tiles = (c_padded + j.span - 1) / j.span;
+  } else {
+    j.span = 0;
+    j.hw_tiles = (hw + 63) / 64;
+    j.c_tiles = (c_padded + 31) / 32;
+  }
+  j.blocks = unsigned(int64_t(j.hw_tiles) * j.c_tiles * batch);
+  return j;
 }
 
 // 1-byte elements (FP8 bit patterns): [B][C][HW] -> [B][HW][Cp], channels zero-padded to Cp (a multiple of 32).  Pure data
@@ -720,11 +810,13 @@ cudaError_t repack_bytes_pair_launch(const void* src_a, void* dst_a, int batch_a
   return cudaGetLastError();
 }
 
-cudaError_t repack_tf32_launch(const void* src, void* dst, int batch, int channels, int hw, int c_padded, cudaStream_t stream) {
-  const dim3 grid(unsigned((hw + 31) / 32), unsigned((c_padded + 31) / 32), unsigned(batch));
-  if (grid.y > 65535 || grid.z > 65535) return cudaErrorInvalidValue;
-  const cudaError_t e = launch_pdl(repack_tf32_kernel, grid, dim3(256), 0, stream, static_cast<const float*>(src), static_cast<float*>(dst),
-                                   channels, hw, c_padded);
+cudaError_t repack_tf32_pair_launch(const void* src_a, void* dst_a, int batch_a, int ch_a, int hw_a, int cp_a, const void* src_b,
+                                    void* dst_b, int batch_b, int ch_b, int hw_b, int cp_b, cudaStream_t stream) {
+  if (int64_t((hw_a + 63) / 64) * ((cp_a + 31) / 32) * batch_a + int64_t((hw_b + 63) / 64) * ((cp_b + 31) / 32) * batch_b > 2147483647LL)
+    return cudaErrorInvalidValue;
+  const Tf32Job a = make_tf32_job(src_a, dst_a, batch_a, ch_a, hw_a, cp_a);
+  const Tf32Job b = make_tf32_job(src_b, dst_b, batch_b, ch_b, hw_b, cp_b);
+  const cudaError_t e = launch_pdl(repack_tf32_kernel, dim3(a.blocks + b.blocks), dim3(256), 0, stream, a, b, prefetch_enabled() ? 1 : 0);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();
 }
