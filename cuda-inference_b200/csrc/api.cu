@@ -123,6 +123,13 @@ struct Resolved {
   size_t smem;
   int epi_warps;  // 8, or 16 when the CTA has its SM to itself (see conv_tc_kernel)
   size_t ws_x, ws_w, ws_part, ws_total;  // workspace layout (bytes; offsets are cumulative in this order)
+  // The halo-tile kernel (conv_halo.cu) instead of the slab kernels: tile_m, tile_n, split_k, pair, stages (of the weight
+  // ring), epi_warps (worker warps) and smem above are its own, and:
+  int halo;
+  int h_hs, h_ws, h_phases, h_phases_w, h_rows;  // padded grid per image, phases of a tile and rows of each
+  int h_box_h, h_boxes;                          // padded rows per TMA box, boxes per phase
+  int h_a_stages, h_taps_per_load, h_tap_groups, h_total_loads, h_loads_per_split, h_last_ksteps, h_resident;
+  size_t h_stage_bytes;
 };
 
 // Slab width for a channel count in 2-byte units: the narrowest of 16, 32 and 64 that holds all of it, else 64.  Channels are
@@ -288,6 +295,11 @@ bool pairs_enabled() {
   }();
   return on;
 }
+// GIEB_HALO (a debugging aid): 0 keeps every layer on the slab kernels, 2 takes the halo-tile kernel wherever it is possible.
+int halo_mode() {
+  const char* e = getenv("GIEB_HALO");
+  return e ? atoi(e) : 1;
+}
 // GIEB_DISABLE_PREFETCH=1 switches the L2 prefetches that precede the dependency waits off (a debugging aid).
 bool prefetch_enabled() {
   static const bool on = [] {
@@ -299,6 +311,125 @@ bool prefetch_enabled() {
 }  // namespace gieb
 
 namespace {
+
+// Configuration of the halo-tile kernel for a problem whose route and padding resolve() has settled, when it is expected to be
+// faster than the `slab` cycles of the best slab configuration; false: not for this problem.
+bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, double slab, Resolved* r) {
+  const int mode = halo_mode();
+  if (mode == 0) return false;
+  const bool nhwc = (d.flags & GIEB_FLAG_INPUT_NHWC) != 0;
+  const int taps = d.kernel_h * d.kernel_w;
+  if (r->variant != 1 || taps == 1) return false;
+  if (d.stride_h > 2 || d.stride_w > 2 || d.pad_h > d.kernel_h - 1 || d.pad_w > d.kernel_w - 1) return false;
+  if (g.pq < 16 || taps > 64) return false;
+  const int ph = d.stride_h < d.kernel_h ? d.stride_h : d.kernel_h, pw = d.stride_w < d.kernel_w ? d.stride_w : d.kernel_w;
+  // stride 1: neighbours share their padding; larger strides: a row of a phase holds every position that some tap reads
+  const int ws = d.stride_w == 1 ? d.in_w + d.pad_w : g.out_w + (d.kernel_w - 1) / d.stride_w;
+  const int hs = d.stride_h == 1 ? d.in_h + d.pad_h : g.out_h + (d.kernel_h - 1) / d.stride_h;
+  const int64_t rows = int64_t(d.batch) * hs * ws;
+  const int need = kTileM + (d.kernel_h - 1) / d.stride_h * ws + (d.kernel_w - 1) / d.stride_w;  // rows of one phase that the taps read
+  const int blocks = ceil_div(r->c_padded, 64), last = (r->c_padded - (blocks - 1) * 64) / 16;
+  const double ksteps = (blocks - 1) * 4.0 + last;  // MMA steps per tap
+
+  auto taps_per_load = [&](int b_rows) { return size_t(d.kernel_w) * b_rows * 128 <= 48 * 1024 ? d.kernel_w : 1; };
+  // shared memory: halo tiles, weight stages
+  struct Fit { int a, b, resident; size_t smem; };
+  auto fit = [&](int bn, bool pair, int workers, size_t stage, int tpl, int loads, bool one_n, size_t budget, Fit* f) {
+    const bool staging = (d.flags & GIEB_FLAG_OUTPUT_NHWC) != 0;
+    for (int a = 2; a >= 1; --a) {
+      const size_t fixed = conv_halo_smem_bytes(bn, pair, workers, tpl, a, stage, 0, staging);
+      if (fixed >= budget) continue;
+      const int room = int((budget - fixed) / (size_t(tpl) * (pair ? bn / 2 : bn) * 128));
+      if (room < 2) continue;
+      f->a = a;
+      f->b = room > kMaxStages ? kMaxStages : room;
+      f->resident = one_n && loads <= f->b;
+      if (loads < f->b) f->b = loads < 2 ? 2 : loads;
+      f->smem = conv_halo_smem_bytes(bn, pair, workers, tpl, a, stage, f->b, staging);
+      return true;
+    }
+    return false;
+  };
+  double best = 1e300, best_load = 1;
+  Resolved b = *r;
+  // TMA boxes: whole padded rows of one image, as many as an even split allows in 64 grid rows
+  int box_h = 1;
+  for (int k = 2; k <= 16; ++k)
+    if (hs % k == 0 && k * ws <= 64) box_h = k;
+  const int box_rows = box_h * ws, boxes = ceil_div(box_rows - 1 + need, box_rows);
+  if (ws * d.stride_w > 256 || box_h * d.stride_h > 256 || boxes > 64) return false;  // (limits of a TMA box)
+  for (int pair = 0; pair <= (d.precision == GIEB_TF32 ? 0 : 1); ++pair) {
+    // (the CTAs of a pair shift their boxes to a common first row)
+    const int phase_rows = (boxes + pair) * box_rows;
+    const size_t stage = (size_t(ph) * pw * phase_rows * 128 + 1023) / 1024 * 1024;
+    if (rows + int64_t(ph) * pw * phase_rows + 2 * kTileM > 2147483647LL || stage > 160 * 1024) continue;
+    for (int bn = pair ? 128 : 32; bn <= 256; bn *= 2) {
+      if (bn > 32 && bn / 2 >= d.out_channels) continue;
+      const int workers = pair || bn == 256 ? 16 : 8, tiles_n = ceil_div(d.out_channels, bn);
+      const int tpl = taps_per_load(pair ? bn / 2 : bn), groups = ceil_div(taps, tpl);
+      const int64_t tiles = int64_t(ceil_div(rows, pair ? 2 * kTileM : kTileM)) * tiles_n;
+      const int sms = pair ? kNumSmPairs : kNumSms;
+      if (pair && (rows <= 2 * kTileM || tiles < sms / 2)) continue;
+      for (int s = 1; s <= (pair ? 1 : 8); s *= 2) {
+        const int loads = blocks * groups, per = ceil_div(loads, s);
+        if (s > 1 && (tiles * s > kNumSms || loads < 2 * s || ceil_div(loads, per) != s)) continue;
+        Fit f;
+        if (!fit(bn, pair != 0, workers, stage, tpl, per, s == 1 && tiles_n == 1, kMaxDynamicSmem, &f)) continue;
+        const double load = double((tiles * s + sms - 1) / sms);
+        // Cycles, in the terms of estimate_cycles(), fitted to clock stamps and to the times of ~90 layers: an instruction of
+        // 32 bytes along K takes `step` cycles (shared-memory reads of shifted rows), a round of up to two weight loads ~230
+        // on top (one round per channel block when the weights stay), a tile ~900; the feed is shared with the weights.
+        const double step = pair ? (bn == 128 ? 76.0 : 138.0) : (bn <= 64 ? 60.0 : (bn == 128 ? 84.0 : 138.0));
+        const double blocks_s = s == 1 ? blocks : fmin(blocks, (per + groups - 2) / groups + 1);  // (a slice may begin inside a block)
+        const double rounds = f.resident ? blocks : double(per) / (f.b >= 4 ? 1.7 : 1.0);
+        const double mma = taps * ksteps * step / s + rounds * 230.0;
+        const double a_time = 300.0 + stage / 60.0;  // one halo tile in place
+        const double b_time = f.resident ? 0.0 : double(taps) * (pair ? bn / 2 : bn) * 128.0 / 60.0;
+        double main = fmax(mma, blocks_s * (a_time + b_time));
+        if (f.a == 1 && blocks_s > 1) main = mma + blocks_s * a_time;
+        if (f.b < 3 && !f.resident) main *= 1.5;  // (two weight stages do not cover a load)
+        const double drain = 800.0 + 18.0 * bn * (workers == 16 ? 0.6 : 1.0);
+        double t = (load > 1 ? 4500.0 : 3500.0) + a_time + load * fmax(main, load > 1 ? drain : 0.0) + (load - 1) * 600.0 + drain;
+        if (s > 1) t += 3500.0;
+        if (ph * pw > 1) t += 0.15 * load * main;  // (the phases are loaded whole)
+        if (t < best) {
+          best = t;
+          best_load = load;
+          b.pair = pair; b.tile_n = bn; b.tile_m = pair ? 2 * kTileM : kTileM;
+          b.split_k = s; b.epi_warps = workers; b.h_taps_per_load = tpl; b.h_tap_groups = groups; b.h_total_loads = loads;
+          b.h_loads_per_split = per; b.h_a_stages = f.a; b.stages = f.b; b.h_resident = f.resident; b.smem = f.smem;
+          b.h_rows = phase_rows; b.h_stage_bytes = stage; b.h_box_h = box_h; b.h_boxes = boxes;
+          b.tiles_n = tiles_n;
+        }
+      }
+    }
+  }
+  // Where the two estimates are to be compared at par, by measurement over ~150 layers of both kernels: one wave of tiles needs a
+  // margin of 5 %; with many waves of tiles of at most 64 channels the slab model is ~30 % too short (co-resident CTAs do not
+  // double the issue rate there), except for FP8.
+  double margin = 0.95;
+  if (best_load >= 3) margin = (b.tile_n <= 64 && ph * pw == 1 && d.precision != GIEB_FP8_E4M3) ? 1.3 : 1.0;
+  if (best >= 1e299 || (mode == 1 && best >= margin * slab)) return false;
+  const size_t exchange = 1024 + 3072 + size_t(b.tile_n) * 512;  // a cluster's partial columns land in the idle stages
+  if (b.split_k > 1 && b.smem < exchange) b.smem = exchange;
+  if (b.pair && b.smem < kMaxDynamicSmem / 2 + 2048) b.smem = kMaxDynamicSmem / 2 + 2048;  // (see resolve())
+  b.halo = 1;
+  b.tile_k = 64;
+  b.kb_per_tap = blocks;
+  b.total_kb = taps * blocks;
+  b.reduce = b.split_k > 1 ? 2 : 0;
+  b.est_cycles = best;
+  b.h_hs = hs; b.h_ws = ws;
+  b.h_phases = ph * pw; b.h_phases_w = pw;
+  b.h_last_ksteps = last;
+  b.tiles_m = ceil_div(g.pixels, b.tile_m);  // (as reported; the kernel's own tiles cover the padded grid)
+  b.ws_x = nhwc ? 0 : align256(size_t(d.batch) * d.in_h * d.in_w * b.c_padded * 2);
+  b.ws_w = (d.flags & GIEB_FLAG_WEIGHTS_PREPACKED) ? 0 : align256(size_t(d.out_channels) * taps * b.c_padded * 2);
+  b.ws_total = b.ws_x + b.ws_w;
+  if (b.ws_total > (size_t(180) << 30) / 4) return false;
+  *r = b;
+  return true;
+}
 
 int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, char* why, size_t why_len) {
   auto no = [&](const char* m) { snprintf(why, why_len, "%s", m); return GIEB_UNSUPPORTED; };
@@ -485,6 +616,8 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
       }
     }
   }
+  const bool untouched = c.tile_n == 0 && c.tile_k == 0 && c.stages == 0 && c.split_k == 0 && c.variant == 0 && c.tile_m == 0 && c.reduce == 0 && c.cta_pair == 0;
+  if (untouched && resolve_halo(d, g, best, r)) return GIEB_OK;
   if (best_n == 0) {
     if (c.reduce == 2) return no("cluster reduction needs tile_m 128, split_k 2, 4 or 8 dividing tile_n / 32 with no empty slice, and a ring that holds the received slices");
     if (c.split_k > 1) return no("reduction too short for this split-K factor");
@@ -732,6 +865,96 @@ int encode_epilogue_map(const gieb_conv_plan* pl, const void* ptr, CUtensorMap* 
   return GIEB_OK;
 }
 
+// Tensor maps of the halo-tile kernel: the channel-contiguous activations `xn` as {channels, W, H, N} with boxes of box_h padded
+// rows (read with the convolution's strides), and the weights as {channels, output channels, taps} with boxes of taps_per_load taps.
+int encode_halo_maps(const gieb_conv_plan* pl, const void* xn, const void* wk, CUtensorMap* tm_act, CUtensorMap* tm_wgt) {
+  const gieb_conv_desc& d = pl->desc;
+  const Resolved& r = pl->r;
+  const bool tf32 = d.precision == GIEB_TF32, fp8 = d.precision == GIEB_FP8_E4M3;
+  const CUtensorMapDataType dt = tf32  ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+                                 : fp8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8
+                                       : (d.precision == GIEB_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16);
+  auto el = [&](uint64_t units) { return tf32 ? units >> 1 : (fp8 ? units << 1 : units); };  // elements from counts of 2-byte units
+  const cuuint64_t cb = cuuint64_t(r.c_padded) * 2;  // bytes of one pixel
+  const int taps = d.kernel_h * d.kernel_w;
+  {
+    const cuuint64_t dims[4] = {cuuint64_t(el(r.c_padded)), cuuint64_t(d.in_w), cuuint64_t(d.in_h), cuuint64_t(d.batch)};
+    const cuuint64_t strides[3] = {cb, cb * d.in_w, cb * d.in_w * d.in_h};
+    const cuuint32_t box[4] = {cuuint32_t(el(64)), cuuint32_t(r.h_ws * d.stride_w), cuuint32_t(r.h_box_h * d.stride_h), 1};
+    const cuuint32_t estr[4] = {1, cuuint32_t(d.stride_w), cuuint32_t(d.stride_h), 1};
+    const CUresult res = g_encode_tiled(tm_act, dt, 4, const_cast<void*>(xn), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (res != CUDA_SUCCESS) return fail(GIEB_CUDA_ERROR, "cuTensorMapEncodeTiled (halo rows) failed with CUresult %d", int(res));
+    small_tensor_fixup(tm_act, size_t(d.batch) * d.in_h * d.in_w * cb);
+  }
+  const cuuint64_t dims[3] = {cuuint64_t(el(r.c_padded)), cuuint64_t(d.out_channels), cuuint64_t(taps)};
+  const cuuint64_t strides[2] = {cb * taps, cb};
+  const cuuint32_t box[3] = {cuuint32_t(el(64)), cuuint32_t(r.pair ? r.tile_n / 2 : r.tile_n), cuuint32_t(r.h_taps_per_load)};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult res = g_encode_tiled(tm_wgt, dt, 3, const_cast<void*>(wk), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (res != CUDA_SUCCESS) return fail(GIEB_CUDA_ERROR, "cuTensorMapEncodeTiled (filter taps) failed with CUresult %d", int(res));
+  small_tensor_fixup(tm_wgt, size_t(cb) * taps * d.out_channels);
+  return GIEB_OK;
+}
+
+// The convolution launch of a plan on the halo-tile kernel; the arguments have been checked and what needs repacking has been.
+int launch_halo(const gieb_conv_plan* pl, const CUtensorMap& tm_act, const CUtensorMap& tm_wgt, const void* bias, const void* residual,
+                void* y, cudaStream_t st, cudaEvent_t* ev, unsigned stage_mask) {
+  const gieb_conv_desc& d = pl->desc;
+  const Resolved& r = pl->r;
+  ConvHaloParams p;
+  memset(&p, 0, sizeof(p));
+  p.bias = bias; p.residual = residual; p.y = y;
+  p.status = pl->d_status;
+  p.wait_limit = pl->wait_limit;
+  p.debug_skip = pl->debug_skip;
+  p.batch = d.batch;
+  p.out_channels = d.out_channels; p.out_h = pl->g.out_h; p.out_w = pl->g.out_w; p.pq = pl->g.pq;
+  p.kernel_w = d.kernel_w; p.taps = d.kernel_h * d.kernel_w;
+  p.stride_h = d.stride_h; p.stride_w = d.stride_w; p.pad_h = d.pad_h; p.pad_w = d.pad_w;
+  p.hs = r.h_hs; p.ws = r.h_ws;
+  p.rows_total = d.batch * r.h_hs * r.h_ws;
+  p.phases = r.h_phases; p.phases_w = r.h_phases_w;
+  p.halo_rows = r.h_rows;
+  p.a_stage_bytes = uint32_t(r.h_stage_bytes);
+  p.a_stages = r.h_a_stages; p.b_stages = r.stages;
+  p.resident = r.h_resident;
+  p.boxes = r.h_boxes; p.box_h = r.h_box_h; p.box_rows = r.h_box_h * r.h_ws;
+  p.box_bytes = uint32_t(p.box_rows) * 128;
+  p.is_bf16 = d.precision == GIEB_BF16; p.is_tf32 = d.precision == GIEB_TF32; p.is_fp8 = d.precision == GIEB_FP8_E4M3;
+  p.row_elems = p.is_tf32 ? 32 : (p.is_fp8 ? 128 : 64);
+  p.c_blocks = r.kb_per_tap; p.last_ksteps = r.h_last_ksteps;
+  p.taps_per_load = r.h_taps_per_load; p.tap_groups = r.h_tap_groups;
+  p.total_loads = r.h_total_loads; p.loads_per_split = r.h_loads_per_split;
+  p.tiles_n = r.tiles_n;
+  p.num_tiles = ceil_div(p.rows_total, r.tile_m) * r.tiles_n * r.split_k;
+  p.split = r.split_k;
+  p.out_nhwc = (d.flags & GIEB_FLAG_OUTPUT_NHWC) != 0;
+  const uintptr_t both = reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(residual);
+  p.out_cells = p.out_nhwc && both % 16 == 0 && d.out_channels % 8 == 0;
+  p.out_rows = (both % 4 == 0 && d.out_channels % 2 == 0) ? 2 : 1;
+  p.relu = d.relu;
+  p.bias_fp32 = p.is_tf32 || p.is_fp8 || (d.flags & GIEB_FLAG_BIAS_FP32);
+  p.idesc = p.is_tf32 ? ptx::make_idesc_tf32(kTileM, r.tile_n, false, false)
+                      : ptx::make_idesc_f16(r.pair ? 2 * kTileM : kTileM, r.tile_n, p.is_bf16, false, false);
+  p.fd_split = FastDiv::make(p.split);
+  p.fd_tiles_n = FastDiv::make(p.tiles_n);
+  p.fd_groups = FastDiv::make(p.tap_groups);
+  p.fd_kernel_w = FastDiv::make(p.kernel_w);
+  p.fd_ws = FastDiv::make(p.ws);
+  p.fd_hs = FastDiv::make(p.hs);
+  p.fd_gpo = FastDiv::make(r.tile_n / 4 / p.split);
+  p.fd_boxes = FastDiv::make(p.boxes);
+  p.fd_box_rows = FastDiv::make(p.box_rows);
+  const int64_t resident = r.pair ? kNumSmPairs : int64_t(kNumSms) * resident_ctas(kTileM, r.epi_warps == 16 ? 256 : r.tile_n, r.smem);
+  const dim3 grid(unsigned(p.split > 1 || p.num_tiles < resident ? p.num_tiles : resident) * (r.pair ? 2u : 1u));
+  if (ev) GIEB_CUDA(cudaEventRecord(ev[1], st));
+  if (stage_mask & 2u) GIEB_CUDA(conv_halo_launch(r.tile_n, r.epi_warps, r.pair != 0, tm_act, tm_wgt, p, grid, r.smem, st));
+  if (ev) { GIEB_CUDA(cudaEventRecord(ev[2], st)); GIEB_CUDA(cudaEventRecord(ev[3], st)); }
+  return GIEB_OK;
+}
+
 // `ev`, when given, receives four stage marks: before the repack, before the convolution kernel, after it, and
 // after the split-K reduction (LaunchArgs::stage_events analogue, include/gpu_inference/kernel_registry.h:38-40).
 int launch_impl(const gieb_conv_plan* pl, const void* x, const void* w, const void* bias, void* y, void* ws, size_t ws_bytes,
@@ -791,7 +1014,7 @@ int launch_impl(const gieb_conv_plan* pl, const void* x, const void* w, const vo
   if (w_direct) wk = w;
 
   CUtensorMap tm_act, tm_wgt;
-  const int st_maps = encode_maps(pl, mode, mode == 2 ? x : xn, wk, &tm_act, &tm_wgt);
+  const int st_maps = r.halo ? encode_halo_maps(pl, xn, wk, &tm_act, &tm_wgt) : encode_maps(pl, mode, mode == 2 ? x : xn, wk, &tm_act, &tm_wgt);
   if (st_maps != GIEB_OK) return st_maps;
 
   if (ev) GIEB_CUDA(cudaEventRecord(ev[0], st));
@@ -822,6 +1045,8 @@ int launch_impl(const gieb_conv_plan* pl, const void* x, const void* w, const vo
   else
     GIEB_CUDA(repack_pair_launch(x, xn, d.batch, d.in_channels, d.in_h * d.in_w, r.c_padded, w, const_cast<void*>(wk),
                                  d.out_channels, d.in_channels, d.kernel_h * d.kernel_w, r.c_padded, st));
+
+  if (r.halo) return launch_halo(pl, tm_act, tm_wgt, bias, residual, y, st, ev, stage_mask);
 
   ConvTcParams p;
   memset(&p, 0, sizeof(p));
@@ -994,7 +1219,8 @@ int gieb_conv_plan_create(const gieb_conv_desc* desc, const gieb_conv_cfg* cfg, 
     }
   }
   if (e == cudaSuccess && r.variant != 3)
-    e = r.swap ? conv_tc_swap_prepare(r.tile_m, r.tile_n, r.tile_k, r.epi_warps, kMaxDynamicSmem)
+    e = r.halo ? conv_halo_prepare(r.tile_n, r.epi_warps, r.pair != 0, kMaxDynamicSmem)
+        : r.swap ? conv_tc_swap_prepare(r.tile_m, r.tile_n, r.tile_k, r.epi_warps, kMaxDynamicSmem)
         : r.pair ? conv_tc_pair_prepare(r.tile_n, r.tile_k, kMaxDynamicSmem)
                  : conv_tc_prepare(r.tile_m, r.tile_n, r.tile_k, r.epi_warps, kMaxDynamicSmem);
   if (e != cudaSuccess) {
@@ -1146,7 +1372,8 @@ int gieb_conv_forward_static(const gieb_conv_desc* desc, const gieb_conv_cfg* cf
   pl.d_status = reinterpret_cast<uint32_t*>(base);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (pl.r.variant != 3)
-    GIEB_CUDA(pl.r.swap ? conv_tc_swap_prepare(pl.r.tile_m, pl.r.tile_n, pl.r.tile_k, pl.r.epi_warps, kMaxDynamicSmem)
+    GIEB_CUDA(pl.r.halo ? conv_halo_prepare(pl.r.tile_n, pl.r.epi_warps, pl.r.pair != 0, kMaxDynamicSmem)
+              : pl.r.swap ? conv_tc_swap_prepare(pl.r.tile_m, pl.r.tile_n, pl.r.tile_k, pl.r.epi_warps, kMaxDynamicSmem)
               : pl.r.pair ? conv_tc_pair_prepare(pl.r.tile_n, pl.r.tile_k, kMaxDynamicSmem)
                           : conv_tc_prepare(pl.r.tile_m, pl.r.tile_n, pl.r.tile_k, pl.r.epi_warps, kMaxDynamicSmem));
   // The array keeps whatever the previous call left: the status word must start at zero.  Everything else in the

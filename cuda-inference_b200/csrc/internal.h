@@ -149,6 +149,41 @@ struct ConvTcParams {
   uint32_t debug_skip;   // test hook, 0 in production: bit 0 = the producers load nothing, bit 1 = the MMA warp issues nothing
 };
 
+// Everything conv_halo_kernel needs besides the tensor maps (see conv_halo.cu for the padded grid and the halo tile).
+struct ConvHaloParams {
+  const void* bias;      // or null
+  const void* residual;  // or null; shape, layout and type of y
+  void* y;
+  uint32_t* status;
+  long long wait_limit;
+  int batch;
+  int out_channels, out_h, out_w, pq;
+  int kernel_w, taps, stride_h, stride_w, pad_h, pad_w;
+  int hs, ws;            // rows and columns of the padded grid per image
+  int rows_total;        // batch * hs * ws
+  int phases, phases_w;  // phases of a halo tile (1 at stride 1)
+  int halo_rows;         // rows of one phase in shared memory
+  uint32_t a_stage_bytes;
+  int a_stages, b_stages;
+  int resident;          // the weights of a tile fit b_stages and are the same for all tiles of a CTA: loaded once
+  // a phase is `boxes` boxes of box_h padded rows (box_rows = box_h * ws grid rows, box_bytes = 128 * box_rows)
+  int boxes, box_h, box_rows;
+  uint32_t box_bytes;
+  int row_elems;                          // elements of a 128-byte row: 64, or 32 (TF32) or 128 (FP8)
+  int c_blocks, last_ksteps;              // blocks of row_elems channels; MMA steps (32 bytes) of the last one
+  int taps_per_load, tap_groups;          // filter taps per weight load, loads per channel block
+  int total_loads, loads_per_split;       // the reduction in weight loads
+  int tiles_n, num_tiles, split;
+  int out_nhwc, out_cells, out_rows;      // channel-contiguous output: 16-byte cells allowed; 2 = else channel pairs, 1 = singly
+  int relu, is_bf16, is_tf32, is_fp8, bias_fp32;
+  uint32_t idesc, debug_skip;
+  FastDiv fd_split, fd_tiles_n, fd_groups, fd_kernel_w, fd_ws, fd_hs, fd_gpo, fd_boxes, fd_box_rows;
+};
+size_t conv_halo_smem_bytes(int tile_n, bool pair, int workers, int taps_per_load, int a_stages, size_t a_stage_bytes, int b_stages, bool staging);
+cudaError_t conv_halo_prepare(int tile_n, int workers, bool pair, size_t smem);
+cudaError_t conv_halo_launch(int tile_n, int workers, bool pair, const CUtensorMap& tm_act, const CUtensorMap& tm_wgt,
+                             const ConvHaloParams& p, dim3 grid, size_t smem, cudaStream_t stream);
+
 // tile_m is 128 or 256 output pixels per CTA (one or two TMEM accumulators sharing each weight tile).
 // pair: the tile belongs to a CTA pair (tile_m = 256), each CTA stages 128 activation rows and tile_n / 2 weight rows.
 // epilogue_bytes: staging of the epilogue behind the ring (TMA-store boxes, or the NCHW transposition tiles).
