@@ -40,7 +40,7 @@ int fail_cuda(cudaError_t e, const char* what) {
   } while (0)
 
 // ---- hardware constants of the one supported target (B200, sm_100a) -------------------------------------------------
-constexpr size_t kMaxDynamicSmem = 232448;  // 227 KiB opt-in limit per CTA
+constexpr size_t kMaxDynamicSmem = kCtaSmemLimit;
 
 size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 int ceil_div(int64_t a, int64_t b) { return int((a + b - 1) / b); }
@@ -121,6 +121,7 @@ struct Resolved {
   int c_padded, kb_per_tap, total_kb, kb_per_split;
   int tiles_m, tiles_n;
   size_t smem;
+  int epi_boxes;  // staging boxes per epilogue warp (see ConvTcParams)
   int epi_warps;  // 8, or 16 when the CTA has its SM to itself (see conv_tc_kernel)
   size_t ws_x, ws_w, ws_part, ws_total;  // workspace layout (bytes; offsets are cumulative in this order)
   // The halo-tile kernel (conv_halo.cu) instead of the slab kernels: tile_m, tile_n, split_k, pair, stages (of the weight
@@ -171,7 +172,7 @@ int pick_stages(int tile_m, int tile_n, int tile_k, int kb_per_split, int64_t ct
   int want = 1;
   if (ctas > kNumSms) want = 2;  // two CTAs per SM (the register file holds no more)
   if (want > by_tmem) want = by_tmem;
-  const size_t budget = want == 1 ? kMaxDynamicSmem - 1024 : (kMaxDynamicSmem / want - 2048);
+  const size_t budget = want == 1 ? kMaxDynamicSmem : kMaxDynamicSmem / want - 2048;
   int stages = budget > 3072 + extra_smem + sb ? int((budget - 3072 - extra_smem) / sb) : 1;
   if (stages > 6) stages = 6;
   if (stages > kb_per_split) stages = kb_per_split;
@@ -231,7 +232,7 @@ double estimate_cycles(const gieb_conv_desc& d, const Geometry& g, int tile_m, i
 // Ring depth of a CTA pair: each CTA owns its SM, so the ring takes what shared memory is left.
 int pick_pair_stages(int tile_n, int tile_k, int kb_per_split, size_t extra_smem) {
   const size_t sb = pair_stage_bytes_of(tile_n, tile_k);
-  int stages = int((kMaxDynamicSmem - 1024 - 3072 - extra_smem) / sb);
+  int stages = int((kMaxDynamicSmem - 3072 - extra_smem) / sb);
   if (stages > kMaxStages) stages = kMaxStages;
   if (stages > kb_per_split) stages = kb_per_split;
   if (stages < 2) stages = 2;
@@ -390,7 +391,7 @@ bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, double slab, Resol
         if (f.b < 3 && !f.resident) main *= 1.5;  // (two weight stages do not cover a load)
         const double drain = 800.0 + 18.0 * bn * (workers == 16 ? 0.6 : 1.0);
         double t = (load > 1 ? 4500.0 : 3500.0) + a_time + load * fmax(main, load > 1 ? drain : 0.0) + (load - 1) * 600.0 + drain;
-        if (s > 1) t += 3500.0;
+        if (s > 1) t += 2000.0 + double(s - 1) / s * (double(kTileM) * bn * 4.0) / 5.0;  // exchange of the partial columns in the cluster
         if (ph * pw > 1) t += 0.15 * load * main;  // (the phases are loaded whole)
         if (t < best) {
           best = t;
@@ -647,7 +648,15 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
     // keeps more loads in flight than two shallow ones (measured on 512 -> 128 channels at 28x28: 17.5 vs 18.4 us).
     if (!c.stages && !r->pair && r->variant == 2 && r->kb_per_split >= 8) {
       const size_t sb = stage_bytes_of(r->tile_m, r->tile_n, r->tile_k);
-      if (3072 + 1024 + 6 * sb + epi_smem <= kMaxDynamicSmem) st = 6;
+      if (3072 + 6 * sb + epi_smem <= kMaxDynamicSmem) st = 6;
+    }
+    // The same for channel-contiguous tensors, where the epilogue's staging leaves two co-resident CTAs of 128 columns two slabs each:
+    // 64 x 512 -> 128 at 56 x 56 takes 52.0 us that way, 44.2 with one CTA and six slabs (256 -> 128: 31.5 and 27.5; 128 -> 128, two
+    // slabs per tile: 21.6 and 25.3).  Tiles of 64 columns gain when nothing is read twice (1x1: 256 -> 64 25.9 and 23.8 us).
+    if (!c.stages && !r->pair && (r->tma_epilogue || r->row_epilogue) && r->tile_m == kTileM && r->kb_per_split * r->tile_k >= 256 && total_tiles > kNumSms &&
+        (r->tile_n == 128 || (r->tile_n == 64 && r->variant == 4))) {
+      const int most = int((kMaxDynamicSmem - 3072 - epi_smem) / stage_bytes_of(r->tile_m, r->tile_n, r->tile_k));
+      st = most < 6 ? most : 6;
     }
     return st;
   };
@@ -661,7 +670,12 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
     const bool single_tile = total_tiles <= kNumSms;
     return (alone && (r->tile_n >= 256 || (r->tile_n >= 128 && single_tile && best_mode != 2))) ? 16 : 8;
   };
-  size_t epi_smem = r->tma_epilogue || r->row_epilogue ? conv_tc_epilogue_staging_bytes(r->tile_n) : (swap ? size_t(8) * 2048 : 0);
+  // Staging of the epilogue: a box of 2 KiB per chunk of 32 channels and 32 pixels; a tile of 256 channels without residual makes do
+  // with one box per warp, and its ring has four slabs instead of three (six instead of four in a pair): the loop over 7 slabs of
+  // 448 -> 640 channels is 5 % shorter, while with fewer than four slabs the epilogue is what counts.
+  const bool one_box = r->tile_n == 256 && (r->row_epilogue || (!(d.flags & GIEB_FLAG_RESIDUAL) && r->kb_per_split >= 4));
+  const int boxes = one_box ? 16 : (r->tile_n / 8 > 8 ? r->tile_n / 8 : 8);
+  size_t epi_smem = r->tma_epilogue || r->row_epilogue ? size_t(boxes) * 2048 : (swap ? size_t(8) * 2048 : 0);
   int stages = stages_for(epi_smem);
   if (stages < 2 || stages > kMaxStages) return no("stages must be in [2, 8]");
   r->smem = conv_tc_smem_bytes(r->tile_m, r->tile_n, r->tile_k, stages, epi_smem, r->pair != 0);
@@ -672,6 +686,7 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
     r->smem = conv_tc_smem_bytes(r->tile_m, r->tile_n, r->tile_k, stages, 0, r->pair != 0);
     r->epi_warps = epi_warps_for(r->smem);
   }
+  r->epi_boxes = one_box ? 1 : conv_tc_epilogue_boxes(r->tile_n, r->epi_warps);
   r->swap = swap;
   r->stages = stages;
   if (r->smem > kMaxDynamicSmem) return no("configuration needs more shared memory than one CTA may have (227 KiB)");
@@ -1086,6 +1101,7 @@ int launch_impl(const gieb_conv_plan* pl, const void* x, const void* w, const vo
   p.tiles_n = r.tiles_n;
   p.num_tiles = p.tiles_m * p.tiles_n * r.split_k;
   p.cluster_split = r.reduce == 2 ? r.split_k : 1;
+  p.epi_boxes = r.epi_boxes;
   p.fd_cluster = FastDiv::make(p.cluster_split);
   p.fd_tiles_mn = FastDiv::make(p.tiles_m * p.tiles_n);
   p.fd_tiles_n = FastDiv::make(p.tiles_n);
@@ -1140,7 +1156,7 @@ int launch_impl(const gieb_conv_plan* pl, const void* x, const void* w, const vo
     }
   }
   if (!(stage_mask & 2u)) {
-  } else if (r.swap) GIEB_CUDA(conv_tc_swap_launch(r.tile_m, r.tile_n, r.tile_k, r.epi_warps, tm_act, tm_wgt, tm_out, p, grid, r.smem, st));
+  } else if (r.swap) GIEB_CUDA(conv_tc_swap_launch(r.tile_m, r.tile_n, r.tile_k, tm_act, tm_wgt, tm_out, p, grid, r.smem, st));
   else if (r.pair) GIEB_CUDA(conv_tc_pair_launch(r.tile_n, r.tile_k, tm_act, tm_wgt, tm_out, tm_res, p, grid, r.smem, st));
   else GIEB_CUDA(conv_tc_launch(r.tile_m, r.tile_n, r.tile_k, r.epi_warps, tm_act, tm_wgt, tm_out, tm_res, p, grid, r.smem, st));
   if (ev) GIEB_CUDA(cudaEventRecord(ev[2], st));
@@ -1220,7 +1236,7 @@ int gieb_conv_plan_create(const gieb_conv_desc* desc, const gieb_conv_cfg* cfg, 
   }
   if (e == cudaSuccess && r.variant != 3)
     e = r.halo ? conv_halo_prepare(r.tile_n, r.epi_warps, r.pair != 0, kMaxDynamicSmem)
-        : r.swap ? conv_tc_swap_prepare(r.tile_m, r.tile_n, r.tile_k, r.epi_warps, kMaxDynamicSmem)
+        : r.swap ? conv_tc_swap_prepare(r.tile_m, r.tile_n, r.tile_k, kMaxDynamicSmem)
         : r.pair ? conv_tc_pair_prepare(r.tile_n, r.tile_k, kMaxDynamicSmem)
                  : conv_tc_prepare(r.tile_m, r.tile_n, r.tile_k, r.epi_warps, kMaxDynamicSmem);
   if (e != cudaSuccess) {
@@ -1373,7 +1389,7 @@ int gieb_conv_forward_static(const gieb_conv_desc* desc, const gieb_conv_cfg* cf
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (pl.r.variant != 3)
     GIEB_CUDA(pl.r.halo ? conv_halo_prepare(pl.r.tile_n, pl.r.epi_warps, pl.r.pair != 0, kMaxDynamicSmem)
-              : pl.r.swap ? conv_tc_swap_prepare(pl.r.tile_m, pl.r.tile_n, pl.r.tile_k, pl.r.epi_warps, kMaxDynamicSmem)
+              : pl.r.swap ? conv_tc_swap_prepare(pl.r.tile_m, pl.r.tile_n, pl.r.tile_k, kMaxDynamicSmem)
               : pl.r.pair ? conv_tc_pair_prepare(pl.r.tile_n, pl.r.tile_k, kMaxDynamicSmem)
                           : conv_tc_prepare(pl.r.tile_m, pl.r.tile_n, pl.r.tile_k, pl.r.epi_warps, kMaxDynamicSmem));
   // The array keeps whatever the previous call left: the status word must start at zero.  Everything else in the

@@ -1,5 +1,5 @@
 // Instantiations and host-side dispatch of the single-CTA points of the tensor-core convolution kernel
-// (conv_tc_kernel.cuh), and the split-K reduction kernel.
+// (conv_tc_kernel.cuh; those of 128 and 256 channels are in conv_tc_wide.cu), and the split-K reduction kernel.
 #include "conv_tc_kernel.cuh"
 
 namespace gieb {
@@ -20,43 +20,19 @@ cudaError_t launch_one(const CUtensorMap& ta, const CUtensorMap& tw, const CUten
 }
 
 #define GIEB_TC_DISPATCH(FN, ...) \
-  switch ((epi_warps == 16 ? 1000000 : 0) + tile_m / 128 * 100000 + tile_n * 100 + tile_k) { \
-    case 0 + 1 * 100000 + 32 * 100 + 16: return FN<32, 16, 1, 8>(__VA_ARGS__); \
-    case 0 + 2 * 100000 + 32 * 100 + 16: return FN<32, 16, 2, 8>(__VA_ARGS__); \
-    case 0 + 1 * 100000 + 32 * 100 + 32: return FN<32, 32, 1, 8>(__VA_ARGS__); \
-    case 0 + 2 * 100000 + 32 * 100 + 32: return FN<32, 32, 2, 8>(__VA_ARGS__); \
-    case 0 + 1 * 100000 + 32 * 100 + 64: return FN<32, 64, 1, 8>(__VA_ARGS__); \
-    case 0 + 2 * 100000 + 32 * 100 + 64: return FN<32, 64, 2, 8>(__VA_ARGS__); \
-    case 0 + 1 * 100000 + 64 * 100 + 16: return FN<64, 16, 1, 8>(__VA_ARGS__); \
-    case 0 + 2 * 100000 + 64 * 100 + 16: return FN<64, 16, 2, 8>(__VA_ARGS__); \
-    case 0 + 1 * 100000 + 64 * 100 + 32: return FN<64, 32, 1, 8>(__VA_ARGS__); \
-    case 0 + 2 * 100000 + 64 * 100 + 32: return FN<64, 32, 2, 8>(__VA_ARGS__); \
-    case 0 + 1 * 100000 + 64 * 100 + 64: return FN<64, 64, 1, 8>(__VA_ARGS__); \
-    case 0 + 2 * 100000 + 64 * 100 + 64: return FN<64, 64, 2, 8>(__VA_ARGS__); \
-    case 0 + 1 * 100000 + 128 * 100 + 16: return FN<128, 16, 1, 8>(__VA_ARGS__); \
-    case 0 + 2 * 100000 + 128 * 100 + 16: return FN<128, 16, 2, 8>(__VA_ARGS__); \
-    case 0 + 1 * 100000 + 128 * 100 + 32: return FN<128, 32, 1, 8>(__VA_ARGS__); \
-    case 0 + 2 * 100000 + 128 * 100 + 32: return FN<128, 32, 2, 8>(__VA_ARGS__); \
-    case 0 + 1 * 100000 + 128 * 100 + 64: return FN<128, 64, 1, 8>(__VA_ARGS__); \
-    case 0 + 2 * 100000 + 128 * 100 + 64: return FN<128, 64, 2, 8>(__VA_ARGS__); \
-    case 0 + 1 * 100000 + 256 * 100 + 16: return FN<256, 16, 1, 8>(__VA_ARGS__); \
-    case 0 + 2 * 100000 + 256 * 100 + 16: return FN<256, 16, 2, 8>(__VA_ARGS__); \
-    case 0 + 1 * 100000 + 256 * 100 + 32: return FN<256, 32, 1, 8>(__VA_ARGS__); \
-    case 0 + 2 * 100000 + 256 * 100 + 32: return FN<256, 32, 2, 8>(__VA_ARGS__); \
-    case 0 + 1 * 100000 + 256 * 100 + 64: return FN<256, 64, 1, 8>(__VA_ARGS__); \
-    case 0 + 2 * 100000 + 256 * 100 + 64: return FN<256, 64, 2, 8>(__VA_ARGS__); \
-    case 1000000 + 1 * 100000 + 128 * 100 + 16: return FN<128, 16, 1, 16>(__VA_ARGS__); \
-    case 1000000 + 2 * 100000 + 128 * 100 + 16: return FN<128, 16, 2, 16>(__VA_ARGS__); \
-    case 1000000 + 1 * 100000 + 128 * 100 + 32: return FN<128, 32, 1, 16>(__VA_ARGS__); \
-    case 1000000 + 2 * 100000 + 128 * 100 + 32: return FN<128, 32, 2, 16>(__VA_ARGS__); \
-    case 1000000 + 1 * 100000 + 128 * 100 + 64: return FN<128, 64, 1, 16>(__VA_ARGS__); \
-    case 1000000 + 2 * 100000 + 128 * 100 + 64: return FN<128, 64, 2, 16>(__VA_ARGS__); \
-    case 1000000 + 1 * 100000 + 256 * 100 + 16: return FN<256, 16, 1, 16>(__VA_ARGS__); \
-    case 1000000 + 2 * 100000 + 256 * 100 + 16: return FN<256, 16, 2, 16>(__VA_ARGS__); \
-    case 1000000 + 1 * 100000 + 256 * 100 + 32: return FN<256, 32, 1, 16>(__VA_ARGS__); \
-    case 1000000 + 2 * 100000 + 256 * 100 + 32: return FN<256, 32, 2, 16>(__VA_ARGS__); \
-    case 1000000 + 1 * 100000 + 256 * 100 + 64: return FN<256, 64, 1, 16>(__VA_ARGS__); \
-    case 1000000 + 2 * 100000 + 256 * 100 + 64: return FN<256, 64, 2, 16>(__VA_ARGS__); \
+  switch (tile_m / 128 * 100000 + tile_n * 100 + tile_k) { \
+    case 1 * 100000 + 32 * 100 + 16: return FN<32, 16, 1, 8>(__VA_ARGS__); \
+    case 2 * 100000 + 32 * 100 + 16: return FN<32, 16, 2, 8>(__VA_ARGS__); \
+    case 1 * 100000 + 32 * 100 + 32: return FN<32, 32, 1, 8>(__VA_ARGS__); \
+    case 2 * 100000 + 32 * 100 + 32: return FN<32, 32, 2, 8>(__VA_ARGS__); \
+    case 1 * 100000 + 32 * 100 + 64: return FN<32, 64, 1, 8>(__VA_ARGS__); \
+    case 2 * 100000 + 32 * 100 + 64: return FN<32, 64, 2, 8>(__VA_ARGS__); \
+    case 1 * 100000 + 64 * 100 + 16: return FN<64, 16, 1, 8>(__VA_ARGS__); \
+    case 2 * 100000 + 64 * 100 + 16: return FN<64, 16, 2, 8>(__VA_ARGS__); \
+    case 1 * 100000 + 64 * 100 + 32: return FN<64, 32, 1, 8>(__VA_ARGS__); \
+    case 2 * 100000 + 64 * 100 + 32: return FN<64, 32, 2, 8>(__VA_ARGS__); \
+    case 1 * 100000 + 64 * 100 + 64: return FN<64, 64, 1, 8>(__VA_ARGS__); \
+    case 2 * 100000 + 64 * 100 + 64: return FN<64, 64, 2, 8>(__VA_ARGS__); \
     default: return cudaErrorInvalidValue;                                            \
   }
 
@@ -137,23 +113,25 @@ splitk_reduce_kernel(const float* __restrict__ partial, int splits, int64_t tota
 
 }  // namespace
 
-// 8 epilogue warps x ceil(chunks / 2) boxes = 16 warps x ceil(chunks / 4) boxes for the tile widths that may run 16 warps
-size_t conv_tc_epilogue_staging_bytes(int tile_n) { return size_t(8) * (tile_n >= 64 ? tile_n / 64 : 1) * 2048; }
+int conv_tc_epilogue_boxes(int tile_n, int epi_warps) { return tile_n / 32 * 4 > epi_warps ? tile_n / 32 * 4 / epi_warps : 1; }
 
 int conv_tc_threads(int epi_warps) { return 32 * (kProducerWarps + 1 + epi_warps); }
 
 size_t conv_tc_smem_bytes(int tile_m, int tile_n, int tile_k, int stages, size_t epilogue_bytes, bool pair) {
   const size_t rows = pair ? size_t(kTileM) + tile_n / 2 : size_t(tile_m) + tile_n;  // operand rows one CTA stages per slab
-  return 1024 + kCtrlBytes + size_t(stages) * rows * tile_k * 2 + epilogue_bytes;
+  const size_t bytes = kCtrlBytes + size_t(stages) * rows * tile_k * 2 + epilogue_bytes;
+  return bytes + 1024 <= kCtaSmemLimit ? bytes + 1024 : bytes;  // a KiB of reserve that a ring filling the last byte does without
 }
 
 cudaError_t conv_tc_prepare(int tile_m, int tile_n, int tile_k, int epi_warps, size_t smem_bytes) {
+  if (tile_n >= 128) return conv_tc_wide_prepare(tile_m, tile_n, tile_k, epi_warps, smem_bytes);
   GIEB_TC_DISPATCH(prepare_one, smem_bytes)
 }
 
 cudaError_t conv_tc_launch(int tile_m, int tile_n, int tile_k, int epi_warps, const CUtensorMap& tm_act, const CUtensorMap& tm_wgt,
                            const CUtensorMap& tm_out, const CUtensorMap& tm_res, const ConvTcParams& p, dim3 grid, size_t smem_bytes,
                            cudaStream_t stream) {
+  if (tile_n >= 128) return conv_tc_wide_launch(tile_m, tile_n, tile_k, epi_warps, tm_act, tm_wgt, tm_out, tm_res, p, grid, smem_bytes, stream);
   GIEB_TC_DISPATCH(launch_one, tm_act, tm_wgt, tm_out, tm_res, p, grid, smem_bytes, stream)
 }
 

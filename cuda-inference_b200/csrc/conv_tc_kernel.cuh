@@ -48,6 +48,30 @@ __device__ __forceinline__ T round_to(float a) {
   else return __float2bfloat16_rn(a);
 }
 
+// Two sums to storage type in one word: one rounding each, then the ReLU on the rounded pair (rounding is monotonic and keeps
+// zero, so this is the ReLU of the sums; a NaN becomes zero either way).
+template <typename T, bool RELU>
+__device__ __forceinline__ uint32_t round_pair(float2 a) {
+  if constexpr (std::is_same<T, __half>::value) {
+    __half2 o = __floats2half2_rn(a.x, a.y);
+    if (RELU) o = __hmax2(o, __half2half2(__ushort_as_half(0)));
+    return *reinterpret_cast<const uint32_t*>(&o);
+  } else {
+    __nv_bfloat162 o = __floats2bfloat162_rn(a.x, a.y);
+    if (RELU) o = __hmax2(o, __bfloat162bfloat162(__ushort_as_bfloat16(0)));
+    return *reinterpret_cast<const uint32_t*>(&o);
+  }
+}
+
+// A stored pair as two floats.
+template <typename T>
+__device__ __forceinline__ float2 pair_to_float(uint32_t w) {
+  if constexpr (std::is_same<T, __half>::value) return __half22float2(*reinterpret_cast<const __half2*>(&w));
+  else return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w));
+}
+
+__device__ __forceinline__ float2 acc_pair(const uint32_t (&v)[32], int i) { return make_float2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])); }
+
 // Epilogue of one 32-column chunk for one accumulator row (= one output pixel): + bias, optional ReLU, one rounding,
 // 32 stores that are `stride` elements apart (consecutive output channels of an NCHW tensor).  Branch-free body:
 // the ReLU / storage-type / full-chunk decisions are made once per chunk by the caller.
@@ -58,14 +82,20 @@ __device__ __forceinline__ void store_chunk_full(const uint32_t (&v)[32], const 
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
     const float4 b = b4[q];
-    const float bb[4] = {b.x, b.y, b.z, b.w};
+    const float2 lo = ptx::add_f32x2(acc_pair(v, q * 4), make_float2(b.x, b.y)), hi = ptx::add_f32x2(acc_pair(v, q * 4 + 2), make_float2(b.z, b.w));
+    if constexpr (sizeof(T) == 2) {
+      const uint32_t w0 = round_pair<T, RELU>(lo), w1 = round_pair<T, RELU>(hi);
+      uint16_t* d = reinterpret_cast<uint16_t*>(dst);
+      d[0] = uint16_t(w0);
+      d[stride] = uint16_t(w0 >> 16);
+      d[2 * stride] = uint16_t(w1);
+      d[3 * stride] = uint16_t(w1 >> 16);
+    } else {
+      const float a[4] = {lo.x, lo.y, hi.x, hi.y};
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      float a = __uint_as_float(v[q * 4 + t]) + bb[t];
-      if (RELU) a = fmaxf(a, 0.f);
-      *dst = round_to<T>(a);
-      dst += stride;
+      for (int t = 0; t < 4; ++t) dst[t * stride] = RELU ? fmaxf(a[t], 0.f) : a[t];
     }
+    dst += 4 * stride;
   }
 }
 
@@ -113,30 +143,13 @@ __device__ __forceinline__ uint4 finish8(const uint32_t (&v)[32], int q, const f
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const float4 b = b4[q * 2 + h];
-    const float bb[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-      float a0 = __uint_as_float(v[q * 8 + h * 4 + t * 2]) + bb[t * 2];
-      float a1 = __uint_as_float(v[q * 8 + h * 4 + t * 2 + 1]) + bb[t * 2 + 1];
-      if (RES) {
-        const uint32_t w = rw[h * 2 + t];
-        if constexpr (std::is_same<T, __half>::value) {
-          const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
-          a0 += f.x; a1 += f.y;
-        } else {
-          const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w));
-          a0 += f.x; a1 += f.y;
-        }
-      }
-      if (RELU) { a0 = fmaxf(a0, 0.f); a1 = fmaxf(a1, 0.f); }
-      if constexpr (std::is_same<T, __half>::value) {
-        const __half2 o = __floats2half2_rn(a0, a1);
-        ow[h * 2 + t] = *reinterpret_cast<const uint32_t*>(&o);
-      } else {
-        const __nv_bfloat162 o = __floats2bfloat162_rn(a0, a1);
-        ow[h * 2 + t] = *reinterpret_cast<const uint32_t*>(&o);
-      }
+    float2 lo = ptx::add_f32x2(acc_pair(v, q * 8 + h * 4), make_float2(b.x, b.y)), hi = ptx::add_f32x2(acc_pair(v, q * 8 + h * 4 + 2), make_float2(b.z, b.w));
+    if (RES) {
+      lo = ptx::add_f32x2(lo, pair_to_float<T>(rw[h * 2]));
+      hi = ptx::add_f32x2(hi, pair_to_float<T>(rw[h * 2 + 1]));
     }
+    ow[h * 2] = round_pair<T, RELU>(lo);
+    ow[h * 2 + 1] = round_pair<T, RELU>(hi);
   }
   return make_uint4(ow[0], ow[1], ow[2], ow[3]);
 }
@@ -229,27 +242,13 @@ __device__ __forceinline__ void row_to_staging(const uint32_t (&v)[32], float bi
   uint32_t w[16];
 #pragma unroll
   for (int j = 0; j < 16; ++j) {
-    float a0 = __uint_as_float(v[2 * j]) + bias, a1 = __uint_as_float(v[2 * j + 1]) + bias;
+    float2 a = ptx::add_f32x2(acc_pair(v, 2 * j), make_float2(bias, bias));
     if constexpr (RES) {  // the residual's 32 pixels of this lane's channel, in storage type
       const uint4& r4 = res[j >> 2];
-      const uint32_t rw = (j & 3) == 0 ? r4.x : ((j & 3) == 1 ? r4.y : ((j & 3) == 2 ? r4.z : r4.w));
-      if constexpr (std::is_same<T, __half>::value) {
-        const float2 rf = __half22float2(*reinterpret_cast<const __half2*>(&rw));
-        a0 += rf.x; a1 += rf.y;
-      } else {
-        const float2 rf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&rw));
-        a0 += rf.x; a1 += rf.y;
-      }
+      a = ptx::add_f32x2(a, pair_to_float<T>((j & 3) == 0 ? r4.x : ((j & 3) == 1 ? r4.y : ((j & 3) == 2 ? r4.z : r4.w))));
     }
-    if constexpr (std::is_same<T, __half>::value) {
-      __half2 o = __floats2half2_rn(a0, a1);
-      const __half2 oz = __hmax2(o, __half2half2(__ushort_as_half(0)));
-      w[j] = relu ? *reinterpret_cast<const uint32_t*>(&oz) : *reinterpret_cast<const uint32_t*>(&o);
-    } else {
-      __nv_bfloat162 o = __floats2bfloat162_rn(a0, a1);
-      const __nv_bfloat162 oz = __hmax2(o, __bfloat162bfloat162(__ushort_as_bfloat16(0)));
-      w[j] = relu ? *reinterpret_cast<const uint32_t*>(&oz) : *reinterpret_cast<const uint32_t*>(&o);
-    }
+    const uint32_t plain = round_pair<T, false>(a), clamped = round_pair<T, true>(a);
+    w[j] = relu ? clamped : plain;
   }
   const int sw = (lane >> 1) & 3;
 #pragma unroll
@@ -336,8 +335,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
   constexpr uint32_t TMEM_COLS = ACC_COLS * ACC_BUFS < 32 ? 32 : ACC_COLS * ACC_BUFS;
   static_assert(TMEM_COLS <= 512, "accumulators must fit the 512 TMEM columns");
 
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = smem_raw + ((1024u - (ptx::smem_u32(smem_raw) & 1023u)) & 1023u);
+  extern __shared__ __align__(1024) uint8_t smem[];
   float* bias_s = reinterpret_cast<float*>(smem);  // [2][256]
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + 2048);
   uint64_t* empty_bar = full_bar + kMaxStages;
@@ -348,7 +346,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
   uint64_t* res_bar = acc_empty + 2;               // [EW epilogue warps][kEpiBufs] residual tile landed (TMA epilogue only)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(res_bar + EW * kEpiBufs);
   uint8_t* stage_base = smem + kCtrlBytes;
-  // TMA epilogue staging: per epilogue warp kEpiBufs boxes of 32 pixels x 32 channels (2 KiB, 64-byte swizzle)
+  // Epilogue staging: per epilogue warp p.epi_boxes (1 or kEpiBufs) boxes of 32 pixels x 32 channels (2 KiB, 64-byte swizzle)
   uint8_t* epi_base = stage_base + size_t(p.stages) * STAGE_BYTES;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -667,6 +665,23 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
     const int par = (warp - kProducerWarps - 1) >> 2;  // 0 .. EG-1: which chunks this warp owns
     const int et = threadIdx.x - 32 * (kProducerWarps + 1);  // index among the epilogue threads
     const int we = warp - kProducerWarps - 1;                // index among the epilogue warps
+    int box_turn = 0;                                        // staging box of the next TMA store (without residual)
+    // The bias of a channel tile is staged as floats, in two buffers taken in turn: when a warp fills one, every warp has passed
+    // the barrier of the other and has therefore finished with what it overwrites.  The value is loaded one tile ahead, and a
+    // CTA whose next tile has the same channels keeps what is there, without a barrier.
+    int staged_n0 = -1, bias_buf = 0;
+    float bias_next = 0.f;
+    auto load_bias = [&](int n0) {
+      const int oc = n0 + et;
+      float b = 0.f;
+      if (et < BN && p.has_bias && p.partial == nullptr && oc < p.out_channels) {
+        if (p.bias_fp32) b = static_cast<const float*>(p.bias)[oc];
+        else if (p.is_bf16) b = __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[oc]);
+        else b = __half2float(static_cast<const __half*>(p.bias)[oc]);
+      }
+      return b;
+    };
+    static_assert(BN <= 32 * EW, "one bias value per epilogue thread");
     uint32_t res_phase = 0;                                  // bit k: parity of this warp's residual barrier k (TMA epilogue)
     // GEMM row -> (image, pixel within the image, row holds an output pixel at all)
     auto decode_row = [&](int m, bool& m_ok, int& img, int& pix) {
@@ -707,30 +722,24 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
       const int halves = (MH == 2 && m0 + kTileM < p.m_total) ? 2 : 1;
       const int buf = tcount % ACC_BUFS;
       const uint32_t acc_phase = (tcount / ACC_BUFS) & 1;
-      float* bias_t = bias_s + (tcount & 1) * 256;
 
       join_setup();
-      // stage this tile's bias as float (two buffers: a fast warp may already be one tile ahead of a slow one)
-      for (int i = et; i < BN; i += 32 * EW) {
-        const int oc = n0 + i;
-        float b = 0.f;
-        if (p.has_bias && p.partial == nullptr && oc < p.out_channels) {
-          if (p.bias_fp32) b = static_cast<const float*>(p.bias)[oc];
-          else if (p.is_bf16) b = __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[oc]);
-          else b = __half2float(static_cast<const __half*>(p.bias)[oc]);
-        }
-        bias_t[i] = b;
+      if (n0 != staged_n0) {
+        if (staged_n0 < 0) bias_next = load_bias(n0);
+        staged_n0 = n0;
+        bias_buf ^= 256;
+        if (et < BN) bias_s[bias_buf + et] = bias_next;
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * EW) : "memory");  // epilogue warps only
       }
-      asm volatile("bar.sync 1, %0;" ::"n"(32 * EW) : "memory");  // epilogue warps only
+      const float* bias_t = bias_s + bias_buf;
 
       // TMA epilogue (channel-contiguous output): this warp's chunk c of half h is staged in its own 2 KiB box and
       // leaves as one TMA store; with a residual, TMA first loads the residual box into the same place, issued here
       // (before the accumulator is even complete) so that the load overlaps the main loop.
-      auto stage_box = [&](int k) { return epi_base + size_t(we * kEpiBufs + k) * 2048; };
+      auto stage_box = [&](int k) { return epi_base + size_t(we * p.epi_boxes + k) * 2048; };
       auto prefetch_residual = [&](int h) {
-        if (lane == 0) ptx::bulk_wait_group_read0();  // earlier stores of this warp have left the boxes
-        __syncwarp();
         if (p.res_tma && lane == 0) {
+          ptx::bulk_wait_group_read0();  // earlier stores of this warp have left the boxes
           for (int k = 0; k < kEpiBufs; ++k) {
             const int chunk = par + EG * k;
             if (chunk >= BN / 32 || n0 + chunk * 32 >= p.out_channels) break;
@@ -739,7 +748,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
           }
         }
       };
-      if (p.out_tma) prefetch_residual(0);
+      prefetch_residual(0);
 
       // Row decode and output addresses, done while the main loop still runs (the accumulator is not needed for them).
       const int64_t cstride = p.out_nhwc ? 1 : p.pq;
@@ -782,6 +791,11 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
           ptx::cluster_sync_all();
         }
         break;
+      }
+      if (!cluster && p.tiles_n > 1 && tile + tile_step < p.num_tiles) {
+        const int next = tile + tile_step - p.fd_tiles_mn.div(tile + tile_step) * tiles_mn;
+        const int next_n0 = (next - p.fd_tiles_n.div(next) * p.tiles_n) * BN;
+        if (next_n0 != n0) bias_next = load_bias(next_n0);
       }
       const uint32_t acc = tmem_base + buf * ACC_COLS;
       if (cluster) {
@@ -948,7 +962,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
         if (h >= halves) break;
         const bool m_ok = m_ok_h[h];
         const int64_t base = base_h[h];
-        if (p.out_tma && h > 0) prefetch_residual(h);
+        if (h > 0) prefetch_residual(h);
 #pragma unroll 1
         for (int chunk = par; chunk < BN / 32; chunk += EG) {
           if (n0 + chunk * 32 >= p.out_channels) break;  // warp-uniform
@@ -956,10 +970,17 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
           ptx::tmem_ld_32x32b_x32(acc + (uint32_t(quad * 32) << 16) + uint32_t(h * BN + chunk * 32), v);
           ptx::tmem_ld_wait();
           if (p.out_tma) {
-            const int k = chunk / EG;
+            const int k = p.res_tma ? chunk / EG : box_turn;
             uint8_t* box = stage_box(k);
             bool landed = true;
-            if (p.res_tma) {
+            if (!p.res_tma) {  // the boxes are used in turn: the store that used this one last has read it
+              if (lane == 0) {
+                if (p.epi_boxes == 1) ptx::bulk_wait_group_read<0>();
+                else ptx::bulk_wait_group_read<kEpiBufs - 1>();
+              }
+              __syncwarp();
+              box_turn = box_turn + 1 == p.epi_boxes ? 0 : box_turn + 1;
+            } else {
               landed = ptx::mbar_wait(&res_bar[we * kEpiBufs + k], (res_phase >> k) & 1u, p.status, kStatusEpilogueTimeout, p.wait_limit);
               res_phase ^= 1u << k;  // barrier k has been used once more (a tile at the channel edge skips some)
             }

@@ -21,41 +21,29 @@ cudaError_t launch_swap(const CUtensorMap& ta, const CUtensorMap& tw, const CUte
 }
 
 #define GIEB_TC_SWAP_DISPATCH(FN, ...)                                                        \
-  switch ((epi_warps == 16 ? 1000000 : 0) + tile_m / 128 * 100000 + tile_n * 100 + tile_k) {  \
-    case 0 + 1 * 100000 + 128 * 100 + 16: return FN<128, 16, 1, 8>(__VA_ARGS__);              \
-    case 0 + 2 * 100000 + 128 * 100 + 16: return FN<128, 16, 2, 8>(__VA_ARGS__);              \
-    case 0 + 1 * 100000 + 128 * 100 + 32: return FN<128, 32, 1, 8>(__VA_ARGS__);              \
-    case 0 + 2 * 100000 + 128 * 100 + 32: return FN<128, 32, 2, 8>(__VA_ARGS__);              \
-    case 0 + 1 * 100000 + 128 * 100 + 64: return FN<128, 64, 1, 8>(__VA_ARGS__);              \
-    case 0 + 2 * 100000 + 128 * 100 + 64: return FN<128, 64, 2, 8>(__VA_ARGS__);              \
-    case 0 + 1 * 100000 + 256 * 100 + 16: return FN<256, 16, 1, 8>(__VA_ARGS__);              \
-    case 0 + 2 * 100000 + 256 * 100 + 16: return FN<256, 16, 2, 8>(__VA_ARGS__);              \
-    case 0 + 1 * 100000 + 256 * 100 + 32: return FN<256, 32, 1, 8>(__VA_ARGS__);              \
-    case 0 + 2 * 100000 + 256 * 100 + 32: return FN<256, 32, 2, 8>(__VA_ARGS__);              \
-    case 0 + 1 * 100000 + 256 * 100 + 64: return FN<256, 64, 1, 8>(__VA_ARGS__);              \
-    case 0 + 2 * 100000 + 256 * 100 + 64: return FN<256, 64, 2, 8>(__VA_ARGS__);              \
-    case 1000000 + 1 * 100000 + 128 * 100 + 16: return FN<128, 16, 1, 16>(__VA_ARGS__);       \
-    case 1000000 + 2 * 100000 + 128 * 100 + 16: return FN<128, 16, 2, 16>(__VA_ARGS__);       \
-    case 1000000 + 1 * 100000 + 128 * 100 + 32: return FN<128, 32, 1, 16>(__VA_ARGS__);       \
-    case 1000000 + 2 * 100000 + 128 * 100 + 32: return FN<128, 32, 2, 16>(__VA_ARGS__);       \
-    case 1000000 + 1 * 100000 + 128 * 100 + 64: return FN<128, 64, 1, 16>(__VA_ARGS__);       \
-    case 1000000 + 2 * 100000 + 128 * 100 + 64: return FN<128, 64, 2, 16>(__VA_ARGS__);       \
-    case 1000000 + 1 * 100000 + 256 * 100 + 16: return FN<256, 16, 1, 16>(__VA_ARGS__);       \
-    case 1000000 + 2 * 100000 + 256 * 100 + 16: return FN<256, 16, 2, 16>(__VA_ARGS__);       \
-    case 1000000 + 1 * 100000 + 256 * 100 + 32: return FN<256, 32, 1, 16>(__VA_ARGS__);       \
-    case 1000000 + 2 * 100000 + 256 * 100 + 32: return FN<256, 32, 2, 16>(__VA_ARGS__);       \
-    case 1000000 + 1 * 100000 + 256 * 100 + 64: return FN<256, 64, 1, 16>(__VA_ARGS__);       \
-    case 1000000 + 2 * 100000 + 256 * 100 + 64: return FN<256, 64, 2, 16>(__VA_ARGS__);       \
+  switch (tile_m / 128 * 100000 + tile_n * 100 + tile_k) {                                    \
+    case 1 * 100000 + 128 * 100 + 16: return FN<128, 16, 1, 8>(__VA_ARGS__);              \
+    case 2 * 100000 + 128 * 100 + 16: return FN<128, 16, 2, 8>(__VA_ARGS__);              \
+    case 1 * 100000 + 128 * 100 + 32: return FN<128, 32, 1, 8>(__VA_ARGS__);              \
+    case 2 * 100000 + 128 * 100 + 32: return FN<128, 32, 2, 8>(__VA_ARGS__);              \
+    case 1 * 100000 + 128 * 100 + 64: return FN<128, 64, 1, 8>(__VA_ARGS__);              \
+    case 2 * 100000 + 128 * 100 + 64: return FN<128, 64, 2, 8>(__VA_ARGS__);              \
+    case 1 * 100000 + 256 * 100 + 16: return FN<256, 16, 1, 8>(__VA_ARGS__);              \
+    case 2 * 100000 + 256 * 100 + 16: return FN<256, 16, 2, 8>(__VA_ARGS__);              \
+    case 1 * 100000 + 256 * 100 + 32: return FN<256, 32, 1, 8>(__VA_ARGS__);              \
+    case 2 * 100000 + 256 * 100 + 32: return FN<256, 32, 2, 8>(__VA_ARGS__);              \
+    case 1 * 100000 + 256 * 100 + 64: return FN<256, 64, 1, 8>(__VA_ARGS__);              \
+    case 2 * 100000 + 256 * 100 + 64: return FN<256, 64, 2, 8>(__VA_ARGS__);              \
     default: return cudaErrorInvalidValue;                                                    \
   }
 
 }  // namespace
 
-cudaError_t conv_tc_swap_prepare(int tile_m, int tile_n, int tile_k, int epi_warps, size_t smem_bytes) {
+cudaError_t conv_tc_swap_prepare(int tile_m, int tile_n, int tile_k, size_t smem_bytes) {
   GIEB_TC_SWAP_DISPATCH(prepare_swap, smem_bytes)
 }
 
-cudaError_t conv_tc_swap_launch(int tile_m, int tile_n, int tile_k, int epi_warps, const CUtensorMap& tm_act, const CUtensorMap& tm_wgt,
+cudaError_t conv_tc_swap_launch(int tile_m, int tile_n, int tile_k, const CUtensorMap& tm_act, const CUtensorMap& tm_wgt,
                                 const CUtensorMap& tm_out, const ConvTcParams& p, dim3 grid, size_t smem_bytes, cudaStream_t stream) {
   GIEB_TC_SWAP_DISPATCH(launch_swap, tm_act, tm_wgt, tm_out, tm_out, p, grid, smem_bytes, stream)
 }

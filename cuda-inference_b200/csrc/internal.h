@@ -18,6 +18,7 @@ enum : uint32_t {
 constexpr int kNumSms = 148;       // streaming multiprocessors of the one supported target (B200): grids are sized in multiples of it
 constexpr int kTileM = 128;        // output pixels per CTA tile = TMEM lanes = UMMA M
 constexpr int kMaxStages = 8;
+constexpr size_t kCtaSmemLimit = 232448;  // 227 KiB opt-in limit of dynamic shared memory per CTA
 constexpr int kProducerWarps = 3;  // warps 0..2 issue the TMA loads, slab by slab in turn
 // warp 3: MMA issuer and TMEM owner; warps 4..11 (4..19 with 16 epilogue warps): epilogue
 static_assert((kProducerWarps + 1) % 4 == 0, "epilogue warp w must sit on TMEM lane quarter w % 4");
@@ -136,6 +137,7 @@ struct ConvTcParams {
   const void* residual;  // optional tensor of the output's shape, layout and type, added before the activation
   int out_nhwc;          // 0: y (and residual, partials) are NCHW; 1: channel-contiguous [B][P][Q][O]
   int out_rows;          // channel-contiguous output goes through shared memory and leaves row by row: 2 = in channel pairs, 1 = singly
+  int epi_boxes;         // 2 KiB staging boxes per epilogue warp: 1, or one per chunk that a warp owns (a residual needs those)
   int out_tma, res_tma;  // channel-contiguous output leaves through TMA stores / the residual arrives through TMA loads
   // Transposed-accumulator kernels: swap_tma = y may be written by TMA stores over its {P*Q, O, N} view (16-byte aligned y,
   // P*Q % 8 == 0); out_vec = pixels per store (4, 2 or 1) of the path that handles everything else (a unit that crosses
@@ -188,7 +190,7 @@ cudaError_t conv_halo_launch(int tile_n, int workers, bool pair, const CUtensorM
 // pair: the tile belongs to a CTA pair (tile_m = 256), each CTA stages 128 activation rows and tile_n / 2 weight rows.
 // epilogue_bytes: staging of the epilogue behind the ring (TMA-store boxes, or the NCHW transposition tiles).
 size_t conv_tc_smem_bytes(int tile_m, int tile_n, int tile_k, int stages, size_t epilogue_bytes, bool pair = false);
-size_t conv_tc_epilogue_staging_bytes(int tile_n);
+int conv_tc_epilogue_boxes(int tile_n, int epi_warps);  // chunks of 32 channels one epilogue warp owns per 128 pixels
 // epi_warps: 8, or 16 for CTAs that have an SM to themselves (tile_n >= 128 only)
 int conv_tc_threads(int epi_warps);
 cudaError_t conv_tc_prepare(int tile_m, int tile_n, int tile_k, int epi_warps, size_t smem_bytes);  // opt in to large dynamic shared memory
@@ -197,6 +199,11 @@ cudaError_t conv_tc_prepare(int tile_m, int tile_n, int tile_k, int epi_warps, s
 cudaError_t conv_tc_launch(int tile_m, int tile_n, int tile_k, int epi_warps, const CUtensorMap& tm_act, const CUtensorMap& tm_wgt,
                            const CUtensorMap& tm_out, const CUtensorMap& tm_res, const ConvTcParams& p, dim3 grid, size_t smem_bytes,
                            cudaStream_t stream);
+// (their points of 128 and 256 channels, a translation unit of their own)
+cudaError_t conv_tc_wide_prepare(int tile_m, int tile_n, int tile_k, int epi_warps, size_t smem_bytes);
+cudaError_t conv_tc_wide_launch(int tile_m, int tile_n, int tile_k, int epi_warps, const CUtensorMap& tm_act, const CUtensorMap& tm_wgt,
+                                const CUtensorMap& tm_out, const CUtensorMap& tm_res, const ConvTcParams& p, dim3 grid, size_t smem_bytes,
+                                cudaStream_t stream);
 
 // CTA-pair points (tcgen05.mma.cta_group::2): tile_m = 256, tile_n 64 / 128 / 256; `grid` = 2 x the number of pairs.
 int conv_tc_pair_epi_warps(int tile_n);
@@ -204,10 +211,10 @@ cudaError_t conv_tc_pair_prepare(int tile_n, int tile_k, size_t smem_bytes);
 cudaError_t conv_tc_pair_launch(int tile_n, int tile_k, const CUtensorMap& tm_act, const CUtensorMap& tm_wgt, const CUtensorMap& tm_out,
                                 const CUtensorMap& tm_res, const ConvTcParams& p, dim3 grid, size_t smem_bytes, cudaStream_t stream);
 
-// Transposed-accumulator points (lane = output channel): NCHW output through TMA stores; tile_n 128 or 256, 16-bit types.
+// Transposed-accumulator points (lane = output channel): NCHW output through TMA stores; tile_n 128 or 256, 16-bit types, 8 epilogue warps.
 // tm_out: y as the 3-D tensor {P*Q, O, N} with a 32-pixel x 32-channel box and 64-byte swizzle (read when p.swap_tma).
-cudaError_t conv_tc_swap_prepare(int tile_m, int tile_n, int tile_k, int epi_warps, size_t smem_bytes);
-cudaError_t conv_tc_swap_launch(int tile_m, int tile_n, int tile_k, int epi_warps, const CUtensorMap& tm_act, const CUtensorMap& tm_wgt,
+cudaError_t conv_tc_swap_prepare(int tile_m, int tile_n, int tile_k, size_t smem_bytes);
+cudaError_t conv_tc_swap_launch(int tile_m, int tile_n, int tile_k, const CUtensorMap& tm_act, const CUtensorMap& tm_wgt,
                                 const CUtensorMap& tm_out, const ConvTcParams& p, dim3 grid, size_t smem_bytes, cudaStream_t stream);
 
 // Sum of split-K partials + bias (+ residual) + ReLU + one rounding; `total` = B*O*P*Q elements in the output's order.

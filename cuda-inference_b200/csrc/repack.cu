@@ -4,7 +4,7 @@
 // permutation of 16-bit words: results are bit-exact whatever the bit patterns (NaN payloads included).
 //
 // The source may have any 2-byte alignment (tests/test_tensor_core.cpp:38-57 offsets X and W by one element);
-// a 128-bit load path is taken when the source is 16-byte aligned and HW is a multiple of 8.  The destination is
+// it is read in aligned words or vectors.  The destination is
 // always written with 128-bit stores (Cp % 8 == 0, 16-byte aligned base).
 #include <stdint.h>
 
@@ -15,73 +15,103 @@ namespace gieb {
 namespace {
 
 constexpr int kTile = 64;          // channels and pixels per CTA tile
-constexpr int kLdWords = 33;       // 32-bit words per shared-memory row (64 px + 1 word of padding)
 
-// Tiled transpose of one 64-channel x 64-pixel tile by 256 threads; `tile` is kTile * kLdWords words of shared memory.
-// LOAD: 0 = 2-byte loads (any alignment), 1 = 16-byte loads (HW % 8 == 0, 16-byte aligned source), 2 = 4-byte loads
-// (HW even, 4-byte aligned source).
-template <int LOAD>
-__device__ __forceinline__ void repack_tile(uint32_t* tile, const uint16_t* __restrict__ src, uint16_t* __restrict__ dst, int C,
-                                            int HW, int Cp, int hw_tile, int c_tile, int b) {
-  const int px0 = hw_tile * kTile;
-  const int c0 = c_tile * kTile;
-  const uint16_t* s = src + (size_t(b) * C + c0) * HW + px0;
-  const int t = threadIdx.x;
+// One repack job: a whole tensor.  mode 0, 1, 3 = tiled (see repack_tile), 2 = small-HW slab, 4 = see below.
+struct RepackJob {
+  const uint16_t* src;
+  uint16_t* dst;
+  int C, HW, Cp, batch;
+  int mode;
+  int hw_tiles, c_tiles;
+  FastDiv fd_hw_tiles, fd_c_tiles;
+  int span;  // mode 2: channels per CTA
+  unsigned blocks;  // hw_tiles * c_tiles * batch
+  int prefetch;     // (read from the first job) L2 prefetch of the source lines before the dependency wait
+  // mode 4 (pixel subsampling for strided 1x1 convolutions): HW = out_h * out_w pixels are taken from a source plane of
+  // src_hw = h * w elements, destination pixel (p, q) from source pixel (p * sub_sh, q * sub_sw)
+  int src_hw, src_w, sub_ow, sub_sh, sub_sw;
+  void set_tiles(int64_t tiles) {
+    blocks = unsigned(tiles);
+    fd_hw_tiles = FastDiv::make(hw_tiles);
+    fd_c_tiles = FastDiv::make(c_tiles);
+  }
+};
 
-  if (LOAD == 1) {
-    // 64 channels x 8 vectors of 8 pixels; a vector never straddles HW because HW % 8 == 0.
+// Tiled transpose of one 64-channel x 64-pixel tile by 256 threads.  A tile sits in shared memory as pixel pairs, a row per channel.
+// MODE (of the job) 1: 16-byte loads of aligned rows; 3: 4-byte loads (even planes); 0: planes of odd size or a source off its
+// alignment: the nine 16-byte vectors that cover a row, which then begins `shift` elements into its words.  Bound by latency and by
+// the loads and shared-memory accesses per byte, so registers are held to 32 (eight blocks per SM).  46 x 430 x 57 x 57: 63.6 us with
+// 2-byte accesses, 73.9 with 4-byte loads that are shifted on their way, 82.9 with asynchronous copies, 52.6 now; even planes
+// (64 x 256 x 58 x 57): 45.3 with nine vectors, 35.9 with words.
+constexpr int kLdWords = 37;       // 32-bit words per shared-memory row: nine vectors and one word of padding
+
+// Elements between the 16-byte boundary before row `row` of a tile and the row; s0: the tile's first element.
+__device__ __forceinline__ int shift_of(const uint16_t* s0, int row, int HW) {
+  return (int(reinterpret_cast<uintptr_t>(s0) >> 1) + row * HW) & 7;
+}
+
+template <int MODE>
+__device__ __forceinline__ void repack_tile(uint32_t* tile, const RepackJob& j, int px0, int c0, int b) {
+  const int C = j.C, HW = j.HW, t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const uint16_t* s = j.src + (size_t(b) * C + c0) * HW + px0;
+  if (MODE == 3) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int v = t + i * 256;
-      const int ch = v >> 3, pv = v & 7;
-      uint4 q = make_uint4(0, 0, 0, 0);
-      if (c0 + ch < C && px0 + pv * 8 < HW) q = *reinterpret_cast<const uint4*>(s + size_t(ch) * HW + pv * 8);
-      uint32_t* d = &tile[ch * kLdWords + pv * 4];
-      d[0] = q.x; d[1] = q.y; d[2] = q.z; d[3] = q.w;
-    }
-  } else if (LOAD == 2) {
-    // 64 channels x 32 pixel pairs; a pair never straddles HW because HW is even, and every row starts 4-byte aligned
-    const int pp = t & 31;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int ch = (t >> 5) + i * 8;
+    for (int i = 0; i < 8; ++i) {  // a warp per row
+      const int ch = warp + i * 8;
       uint32_t v = 0;
-      if (c0 + ch < C && px0 + 2 * pp < HW) v = *reinterpret_cast<const uint32_t*>(s + size_t(ch) * HW + 2 * pp);
-      tile[ch * kLdWords + pp] = v;
+      if (c0 + ch < C && px0 + 2 * lane < HW) v = *reinterpret_cast<const uint32_t*>(s + size_t(ch) * HW + 2 * lane);
+      tile[ch * kLdWords + lane] = v;
     }
   } else {
-    uint16_t* tile16 = reinterpret_cast<uint16_t*>(tile);
-    const int px = t & 63;
+    constexpr int VECS = MODE == 1 ? 8 : 9;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const int ch = (t >> 6) + i * 4;
-      uint16_t v = 0;
-      if (c0 + ch < C && px0 + px < HW) v = s[size_t(ch) * HW + px];
-      tile16[ch * (kLdWords * 2) + px] = v;
+    for (int i = 0; i < (64 * VECS + 255) / 256; ++i) {
+      const int v = t + i * 256;
+      const int ch = v / VECS, pv = v - ch * VECS;
+      if (MODE == 0 && v >= 64 * VECS) break;
+      const int shift = MODE == 1 ? 0 : shift_of(s, ch, HW);
+      uint4 q = make_uint4(0, 0, 0, 0);
+      if (c0 + ch < C && px0 + pv * 8 - shift < HW && (MODE == 1 || pv * 8 < 64 + shift)) {
+        const uint16_t* at = s + size_t(ch) * HW + pv * 8 - shift;
+        const uint16_t* end = j.src + size_t(j.batch) * C * HW;
+        if (MODE == 1 || (at >= j.src && at + 8 <= end)) q = *reinterpret_cast<const uint4*>(at);
+        else {  // the first or the last vector of the tensor
+          uint32_t w[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            if (at + e >= j.src && at + e < end) w[e >> 1] |= uint32_t(at[e]) << (16 * (e & 1));
+          q = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+      }
+      uint32_t* d = &tile[ch * kLdWords + pv * 4];
+      d[0] = q.x; d[1] = q.y; d[2] = q.z; d[3] = q.w;
     }
   }
   __syncthreads();
 
-  // Each thread emits one 16-byte vector = 8 consecutive channels of one pixel.  A warp covers 8 pixels x 4
-  // channel groups (64 contiguous bytes per pixel) which is bank-conflict free with the 33-word row pitch.
-  const uint16_t* tile16 = reinterpret_cast<const uint16_t*>(tile);
-  const int lane = t & 31, warp = t >> 5;
+  // Each thread emits 8 consecutive channels of two neighbouring pixels.  A warp covers 8 pixel pairs x 4 channel groups (64
+  // contiguous bytes per pixel), which is bank-conflict free with the odd row pitch.
   const int cg = (warp & 1) * 4 + (lane & 3);
+  const int pair = (warp >> 1) * 8 + (lane >> 2);
+  const int px = px0 + 2 * pair;
+  if (px >= HW || c0 + cg * 8 >= j.Cp) return;
+  const uint32_t* row = tile + cg * 8 * kLdWords + pair;
+  uint32_t w[8];
 #pragma unroll
-  for (int it = 0; it < 2; ++it) {
-    const int px = ((warp >> 1) + it * 4) * 8 + (lane >> 2);
-    if (px0 + px < HW && c0 + cg * 8 < Cp) {
-      uint16_t o[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = tile16[(cg * 8 + j) * (kLdWords * 2) + px];
-      uint4 q;
-      q.x = uint32_t(o[0]) | (uint32_t(o[1]) << 16);
-      q.y = uint32_t(o[2]) | (uint32_t(o[3]) << 16);
-      q.z = uint32_t(o[4]) | (uint32_t(o[5]) << 16);
-      q.w = uint32_t(o[6]) | (uint32_t(o[7]) << 16);
-      *reinterpret_cast<uint4*>(dst + (size_t(b) * HW + px0 + px) * Cp + c0 + cg * 8) = q;
+  for (int k = 0; k < 8; ++k) {
+    if (MODE != 0) w[k] = row[k * kLdWords];
+    else {
+      const int shift = shift_of(s, k, HW);  // (of row cg * 8 + k as well: eight rows are whole vectors)
+      w[k] = row[k * kLdWords + (shift >> 1)];
+      if (shift & 1) w[k] = __funnelshift_r(w[k], row[k * kLdWords + (shift >> 1) + 1], 16);
     }
   }
+  uint16_t* d = j.dst + (size_t(b) * HW + px) * j.Cp + c0 + cg * 8;
+  *reinterpret_cast<uint4*>(d) =
+      make_uint4(__byte_perm(w[0], w[1], 0x5410), __byte_perm(w[2], w[3], 0x5410), __byte_perm(w[4], w[5], 0x5410), __byte_perm(w[6], w[7], 0x5410));
+  if (px + 1 < HW)
+    *reinterpret_cast<uint4*>(d + j.Cp) =
+        make_uint4(__byte_perm(w[0], w[1], 0x7632), __byte_perm(w[2], w[3], 0x7632), __byte_perm(w[4], w[5], 0x7632), __byte_perm(w[6], w[7], 0x7632));
 }
 
 // Small-HW variant (filter taps: HW = R*S <= 64).  One CTA handles `span` channels of one batch entry (a multiple of
@@ -118,22 +148,6 @@ __device__ __forceinline__ void repack_small_hw(uint16_t* slab, const uint16_t* 
     *reinterpret_cast<uint4*>(dst + (size_t(b) * HW + px) * Cp + c0 + cg * 8) = q;
   }
 }
-
-// One repack job: a whole tensor.  mode 0 = tiled with 2-byte loads, 1 = tiled with 128-bit loads, 2 = small-HW slab,
-// 3 = tiled with 32-bit loads.
-struct RepackJob {
-  const uint16_t* src;
-  uint16_t* dst;
-  int C, HW, Cp, batch;
-  int mode;
-  int hw_tiles, c_tiles;
-  int span;  // mode 2: channels per CTA
-  unsigned blocks;  // hw_tiles * c_tiles * batch
-  int prefetch;     // (read from the first job) L2 prefetch of the source lines before the dependency wait
-  // mode 4 (pixel subsampling for strided 1x1 convolutions): HW = out_h * out_w pixels are taken from a source plane of
-  // src_hw = h * w elements, destination pixel (p, q) from source pixel (p * sub_sh, q * sub_sw)
-  int src_hw, src_w, sub_ow, sub_sh, sub_sw;
-};
 
 // The 128-byte lines one CTA is about to read, one prefetch per line, never outside the source tensor.
 __device__ __forceinline__ void prefetch_source(const RepackJob& j, int hw_tile, int c_tile, int bi) {
@@ -194,15 +208,16 @@ __device__ __forceinline__ void repack_tile_sub(uint32_t* tile, const RepackJob&
 }
 
 // Up to two jobs in one launch (activations + weights): block indices [0, a.blocks) belong to job a, the rest to job b.
-__global__ void __launch_bounds__(256) repack_jobs_kernel(const RepackJob a, const RepackJob b) {
-  __shared__ __align__(16) uint32_t smem[kTile * kLdWords];  // 8448 B >= kTile * kSmallHwMax * 2 = 8192 B
+__global__ void __launch_bounds__(256, 8) repack_jobs_kernel(const RepackJob a, const RepackJob b) {
+  __shared__ __align__(16) uint32_t smem[kTile * kLdWords];
+  static_assert(kTile * kLdWords * 4 >= kTile * kSmallHwMax * 2, "the slab must fit");
   const bool first = blockIdx.x < a.blocks;
   const RepackJob& j = first ? a : b;
-  unsigned id = first ? blockIdx.x : blockIdx.x - a.blocks;
-  const int hw_tile = int(id % unsigned(j.hw_tiles));
-  id /= unsigned(j.hw_tiles);
-  const int c_tile = int(id % unsigned(j.c_tiles));
-  const int bi = int(id / unsigned(j.c_tiles));
+  const int id = int(first ? blockIdx.x : blockIdx.x - a.blocks);
+  const int row = j.fd_hw_tiles.div(id);
+  const int hw_tile = id - row * j.hw_tiles;
+  const int bi = j.fd_c_tiles.div(row);
+  const int c_tile = row - bi * j.c_tiles;
   // Launched with programmatic stream serialization, so this CTA may be resident well before the previous kernel of the
   // stream has finished.  Meanwhile it starts its source lines on their way from HBM into L2 (a cache fill at the
   // coherence point: harmless even if that kernel still writes them), so that the loads below hit L2.
@@ -213,9 +228,9 @@ __global__ void __launch_bounds__(256) repack_jobs_kernel(const RepackJob a, con
   ptx::grid_dep_launch();
   if (j.mode == 4) repack_tile_sub(smem, j, hw_tile, c_tile, bi);
   else if (j.mode == 2) repack_small_hw(reinterpret_cast<uint16_t*>(smem), j.src, j.dst, j.C, j.HW, j.Cp, j.span, c_tile, bi);
-  else if (j.mode == 1) repack_tile<1>(smem, j.src, j.dst, j.C, j.HW, j.Cp, hw_tile, c_tile, bi);
-  else if (j.mode == 3) repack_tile<2>(smem, j.src, j.dst, j.C, j.HW, j.Cp, hw_tile, c_tile, bi);
-  else repack_tile<0>(smem, j.src, j.dst, j.C, j.HW, j.Cp, hw_tile, c_tile, bi);
+  else if (j.mode == 1) repack_tile<1>(smem, j, hw_tile * kTile, c_tile * kTile, bi);
+  else if (j.mode == 3) repack_tile<3>(smem, j, hw_tile * kTile, c_tile * kTile, bi);
+  else repack_tile<0>(smem, j, hw_tile * kTile, c_tile * kTile, bi);
 }
 
 // ---- row gather for convolutions with very few input channels ------------------------------------------------------
@@ -395,6 +410,12 @@ RepackJob make_job(const void* src, void* dst, int batch, int channels, int hw, 
   return j;
 }
 
+cudaError_t launch_jobs(RepackJob a, int64_t tiles_a, RepackJob b, int64_t tiles_b, cudaStream_t stream) {
+  a.set_tiles(tiles_a);
+  b.set_tiles(tiles_b);
+  return launch_pdl(repack_jobs_kernel, dim3(a.blocks + b.blocks), dim3(256), 0, stream, a, b);
+}
+
 }  // namespace
 
 cudaError_t repack_pair_launch(const void* src_a, void* dst_a, int batch_a, int ch_a, int hw_a, int cp_a, const void* src_b,
@@ -408,11 +429,7 @@ cudaError_t repack_pair_launch(const void* src_a, void* dst_a, int batch_a, int 
     nb = int64_t(b.hw_tiles) * b.c_tiles * batch_b;
   }
   if (na + nb > 2147483647LL) return cudaErrorInvalidValue;
-  a.blocks = unsigned(na);
-  b.blocks = unsigned(nb);
-  const cudaError_t e = launch_pdl(repack_jobs_kernel, dim3(unsigned(na + nb)), dim3(256), 0, stream, a, b);
-  if (e != cudaSuccess) return e;
-  return cudaGetLastError();
+  return launch_jobs(a, na, b, nb, stream);
 }
 
 cudaError_t repack_subsampled_launch(const void* x, void* xn, int batch, int channels, int h, int w, int out_h, int out_w, int stride_h,
@@ -431,11 +448,7 @@ cudaError_t repack_subsampled_launch(const void* x, void* xn, int batch, int cha
     nb = int64_t(b.hw_tiles) * b.c_tiles * out_channels;
   }
   if (na + nb > 2147483647LL) return cudaErrorInvalidValue;
-  a.blocks = unsigned(na);
-  b.blocks = unsigned(nb);
-  const cudaError_t e = launch_pdl(repack_jobs_kernel, dim3(unsigned(na + nb)), dim3(256), 0, stream, a, b);
-  if (e != cudaSuccess) return e;
-  return cudaGetLastError();
+  return launch_jobs(a, na, b, nb, stream);
 }
 
 // ---- column-pair gather: the row gather for stride_w = 2 and at most 4 channels, four times smaller --------------------
@@ -689,30 +702,43 @@ Tf32Job make_tf32_job(const void* src, void* dst, int batch, int channels, int h
 // 1-byte elements (FP8 bit patterns): [B][C][HW] -> [B][HW][Cp], channels zero-padded to Cp (a multiple of 32).  Pure data
 // movement, bit-exact.  Up to two tensors per launch (activations and weights), like repack_jobs_kernel, and the same
 // two shapes of work:
-//   tile mode: one CTA transposes a 64-channel x 64-pixel tile: 4-byte loads along the pixels where the plane size and the
-//     source address allow it, 16-byte stores of 16 consecutive channels (a warp writes 8 pixels x 64 bytes);
+//   tile mode: one CTA transposes a 64-channel x 128-pixel tile: 4-byte loads along the pixels (a row that starts inside a word is
+//     shifted into place by a shuffle and a funnel shift), 4 x 4 bytes transposed in registers, 8-byte stores of 8 consecutive
+//     channels (a warp writes 16 pixels x 64 bytes).  Bound by its instruction count: with 1-byte reads of a 64 x 64 tile the copy
+//     of 160 x 64 x 44 x 27 took 12.8 us, now 9.7;
 //   slab mode (planes of at most 16 elements: filter taps): one CTA takes `span` channels of one batch entry; the source
 //     slab [span][HW] is contiguous and is read linearly, then written as [HW][span].
 // Both prefetch their source lines into L2 before the dependency wait (see repack_jobs_kernel).
 struct ByteJob {
   const uint8_t* src;
   uint8_t* dst;
-  int C, HW, Cp, hw_tiles, c_tiles, span;  // span > 0: slab mode
+  int C, HW, Cp, batch, hw_tiles, c_tiles, span;  // span > 0: slab mode
+  FastDiv fd_hw_tiles, fd_c_tiles;
   unsigned blocks;
 };
-constexpr int kBytePitch = 68;
-constexpr int kByteSlab = 8192;  // bytes of shared memory a slab may take
+constexpr int kBytePitch = 33;   // words per channel of a tile
+constexpr int kByteSlab = 8448;  // bytes of shared memory: a tile, or a slab
+
+// The word at `at` (4-byte aligned), of which only the bytes inside [src, end) are read.
+__device__ __forceinline__ uint32_t load_word_within(const uint8_t* at, const uint8_t* src, const uint8_t* end) {
+  if (at >= src && at + 4 <= end) return *reinterpret_cast<const uint32_t*>(at);
+  uint32_t v = 0;
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+    if (at + e >= src && at + e < end) v |= uint32_t(at[e]) << (8 * e);
+  return v;
+}
 
 __global__ void __launch_bounds__(256) repack_bytes_kernel(const ByteJob a, const ByteJob b, int prefetch) {
   __shared__ __align__(16) uint8_t tile[kByteSlab];
-  static_assert(64 * kBytePitch <= kByteSlab, "the tile mode's 64 x 64 tile must fit the slab buffer");
+  static_assert(64 * kBytePitch * 4 <= kByteSlab, "the tile must fit the slab buffer");
   const bool first = blockIdx.x < a.blocks;
   const ByteJob& j = first ? a : b;
-  unsigned id = first ? blockIdx.x : blockIdx.x - a.blocks;
-  const int hw_tile = int(id % unsigned(j.hw_tiles));
-  id /= unsigned(j.hw_tiles);
-  const int c_tile = int(id % unsigned(j.c_tiles));
-  const int bi = int(id / unsigned(j.c_tiles));
+  const unsigned id = first ? blockIdx.x : blockIdx.x - a.blocks;
+  const int row = j.fd_hw_tiles.div(int(id));
+  const int hw_tile = int(id) - row * j.hw_tiles;
+  const int bi = j.fd_c_tiles.div(row);
+  const int c_tile = row - bi * j.c_tiles;
   const int t = threadIdx.x;
   if (j.span > 0) {
     const int c0 = c_tile * j.span;
@@ -742,39 +768,59 @@ __global__ void __launch_bounds__(256) repack_bytes_kernel(const ByteJob a, cons
     }
     return;
   }
-  const int c0 = c_tile * 64, px0 = hw_tile * 64;
+  const int c0 = c_tile * 64, px0 = hw_tile * 128;
   const uint8_t* s = j.src + (size_t(bi) * j.C + c0) * j.HW + px0;
-  if (prefetch && t < 64 && c0 + t < j.C && px0 < j.HW) ptx::prefetch_l2(s + size_t(t) * j.HW);  // 64 bytes: one line, or the first of two
+  if (prefetch && t < 128 && c0 + (t >> 1) < j.C)  // 128 bytes: at most two lines
+    ptx::prefetch_l2(s + size_t(t >> 1) * j.HW + ((t & 1) ? min(128, j.HW - px0) - 1 : 0));
   ptx::grid_dep_wait();
   ptx::grid_dep_launch();
-  const bool words = (j.HW & 3) == 0 && (reinterpret_cast<uintptr_t>(j.src) & 3u) == 0;
+  const uint8_t* end = j.src + size_t(j.batch) * j.C * j.HW;
+  const int lane = t & 31, warp = t >> 5;
+  uint32_t* words = reinterpret_cast<uint32_t*>(tile);
+  uint32_t word[8], last[8];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int idx = t + i * 256, ch = idx >> 4, q = (idx & 15) * 4;
-    uint32_t v = 0;
-    if (c0 + ch < j.C && px0 + q < j.HW) {
-      const uint8_t* p = s + size_t(ch) * j.HW + q;
-      if (words) v = *reinterpret_cast<const uint32_t*>(p);   // a group of four never straddles the plane (HW % 4 == 0)
-      else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (px0 + q + e < j.HW) v |= uint32_t(p[e]) << (8 * e);
-      }
+  for (int i = 0; i < 8; ++i) {
+    const int ch = warp + i * 8;
+    const uint8_t* r = s + size_t(ch) * j.HW;
+    const int off = int(reinterpret_cast<uintptr_t>(r) & 3u);
+    word[i] = last[i] = 0;
+    if (c0 + ch < j.C && px0 + 4 * lane - off < j.HW) {
+      word[i] = load_word_within(r - off + 4 * lane, j.src, end);
+      if (off != 0 && lane == 31) last[i] = load_word_within(r - off + 128, j.src, end);
     }
-    *reinterpret_cast<uint32_t*>(tile + ch * kBytePitch + q) = v;
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int ch = warp + i * 8;
+    const int off = int(reinterpret_cast<uintptr_t>(s + size_t(ch) * j.HW) & 3u);
+    if (off != 0) {  // (the same for the whole warp)
+      uint32_t next = __shfl_down_sync(0xffffffffu, word[i], 1);
+      if (lane == 31) next = last[i];
+      word[i] = __funnelshift_r(word[i], next, 8 * off);
+    }
+    words[ch * kBytePitch + lane] = word[i];
   }
   __syncthreads();
-  const int cg = t & 3, px = t >> 2;
-  if (px0 + px < j.HW && c0 + cg * 16 < j.Cp) {
-    uint32_t o[4];
+  const int cg = t & 7, quad = t >> 3;  // 8 channels, 4 pixels
+  const int px = px0 + 4 * quad;
+  if (px < j.HW && c0 + cg * 8 < j.Cp) {
+    uint32_t o[2][4];
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      uint32_t v = 0;
+    for (int h = 0; h < 2; ++h) {
+      uint32_t w[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) v |= uint32_t(tile[(cg * 16 + w * 4 + e) * kBytePitch + px]) << (8 * e);
-      o[w] = v;
+      for (int e = 0; e < 4; ++e) w[e] = words[(cg * 8 + h * 4 + e) * kBytePitch + quad];
+      const uint32_t lo01 = __byte_perm(w[0], w[1], 0x5140), lo23 = __byte_perm(w[2], w[3], 0x5140);
+      const uint32_t hi01 = __byte_perm(w[0], w[1], 0x7362), hi23 = __byte_perm(w[2], w[3], 0x7362);
+      o[h][0] = __byte_perm(lo01, lo23, 0x5410);
+      o[h][1] = __byte_perm(lo01, lo23, 0x7632);
+      o[h][2] = __byte_perm(hi01, hi23, 0x5410);
+      o[h][3] = __byte_perm(hi01, hi23, 0x7632);
     }
-    *reinterpret_cast<uint4*>(j.dst + (size_t(bi) * j.HW + px0 + px) * j.Cp + c0 + cg * 16) = make_uint4(o[0], o[1], o[2], o[3]);
+    uint8_t* d = j.dst + (size_t(bi) * j.HW + px) * j.Cp + c0 + cg * 8;
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (px + e < j.HW) *reinterpret_cast<uint2*>(d + size_t(e) * j.Cp) = make_uint2(o[0][e], o[1][e]);
   }
 }
 
@@ -782,17 +828,19 @@ ByteJob make_byte_job(const void* src, void* dst, int batch, int channels, int h
   ByteJob j;
   j.src = static_cast<const uint8_t*>(src);
   j.dst = static_cast<uint8_t*>(dst);
-  j.C = channels; j.HW = hw; j.Cp = c_padded;
+  j.C = channels; j.HW = hw; j.Cp = c_padded; j.batch = batch;
   if (hw <= 16) {   // filter taps: as many 64-channel groups per CTA as the slab holds
-    j.span = (kByteSlab / hw) / 64 * 64;
+    j.span = (8192 / hw) / 64 * 64;
     if (j.span > (c_padded + 63) / 64 * 64) j.span = (c_padded + 63) / 64 * 64;
     j.hw_tiles = 1;
     j.c_tiles = (c_padded + j.span - 1) / j.span;
   } else {
     j.span = 0;
-    j.hw_tiles = (hw + 63) / 64;
+    j.hw_tiles = (hw + 127) / 128;
     j.c_tiles = (c_padded + 63) / 64;
   }
+  j.fd_hw_tiles = FastDiv::make(j.hw_tiles);
+  j.fd_c_tiles = FastDiv::make(j.c_tiles);
   j.blocks = unsigned(int64_t(j.hw_tiles) * j.c_tiles * batch);
   return j;
 }
