@@ -378,7 +378,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_consta
         with_type([&](auto* yp, auto* rp) {
           using T = std::remove_pointer_t<decltype(yp)>;
           if constexpr (sizeof(T) == 2) {
-            if (p.out_nhwc) {
+            if (p.out_nhwc && rows_pay(nvalid, p.out_rows == 2)) {
               const bool cells = p.out_cells && nvalid == 32;
               if (rp != nullptr) {
                 if (cells) staging_cells<true>(box, lane, rp, o.rows, uint32_t(chunk) * 4u);

@@ -39,8 +39,10 @@ struct RepackJob {
 
 // Tiled transpose of one 64-channel x 64-pixel tile by 256 threads.  A tile sits in shared memory as pixel pairs, a row per channel.
 // MODE (of the job) 1: 16-byte loads of aligned rows; 3: 4-byte loads (even planes); 0: planes of odd size or a source off its
-// alignment: the nine 16-byte vectors that cover a row, which then begins `shift` elements into its words.  Bound by latency and by
-// the loads and shared-memory accesses per byte, so registers are held to 32 (eight blocks per SM).  46 x 430 x 57 x 57: 63.6 us with
+// alignment: the nine 16-byte vectors that cover a row, which then begins `shift` elements into its words; 5: the same planes by
+// 2-byte loads, a shorter way for a block that has nothing beside it (64 -> 253 at 35 x 35, 2 images: 8.5 us a pass, 9.5 with vectors).  Bound by latency and by
+// the loads and shared-memory accesses per byte: a large tensor takes the kernel that is cut to 32 registers, eight blocks per SM
+// (see launch_jobs).  46 x 430 x 57 x 57: 63.6 us with
 // 2-byte accesses, 73.9 with 4-byte loads that are shifted on their way, 82.9 with asynchronous copies, 52.6 now; even planes
 // (64 x 256 x 58 x 57): 45.3 with nine vectors, 35.9 with words.
 constexpr int kLdWords = 37;       // 32-bit words per shared-memory row: nine vectors and one word of padding
@@ -54,7 +56,17 @@ template <int MODE>
 __device__ __forceinline__ void repack_tile(uint32_t* tile, const RepackJob& j, int px0, int c0, int b) {
   const int C = j.C, HW = j.HW, t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const uint16_t* s = j.src + (size_t(b) * C + c0) * HW + px0;
-  if (MODE == 3) {
+  if (MODE == 5) {
+    uint16_t* tile16 = reinterpret_cast<uint16_t*>(tile);
+    const int px = t & 63;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int ch = (t >> 6) + i * 4;
+      uint16_t v = 0;
+      if (c0 + ch < C && px0 + px < HW) v = s[size_t(ch) * HW + px];
+      tile16[ch * (kLdWords * 2) + px] = v;
+    }
+  } else if (MODE == 3) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {  // a warp per row
       const int ch = warp + i * 8;
@@ -208,7 +220,8 @@ __device__ __forceinline__ void repack_tile_sub(uint32_t* tile, const RepackJob&
 }
 
 // Up to two jobs in one launch (activations + weights): block indices [0, a.blocks) belong to job a, the rest to job b.
-__global__ void __launch_bounds__(256, 8) repack_jobs_kernel(const RepackJob a, const RepackJob b) {
+template <int RESIDENT>  // blocks per SM that the registers are cut for; 0: as they come
+__global__ void __launch_bounds__(256, RESIDENT) repack_jobs_kernel(const RepackJob a, const RepackJob b) {
   __shared__ __align__(16) uint32_t smem[kTile * kLdWords];
   static_assert(kTile * kLdWords * 4 >= kTile * kSmallHwMax * 2, "the slab must fit");
   const bool first = blockIdx.x < a.blocks;
@@ -230,7 +243,7 @@ __global__ void __launch_bounds__(256, 8) repack_jobs_kernel(const RepackJob a, 
   else if (j.mode == 2) repack_small_hw(reinterpret_cast<uint16_t*>(smem), j.src, j.dst, j.C, j.HW, j.Cp, j.span, c_tile, bi);
   else if (j.mode == 1) repack_tile<1>(smem, j, hw_tile * kTile, c_tile * kTile, bi);
   else if (j.mode == 3) repack_tile<3>(smem, j, hw_tile * kTile, c_tile * kTile, bi);
-  else repack_tile<0>(smem, j, hw_tile * kTile, c_tile * kTile, bi);
+  else repack_tile<RESIDENT ? 0 : 5>(smem, j, hw_tile * kTile, c_tile * kTile, bi);
 }
 
 // ---- row gather for convolutions with very few input channels ------------------------------------------------------
@@ -413,7 +426,11 @@ RepackJob make_job(const void* src, void* dst, int batch, int channels, int hw, 
 cudaError_t launch_jobs(RepackJob a, int64_t tiles_a, RepackJob b, int64_t tiles_b, cudaStream_t stream) {
   a.set_tiles(tiles_a);
   b.set_tiles(tiles_b);
-  return launch_pdl(repack_jobs_kernel, dim3(a.blocks + b.blocks), dim3(256), 0, stream, a, b);
+  // More than one wave: eight blocks per SM (46 x 430 x 57 x 57: 52.6 us, 60.1 with six).  A small job does not want them: its blocks
+  // begin on the SMs that the kernel before it leaves idle, and the more those take the longer they are at it when all the others
+  // have finished (32 x 256 x 14 x 14 and its weights under a 100-block convolution: 0.6 us a pass).
+  const auto kernel = a.blocks + b.blocks > unsigned(kNumSms) * 8 ? repack_jobs_kernel<8> : repack_jobs_kernel<0>;
+  return launch_pdl(kernel, dim3(a.blocks + b.blocks), dim3(256), 0, stream, a, b);
 }
 
 }  // namespace
@@ -702,9 +719,9 @@ Tf32Job make_tf32_job(const void* src, void* dst, int batch, int channels, int h
 // 1-byte elements (FP8 bit patterns): [B][C][HW] -> [B][HW][Cp], channels zero-padded to Cp (a multiple of 32).  Pure data
 // movement, bit-exact.  Up to two tensors per launch (activations and weights), like repack_jobs_kernel, and the same
 // two shapes of work:
-//   tile mode: one CTA transposes a 64-channel x 128-pixel tile: 4-byte loads along the pixels (a row that starts inside a word is
-//     shifted into place by a shuffle and a funnel shift), 4 x 4 bytes transposed in registers, 8-byte stores of 8 consecutive
-//     channels (a warp writes 16 pixels x 64 bytes).  Bound by its instruction count: with 1-byte reads of a 64 x 64 tile the copy
+//   tile mode: one CTA transposes a 64-channel x PX-pixel tile (PX 128 where that leaves more than a wave of blocks, else 64): 4-byte loads along the pixels (a row that starts inside a word is
+//     shifted into place by a shuffle and a funnel shift), bytes transposed in registers, 8-byte stores of 8 consecutive
+//     channels.  Bound by its instruction count: with 1-byte reads of a 64 x 64 tile the copy
 //     of 160 x 64 x 44 x 27 took 12.8 us, now 9.7;
 //   slab mode (planes of at most 16 elements: filter taps): one CTA takes `span` channels of one batch entry; the source
 //     slab [span][HW] is contiguous and is read linearly, then written as [HW][span].
@@ -716,7 +733,6 @@ struct ByteJob {
   FastDiv fd_hw_tiles, fd_c_tiles;
   unsigned blocks;
 };
-constexpr int kBytePitch = 33;   // words per channel of a tile
 constexpr int kByteSlab = 8448;  // bytes of shared memory: a tile, or a slab
 
 // The word at `at` (4-byte aligned), of which only the bytes inside [src, end) are read.
@@ -729,9 +745,11 @@ __device__ __forceinline__ uint32_t load_word_within(const uint8_t* at, const ui
   return v;
 }
 
+template <int PX>
 __global__ void __launch_bounds__(256) repack_bytes_kernel(const ByteJob a, const ByteJob b, int prefetch) {
   __shared__ __align__(16) uint8_t tile[kByteSlab];
-  static_assert(64 * kBytePitch * 4 <= kByteSlab, "the tile must fit the slab buffer");
+  constexpr int LANES = PX / 4, PITCH = LANES + 1;  // words of a row, and of a row with its padding
+  static_assert(64 * PITCH * 4 <= kByteSlab, "the tile must fit the slab buffer");
   const bool first = blockIdx.x < a.blocks;
   const ByteJob& j = first ? a : b;
   const unsigned id = first ? blockIdx.x : blockIdx.x - a.blocks;
@@ -768,63 +786,59 @@ __global__ void __launch_bounds__(256) repack_bytes_kernel(const ByteJob a, cons
     }
     return;
   }
-  const int c0 = c_tile * 64, px0 = hw_tile * 128;
+  const int c0 = c_tile * 64, px0 = hw_tile * PX;
   const uint8_t* s = j.src + (size_t(bi) * j.C + c0) * j.HW + px0;
-  if (prefetch && t < 128 && c0 + (t >> 1) < j.C)  // 128 bytes: at most two lines
-    ptx::prefetch_l2(s + size_t(t >> 1) * j.HW + ((t & 1) ? min(128, j.HW - px0) - 1 : 0));
+  if (prefetch && t < PX && c0 + (t & 63) < j.C && px0 + (t & 64) < j.HW) ptx::prefetch_l2(s + size_t(t & 63) * j.HW + (t & 64));
   ptx::grid_dep_wait();
   ptx::grid_dep_launch();
   const uint8_t* end = j.src + size_t(j.batch) * j.C * j.HW;
-  const int lane = t & 31, warp = t >> 5;
+  constexpr int ROWS = 256 / LANES, PASSES = 64 / ROWS;
+  const int lane = t & (LANES - 1), row0 = t / LANES;  // (half) a warp per row
   uint32_t* words = reinterpret_cast<uint32_t*>(tile);
-  uint32_t word[8], last[8];
+  uint32_t word[PASSES], last[PASSES];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int ch = warp + i * 8;
+  for (int i = 0; i < PASSES; ++i) {
+    const int ch = row0 + i * ROWS;
     const uint8_t* r = s + size_t(ch) * j.HW;
     const int off = int(reinterpret_cast<uintptr_t>(r) & 3u);
     word[i] = last[i] = 0;
     if (c0 + ch < j.C && px0 + 4 * lane - off < j.HW) {
       word[i] = load_word_within(r - off + 4 * lane, j.src, end);
-      if (off != 0 && lane == 31) last[i] = load_word_within(r - off + 128, j.src, end);
+      if (off != 0 && lane == LANES - 1) last[i] = load_word_within(r - off + PX, j.src, end);
     }
   }
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int ch = warp + i * 8;
+  for (int i = 0; i < PASSES; ++i) {
+    const int ch = row0 + i * ROWS;
     const int off = int(reinterpret_cast<uintptr_t>(s + size_t(ch) * j.HW) & 3u);
-    if (off != 0) {  // (the same for the whole warp)
-      uint32_t next = __shfl_down_sync(0xffffffffu, word[i], 1);
-      if (lane == 31) next = last[i];
-      word[i] = __funnelshift_r(word[i], next, 8 * off);
-    }
-    words[ch * kBytePitch + lane] = word[i];
+    uint32_t next = __shfl_down_sync(0xffffffffu, word[i], 1, LANES);
+    if (lane == LANES - 1) next = last[i];
+    words[ch * PITCH + lane] = __funnelshift_r(word[i], next, 8 * off);
   }
   __syncthreads();
-  const int cg = t & 7, quad = t >> 3;  // 8 channels, 4 pixels
-  const int px = px0 + 4 * quad;
-  if (px < j.HW && c0 + cg * 8 < j.Cp) {
-    uint32_t o[2][4];
+  const int cg = t & 7;  // 8 channels
+#pragma unroll
+  for (int pair = t >> 3; pair < PX / 2; pair += 32) {  // 2 pixels
+    const int px = px0 + 2 * pair;
+    if (px >= j.HW || c0 + cg * 8 >= j.Cp) break;
+    uint32_t even[2], odd[2];
+    const unsigned pick = (pair & 1) ? 0x7362u : 0x5140u;  // the two pixels of both words, side by side
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       uint32_t w[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) w[e] = words[(cg * 8 + h * 4 + e) * kBytePitch + quad];
-      const uint32_t lo01 = __byte_perm(w[0], w[1], 0x5140), lo23 = __byte_perm(w[2], w[3], 0x5140);
-      const uint32_t hi01 = __byte_perm(w[0], w[1], 0x7362), hi23 = __byte_perm(w[2], w[3], 0x7362);
-      o[h][0] = __byte_perm(lo01, lo23, 0x5410);
-      o[h][1] = __byte_perm(lo01, lo23, 0x7632);
-      o[h][2] = __byte_perm(hi01, hi23, 0x5410);
-      o[h][3] = __byte_perm(hi01, hi23, 0x7632);
+      for (int e = 0; e < 4; ++e) w[e] = words[(cg * 8 + h * 4 + e) * PITCH + (pair >> 1)];
+      const uint32_t p01 = __byte_perm(w[0], w[1], pick), p23 = __byte_perm(w[2], w[3], pick);
+      even[h] = __byte_perm(p01, p23, 0x5410);
+      odd[h] = __byte_perm(p01, p23, 0x7632);
     }
     uint8_t* d = j.dst + (size_t(bi) * j.HW + px) * j.Cp + c0 + cg * 8;
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if (px + e < j.HW) *reinterpret_cast<uint2*>(d + size_t(e) * j.Cp) = make_uint2(o[0][e], o[1][e]);
+    *reinterpret_cast<uint2*>(d) = make_uint2(even[0], even[1]);
+    if (px + 1 < j.HW) *reinterpret_cast<uint2*>(d + j.Cp) = make_uint2(odd[0], odd[1]);
   }
 }
 
-ByteJob make_byte_job(const void* src, void* dst, int batch, int channels, int hw, int c_padded) {
+ByteJob make_byte_job(const void* src, void* dst, int batch, int channels, int hw, int c_padded, int tile_px) {
   ByteJob j;
   j.src = static_cast<const uint8_t*>(src);
   j.dst = static_cast<uint8_t*>(dst);
@@ -836,7 +850,7 @@ ByteJob make_byte_job(const void* src, void* dst, int batch, int channels, int h
     j.c_tiles = (c_padded + j.span - 1) / j.span;
   } else {
     j.span = 0;
-    j.hw_tiles = (hw + 127) / 128;
+    j.hw_tiles = (hw + tile_px - 1) / tile_px;
     j.c_tiles = (c_padded + 63) / 64;
   }
   j.fd_hw_tiles = FastDiv::make(j.hw_tiles);
@@ -851,9 +865,11 @@ cudaError_t repack_bytes_pair_launch(const void* src_a, void* dst_a, int batch_a
                                      void* dst_b, int batch_b, int ch_b, int hw_b, int cp_b, cudaStream_t stream) {
   if (int64_t((hw_a + 63) / 64) * ((cp_a + 63) / 64) * batch_a + int64_t((hw_b + 63) / 64) * ((cp_b + 63) / 64) * batch_b > 2147483647LL)
     return cudaErrorInvalidValue;
-  const ByteJob a = make_byte_job(src_a, dst_a, batch_a, ch_a, hw_a, cp_a);
-  const ByteJob b = make_byte_job(src_b, dst_b, batch_b, ch_b, hw_b, cp_b);
-  const cudaError_t e = launch_pdl(repack_bytes_kernel, dim3(a.blocks + b.blocks), dim3(256), 0, stream, a, b, prefetch_enabled() ? 1 : 0);
+  const bool wide = int64_t((hw_a + 127) / 128) * ((cp_a + 63) / 64) * batch_a > kNumSms * 8;
+  const ByteJob a = make_byte_job(src_a, dst_a, batch_a, ch_a, hw_a, cp_a, wide ? 128 : 64);
+  const ByteJob b = make_byte_job(src_b, dst_b, batch_b, ch_b, hw_b, cp_b, wide ? 128 : 64);
+  // (shared memory nobody uses keeps a small job at six blocks per SM: see launch_jobs)
+  const cudaError_t e = launch_pdl(wide ? repack_bytes_kernel<128> : repack_bytes_kernel<64>, dim3(a.blocks + b.blocks), dim3(256), wide ? 0 : 28 * 1024, stream, a, b, prefetch_enabled() ? 1 : 0);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();
 }

@@ -170,9 +170,9 @@ def build(ref: bool = True, quiet: bool = True) -> None:
     """Compile the C restatement and, where the reference checkout exists, the reference's own oracle."""
     out = subprocess.DEVNULL if quiet else None
     subprocess.check_call(["make", "-C", HERE], stdout=out)
-    if ref and os.path.isdir(os.environ.get("GIE_REFERENCE_DIR", "/root/reference")):
-        subprocess.check_call(["make", "-C", HERE, "ref", "REF=" + os.environ.get("GIE_REFERENCE_DIR", "/root/reference")],
-                              stdout=out)
+    checkout = os.environ.get("GIE_REFERENCE_DIR", "/root/reference")
+    if ref and os.path.isdir(os.path.join(checkout, "src")):  # (the directory may be there and empty)
+        subprocess.check_call(["make", "-C", HERE, "ref", "REF=" + checkout], stdout=out)
 
 
 class Oracle:
