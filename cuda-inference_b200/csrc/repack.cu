@@ -429,7 +429,8 @@ cudaError_t launch_jobs(RepackJob a, int64_t tiles_a, RepackJob b, int64_t tiles
   // More than one wave: eight blocks per SM (46 x 430 x 57 x 57: 52.6 us, 60.1 with six).  A small job does not want them: its blocks
   // begin on the SMs that the kernel before it leaves idle, and the more those take the longer they are at it when all the others
   // have finished (32 x 256 x 14 x 14 and its weights under a 100-block convolution: 0.6 us a pass).
-  const auto kernel = a.blocks + b.blocks > unsigned(kNumSms) * 8 ? repack_jobs_kernel<8> : repack_jobs_kernel<0>;
+  // (A strided selection keeps sixteen loads in flight per thread, which 32 registers do not hold.)
+  const auto kernel = a.blocks + b.blocks > unsigned(kNumSms) * 8 && a.mode != 4 ? repack_jobs_kernel<8> : repack_jobs_kernel<0>;
   return launch_pdl(kernel, dim3(a.blocks + b.blocks), dim3(256), 0, stream, a, b);
 }
 
@@ -796,6 +797,15 @@ __global__ void __launch_bounds__(256) repack_bytes_kernel(const ByteJob a, cons
   const int lane = t & (LANES - 1), row0 = t / LANES;  // (half) a warp per row
   uint32_t* words = reinterpret_cast<uint32_t*>(tile);
   uint32_t word[PASSES], last[PASSES];
+  if ((j.HW & 3) == 0 && (reinterpret_cast<uintptr_t>(j.src) & 3u) == 0) {  // rows of whole words
+#pragma unroll
+    for (int i = 0; i < PASSES; ++i) {
+      const int ch = row0 + i * ROWS;
+      word[i] = c0 + ch < j.C && px0 + 4 * lane < j.HW ? *reinterpret_cast<const uint32_t*>(s + size_t(ch) * j.HW + 4 * lane) : 0u;
+    }
+#pragma unroll
+    for (int i = 0; i < PASSES; ++i) words[(row0 + i * ROWS) * PITCH + lane] = word[i];
+  } else {
 #pragma unroll
   for (int i = 0; i < PASSES; ++i) {
     const int ch = row0 + i * ROWS;
@@ -814,6 +824,7 @@ __global__ void __launch_bounds__(256) repack_bytes_kernel(const ByteJob a, cons
     uint32_t next = __shfl_down_sync(0xffffffffu, word[i], 1, LANES);
     if (lane == LANES - 1) next = last[i];
     words[ch * PITCH + lane] = __funnelshift_r(word[i], next, 8 * off);
+  }
   }
   __syncthreads();
   const int cg = t & 7;  // 8 channels
