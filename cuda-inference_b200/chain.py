@@ -193,15 +193,22 @@ class ConvChain:
     def output(self):
         return self.slots[len(self.slots) - 1]
 
-    def _buffers(self):
-        """What a recording holds pointers into."""
-        return [t.data_ptr() for t in self.slots.values()] + [id(c) for c in self.convs] + [self.ws_ptr]
+    def _recordable(self):
+        """Every value that a recording is made from, but for the operations (compared as they are: they cannot change)."""
+        key = [self.precision, self.batch, self.layout, self.fused, self.ws_ptr, self.ws_bytes]
+        for t in self.slots.values():
+            key += (t.data_ptr(), t.numel())
+        for _, plan, w, b in self.convs:
+            key += (plan._plan, w.data_ptr(), b.data_ptr())
+        return key
 
     def _record(self):
         """The launches of one pass with every pointer filled in, for ``enqueue`` to issue from native code: a pass of 107
-        launches spends ~1.7 us of Python per launch otherwise.  The chain's buffers stay where they are; should one have
-        been replaced, ``enqueue`` records again."""
-        self._recorded = self._buffers()
+        launches spends ~1.7 us of Python per launch otherwise.  The chain's plans and buffers stay where they are; should one
+        have been replaced, moved or closed, ``enqueue`` records again.  What is recorded is kept alive with the recording."""
+        self._recorded = self._recordable()
+        self._recorded_ops = list(self.ops)
+        self._kept = (list(self.convs), list(self.slots.values()), self._ws)
         ci = 0
         steps = []
         for op in self.ops:
@@ -224,7 +231,7 @@ class ConvChain:
 
     def enqueue(self, stream: int) -> None:
         """All launches of one forward pass on `stream` (capture-safe: no allocation, no synchronisation)."""
-        if self._recorded != self._buffers():
+        if self._recorded != self._recordable() or self._recorded_ops != self.ops:
             self._steps = self._record()
         check(calls().run_sequence(self._steps, stream))
 
