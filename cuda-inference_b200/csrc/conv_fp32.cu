@@ -22,6 +22,7 @@
 #include <type_traits>
 #include <utility>
 
+#include "conv_fp32_table.h"
 #include "internal.h"
 #include "ptx.cuh"
 
@@ -29,7 +30,6 @@ namespace gieb {
 namespace {
 
 constexpr int kBK = 16;
-constexpr int kLutMax = 4096;  // reduction length of a CTA up to which the (c, r, s) decode of k is tabulated in shared memory
 constexpr int kMaxSmem = 96 * 1024;
 
 struct Fp32Args {
@@ -130,7 +130,7 @@ conv_fp32_kernel(const Fp32Args a) {
   if (LUT) {
     for (int i = t; i < slabs * kBK; i += kThreads) {
       const int k = kbase + i;
-      int2 e = make_int2(0, 0x7fff0000);  // r far outside every image: never loaded
+      int2 e = make_int2(0, kNoRow << 16);  // a row outside the image: never loaded
       if (k < a.k) {
         const int c = a.fd_rs.div(k), q = k - c * rs;
         const int r = a.fd_s.div(q), sx = q - r * a.s;
@@ -374,7 +374,7 @@ cudaError_t conv_fp32_launch(const void* x, const void* w, const void* bias, voi
   a.slabs_per_slice = (slabs + a.slices - 1) / a.slices;
   const bool xvec = r == 1 && s == 1 && stride_h == 1 && stride_w == 1 && pad_h == 0 && pad_w == 0 && (out_h * out_w) % 4 == 0 &&
                     (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
-  const bool lut = !xvec && a.slabs_per_slice * kBK <= kLutMax && int64_t(c) * h * wd < (int64_t(1) << 31) && r < 0x7fff && s <= 0xffff && h < 0x7fff;
+  const bool lut = !xvec && conv_fp32_table_fits(int64_t(a.slabs_per_slice) * kBK, c, h, wd, r, s, pad_h);
   const bool w16 = a.k % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15u) == 0;  // 128-bit copies along k
   const size_t smem = size_t(kRing) * (kBK * tp + to * kWPitch) * sizeof(float) + (lut ? size_t(a.slabs_per_slice) * kBK * sizeof(int2) : 0);
   const dim3 grid(unsigned(tiles_p * a.slices), unsigned(tiles_o));

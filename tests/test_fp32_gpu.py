@@ -19,6 +19,8 @@ CASES = [
     ((2, 816, 13, 31, 80, 1, 1, 1, 1, 0, 0), 0),     # 1x1, planes of 403 pixels
     ((1, 4, 33000, 1, 8, 3, 1, 1, 1, 1, 0), 0),      # taller than the decode table's fields
     ((1, 1, 1, 1, 1, 1, 1, 1, 1, 0, 0), 0),
+    ((1, 1, 32760, 3, 8, 3, 1, 1, 1, 20, 0), 0),     # image and padding together are taller than the decode table's fields; 3 terms
+    ((1, 2, 32700, 1, 4, 3, 1, 1, 1, 67, 0), 0),     # exactly as tall
 ]
 
 
