@@ -76,7 +76,6 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_consta
   const bool leader = pair_rank == 0;
   const int tile_first = PAIR ? int(blockIdx.x >> 1) : int(blockIdx.x);
   const int tile_step = PAIR ? int(gridDim.x >> 1) : int(gridDim.x);
-  ptx::grid_dep_launch();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -107,6 +106,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_consta
       ptx::tmem_alloc(tmem_slot, TMEM_COLS);
       ptx::tmem_relinquish();
     }
+    ptx::grid_dep_launch();  // (behind the allocation: see conv_tc_kernel)
   }
   ptx::tc_fence_before_sync();
   if constexpr (PAIR) ptx::cluster_sync_all();

@@ -362,7 +362,6 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
   // persistent walk over the tile list: by CTA, or by CTA pair
   const int tile_first = PAIR ? int(blockIdx.x >> 1) : int(blockIdx.x);
   const int tile_step = PAIR ? int(gridDim.x >> 1) : int(gridDim.x);
-  ptx::grid_dep_launch();  // the next kernel of the stream may begin its own set-up (it orders itself with grid_dep_wait)
 
   if (threadIdx.x == 0) {
     ptx::prefetch_tensormap(&tm_act);
@@ -393,6 +392,10 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
       ptx::tmem_alloc(tmem_slot, TMEM_COLS);
       ptx::tmem_relinquish();
     }
+    // The next kernel of the stream may begin its own set-up (it orders itself with grid_dep_wait).  Only now: a CTA of it that
+    // came to lie beside this one while this one still waited for columns could take them first, and would then hold them
+    // until this kernel has ended, which it could not without them.
+    ptx::grid_dep_launch();
   }
   // The set-up barrier (mbarriers initialised, TMEM allocated) is joined by every warp exactly once, from inside its
   // role and only after it has decoded its first tile, so the decode overlaps the set-up instead of following it.

@@ -178,3 +178,22 @@ def test_rmsnorm_argument_checks_need_no_gpu(pkg):
         with pytest.raises(pkg.GieError) as e:
             pkg.rmsnorm_forward(rows, hidden, 1e-6, 0, x, g, y, ri, ro, 0)
         assert e.value.code == pkg.INVALID_ARGUMENT
+
+
+def test_dependents_start_behind_the_tensor_memory_allocation():
+    """A kernel that allocates tensor memory lets the next kernel of the stream start only once it has its columns: the
+    signal comes from the allocating warp, after the allocation, and from nowhere else."""
+    csrc = os.path.join(ROOT, "cuda-inference_b200", "csrc")
+    seen = 0
+    for f in sorted(os.listdir(csrc)):
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, f)).read())
+        if f == "ptx.cuh" or not re.search(r"ptx::tmem_alloc\(", text):
+            continue
+        seen += 1
+        signals = [m.start() for m in re.finditer(r"ptx::grid_dep_launch\(\)", text)]
+        allocs = [m.start() for m in re.finditer(r"ptx::tmem_alloc(?:_pair)?\(", text)]
+        assert len(signals) == 1, f
+        assert max(allocs) < signals[0] < text.index("ptx::tc_fence_before_sync()"), f
+        block = text[text.rindex("if (warp == kProducerWarps) {", 0, signals[0]):signals[0]]
+        assert block.count("{") > block.count("}") and "tmem_alloc" in block, f  # still inside the allocating warp's block
+    assert seen == 2
