@@ -156,6 +156,20 @@ int tmem_cols_of(int tile_m, int tile_n) {
   return cols < 32 ? 32 : cols;
 }
 
+// Shared memory that a CTA of `cols` tensor-memory columns asks for at least, so that columns run out on no SM before shared
+// memory does where that would cost anything.  An allocation that finds no columns waits until another CTA of the SM has ended:
+//  * All 512 columns: more than half of an SM.  A persistent kernel launches one such CTA per SM, but while CTAs of the kernel
+//    before it still hold most SMs two could be placed on one; the second then began when the first had walked its whole tile
+//    list and the launch took twice as long (FP16 237 x 64 -> 320 at 81 x 81, 1x1/2, 2 slabs of ring: 337 us, the kernel alone
+//    150; 41 x 41, 1x1/1: 313 us).
+//  * CTAs that wait for one another (pairs, split-K clusters): their columns' share.  Otherwise one CTA each of two such
+//    launches, in two streams, could hold the columns of an SM that the other's peer waits for.
+constexpr size_t kSmSmem = 233472;  // 228 KiB of an SM; every CTA takes 1 KiB besides what it asks for
+size_t smem_floor(int cols, bool waits_for_peers) {
+  if (waits_for_peers) return kSmSmem / 512 * cols - 1024;
+  return cols > 256 ? kSmSmem / 2 : 0;
+}
+
 int resident_ctas(int tile_m, int tile_n, size_t smem) {
   int by_smem = int(kMaxDynamicSmem / (smem + 1024));
   int by_tmem = 512 / tmem_cols_of(tile_m, tile_n);
@@ -415,6 +429,8 @@ bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, double slab, Resol
   const size_t exchange = 1024 + 3072 + size_t(b.tile_n) * 512;  // a cluster's partial columns land in the idle stages
   if (b.split_k > 1 && b.smem < exchange) b.smem = exchange;
   if (b.pair && b.smem < kMaxDynamicSmem / 2 + 2048) b.smem = kMaxDynamicSmem / 2 + 2048;  // (see resolve())
+  const size_t floor = smem_floor(tmem_cols_of(kTileM, b.tile_n), b.pair || b.split_k > 1);
+  if (b.smem < floor) b.smem = floor;
   b.halo = 1;
   b.tile_k = 64;
   b.kb_per_tap = blocks;
@@ -705,6 +721,8 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
   r->reduce = r->split_k > 1 ? best_mode : 0;
   if (r->reduce == 2 && !cluster_reduce_ok(r->tile_m, r->tile_n, r->tile_k, stages, r->split_k))
     return no("cluster reduction needs tile_m 128, split_k 2, 4 or 8 dividing tile_n / 32, and a ring that holds the received slices");
+  const size_t floor = smem_floor(r->pair ? tmem_cols_of(kTileM, r->tile_n) : tmem_cols_of(r->tile_m, r->tile_n), r->pair || r->reduce == 2);
+  if (r->smem < floor) r->smem = floor;
   r->ws_part = r->split_k > 1 && r->reduce == 1 ? align256(size_t(r->split_k) * size_t((g.y_elems + 3) & ~int64_t(3)) * 4) : 0;
   r->ws_total = r->ws_x + r->ws_w + r->ws_part;
   if (r->ws_total > (size_t(180) << 30) / 4) return no("workspace exceeds a quarter of device memory");

@@ -197,3 +197,36 @@ def test_dependents_start_behind_the_tensor_memory_allocation():
         block = text[text.rindex("if (warp == kProducerWarps) {", 0, signals[0]):signals[0]]
         assert block.count("{") > block.count("}") and "tmem_alloc" in block, f  # still inside the allocating warp's block
     assert seen == 2
+
+
+def test_shared_memory_keeps_tensor_memory_from_running_out(pkg):
+    """An allocation of tensor memory waits for another CTA of the SM to end.  CTAs of all 512 columns ask for more than half of
+    an SM's shared memory, so that two never share one; CTAs that wait for one another (pairs, split-K clusters) ask for at
+    least their columns' share of it, so that no set of them that fits an SM wants more than its 512 columns."""
+    sm = 228 * 1024
+    seen = {"full": 0, "pair": 0, "cluster": 0}
+    shapes = [(237, 64, 81, 81, 320, 1, 1, 2, 2, 0, 0), (237, 64, 41, 41, 320, 1, 1, 1, 1, 0, 0), (8, 512, 7, 7, 512, 3, 3, 1, 1, 1, 1),
+              (1, 512, 7, 7, 512, 3, 3, 1, 1, 1, 1), (32, 256, 14, 14, 256, 3, 3, 1, 1, 1, 1), (64, 512, 28, 28, 512, 3, 3, 1, 1, 1, 1),
+              (1, 1024, 7, 7, 512, 1, 1, 1, 1, 0, 0), (2, 320, 8, 8, 40, 5, 5, 1, 1, 2, 2), (8, 64, 31, 31, 512, 3, 3, 1, 1, 1, 1),
+              (2, 256, 67, 67, 512, 1, 3, 1, 1, 0, 1), (1, 2048, 9, 9, 256, 3, 3, 1, 1, 1, 1), (4, 64, 12, 12, 256, 1, 1, 1, 1, 0, 0)]
+    cfgs = [None] + [dict(tile_m=m, tile_n=n, stages=2, cta_pair=1) for m in (128, 256) for n in (32, 64, 128, 256)]
+    cfgs += [dict(tile_n=n, stages=2, cta_pair=2) for n in (64, 128, 256)] + [dict(tile_n=n, split_k=2, reduce=2) for n in (64, 128, 256)]
+    for a in shapes:
+        for prec in (pkg.FP16, pkg.BF16, pkg.FP8_E4M3):
+            for kw in cfgs:
+                info = pkg.query(P(pkg, *a, precision=prec, has_bias=True, relu=True), pkg.make_cfg(**kw) if kw else None)
+                if not info.supported:
+                    continue
+                c = info.cfg
+                one = c.tile_n * (1 if c.cta_pair == 2 else c.tile_m // 128)   # columns of one accumulator; two when they fit
+                cols = max(32, 2 * one if one <= 256 else one)
+                smem = info.dynamic_smem_bytes
+                assert smem <= 227 * 1024
+                if cols == 512:
+                    seen["full"] += 1
+                    assert 2 * (smem + 1024) > sm, (a, prec, kw, smem)
+                waits = "pair" if c.cta_pair == 2 else ("cluster" if c.reduce == 2 else None)
+                if waits:
+                    seen[waits] += 1
+                    assert (smem + 1024) * 512 >= sm * cols, (a, prec, kw, smem, cols)
+    assert min(seen.values()) > 10, seen
