@@ -310,11 +310,6 @@ bool pairs_enabled() {
   }();
   return on;
 }
-// GIEB_HALO (a debugging aid): 0 keeps every layer on the slab kernels, 2 takes the halo-tile kernel wherever it is possible.
-int halo_mode() {
-  const char* e = getenv("GIEB_HALO");
-  return e ? atoi(e) : 1;
-}
 // GIEB_DISABLE_PREFETCH=1 switches the L2 prefetches that precede the dependency waits off (a debugging aid).
 bool prefetch_enabled() {
   static const bool on = [] {
@@ -327,11 +322,11 @@ bool prefetch_enabled() {
 
 namespace {
 
-// Configuration of the halo-tile kernel for a problem whose route and padding resolve() has settled, when it is expected to be
-// faster than the `slab` cycles of the best slab configuration; false: not for this problem.
-bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, double slab, Resolved* r) {
-  const int mode = halo_mode();
-  if (mode == 0) return false;
+// Configuration of the halo-tile kernel for a problem whose route and padding resolve() has settled: unasked (c.variant 0) when it
+// is expected to be faster than the `slab` cycles of the best slab configuration, else the best one that has the fields set in
+// `c`.  False: not for this problem.
+bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, const gieb_conv_cfg& c, double slab, Resolved* r) {
+  const bool asked = c.variant == 6;
   const bool nhwc = (d.flags & GIEB_FLAG_INPUT_NHWC) != 0;
   const int taps = d.kernel_h * d.kernel_w;
   if (r->variant != 1 || taps == 1) return false;
@@ -355,11 +350,11 @@ bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, double slab, Resol
       const size_t fixed = conv_halo_smem_bytes(bn, pair, workers, tpl, a, stage, 0, staging);
       if (fixed >= budget) continue;
       const int room = int((budget - fixed) / (size_t(tpl) * (pair ? bn / 2 : bn) * 128));
-      if (room < 2) continue;
+      if (room < 2 || room < c.stages) continue;
       f->a = a;
-      f->b = room > kMaxStages ? kMaxStages : room;
+      f->b = c.stages ? c.stages : (room > kMaxStages ? kMaxStages : room);
       f->resident = one_n && loads <= f->b;
-      if (loads < f->b) f->b = loads < 2 ? 2 : loads;
+      if (!c.stages && loads < f->b) f->b = loads < 2 ? 2 : loads;
       f->smem = conv_halo_smem_bytes(bn, pair, workers, tpl, a, stage, f->b, staging);
       return true;
     }
@@ -374,18 +369,20 @@ bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, double slab, Resol
   const int box_rows = box_h * ws, boxes = ceil_div(box_rows - 1 + need, box_rows);
   if (ws * d.stride_w > 256 || box_h * d.stride_h > 256 || boxes > 64) return false;  // (limits of a TMA box)
   for (int pair = 0; pair <= (d.precision == GIEB_TF32 ? 0 : 1); ++pair) {
+    if ((c.cta_pair && pair != c.cta_pair - 1) || (c.tile_m && pair != c.tile_m / kTileM - 1)) continue;
     // (the CTAs of a pair shift their boxes to a common first row)
     const int phase_rows = (boxes + pair) * box_rows;
     const size_t stage = (size_t(ph) * pw * phase_rows * 128 + 1023) / 1024 * 1024;
     if (rows + int64_t(ph) * pw * phase_rows + 2 * kTileM > 2147483647LL || stage > 160 * 1024) continue;
     for (int bn = pair ? 128 : 32; bn <= 256; bn *= 2) {
-      if (bn > 32 && bn / 2 >= d.out_channels) continue;
+      if (c.tile_n ? bn != c.tile_n : bn > 32 && bn / 2 >= d.out_channels) continue;
       const int workers = pair || bn == 256 ? 16 : 8, tiles_n = ceil_div(d.out_channels, bn);
       const int tpl = taps_per_load(pair ? bn / 2 : bn), groups = ceil_div(taps, tpl);
       const int64_t tiles = int64_t(ceil_div(rows, pair ? 2 * kTileM : kTileM)) * tiles_n;
       const int sms = pair ? kNumSmPairs : kNumSms;
-      if (pair && (rows <= 2 * kTileM || tiles < sms / 2)) continue;
+      if (pair && (rows <= 2 * kTileM || (!c.cta_pair && tiles < sms / 2))) continue;
       for (int s = 1; s <= (pair ? 1 : 8); s *= 2) {
+        if ((c.split_k && s != c.split_k) || (c.reduce && s == 1)) continue;
         const int loads = blocks * groups, per = ceil_div(loads, s);
         if (s > 1 && (tiles * s > kNumSms || loads < 2 * s || ceil_div(loads, per) != s)) continue;
         Fit f;
@@ -425,7 +422,7 @@ bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, double slab, Resol
   // double the issue rate there), except for FP8.
   double margin = 0.95;
   if (best_load >= 3) margin = (b.tile_n <= 64 && ph * pw == 1 && d.precision != GIEB_FP8_E4M3) ? 1.3 : 1.0;
-  if (best >= 1e299 || (mode == 1 && best >= margin * slab)) return false;
+  if (best >= 1e299 || (!asked && best >= margin * slab)) return false;
   const size_t exchange = 1024 + 3072 + size_t(b.tile_n) * 512;  // a cluster's partial columns land in the idle stages
   if (b.split_k > 1 && b.smem < exchange) b.smem = exchange;
   if (b.pair && b.smem < kMaxDynamicSmem / 2 + 2048) b.smem = kMaxDynamicSmem / 2 + 2048;  // (see resolve())
@@ -440,7 +437,7 @@ bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, double slab, Resol
   b.h_hs = hs; b.h_ws = ws;
   b.h_phases = ph * pw; b.h_phases_w = pw;
   b.h_last_ksteps = last;
-  b.tiles_m = ceil_div(g.pixels, b.tile_m);  // (as reported; the kernel's own tiles cover the padded grid)
+  b.tiles_m = ceil_div(rows, b.tile_m);  // (tiles cover the padded grid)
   b.ws_x = nhwc ? 0 : align256(size_t(d.batch) * d.in_h * d.in_w * b.c_padded * 2);
   b.ws_w = (d.flags & GIEB_FLAG_WEIGHTS_PREPACKED) ? 0 : align256(size_t(d.out_channels) * taps * b.c_padded * 2);
   b.ws_total = b.ws_x + b.ws_w;
@@ -478,8 +475,9 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
   }
   const bool pointwise = d.kernel_h == 1 && d.kernel_w == 1 && d.stride_h == 1 && d.stride_w == 1 && d.pad_h == 0 && d.pad_w == 0;
   const bool direct_ok = !tf32 && pointwise && (d.in_h * d.in_w) % 8 == 0;
-  if (c.variant != 0 && c.variant != 1 && c.variant != 2 && c.variant != 4 && c.variant != 5)
-    return no("unknown kernel variant for 16-bit precision (1 = im2col-mode TMA, 2 = direct NCHW 1x1, 4 = tiled TMA for 1x1, 5 = row gather)");
+  if (c.variant != 0 && c.variant != 1 && c.variant != 2 && c.variant != 4 && c.variant != 5 && c.variant != 6)
+    return no("unknown kernel variant for 16-bit precision (1 = im2col-mode TMA, 2 = direct NCHW 1x1, 4 = tiled TMA for 1x1, 5 = row gather, 6 = halo tiles)");
+  const bool halo = c.variant == 6;  // the operands of variant 1, read by another kernel
   // Row gather: the S taps of a filter row become channels (c2 = padded S*C <= 64, one slab or less per filter row).
   // Worth it when it at least halves the padded reduction length (a 7x7 stem over 3 channels: 7*32 instead of 49*16).
   const int gather_c2 = round_up(d.kernel_w * d.in_channels, 16);
@@ -496,7 +494,7 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
     if (d.in_channels % 16 != 0) return no("channel-contiguous input needs a channel count that is a multiple of 16");
     if (c.variant == 2) return no("variant 2 reads NCHW activations; a channel-contiguous input takes variant 1 or 4");
   }
-  r->variant = c.variant ? c.variant : (in_nhwc ? (pointwise ? 4 : 1) : (direct_ok ? 2 : ((pointwise || strided_pw) ? 4 : (gather_pays ? 5 : 1))));
+  r->variant = halo ? 1 : c.variant ? c.variant : (in_nhwc ? (pointwise ? 4 : 1) : (direct_ok ? 2 : ((pointwise || strided_pw) ? 4 : (gather_pays ? 5 : 1))));
   r->subsampled = (r->variant == 4 && strided_pw) ? 1 : 0;
   const bool gather = r->variant == 5;
   r->eff_in_w = gather ? g.out_w : d.in_w;
@@ -547,15 +545,20 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
     r->tile_k = c.tile_k ? c.tile_k : pick_tile_k(d.in_channels);
   }
   if (r->tile_k != 16 && r->tile_k != 32 && r->tile_k != 64) return no("tile_k must be 16, 32 or 64");
-  if (in_nhwc && c.tile_k && d.in_channels % r->tile_k != 0) return no("tile_k must divide the channel count of a channel-contiguous input (it is read in place)");
+  // A slab width that was asked for pads to whole slabs.  A configuration with every field set that names the automatic width is
+  // one that gieb_conv_query reported, or as good as one: it stands for the same layout, whose last slab may be a partial one.
+  const int units = fp8 ? (d.in_channels + 1) / 2 : (tf32 ? 2 * d.in_channels : d.in_channels);
+  const bool complete = c.tile_m && c.tile_n && c.stages && c.split_k && c.variant && c.cta_pair && c.tile_k && r->tile_k == pick_tile_k(units);
+  const bool whole_slabs = c.tile_k && !complete && !halo;
+  if (halo && c.tile_k && r->tile_k != 64) return no("variant 6 (halo tiles) takes rows of 128 bytes: tile_k 64 (32 for TF32, 128 for FP8)");
+  if (in_nhwc && whole_slabs && d.in_channels % r->tile_k != 0) return no("tile_k must divide the channel count of a channel-contiguous input (it is read in place)");
   if (gather) {
     const int gc2 = r->gather_pairs ? r->gp_t * 8 : gather_c2;
     if (!c.tile_k) r->tile_k = gc2 % 64 == 0 ? 64 : (gc2 % 32 == 0 ? 32 : 16);
     if (gc2 % r->tile_k != 0) return no("tile_k must divide the gathered row length (padded kernel_w * channels)");
     r->c_padded = gc2;
-  } else {  // (a slab width that was asked for pads to whole slabs)
-    const int units = fp8 ? (d.in_channels + 1) / 2 : (tf32 ? 2 * d.in_channels : d.in_channels);
-    r->c_padded = round_up(units, c.tile_k ? r->tile_k : 16);
+  } else {
+    r->c_padded = round_up(units, whole_slabs ? r->tile_k : 16);
   }
   r->kb_per_tap = ceil_div(r->c_padded, r->tile_k);
   r->total_kb = d.kernel_h * r->eff_kernel_w * r->kb_per_tap;
@@ -572,6 +575,13 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
     if (c.tile_m != 0 && c.tile_m != 256) return no("a CTA pair computes 256-pixel tiles (tile_m 0 or 256)");
     if (c.tile_n != 0 && c.tile_n < 64) return no("CTA-pair tiles are 64, 128 or 256 output channels wide");
     if (c.reduce == 2) return no("a CTA pair is a cluster already: its split-K slices are summed through the workspace (reduce 0 or 1)");
+  }
+  if (halo) {
+    if (c.stages != 0 && (c.stages < 2 || c.stages > kMaxStages)) return no("stages must be in [2, 8]");
+    if (c.reduce < 0 || c.reduce > 2) return no("reduce must be 0 (auto), 1 (workspace) or 2 (cluster)");
+    if (c.reduce != 1 && resolve_halo(d, g, c, 0.0, r)) return GIEB_OK;
+    return no("variant 6 (halo tiles) needs a kernel of 2 to 64 taps, strides up to 2, padding below the kernel's extents, at least 16 output "
+              "pixels, split_k 1, 2, 4 or 8 (in clusters; not in pairs) and tiles that fit shared memory");
   }
   // NCHW output whose planes are 16-byte multiples, 16-bit types: 128- and 256-channel tiles that a CTA finishes alone
   // keep the accumulator transposed (lane = output channel) and write their boxes with TMA stores.
@@ -635,7 +645,7 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
     }
   }
   const bool untouched = c.tile_n == 0 && c.tile_k == 0 && c.stages == 0 && c.split_k == 0 && c.variant == 0 && c.tile_m == 0 && c.reduce == 0 && c.cta_pair == 0;
-  if (untouched && resolve_halo(d, g, best, r)) return GIEB_OK;
+  if (untouched && resolve_halo(d, g, c, best, r)) return GIEB_OK;
   if (best_n == 0) {
     if (c.reduce == 2) return no("cluster reduction needs tile_m 128, split_k 2, 4 or 8 dividing tile_n / 32 with no empty slice, and a ring that holds the received slices");
     if (c.split_k > 1) return no("reduction too short for this split-K factor");
@@ -738,7 +748,7 @@ void fill_info(const gieb_conv_desc& d, const Resolved& r, gieb_conv_info* out) 
   out->cfg.tile_k = d.precision == GIEB_TF32 ? r.tile_k / 2 : (d.precision == GIEB_FP8_E4M3 ? r.tile_k * 2 : r.tile_k);  // in elements of the storage type
   out->cfg.stages = r.stages;
   out->cfg.split_k = r.split_k;
-  out->cfg.variant = r.variant;
+  out->cfg.variant = r.halo ? 6 : r.variant;
   out->cfg.reduce = r.reduce;
   out->cfg.cta_pair = r.variant == 3 ? 0 : (r.pair ? 2 : 1);
   out->workspace_bytes = r.ws_total;

@@ -82,7 +82,10 @@ typedef struct gieb_conv_desc {
  * (src/kernels/tensor_core_mma.cu:369-388, src/kernels/implicit_gemm.cu:243-266).  Zero / NULL = heuristic. */
 typedef struct gieb_conv_cfg {
   int32_t tile_n;   /* output channels per CTA tile: 32, 64, 128 or 256 (tensor path); 0 = auto              */
-  int32_t tile_k;   /* reduction slab in channels: 16, 32 or 64; 0 = auto                                    */
+  int32_t tile_k;   /* reduction slab in channels: 16, 32 or 64; 0 = auto.  Asked for, it pads the channels to whole slabs
+                       (and has to divide those of a channel-contiguous input).  Left to the library, or in a
+                       configuration whose fields are all set as gieb_conv_query reports them, channels are padded to
+                       a multiple of 16 and the last slab of a filter tap may be a partial one                    */
   int32_t stages;   /* shared-memory ring depth, 2..8; 0 = auto                                              */
   int32_t split_k;  /* number of reduction splits, >= 1; 0 = auto                                            */
   int32_t variant;  /* 0 = auto; 1 = tensor path, im2col-mode TMA over the channel-contiguous copy (any geometry);
@@ -93,7 +96,11 @@ typedef struct gieb_conv_cfg {
                        3 = FP32 SIMT;
                        5 = tensor path over row-gathered activations for inputs with few channels (NCHW input,
                            kernel_w > 1, kernel_w * C <= 64): the S taps of a filter row become channels, so a 7x7
-                           stem over 3 channels reduces over 7 x 32 values instead of 49 x 16 padded ones      */
+                           stem over 3 channels reduces over 7 x 32 values instead of 49 x 16 padded ones;
+                       6 = tensor path whose tiles hold every activation once for all filter taps (kernels of 2 to 64
+                           taps, strides 1 or 2, padding below the kernel's extents, 16 output pixels or more);
+                           tile_m 128, or 256 with cta_pair 2; tile_n 128 or 256 in pairs; split_k 1, 2, 4 or 8, summed
+                           in clusters (not in pairs); stages = ring depth of the weights, tile_k 64                 */
   int32_t tile_m;   /* output pixels per CTA tile: 128 or 256 (two accumulators share each weight tile); 0 = auto */
   int32_t reduce;   /* how split-K slices are summed: 0 = auto; 1 = FP32 partials in the workspace + a reduction launch;
                        2 = inside the convolution kernel: the slices of a tile form a thread-block cluster and are
@@ -109,8 +116,8 @@ typedef struct gieb_conv_cfg {
  * (include/gpu_inference/kernel_registry.h:62-70). */
 typedef struct gieb_conv_info {
   int32_t supported;
-  int32_t variant;
-  gieb_conv_cfg cfg;          /* the configuration that would run (heuristic filled in)  */
+  int32_t variant;            /* route of the operands: cfg.variant, but 1 where that is 6 */
+  gieb_conv_cfg cfg;          /* the configuration that would run (heuristic filled in): handed back, it gives the same plan */
   uint64_t workspace_bytes;   /* caller-provided per-call scratch                          */
   uint64_t persistent_bytes;  /* plan-owned device memory                                  */
   uint32_t dynamic_smem_bytes;

@@ -156,6 +156,9 @@ def test_selection_is_deterministic_and_fills_the_machine(pkg):
         rows = a[0] * -(-(a[2] * a[3]) // 64) * 64 if i1.variant == 2 else pixels   # direct NCHW route counts 64-pixel boxes
         if i1.variant == 5 and a[8] == 2 and a[1] <= 4 and p.out_w <= 128:
             rows = a[0] * p.out_h * 128   # position strips: one 128-row box per output row
+        if c.variant == 6:                # halo tiles cover the padded grid; at stride 1 neighbours share their padding
+            assert (a[7], a[8]) == (1, 1)
+            rows = a[0] * (a[2] + a[9]) * (a[3] + a[10])
         ctas_per_tile = 2 if c.cta_pair == 2 else 1   # a 256-pixel tile of a CTA pair is two CTAs
         assert i1.num_blocks == -(-rows // c.tile_m) * -(-a[4] // c.tile_n) * c.split_k * ctas_per_tile
     # the small deep layer gets split-K, the big ones do not
@@ -230,3 +233,68 @@ def test_shared_memory_keeps_tensor_memory_from_running_out(pkg):
                     seen[waits] += 1
                     assert (smem + 1024) * 512 >= sm * cols, (a, prec, kw, smem, cols)
     assert min(seen.values()) > 10, seen
+
+
+def _random_problems(pkg, n, seed):
+    """Convolutions over the sizes, layouts and types that networks have, ragged ones among them."""
+    import random
+    rng = random.Random(seed)
+    made = 0
+    while made < n:
+        k = rng.choice([(1, 1), (3, 3), (3, 3), (5, 5), (7, 7), (1, 3), (3, 2)])
+        stride = rng.choice([1, 1, 1, 2])
+        h = rng.choice([7, 8, 9, 13, 14, 17, 28, 31, 35, 56, 67])
+        w = rng.choice([h, h, rng.randint(5, 80)])
+        c = rng.choice([3, 16, 33, 48, 64, 72, 80, 96, 112, 128, 130, 144, 160, 192, 200, 256, 320, 512, 816])
+        o = rng.choice([8, 17, 32, 40, 64, 70, 96, 128, 131, 144, 192, 200, 256, 320, 512])
+        b = rng.choice([1, 1, 2, 3, 4, 8, 16, 32, 64, 128])
+        prec = rng.choice([pkg.FP16, pkg.FP16, pkg.BF16, pkg.TF32, pkg.FP8_E4M3, pkg.FP32])
+        flags = 0
+        if prec in (pkg.FP16, pkg.BF16):
+            flags = (rng.choice([0, pkg.FLAG_INPUT_NHWC if c % 16 == 0 else 0]) | rng.choice([0, pkg.FLAG_OUTPUT_NHWC]) |
+                     rng.choice([0, pkg.FLAG_RESIDUAL]) | rng.choice([0, pkg.FLAG_WEIGHTS_PREPACKED]))
+        p = P(pkg, b, c, h, w, o, k[0], k[1], stride, stride, k[0] // 2, k[1] // 2, precision=prec, has_bias=True, relu=True, flags=flags)
+        if pkg.query(p).supported:
+            made += 1
+            yield p
+
+
+def _reported(info):
+    return (tuple(getattr(info.cfg, f) for f, _ in info.cfg._fields_), info.variant, info.workspace_bytes, info.dynamic_smem_bytes, info.threads_per_block,
+            info.num_blocks, info.launches, info.padded_channels)
+
+
+def test_reported_configuration_gives_the_same_plan(pkg):
+    """What a query reports as its configuration can be handed back, and then stands for the same plan: tiles, workspace,
+    weight layout and grid (the halo kernel's plans and partial last slabs among them)."""
+    seen = {}
+    for p in _random_problems(pkg, 3000, 5):
+        auto = pkg.query(p)
+        c = auto.cfg
+        again = pkg.query(p, pkg.make_cfg(**{f: getattr(c, f) for f, _ in c._fields_}))
+        assert again.supported, (p, again.reason)
+        assert _reported(again) == _reported(auto), (p, _reported(auto), _reported(again))
+        kind = (c.variant, c.cta_pair, c.split_k > 1, auto.padded_channels % max(1, c.tile_k) != 0)
+        seen[kind] = seen.get(kind, 0) + 1
+    for kind in [(6, 1, False, False), (6, 1, True, False), (6, 2, False, False), (6, 1, False, True), (1, 1, True, False), (1, 1, False, True),
+                 (1, 2, False, False), (4, 1, False, True), (2, 1, False, False), (5, 1, False, False), (3, 0, False, False)]:
+        assert seen.get(kind, 0) >= 3, (kind, seen)
+
+
+def test_halo_variant_takes_and_refuses(pkg):
+    """The halo-tile kernel by name: what it can run it runs with the fields given, what it cannot is refused with a reason."""
+    p = P(pkg, 4, 144, 14, 14, 200, 3, 3, 1, 1, 1, 1, precision=pkg.FP16)
+    for kw in (dict(), dict(tile_n=256), dict(tile_n=64, split_k=2), dict(tile_n=128, split_k=2, reduce=2), dict(cta_pair=2), dict(cta_pair=2, tile_n=256),
+               dict(tile_n=32, stages=3), dict(tile_m=128, tile_k=64)):
+        i = pkg.query(p, pkg.make_cfg(variant=6, **kw))
+        assert i.supported and i.cfg.variant == 6 and i.variant == 1, (kw, i.reason)
+        assert i.padded_channels == 144 and all(getattr(i.cfg, k) == v for k, v in kw.items()), kw
+    for kw in (dict(tile_n=48), dict(split_k=3), dict(cta_pair=2, split_k=2), dict(cta_pair=2, tile_n=64), dict(cta_pair=2, tile_m=128), dict(reduce=1),
+               dict(reduce=2, split_k=1), dict(tile_k=32), dict(stages=1), dict(stages=9), dict(cta_pair=3), dict(tile_m=64)):
+        i = pkg.query(p, pkg.make_cfg(variant=6, **kw))
+        assert not i.supported and i.reason, kw
+    for a in [(2, 64, 14, 14, 64, 1, 1, 1, 1, 0, 0), (2, 64, 40, 40, 64, 3, 3, 3, 3, 1, 1), (2, 64, 14, 14, 64, 3, 3, 1, 1, 3, 1), (2, 64, 3, 3, 64, 3, 3, 1, 1, 1, 1),
+              (2, 64, 30, 30, 64, 9, 9, 1, 1, 4, 4)]:
+        assert not pkg.query(P(pkg, *a, precision=pkg.FP16), pkg.make_cfg(variant=6)).supported, a
+    assert not pkg.query(P(pkg, 1, 64, 14, 14, 64, 3, 3, 1, 1, 1, 1, precision=pkg.TF32), pkg.make_cfg(variant=6, cta_pair=2)).supported
+    assert not pkg.query(P(pkg, 1, 64, 14, 14, 64, 3, 3, 1, 1, 1, 1, precision=pkg.FP32), pkg.make_cfg(variant=6)).supported
