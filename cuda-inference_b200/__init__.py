@@ -1,6 +1,7 @@
 """Python host-side mirror of the C ABI in ``include/gie_b200.h`` (no torch types cross the boundary).  Plans, queries and
 status words go through ctypes; the calls a program makes once per layer go through the extension module ``_calls``
-(csrc/python_calls.cpp), which costs the host a fifth of a ctypes call.
+(csrc/python_calls.cpp), which costs the host a fifth of a ctypes call.  It takes plain ints and None; a call with any other
+argument (a stream object, a ``c_void_p``) is converted, or refused, by ctypes.
 
 The native library ``libgie_b200.so`` and ``_calls.so`` are built in-tree by ``build.py``.  Importing this package never falls back to
 any other implementation: if the library is missing, loading raises.  Device memory and streams come from the caller
@@ -191,7 +192,10 @@ class ConvPlan:
 
     def launch(self, x: int, w: int, bias: int | None, y: int, workspace: int | None, workspace_bytes: int, stream: int = 0) -> None:
         """execute_unchecked: raw device pointers, asynchronous on `stream`."""
-        status = _calls.conv_launch(self._plan, x, w, bias, y, workspace, workspace_bytes, stream)
+        try:
+            status = _calls.conv_launch(self._plan, x, w, bias, y, workspace, workspace_bytes, stream)
+        except TypeError:
+            status = lib().gieb_conv_launch(self._h, x, w, bias, y, workspace, workspace_bytes, stream)
         if status:
             check(status)
 
@@ -209,7 +213,10 @@ class ConvPlan:
                      stream: int = 0) -> None:
         """launch() with a residual tensor (shape, layout and type of y) added before the activation; for plans whose
         problem carries FLAG_RESIDUAL."""
-        status = _calls.conv_launch_fused(self._plan, x, w, bias, residual, y, workspace, workspace_bytes, stream)
+        try:
+            status = _calls.conv_launch_fused(self._plan, x, w, bias, residual, y, workspace, workspace_bytes, stream)
+        except TypeError:
+            status = lib().gieb_conv_launch_fused(self._h, x, w, bias, residual, y, workspace, workspace_bytes, stream)
         if status:
             check(status)
 
@@ -275,25 +282,37 @@ def prepack_weights(src: int, dst: int, out_channels: int, channels: int, rs: in
 def rmsnorm_forward(rows: int, hidden: int, eps: float, dtype: int, x: int, gamma: int, y: int, residual_in: int | None = None,
                     residual_out: int | None = None, stream: int = 0, gamma_fp32: bool = False) -> None:
     """gie::rmsnorm_forward on raw device pointers; dtype uses gie::DataType order (0 fp32, 1 fp16, 2 bf16)."""
-    status = (_calls or calls()).rmsnorm_launch(rows, hidden, eps, dtype, 1 if gamma_fp32 else 0, x, gamma, y, residual_in, residual_out, stream)
+    try:
+        status = (_calls or calls()).rmsnorm_launch(rows, hidden, eps, dtype, 1 if gamma_fp32 else 0, x, gamma, y, residual_in, residual_out, stream)
+    except TypeError:
+        d = RmsNormDesc(rows, hidden, eps, dtype, 1 if gamma_fp32 else 0)
+        status = lib().gieb_rmsnorm_launch(C.byref(d), x, gamma, y, residual_in, residual_out, stream)
     if status:
         check(status)
 
 
+def _glue(name: str, *args) -> None:
+    try:
+        status = getattr(calls(), name)(*args)
+    except TypeError:
+        status = getattr(lib(), "gieb_" + name)(*args)
+    check(status)
+
+
 def bias_act(precision: int, batch: int, channels: int, hw: int, bias: int | None, relu: bool, y: int, stream: int = 0) -> None:
-    check(calls().bias_act_launch(precision, batch, channels, hw, bias, int(relu), y, stream))
+    _glue("bias_act_launch", precision, batch, channels, hw, bias, int(relu), y, stream)
 
 
 def maxpool2d(precision: int, batch: int, channels: int, h: int, w: int, kernel: int, stride: int, pad: int, x: int, y: int,
               stream: int = 0) -> None:
-    check(calls().maxpool2d_launch(precision, batch, channels, h, w, kernel, stride, pad, x, y, stream))
+    _glue("maxpool2d_launch", precision, batch, channels, h, w, kernel, stride, pad, x, y, stream)
 
 
 def maxpool2d_nhwc(precision: int, batch: int, channels: int, h: int, w: int, kernel: int, stride: int, pad: int, x: int, y: int,
                    stream: int = 0) -> None:
     """maxpool2d on channel-contiguous [B][H][W][C] tensors (fp16 / bf16, C % 8 == 0)."""
-    check(calls().maxpool2d_nhwc_launch(precision, batch, channels, h, w, kernel, stride, pad, x, y, stream))
+    _glue("maxpool2d_nhwc_launch", precision, batch, channels, h, w, kernel, stride, pad, x, y, stream)
 
 
 def add_relu(precision: int, relu: bool, a: int, b: int, y: int, n: int, stream: int = 0) -> None:
-    check(calls().add_relu_launch(precision, int(relu), a, b, y, n, stream))
+    _glue("add_relu_launch", precision, int(relu), a, b, y, n, stream)

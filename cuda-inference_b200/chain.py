@@ -5,6 +5,7 @@ Device buffers come from torch (plumbing only); every kernel that runs is this l
 one GPU; multi-GPU runs are independent replicas over a batch shard (no collective, no peer access)."""
 from __future__ import annotations
 
+import ctypes
 import math
 
 from . import (ConvPlan, ConvProblem, GieError, calls, check, make_cfg, FLAG_INPUT_NHWC, FLAG_OUTPUT_NHWC, FLAG_RESIDUAL,
@@ -233,6 +234,8 @@ class ConvChain:
         """All launches of one forward pass on `stream` (capture-safe: no allocation, no synchronisation)."""
         if self._recorded != self._recordable() or self._recorded_ops != self.ops:
             self._steps = self._record()
+        if not isinstance(stream, int):  # what ctypes takes for a pointer (a stream object, a c_void_p, None)
+            stream = ctypes.cast(stream, ctypes.c_void_p).value
         check(calls().run_sequence(self._steps, stream))
 
     def capture(self, stream) -> None:

@@ -13,7 +13,8 @@
 
 namespace {
 
-// What ctypes takes for a void* that is kept as a number: an int, None, or an object with such a `value` (c_void_p).
+// Pointers are ints or None and counts are ints, nothing else: for any other argument the callers in __init__.py go through
+// ctypes, whose conversions (objects with `_as_parameter_`, c_void_p, numpy integers for counts, ..) and refusals then apply.
 bool to_pointer(PyObject* o, void** out) {
   if (PyLong_Check(o)) {
     *out = reinterpret_cast<void*>(static_cast<uintptr_t>(PyLong_AsUnsignedLongLongMask(o)));
@@ -23,22 +24,16 @@ bool to_pointer(PyObject* o, void** out) {
     *out = nullptr;
     return true;
   }
-  PyObject* v = PyIndex_Check(o) ? PyNumber_Index(o) : PyObject_GetAttrString(o, "value");
-  if (v != nullptr && (PyLong_Check(v) || v == Py_None)) {
-    const bool ok = to_pointer(v, out);
-    Py_DECREF(v);
-    return ok;
-  }
-  Py_XDECREF(v);
   PyErr_Format(PyExc_TypeError, "expected a device pointer (int or None), got %.100s", Py_TYPE(o)->tp_name);
   return false;
 }
 
 bool to_int(PyObject* o, long long* out) {
-  PyObject* v = PyLong_Check(o) ? Py_NewRef(o) : PyNumber_Index(o);
-  if (v == nullptr) return false;
-  *out = static_cast<long long>(PyLong_AsUnsignedLongLongMask(v));
-  Py_DECREF(v);
+  if (!PyLong_Check(o)) {
+    PyErr_Format(PyExc_TypeError, "expected an int, got %.100s", Py_TYPE(o)->tp_name);
+    return false;
+  }
+  *out = static_cast<long long>(PyLong_AsUnsignedLongLongMask(o));
   return !PyErr_Occurred();
 }
 

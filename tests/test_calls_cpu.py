@@ -149,3 +149,112 @@ def test_closed_plan_in_a_recorded_pass_is_an_error(pkg):
     with pytest.raises(pkg.GieError) as e:
         c.enqueue(0)
     assert e.value.code == pkg.INVALID_ARGUMENT
+
+
+class Stream:
+    """What torch.cuda.Stream is to a foreign-function call."""
+
+    def __init__(self, value):
+        import ctypes
+        self._as_parameter_ = ctypes.c_void_p(value)
+
+
+def entry_points(pkg):
+    """Every call of the extension module through its wrapper, with one argument left open and one fault that the C side reports
+    before it touches a device (a null plan, no rows, a null tensor)."""
+    closed = pkg.ConvPlan.__new__(pkg.ConvPlan)
+    import ctypes
+    closed._h, closed._plan = ctypes.c_void_p(), None
+    return {
+        "launch": lambda v: closed.launch(v, 256, None, 256, None, 0, 0),
+        "launch stream": lambda v: closed.launch(256, 256, None, 256, None, 0, v),
+        "launch_fused": lambda v: closed.launch_fused(256, 256, None, v, 256, None, 0, 0),
+        "rmsnorm": lambda v: pkg.rmsnorm_forward(0, 64, 1e-6, 2, v, 256, 256, stream=0),
+        "rmsnorm stream": lambda v: pkg.rmsnorm_forward(0, 64, 1e-6, 2, 256, 256, 256, stream=v),
+        "bias_act": lambda v: pkg.bias_act(pkg.FP16, 0, 4, 4, v, True, 256, 0),
+        "maxpool2d": lambda v: pkg.maxpool2d(pkg.FP16, 0, 4, 8, 8, 3, 2, 1, v, 256, 0),
+        "maxpool2d_nhwc": lambda v: pkg.maxpool2d_nhwc(pkg.FP16, 0, 8, 8, 8, 3, 2, 1, v, 256, 0),
+        "add_relu": lambda v: pkg.add_relu(pkg.FP16, True, v, 256, 256, -1, 0),
+    }
+
+
+NAMES = ["launch", "launch stream", "launch_fused", "rmsnorm", "rmsnorm stream", "bias_act", "maxpool2d", "maxpool2d_nhwc", "add_relu"]
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_pointer_arguments_are_those_of_ctypes(pkg, name):
+    """Accepted: ints, None, objects with _as_parameter_, c_void_p.  Refused: floats, numpy integers, other objects."""
+    import ctypes
+
+    import numpy as np
+    call = entry_points(pkg)[name]
+    for v in (256, True, None, Stream(256), Stream(None), ctypes.c_void_p(256), ctypes.c_void_p()):
+        with pytest.raises(pkg.GieError) as e:
+            call(v)
+        assert e.value.code == pkg.INVALID_ARGUMENT, (name, v)
+    for v in (1.0, np.int64(256), object(), [256]):
+        with pytest.raises(ctypes.ArgumentError):
+            call(v)
+
+
+def test_counts_are_those_of_ctypes(pkg):
+    import ctypes
+
+    import numpy as np
+    for rows in (0, np.int32(0), False):
+        with pytest.raises(pkg.GieError) as e:
+            pkg.rmsnorm_forward(rows, 64, np.float32(1e-6), 2, 256, 256, 256)
+        assert e.value.code == pkg.INVALID_ARGUMENT
+    for rows in (1.0, None, "1"):
+        with pytest.raises(TypeError):
+            pkg.rmsnorm_forward(rows, 64, 1e-6, 2, 256, 256, 256)
+    with pytest.raises(TypeError):
+        pkg.rmsnorm_forward(0, 64, "eps", 2, 256, 256, 256)
+    with pytest.raises(ctypes.ArgumentError):
+        pkg.add_relu(pkg.FP16, True, 256, 256, 256, 1.5)
+
+
+def test_recorded_pass_takes_stream_objects(pkg, fake):
+    import ctypes
+    c = small_chain(pkg)
+    c._steps = c._record()
+    streams = []
+    fake.run_sequence = lambda steps, stream: streams.append(stream)
+    for s in (512, Stream(512), ctypes.c_void_p(512), None, Stream(None)):
+        c.enqueue(s)
+    assert streams == [512, 512, 512, None, None]
+    with pytest.raises(ctypes.ArgumentError):
+        c.enqueue(1.5)
+
+
+def test_extension_module_reports_its_own_errors(pkg):
+    calls = pkg.calls()
+    with pytest.raises(TypeError, match="8 arguments, got 2"):
+        calls.conv_launch(None, 1)
+    with pytest.raises(TypeError, match="device pointer"):
+        calls.conv_launch(None, 1.5, None, None, None, None, 0, None)
+    with pytest.raises(TypeError, match="an int"):
+        calls.conv_launch(None, None, None, None, None, None, None, None)
+    assert calls.conv_launch(None, None, None, None, None, None, 0, None) == pkg.INVALID_ARGUMENT and pkg.last_error()
+    with pytest.raises(ValueError, match="unknown call gemm"):
+        calls.record([("gemm", 1)])
+    with pytest.raises(TypeError, match="arguments"):
+        calls.record([("add_relu_launch", 1, 1)])
+    for bad in ([()], [(7, 1)], [("add_relu_launch", 1, 1, 1.5, 1, 1, 1)]):
+        with pytest.raises((TypeError, ValueError)):
+            calls.record(bad)
+    for bad in (5, None):
+        with pytest.raises(TypeError):
+            calls.record(bad)
+    with pytest.raises(TypeError, match="2 arguments"):
+        calls.run_sequence(calls.record([]))
+    with pytest.raises(ValueError):
+        calls.run_sequence(object(), 0)
+    assert calls.run_sequence(calls.record([]), 0) is None
+    # the first failing step ends the pass with its own status: a null tensor, then a precision that does not exist
+    null_add = ("add_relu_launch", pkg.FP16, 1, None, None, None, 16)
+    null_plan = ("conv_launch", None, 256, 256, None, 256, None, 0)
+    assert calls.run_sequence(calls.record([null_add, null_plan]), 0) == pkg.INVALID_ARGUMENT
+    first = pkg.last_error()
+    assert calls.run_sequence(calls.record([null_plan, null_add]), 0) == pkg.INVALID_ARGUMENT
+    assert pkg.last_error() != first
