@@ -332,6 +332,7 @@ bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, const gieb_conv_cf
   if (r->variant != 1 || taps == 1) return false;
   if (d.stride_h > 2 || d.stride_w > 2 || d.pad_h > d.kernel_h - 1 || d.pad_w > d.kernel_w - 1) return false;
   if (g.pq < 16 || taps > 64) return false;
+  if ((d.flags & GIEB_FLAG_OUTPUT_NHWC) && g.y_elems > int64_t(8) * 0xffffffffLL) return false;  // (row offsets are 32-bit counts of 16-byte cells)
   const int ph = d.stride_h < d.kernel_h ? d.stride_h : d.kernel_h, pw = d.stride_w < d.kernel_w ? d.stride_w : d.kernel_w;
   // stride 1: neighbours share their padding; larger strides: a row of a phase holds every position that some tap reads
   const int ws = d.stride_w == 1 ? d.in_w + d.pad_w : g.out_w + (d.kernel_w - 1) / d.stride_w;

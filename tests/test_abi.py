@@ -298,3 +298,14 @@ def test_halo_variant_takes_and_refuses(pkg):
         assert not pkg.query(P(pkg, *a, precision=pkg.FP16), pkg.make_cfg(variant=6)).supported, a
     assert not pkg.query(P(pkg, 1, 64, 14, 14, 64, 3, 3, 1, 1, 1, 1, precision=pkg.TF32), pkg.make_cfg(variant=6, cta_pair=2)).supported
     assert not pkg.query(P(pkg, 1, 64, 14, 14, 64, 3, 3, 1, 1, 1, 1, precision=pkg.FP32), pkg.make_cfg(variant=6)).supported
+
+
+def test_halo_variant_leaves_outputs_beyond_its_row_offsets(pkg):
+    """Rows of a channel-contiguous output are addressed by 32-bit counts of 16-byte cells: 64 GiB and no more."""
+    flags = pkg.FLAG_INPUT_NHWC | pkg.FLAG_OUTPUT_NHWC | pkg.FLAG_WEIGHTS_PREPACKED
+    for o, flag, fits in [(16, flags, True), (24, flags, True), (32, flags, False), (64, flags, False), (64, pkg.FLAG_INPUT_NHWC | pkg.FLAG_WEIGHTS_PREPACKED, True)]:
+        p = P(pkg, 65536, 16, 128, 128, o, 3, 3, 1, 1, 1, 1, precision=pkg.FP16, has_bias=True, relu=True, flags=flag)
+        i = pkg.query(p, pkg.make_cfg(variant=6))
+        assert bool(i.supported) == fits, o
+        auto = pkg.query(p)
+        assert auto.supported and (fits or auto.cfg.variant != 6)
