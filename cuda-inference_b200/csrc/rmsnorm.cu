@@ -259,7 +259,8 @@ cudaError_t run(int rows, int hidden, float eps, const void* x, const void* gamm
   }
   int threads = 32;
   while (threads < hidden && threads < 1024) threads <<= 1;
-  const int staged = hidden <= 12 * 1024 ? hidden : 0;  // <= 48 KiB of dynamic shared memory (no opt-in needed)
+  constexpr int kStagedMax = (48 * 1024 - 32 * int(sizeof(float))) / int(sizeof(float));  // 48 KiB need no opt-in, the kernel's own `red` included
+  const int staged = hidden <= kStagedMax ? hidden : 0;
   return launch_pdl(rmsnorm_generic_kernel<T, FUSED, GAMMA_F32>, dim3(unsigned(rows)), dim3(unsigned(threads)), size_t(staged) * sizeof(float), st, xp,
                     gamma, yp, ri, ro, hidden, eps, staged);
 }

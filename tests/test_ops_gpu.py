@@ -71,6 +71,20 @@ def test_rmsnorm_misaligned_and_options(pkg, orc, oracle):
     _rms_case(pkg, orc, oracle, 4, 4096, 2, True, 10, alias_res=True)  # residual_out may alias x (rmsnorm.h:26)
 
 
+@pytest.mark.parametrize("rows,hidden", [(1190, 128), (1190, 129), (2400, 500), (300, 512), (1190, 72), (300, 1001), (300, 4095), (310, 8190), (300, 12001), (40, 20003)])
+def test_rmsnorm_many_rows(pkg, orc, oracle, rows, hidden):
+    """Eight, four and two rows to a CTA; rows shifted within their vectors with one, two, four and eight vectors a thread."""
+    for dt, fused in ((0, True), (1, False), (2, True)):
+        _rms_case(pkg, orc, oracle, rows, hidden, dt, fused, seed=rows + hidden + dt)
+
+
+def test_rmsnorm_longest_staged_rows(pkg, orc, oracle):
+    """Tensors off their alignment: the row is kept in shared memory up to what a launch may have without asking."""
+    for hidden in (12224, 12256, 12257, 12280, 12288, 12289):
+        _rms_case(pkg, orc, oracle, 3, hidden, 2, True, seed=hidden, off=1)
+        _rms_case(pkg, orc, oracle, 3, hidden, 0, False, seed=hidden + 1, off=1)
+
+
 def test_rmsnorm_full_size_benchmark_shape(pkg, orc, oracle):
     """8192 x 4096 BF16 with residual: gamma = 1 + N(0, 0.02), activations N(0,1), eps 1e-6."""
     import torch
