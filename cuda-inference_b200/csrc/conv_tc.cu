@@ -5,20 +5,6 @@
 namespace gieb {
 namespace {
 
-template <int BN, int BK, int MH, int EW>
-cudaError_t prepare_one(size_t smem_bytes) {
-  return cudaFuncSetAttribute(conv_tc_kernel<BN, BK, MH, EW, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_bytes));
-}
-
-template <int BN, int BK, int MH, int EW>
-cudaError_t launch_one(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& to, const CUtensorMap& tr, const ConvTcParams& p,
-                       dim3 grid, size_t smem, cudaStream_t st) {
-  cudaError_t e = launch_pdl_cluster(conv_tc_kernel<BN, BK, MH, EW, false>, grid, dim3(32 * (kProducerWarps + 1 + EW)), smem, st,
-                                     unsigned(p.cluster_split > 1 ? p.cluster_split : 1), ta, tw, to, tr, p);
-  if (e != cudaSuccess) return e;
-  return cudaGetLastError();
-}
-
 #define GIEB_TC_DISPATCH(FN, ...) \
   switch (tile_m / 128 * 100000 + tile_n * 100 + tile_k) { \
     case 1 * 100000 + 32 * 100 + 16: return FN<32, 16, 1, 8>(__VA_ARGS__); \
@@ -125,14 +111,14 @@ size_t conv_tc_smem_bytes(int tile_m, int tile_n, int tile_k, int stages, size_t
 
 cudaError_t conv_tc_prepare(int tile_m, int tile_n, int tile_k, int epi_warps, size_t smem_bytes) {
   if (tile_n >= 128) return conv_tc_wide_prepare(tile_m, tile_n, tile_k, epi_warps, smem_bytes);
-  GIEB_TC_DISPATCH(prepare_one, smem_bytes)
+  GIEB_TC_DISPATCH(prepare_point, smem_bytes)
 }
 
 cudaError_t conv_tc_launch(int tile_m, int tile_n, int tile_k, int epi_warps, const CUtensorMap& tm_act, const CUtensorMap& tm_wgt,
                            const CUtensorMap& tm_out, const CUtensorMap& tm_res, const ConvTcParams& p, dim3 grid, size_t smem_bytes,
                            cudaStream_t stream) {
   if (tile_n >= 128) return conv_tc_wide_launch(tile_m, tile_n, tile_k, epi_warps, tm_act, tm_wgt, tm_out, tm_res, p, grid, smem_bytes, stream);
-  GIEB_TC_DISPATCH(launch_one, tm_act, tm_wgt, tm_out, tm_res, p, grid, smem_bytes, stream)
+  GIEB_TC_DISPATCH(launch_point, tm_act, tm_wgt, tm_out, tm_res, p, grid, smem_bytes, stream)
 }
 
 cudaError_t splitk_reduce_launch(const float* partial, int splits, int64_t total, int out_channels, int pq, const void* bias,

@@ -1067,5 +1067,22 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
   }
 }
 
+// One point of the family: its opt-in to large dynamic shared memory, and its launch.  Clusters are CTA pairs (blockIdx.x =
+// 2 * pair + rank) or the split-K slices of a tile.
+template <int BN, int BK, int MH, int EW, bool PAIR = false, bool SWAP = false>
+cudaError_t prepare_point(size_t smem_bytes) {
+  return cudaFuncSetAttribute(conv_tc_kernel<BN, BK, MH, EW, PAIR, SWAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_bytes));
+}
+
+template <int BN, int BK, int MH, int EW, bool PAIR = false, bool SWAP = false>
+cudaError_t launch_point(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& to, const CUtensorMap& tr, const ConvTcParams& p,
+                         dim3 grid, size_t smem, cudaStream_t st) {
+  const unsigned cluster = PAIR ? 2u : unsigned(p.cluster_split > 1 ? p.cluster_split : 1);
+  const cudaError_t e = launch_pdl_cluster(conv_tc_kernel<BN, BK, MH, EW, PAIR, SWAP>, grid, dim3(32 * (kProducerWarps + 1 + EW)), smem, st,
+                                           cluster, ta, tw, to, tr, p);
+  if (e != cudaSuccess) return e;
+  return cudaGetLastError();
+}
+
 }  // namespace
 }  // namespace gieb

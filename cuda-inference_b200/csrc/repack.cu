@@ -720,10 +720,10 @@ Tf32Job make_tf32_job(const void* src, void* dst, int batch, int channels, int h
 // 1-byte elements (FP8 bit patterns): [B][C][HW] -> [B][HW][Cp], channels zero-padded to Cp (a multiple of 32).  Pure data
 // movement, bit-exact.  Up to two tensors per launch (activations and weights), like repack_jobs_kernel, and the same
 // two shapes of work:
-//   tile mode: one CTA transposes a 64-channel x PX-pixel tile (PX 128 where that leaves more than a wave of blocks, else 64): 4-byte loads along the pixels (a row that starts inside a word is
-//     shifted into place by a shuffle and a funnel shift), bytes transposed in registers, 8-byte stores of 8 consecutive
-//     channels.  Bound by its instruction count: with 1-byte reads of a 64 x 64 tile the copy
-//     of 160 x 64 x 44 x 27 took 12.8 us, now 9.7;
+//   tile mode: one CTA transposes a 64-channel x PX-pixel tile (PX 128 where that leaves more than a wave of blocks, else 64):
+//     4-byte loads along the pixels (a row that starts inside a word is shifted into place by a shuffle and a funnel shift),
+//     bytes transposed in registers, 8-byte stores of 8 consecutive channels.  Bound by its instruction count: with 1-byte
+//     reads of a 64 x 64 tile the copy of 160 x 64 x 44 x 27 took 12.8 us, now 9.7;
 //   slab mode (planes of at most 16 elements: filter taps): one CTA takes `span` channels of one batch entry; the source
 //     slab [span][HW] is contiguous and is read linearly, then written as [HW][span].
 // Both prefetch their source lines into L2 before the dependency wait (see repack_jobs_kernel).
@@ -807,24 +807,24 @@ __global__ void __launch_bounds__(256) repack_bytes_kernel(const ByteJob a, cons
     for (int i = 0; i < PASSES; ++i) words[(row0 + i * ROWS) * PITCH + lane] = word[i];
   } else {
 #pragma unroll
-  for (int i = 0; i < PASSES; ++i) {
-    const int ch = row0 + i * ROWS;
-    const uint8_t* r = s + size_t(ch) * j.HW;
-    const int off = int(reinterpret_cast<uintptr_t>(r) & 3u);
-    word[i] = last[i] = 0;
-    if (c0 + ch < j.C && px0 + 4 * lane - off < j.HW) {
-      word[i] = load_word_within(r - off + 4 * lane, j.src, end);
-      if (off != 0 && lane == LANES - 1) last[i] = load_word_within(r - off + PX, j.src, end);
+    for (int i = 0; i < PASSES; ++i) {
+      const int ch = row0 + i * ROWS;
+      const uint8_t* r = s + size_t(ch) * j.HW;
+      const int off = int(reinterpret_cast<uintptr_t>(r) & 3u);
+      word[i] = last[i] = 0;
+      if (c0 + ch < j.C && px0 + 4 * lane - off < j.HW) {
+        word[i] = load_word_within(r - off + 4 * lane, j.src, end);
+        if (off != 0 && lane == LANES - 1) last[i] = load_word_within(r - off + PX, j.src, end);
+      }
     }
-  }
 #pragma unroll
-  for (int i = 0; i < PASSES; ++i) {
-    const int ch = row0 + i * ROWS;
-    const int off = int(reinterpret_cast<uintptr_t>(s + size_t(ch) * j.HW) & 3u);
-    uint32_t next = __shfl_down_sync(0xffffffffu, word[i], 1, LANES);
-    if (lane == LANES - 1) next = last[i];
-    words[ch * PITCH + lane] = __funnelshift_r(word[i], next, 8 * off);
-  }
+    for (int i = 0; i < PASSES; ++i) {
+      const int ch = row0 + i * ROWS;
+      const int off = int(reinterpret_cast<uintptr_t>(s + size_t(ch) * j.HW) & 3u);
+      uint32_t next = __shfl_down_sync(0xffffffffu, word[i], 1, LANES);
+      if (lane == LANES - 1) next = last[i];
+      words[ch * PITCH + lane] = __funnelshift_r(word[i], next, 8 * off);
+    }
   }
   __syncthreads();
   const int cg = t & 7;  // 8 channels
@@ -880,7 +880,8 @@ cudaError_t repack_bytes_pair_launch(const void* src_a, void* dst_a, int batch_a
   const ByteJob a = make_byte_job(src_a, dst_a, batch_a, ch_a, hw_a, cp_a, wide ? 128 : 64);
   const ByteJob b = make_byte_job(src_b, dst_b, batch_b, ch_b, hw_b, cp_b, wide ? 128 : 64);
   // (shared memory nobody uses keeps a small job at six blocks per SM: see launch_jobs)
-  const cudaError_t e = launch_pdl(wide ? repack_bytes_kernel<128> : repack_bytes_kernel<64>, dim3(a.blocks + b.blocks), dim3(256), wide ? 0 : 28 * 1024, stream, a, b, prefetch_enabled() ? 1 : 0);
+  const cudaError_t e = launch_pdl(wide ? repack_bytes_kernel<128> : repack_bytes_kernel<64>, dim3(a.blocks + b.blocks), dim3(256),
+                                   wide ? 0 : 28 * 1024, stream, a, b, prefetch_enabled() ? 1 : 0);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();
 }
