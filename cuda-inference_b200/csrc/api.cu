@@ -1197,6 +1197,22 @@ int launch_impl(const gieb_conv_plan* pl, const void* x, const void* w, const vo
   return GIEB_OK;
 }
 
+// Opts every kernel that launches of this configuration may take in to large dynamic shared memory.
+cudaError_t prepare_kernels(const Resolved& r) {
+  if (r.variant == 3) return cudaSuccess;
+  if (r.halo) return conv_halo_prepare(r.tile_n, r.epi_warps, r.pair != 0, kMaxDynamicSmem);
+  // The general kernel: a partial last slab, or rows that TMA cannot store (which tensors off their alignment are as well).
+  const bool tail = r.tile_k == 64 && r.c_padded % 64 != 0;
+  for (int general = 0; general < 2; ++general) {
+    if (general ? !(tail || r.row_epilogue || r.tma_epilogue) : (tail || r.row_epilogue)) continue;
+    const cudaError_t e = r.swap   ? conv_tc_swap_prepare(r.tile_m, r.tile_n, r.tile_k, general != 0, kMaxDynamicSmem)
+                          : r.pair ? conv_tc_pair_prepare(r.tile_n, r.tile_k, general != 0, kMaxDynamicSmem)
+                                   : conv_tc_prepare(r.tile_m, r.tile_n, r.tile_k, r.epi_warps, general != 0, kMaxDynamicSmem);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1264,11 +1280,7 @@ int gieb_conv_plan_create(const gieb_conv_desc* desc, const gieb_conv_cfg* cfg, 
       cudaStreamDestroy(s);
     }
   }
-  if (e == cudaSuccess && r.variant != 3)
-    e = r.halo ? conv_halo_prepare(r.tile_n, r.epi_warps, r.pair != 0, kMaxDynamicSmem)
-        : r.swap ? conv_tc_swap_prepare(r.tile_m, r.tile_n, r.tile_k, kMaxDynamicSmem)
-        : r.pair ? conv_tc_pair_prepare(r.tile_n, r.tile_k, kMaxDynamicSmem)
-                 : conv_tc_prepare(r.tile_m, r.tile_n, r.tile_k, r.epi_warps, kMaxDynamicSmem);
+  if (e == cudaSuccess) e = prepare_kernels(r);
   if (e != cudaSuccess) {
     if (pl->d_status) cudaFree(pl->d_status);
     delete pl;
@@ -1417,11 +1429,7 @@ int gieb_conv_forward_static(const gieb_conv_desc* desc, const gieb_conv_cfg* cf
   if (cc_major != 10) return fail(GIEB_UNSUPPORTED, "this library contains sm_100a code only; device %d has compute capability %d.x", pl.device, cc_major);
   pl.d_status = reinterpret_cast<uint32_t*>(base);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (pl.r.variant != 3)
-    GIEB_CUDA(pl.r.halo ? conv_halo_prepare(pl.r.tile_n, pl.r.epi_warps, pl.r.pair != 0, kMaxDynamicSmem)
-              : pl.r.swap ? conv_tc_swap_prepare(pl.r.tile_m, pl.r.tile_n, pl.r.tile_k, kMaxDynamicSmem)
-              : pl.r.pair ? conv_tc_pair_prepare(pl.r.tile_n, pl.r.tile_k, kMaxDynamicSmem)
-                          : conv_tc_prepare(pl.r.tile_m, pl.r.tile_n, pl.r.tile_k, pl.r.epi_warps, kMaxDynamicSmem));
+  GIEB_CUDA(prepare_kernels(pl.r));
   // The array keeps whatever the previous call left: the status word must start at zero.  Everything else in the
   // scratch is fully rewritten by the repack kernels (padding channels included) and the split-K slices before use.
   GIEB_CUDA(cudaMemsetAsync(base, 0, kStaticScratchHeader, s));

@@ -1,5 +1,5 @@
 // Instantiations and host-side dispatch of the single-CTA points of the tensor-core convolution kernel
-// (conv_tc_kernel.cuh; those of 128 and 256 channels are in conv_tc_wide.cu), and the split-K reduction kernel.
+// (conv_tc_kernel.cuh; those of 128 and 256 channels are in conv_tc_wide.cu and conv_tc_wide16.cu), and the split-K reduction kernel.
 #include "conv_tc_kernel.cuh"
 
 namespace gieb {
@@ -7,18 +7,18 @@ namespace {
 
 #define GIEB_TC_DISPATCH(FN, ...) \
   switch (tile_m / 128 * 100000 + tile_n * 100 + tile_k) { \
-    case 1 * 100000 + 32 * 100 + 16: return FN<32, 16, 1, 8>(__VA_ARGS__); \
-    case 2 * 100000 + 32 * 100 + 16: return FN<32, 16, 2, 8>(__VA_ARGS__); \
-    case 1 * 100000 + 32 * 100 + 32: return FN<32, 32, 1, 8>(__VA_ARGS__); \
-    case 2 * 100000 + 32 * 100 + 32: return FN<32, 32, 2, 8>(__VA_ARGS__); \
-    case 1 * 100000 + 32 * 100 + 64: return FN<32, 64, 1, 8>(__VA_ARGS__); \
-    case 2 * 100000 + 32 * 100 + 64: return FN<32, 64, 2, 8>(__VA_ARGS__); \
-    case 1 * 100000 + 64 * 100 + 16: return FN<64, 16, 1, 8>(__VA_ARGS__); \
-    case 2 * 100000 + 64 * 100 + 16: return FN<64, 16, 2, 8>(__VA_ARGS__); \
-    case 1 * 100000 + 64 * 100 + 32: return FN<64, 32, 1, 8>(__VA_ARGS__); \
-    case 2 * 100000 + 64 * 100 + 32: return FN<64, 32, 2, 8>(__VA_ARGS__); \
-    case 1 * 100000 + 64 * 100 + 64: return FN<64, 64, 1, 8>(__VA_ARGS__); \
-    case 2 * 100000 + 64 * 100 + 64: return FN<64, 64, 2, 8>(__VA_ARGS__); \
+    case 1 * 100000 + 32 * 100 + 16: GIEB_TC_EITHER(FN, 32, 16, 1, 8, false, false, __VA_ARGS__); \
+    case 2 * 100000 + 32 * 100 + 16: GIEB_TC_EITHER(FN, 32, 16, 2, 8, false, false, __VA_ARGS__); \
+    case 1 * 100000 + 32 * 100 + 32: GIEB_TC_EITHER(FN, 32, 32, 1, 8, false, false, __VA_ARGS__); \
+    case 2 * 100000 + 32 * 100 + 32: GIEB_TC_EITHER(FN, 32, 32, 2, 8, false, false, __VA_ARGS__); \
+    case 1 * 100000 + 32 * 100 + 64: GIEB_TC_EITHER(FN, 32, 64, 1, 8, false, false, __VA_ARGS__); \
+    case 2 * 100000 + 32 * 100 + 64: GIEB_TC_EITHER(FN, 32, 64, 2, 8, false, false, __VA_ARGS__); \
+    case 1 * 100000 + 64 * 100 + 16: GIEB_TC_EITHER(FN, 64, 16, 1, 8, false, false, __VA_ARGS__); \
+    case 2 * 100000 + 64 * 100 + 16: GIEB_TC_EITHER(FN, 64, 16, 2, 8, false, false, __VA_ARGS__); \
+    case 1 * 100000 + 64 * 100 + 32: GIEB_TC_EITHER(FN, 64, 32, 1, 8, false, false, __VA_ARGS__); \
+    case 2 * 100000 + 64 * 100 + 32: GIEB_TC_EITHER(FN, 64, 32, 2, 8, false, false, __VA_ARGS__); \
+    case 1 * 100000 + 64 * 100 + 64: GIEB_TC_EITHER(FN, 64, 64, 1, 8, false, false, __VA_ARGS__); \
+    case 2 * 100000 + 64 * 100 + 64: GIEB_TC_EITHER(FN, 64, 64, 2, 8, false, false, __VA_ARGS__); \
     default: return cudaErrorInvalidValue;                                            \
   }
 
@@ -109,15 +109,20 @@ size_t conv_tc_smem_bytes(int tile_m, int tile_n, int tile_k, int stages, size_t
   return bytes + 1024 <= kCtaSmemLimit ? bytes + 1024 : bytes;  // a KiB of reserve that a ring filling the last byte does without
 }
 
-cudaError_t conv_tc_prepare(int tile_m, int tile_n, int tile_k, int epi_warps, size_t smem_bytes) {
-  if (tile_n >= 128) return conv_tc_wide_prepare(tile_m, tile_n, tile_k, epi_warps, smem_bytes);
+bool conv_tc_general(const ConvTcParams& p, int tile_k) { return p.out_rows != 0 || (tile_k == 64 && p.last_ksteps != 4); }
+
+cudaError_t conv_tc_prepare(int tile_m, int tile_n, int tile_k, int epi_warps, bool general, size_t smem_bytes) {
+  if (tile_n >= 128 && epi_warps == 16) return conv_tc_wide16_prepare(tile_m, tile_n, tile_k, general, smem_bytes);
+  if (tile_n >= 128) return conv_tc_wide_prepare(tile_m, tile_n, tile_k, general, smem_bytes);
   GIEB_TC_DISPATCH(prepare_point, smem_bytes)
 }
 
 cudaError_t conv_tc_launch(int tile_m, int tile_n, int tile_k, int epi_warps, const CUtensorMap& tm_act, const CUtensorMap& tm_wgt,
                            const CUtensorMap& tm_out, const CUtensorMap& tm_res, const ConvTcParams& p, dim3 grid, size_t smem_bytes,
                            cudaStream_t stream) {
-  if (tile_n >= 128) return conv_tc_wide_launch(tile_m, tile_n, tile_k, epi_warps, tm_act, tm_wgt, tm_out, tm_res, p, grid, smem_bytes, stream);
+  const bool general = conv_tc_general(p, tile_k);
+  if (tile_n >= 128 && epi_warps == 16) return conv_tc_wide16_launch(tile_m, tile_n, tile_k, general, tm_act, tm_wgt, tm_out, tm_res, p, grid, smem_bytes, stream);
+  if (tile_n >= 128) return conv_tc_wide_launch(tile_m, tile_n, tile_k, general, tm_act, tm_wgt, tm_out, tm_res, p, grid, smem_bytes, stream);
   GIEB_TC_DISPATCH(launch_point, tm_act, tm_wgt, tm_out, tm_res, p, grid, smem_bytes, stream)
 }
 

@@ -320,7 +320,10 @@ __device__ __forceinline__ void with_output_type(const ConvTcParams& p, F&& f) {
 // contiguous bytes of an NCHW tensor: the warp stages its 32 channels x 32 pixels as one box and a TMA store writes it
 // (tensor {P*Q, O, N}); for NCHW output whose planes are 16-byte multiples.  BN 128 or 256, 16-bit types, no split-K,
 // no pair.
-template <int BN, int BK, int MH, int EW, bool PAIR, bool SWAP = false>
+// GENERAL: with the slab loops over partial last slabs and the row-wise output.  Kernels without them are what a layer takes that
+// needs neither: carried along unused, the two cost every launch 0.2-0.4 us and odd NCHW planes 3-4 % (instruction fetch and
+// spilled registers: 64 -> 288 at 37 x 18, 3x3, 3 images 5.42 us, 5.23 without; 128 -> 284 at 35 x 35, 1x1, 45 images 21.3, 19.9).
+template <int BN, int BK, int MH, int EW, bool PAIR, bool SWAP, bool GENERAL>
 __global__ void __launch_bounds__(32 * (kProducerWarps + 1 + EW), (EW == 16 || PAIR) ? 1 : 2)  // EW = 8: at most 80 registers, two CTAs per SM
 conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__ CUtensorMap tm_wgt,
                const __grid_constant__ CUtensorMap tm_out, const __grid_constant__ CUtensorMap tm_res, const ConvTcParams p) {
@@ -645,7 +648,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
         }
       };
       auto with_tail = [&](auto form_tag) {
-        if (BK == 64 && p.last_ksteps != MMAS_PER_SLAB) slab_loop(form_tag, std::integral_constant<bool, BK == 64>{});
+        if (GENERAL && BK == 64 && p.last_ksteps != MMAS_PER_SLAB) slab_loop(form_tag, std::integral_constant<bool, GENERAL && BK == 64>{});
         else slab_loop(form_tag, std::integral_constant<bool, false>{});
       };
       if (!PAIR && !SWAP && p.is_tf32) with_tail(std::integral_constant<int, 2>{});
@@ -1004,16 +1007,18 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
             }
             continue;
           }
-          if (p.out_rows && rows_pay(p.out_channels - (n0 + chunk * 32), p.out_rows == 2)) {
-            const int nvalid = min(32, p.out_channels - (n0 + chunk * 32));
-            const int64_t off = base + chunk * 32;
-            if (p.is_bf16)
-              store_chunk_rows(v, bias_t + chunk * 32, stage_box(0), lane, static_cast<__nv_bfloat16*>(p.y),
-                               const_cast<__nv_bfloat16*>(static_cast<const __nv_bfloat16*>(p.residual)), off, m_ok, nvalid, p.out_rows == 2, p.relu);
-            else
-              store_chunk_rows(v, bias_t + chunk * 32, stage_box(0), lane, static_cast<__half*>(p.y),
-                               const_cast<__half*>(static_cast<const __half*>(p.residual)), off, m_ok, nvalid, p.out_rows == 2, p.relu);
-            continue;
+          if constexpr (GENERAL) {
+            if (p.out_rows && rows_pay(p.out_channels - (n0 + chunk * 32), p.out_rows == 2)) {
+              const int nvalid = min(32, p.out_channels - (n0 + chunk * 32));
+              const int64_t off = base + chunk * 32;
+              if (p.is_bf16)
+                store_chunk_rows(v, bias_t + chunk * 32, stage_box(0), lane, static_cast<__nv_bfloat16*>(p.y),
+                                 const_cast<__nv_bfloat16*>(static_cast<const __nv_bfloat16*>(p.residual)), off, m_ok, nvalid, p.out_rows == 2, p.relu);
+              else
+                store_chunk_rows(v, bias_t + chunk * 32, stage_box(0), lane, static_cast<__half*>(p.y),
+                                 const_cast<__half*>(static_cast<const __half*>(p.residual)), off, m_ok, nvalid, p.out_rows == 2, p.relu);
+              continue;
+            }
           }
           if (m_ok) {
             const int nvalid = min(32, p.out_channels - (n0 + chunk * 32));
@@ -1069,20 +1074,24 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
 
 // One point of the family: its opt-in to large dynamic shared memory, and its launch.  Clusters are CTA pairs (blockIdx.x =
 // 2 * pair + rank) or the split-K slices of a tile.
-template <int BN, int BK, int MH, int EW, bool PAIR = false, bool SWAP = false>
+template <int BN, int BK, int MH, int EW, bool PAIR, bool SWAP, bool GENERAL>
 cudaError_t prepare_point(size_t smem_bytes) {
-  return cudaFuncSetAttribute(conv_tc_kernel<BN, BK, MH, EW, PAIR, SWAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_bytes));
+  return cudaFuncSetAttribute(conv_tc_kernel<BN, BK, MH, EW, PAIR, SWAP, GENERAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_bytes));
 }
 
-template <int BN, int BK, int MH, int EW, bool PAIR = false, bool SWAP = false>
+template <int BN, int BK, int MH, int EW, bool PAIR, bool SWAP, bool GENERAL>
 cudaError_t launch_point(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& to, const CUtensorMap& tr, const ConvTcParams& p,
                          dim3 grid, size_t smem, cudaStream_t st) {
   const unsigned cluster = PAIR ? 2u : unsigned(p.cluster_split > 1 ? p.cluster_split : 1);
-  const cudaError_t e = launch_pdl_cluster(conv_tc_kernel<BN, BK, MH, EW, PAIR, SWAP>, grid, dim3(32 * (kProducerWarps + 1 + EW)), smem, st,
-                                           cluster, ta, tw, to, tr, p);
+  const cudaError_t e = launch_pdl_cluster(conv_tc_kernel<BN, BK, MH, EW, PAIR, SWAP, GENERAL>, grid, dim3(32 * (kProducerWarps + 1 + EW)), smem,
+                                           st, cluster, ta, tw, to, tr, p);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();
 }
+
+// FN for the general or the lean kernel of a point, by the variable `general` of the caller.
+#define GIEB_TC_EITHER(FN, BN, BK, MH, EW, PAIR, SWAP, ...) \
+  return general ? FN<BN, BK, MH, EW, PAIR, SWAP, true>(__VA_ARGS__) : FN<BN, BK, MH, EW, PAIR, SWAP, false>(__VA_ARGS__)
 
 }  // namespace
 }  // namespace gieb

@@ -193,27 +193,33 @@ size_t conv_tc_smem_bytes(int tile_m, int tile_n, int tile_k, int stages, size_t
 int conv_tc_epilogue_boxes(int tile_n, int epi_warps);  // chunks of 32 channels one epilogue warp owns per 128 pixels
 // epi_warps: 8, or 16 for CTAs that have an SM to themselves (tile_n >= 128 only)
 int conv_tc_threads(int epi_warps);
-cudaError_t conv_tc_prepare(int tile_m, int tile_n, int tile_k, int epi_warps, size_t smem_bytes);  // opt in to large dynamic shared memory
+// general: the kernels with partial last slabs and row-wise output (see conv_tc_kernel); a launch takes them when it needs them
+bool conv_tc_general(const ConvTcParams& p, int tile_k);
+cudaError_t conv_tc_prepare(int tile_m, int tile_n, int tile_k, int epi_warps, bool general, size_t smem_bytes);  // opt in to large dynamic shared memory
 // tm_out / tm_res: the output and the residual as 2-D tensors {channels, pixels} with a 32 x 32 box and 64-byte swizzle;
 // read only when p.out_tma / p.res_tma are set.
 cudaError_t conv_tc_launch(int tile_m, int tile_n, int tile_k, int epi_warps, const CUtensorMap& tm_act, const CUtensorMap& tm_wgt,
                            const CUtensorMap& tm_out, const CUtensorMap& tm_res, const ConvTcParams& p, dim3 grid, size_t smem_bytes,
                            cudaStream_t stream);
-// (their points of 128 and 256 channels, a translation unit of their own)
-cudaError_t conv_tc_wide_prepare(int tile_m, int tile_n, int tile_k, int epi_warps, size_t smem_bytes);
-cudaError_t conv_tc_wide_launch(int tile_m, int tile_n, int tile_k, int epi_warps, const CUtensorMap& tm_act, const CUtensorMap& tm_wgt,
-                                const CUtensorMap& tm_out, const CUtensorMap& tm_res, const ConvTcParams& p, dim3 grid, size_t smem_bytes,
-                                cudaStream_t stream);
+// (their points of 128 and 256 channels with 8 and with 16 epilogue warps, translation units of their own)
+cudaError_t conv_tc_wide_prepare(int tile_m, int tile_n, int tile_k, bool general, size_t smem_bytes);
+cudaError_t conv_tc_wide_launch(int tile_m, int tile_n, int tile_k, bool general, const CUtensorMap& tm_act, const CUtensorMap& tm_wgt,
+                              const CUtensorMap& tm_out, const CUtensorMap& tm_res, const ConvTcParams& p, dim3 grid, size_t smem_bytes,
+                              cudaStream_t stream);
+cudaError_t conv_tc_wide16_prepare(int tile_m, int tile_n, int tile_k, bool general, size_t smem_bytes);
+cudaError_t conv_tc_wide16_launch(int tile_m, int tile_n, int tile_k, bool general, const CUtensorMap& tm_act, const CUtensorMap& tm_wgt,
+                              const CUtensorMap& tm_out, const CUtensorMap& tm_res, const ConvTcParams& p, dim3 grid, size_t smem_bytes,
+                              cudaStream_t stream);
 
 // CTA-pair points (tcgen05.mma.cta_group::2): tile_m = 256, tile_n 64 / 128 / 256; `grid` = 2 x the number of pairs.
 int conv_tc_pair_epi_warps(int tile_n);
-cudaError_t conv_tc_pair_prepare(int tile_n, int tile_k, size_t smem_bytes);
+cudaError_t conv_tc_pair_prepare(int tile_n, int tile_k, bool general, size_t smem_bytes);
 cudaError_t conv_tc_pair_launch(int tile_n, int tile_k, const CUtensorMap& tm_act, const CUtensorMap& tm_wgt, const CUtensorMap& tm_out,
                                 const CUtensorMap& tm_res, const ConvTcParams& p, dim3 grid, size_t smem_bytes, cudaStream_t stream);
 
 // Transposed-accumulator points (lane = output channel): NCHW output through TMA stores; tile_n 128 or 256, 16-bit types, 8 epilogue warps.
 // tm_out: y as the 3-D tensor {P*Q, O, N} with a 32-pixel x 32-channel box and 64-byte swizzle (read when p.swap_tma).
-cudaError_t conv_tc_swap_prepare(int tile_m, int tile_n, int tile_k, size_t smem_bytes);
+cudaError_t conv_tc_swap_prepare(int tile_m, int tile_n, int tile_k, bool general, size_t smem_bytes);
 cudaError_t conv_tc_swap_launch(int tile_m, int tile_n, int tile_k, const CUtensorMap& tm_act, const CUtensorMap& tm_wgt,
                                 const CUtensorMap& tm_out, const ConvTcParams& p, dim3 grid, size_t smem_bytes, cudaStream_t stream);
 
