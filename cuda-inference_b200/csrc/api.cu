@@ -344,7 +344,7 @@ bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, const gieb_conv_cf
   const int hs = d.stride_h == 1 ? d.in_h + d.pad_h : g.out_h + (d.kernel_h - 1) / d.stride_h;
   const int64_t rows = int64_t(d.batch) * hs * ws;
   const int need = kTileM + (d.kernel_h - 1) / d.stride_h * ws + (d.kernel_w - 1) / d.stride_w;  // rows of one phase that the taps read
-  const int c_padded = round_up(channel_units(d), 16);
+  const int c_padded = r->c_padded;
   const int blocks = ceil_div(c_padded, 64), last = (c_padded - (blocks - 1) * 64) / 16;
   const double ksteps = (blocks - 1) * 4.0 + last;  // MMA steps per tap
 
@@ -437,7 +437,6 @@ bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, const gieb_conv_cf
   if (b.smem < floor) b.smem = floor;
   b.halo = 1;
   b.tile_k = 64;
-  b.c_padded = c_padded;
   b.kb_per_tap = blocks;
   b.total_kb = taps * blocks;
   b.reduce = b.split_k > 1 ? 2 : 0;
@@ -563,7 +562,7 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
   // the time for 3x3 and 5x5, 0.965 for 1x1, 6 of them slower).  Not where the partial slab lets 1x1 weights be read in place: the
   // copy of the weights is a launch of its own (9 x 240 -> 64 at 54 x 8: 4.8 us, 8.9 with it).
   const bool in_place = in_nhwc || (r->variant == 2 && !(d.flags & GIEB_FLAG_WEIGHTS_PREPACKED) && d.in_channels % 16 == 0);
-  const bool whole_slabs = asked || (!halo && !in_place && r->tile_k == 64 && round_up(units, 64) * 100LL <= round_up(units, 16) * 115LL);
+  const bool whole_slabs = asked || (!in_place && r->tile_k == 64 && round_up(units, 64) * 100LL <= round_up(units, 16) * 115LL);
   if (halo && c.tile_k && r->tile_k != 64) return no("variant 6 (halo tiles) takes rows of 128 bytes: tile_k 64 (32 for TF32, 128 for FP8)");
   if (in_nhwc && asked && d.in_channels % r->tile_k != 0) return no("tile_k must divide the channel count of a channel-contiguous input (it is read in place)");
   if (gather) {
