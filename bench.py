@@ -28,7 +28,7 @@ import __graft_entry__ as entry  # noqa: E402
 
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of the dominant kernel, from one ncu capture of that launch per
 # workload (None where no capture exists).
-NCU_TRAFFIC_BYTES = {"c2": 4470272, "c3_fp16": 52158976, "c4a": 5205760, "c4b": 13514752, "c1": 985856}
+NCU_TRAFFIC_BYTES = {"c2": 4469248, "c3_fp16": 52201728, "c4a": 5212672, "c4b": 13521408, "c1": 1002752}
 
 # The metric both arms report (the same string, so that the two lines can be compared): one step = one forward call =
 # layout repack + weight prepack + convolution with fused bias + ReLU.
@@ -631,7 +631,7 @@ def run_ours(args):
         achieved = shape.flops / (kernel_us * 1e-6) / 1e12
         roof = {"bound": "tensor", "achieved": achieved, "peak": peaks["bf16_tflops"], "unit": "TFLOP/s",
                 "frac": achieved / peaks["bf16_tflops"]}
-    roof.update({"traffic": NCU_TRAFFIC_BYTES.get(args.workload), "kernel": "conv_tc_kernel" if shape.precision else "conv_fp32_kernel",
+    roof.update({"traffic": NCU_TRAFFIC_BYTES.get(args.workload), "kernel": {3: "conv_fp32_kernel", 6: "conv_halo_kernel"}.get(plan.info.cfg.variant, "conv_tc_kernel"),
                  "kernel_us": kernel_us, "kernel_us_p10_p90": [res["kernel"]["p10_us"], res["kernel"]["p90_us"]],
                  "repack_us": res["repack"]["median_us"] if "repack" in res else 0.0,
                  "how": "average launch duration over CUDA-graph replays of that kernel alone, back to back over the rotating "

@@ -413,7 +413,9 @@ bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, const gieb_conv_cf
         const double drain = 800.0 + 18.0 * bn * (workers == 16 ? 0.6 : 1.0);
         double t = (load > 1 ? 4500.0 : 3500.0) + a_time + load * fmax(main, load > 1 ? drain : 0.0) + (load - 1) * 600.0 + drain;
         if (s > 1) t += 2000.0 + double(s - 1) / s * (double(kTileM) * bn * 4.0) / 5.0;  // exchange of the partial columns in the cluster
-        if (s == 2) t *= 1.15;  // (two slices gain less than that: 93 x 768 -> 64 at 7 x 7 21.7 us, 19.2 on the slab kernel)
+        // (two slices gain less than that: 93 x 768 -> 64 at 7 x 7 21.7 us, 19.2 on the slab kernel; nine other layers ran at 0.65 to
+        // 1.05 of what the two models have with this factor)
+        if (s == 2) t *= 1.15;
         if (ph * pw > 1) t += 0.15 * load * main;  // (the phases are loaded whole)
         if (t < best) {
           best = t;
