@@ -138,6 +138,9 @@ int channel_units(const gieb_conv_desc& d) {
   return d.precision == GIEB_FP8_E4M3 ? (d.in_channels + 1) / 2 : (d.precision == GIEB_TF32 ? 2 * d.in_channels : d.in_channels);
 }
 
+// Whether whole slabs of 64 units instead of multiples of 16 cost at most `percent`.
+bool padding_pays(int units, int percent) { return round_up(units, 64) * 100LL <= int64_t(round_up(units, 16)) * percent; }
+
 // Slab width for a channel count in 2-byte units: the narrowest of 16, 32 and 64 that holds all of it, else 64.  Where whole slabs
 // would pad too much (see resolve()) channels are padded to multiples of 16 only: the last slab of a tap reads on into the next
 // tap's columns and the MMA steps over them are left out, so a layer of 144 channels takes 3 slabs per tap (of 4 + 4 + 1 steps) instead of 9 of one step each, every one
@@ -344,7 +347,8 @@ bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, const gieb_conv_cf
   const int hs = d.stride_h == 1 ? d.in_h + d.pad_h : g.out_h + (d.kernel_h - 1) / d.stride_h;
   const int64_t rows = int64_t(d.batch) * hs * ws;
   const int need = kTileM + (d.kernel_h - 1) / d.stride_h * ws + (d.kernel_w - 1) / d.stride_w;  // rows of one phase that the taps read
-  const int c_padded = r->c_padded;
+  // (whole blocks where padding costs at most 15 %: 34 such layers take 0.966 of the time that a partial last block takes)
+  const int units = channel_units(d), c_padded = round_up(units, !nhwc && padding_pays(units, 115) ? 64 : 16);
   const int blocks = ceil_div(c_padded, 64), last = (c_padded - (blocks - 1) * 64) / 16;
   const double ksteps = (blocks - 1) * 4.0 + last;  // MMA steps per tap
 
@@ -445,6 +449,7 @@ bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, const gieb_conv_cf
   if (b.smem < floor) b.smem = floor;
   b.halo = 1;
   b.tile_k = 64;
+  b.c_padded = c_padded;
   b.kb_per_tap = blocks;
   b.total_kb = taps * blocks;
   b.reduce = b.split_k > 1 ? 2 : 0;
@@ -565,12 +570,13 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
   const int units = channel_units(d);
   const bool complete = c.tile_m && c.tile_n && c.stages && c.split_k && c.variant && c.cta_pair && c.tile_k && r->tile_k == pick_tile_k(units);
   const bool asked = c.tile_k && !complete && !halo;
-  // Channels of a copy are padded to whole slabs of 64 as well where that costs at most 15 %: the general kernel with its partial
-  // last slab takes longer than the steps it leaves out (tile_k 64 asked for against the partial slab over 92 such layers: 0.95 of
-  // the time for 3x3 and 5x5, 0.965 for 1x1, 6 of them slower).  Not where the partial slab lets 1x1 weights be read in place: the
-  // copy of the weights is a launch of its own (9 x 240 -> 64 at 54 x 8: 4.8 us, 8.9 with it).
+  // Channels of a copy are padded to whole slabs of 64 as well where that costs little: the general kernel with its partial last
+  // slab takes longer than the steps it leaves out.  tile_k 64 asked for (whole slabs) against the partial slab: padding by up to
+  // 15 %, 0.95 of the time for 3x3 and 5x5 and 0.965 for 1x1 (92 layers, 6 slower); by up to a third, 0.945 for 1x1 and 3x3
+  // (33 to 48 channels: 0.93 over 80 layers, 3 slower), 0.98 for 5x5; by more, nothing.  Not where the partial slab lets 1x1
+  // weights be read in place: the copy of the weights is a launch of its own (9 x 240 -> 64 at 54 x 8: 4.8 us, 8.9 with it).
   const bool in_place = in_nhwc || (r->variant == 2 && !(d.flags & GIEB_FLAG_WEIGHTS_PREPACKED) && d.in_channels % 16 == 0);
-  const bool whole_slabs = asked || (!in_place && r->tile_k == 64 && round_up(units, 64) * 100LL <= round_up(units, 16) * 115LL);
+  const bool whole_slabs = asked || (!in_place && r->tile_k == 64 && padding_pays(units, d.kernel_h * d.kernel_w <= 9 ? 134 : 115));
   if (halo && c.tile_k && r->tile_k != 64) return no("variant 6 (halo tiles) takes rows of 128 bytes: tile_k 64 (32 for TF32, 128 for FP8)");
   if (in_nhwc && asked && d.in_channels % r->tile_k != 0) return no("tile_k must divide the channel count of a channel-contiguous input (it is read in place)");
   if (gather) {

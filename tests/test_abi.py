@@ -312,9 +312,10 @@ def test_halo_variant_leaves_outputs_beyond_its_row_offsets(pkg):
 
 
 def test_channels_of_a_copy_are_padded_to_whole_slabs_where_that_is_cheap(pkg):
-    """At most 15 %: whole slabs of 64.  More, or a tensor that is read in place: multiples of 16."""
+    """At most a third (15 % for more than nine taps): whole slabs of 64.  More, or a tensor that is read in place: multiples of 16."""
     cases = [((3, 605, 29, 29, 256, 1, 1, 1, 1, 0, 0), 0, 640), ((2, 288, 11, 86, 64, 1, 1, 2, 2, 0, 0), 0, 320), ((4, 240, 14, 14, 64, 3, 3, 3, 3, 1, 1), 0, 256),
-             ((4, 144, 14, 14, 64, 3, 3, 3, 3, 1, 1), 0, 144), ((4, 80, 14, 14, 64, 3, 3, 3, 3, 1, 1), 0, 80), ((4, 48, 14, 14, 64, 3, 3, 3, 3, 1, 1), 0, 48),
+             ((4, 144, 14, 14, 64, 3, 3, 3, 3, 1, 1), 0, 192), ((4, 80, 14, 14, 64, 3, 3, 3, 3, 1, 1), 0, 80), ((4, 48, 14, 14, 64, 3, 3, 3, 3, 1, 1), 0, 64),
+             ((4, 144, 14, 14, 64, 5, 5, 3, 3, 2, 2), 0, 144), ((4, 240, 14, 14, 64, 5, 5, 3, 3, 2, 2), 0, 256),
              ((4, 240, 14, 14, 64, 3, 3, 3, 3, 1, 1), pkg.FLAG_INPUT_NHWC, 240),
              ((9, 240, 54, 8, 64, 1, 1, 1, 1, 0, 0), 0, 240), ((9, 240, 54, 8, 64, 1, 1, 1, 1, 0, 0), pkg.FLAG_WEIGHTS_PREPACKED, 256),
              ((9, 245, 54, 8, 64, 1, 1, 1, 1, 0, 0), 0, 256)]
@@ -322,7 +323,7 @@ def test_channels_of_a_copy_are_padded_to_whole_slabs_where_that_is_cheap(pkg):
         p = P(pkg, *args, precision=pkg.FP16, has_bias=True, relu=True, flags=flags)
         i = pkg.query(p)
         assert i.supported and i.padded_channels == padded, (args, flags, i.padded_channels)
-    # the halo kernel pads its blocks by the same rule
+    # the halo kernel, whose steps cost more, pads its blocks by up to 15 %
     for c, padded in ((240, 256), (144, 144)):
         assert pkg.query(P(pkg, 4, c, 14, 14, 64, 3, 3, 1, 1, 1, 1, precision=pkg.FP16), pkg.make_cfg(variant=6)).padded_channels == padded
     # FP8 values count half, TF32 values twice

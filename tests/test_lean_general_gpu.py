@@ -53,7 +53,7 @@ def test_both_forms(pkg, orc, oracle, point, channels, filters):
 
 
 @pytest.mark.parametrize("kw", [dict(tile_m=128, tile_n=128), dict(tile_m=256, tile_n=128), dict(tile_m=128, tile_n=256)])
-@pytest.mark.parametrize("channels", [144, 192])
+@pytest.mark.parametrize("channels", [80, 192])
 def test_transposed_accumulator_with_partial_slab(pkg, orc, oracle, channels, kw, monkeypatch):
     monkeypatch.setenv("GIEB_TRANSPOSED_ACC", "2")
     p = orc.Problem.P(2, channels, 12, 14, 200, 3, 3, 1, 1, 1, 1, precision=orc.FP16, bias=True, relu=True)
