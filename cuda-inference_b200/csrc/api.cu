@@ -434,11 +434,14 @@ bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, const gieb_conv_cf
     }
   }
   // What the ratio of the two estimates has to stay below, by the times of both kernels on 330 layers (sizes, types and layouts
-  // spread over what networks have): with these lines 79 layers take this kernel, at 0.908 of the slab kernels' time on average,
-  // and seven of them lose more than 2 %.  One or two waves need a margin (at 0.95 another 42 layers would come in, 18 of them
-  // slower); with many waves of tiles of at most 64 channels the slab model is too short (co-resident CTAs do not double the issue
-  // rate there), except for FP8; TF32 layers rarely gain (13 of the 15 between 0.85 and 1.05 lose).
-  double margin = 0.90;
+  // spread over what networks have): with these lines 104 layers take this kernel, at 0.922 of the slab kernels' time on average, and
+  // ten of them lose more than 2 %.  One wave of single CTAs gains up to 0.945, one of pairs up to 0.90 (four of seven between
+  // that and 0.95 lose by 4 to 15 %), two waves only well below (0.89 to 0.96: four of five lose); clusters gain at par, most of all against
+  // slices that the slab kernels sum in a launch of their own.  With many waves of tiles of at most 64 channels the slab model is
+  // too short (co-resident CTAs do not double the issue rate there), except for FP8; TF32 layers rarely gain (13 of the 15
+  // between 0.85 and 1.05 lose).
+  double margin = best_load >= 2 ? 0.85 : (b.pair ? 0.90 : 0.945);
+  if (b.split_k > 1) margin = 1.0;
   if (best_load >= 3) margin = (b.tile_n <= 64 && ph * pw == 1 && d.precision != GIEB_FP8_E4M3) ? 1.2 : 1.0;
   if (d.precision == GIEB_TF32) margin = 0.85;
   if (best >= 1e299 || (!asked && best >= margin * slab)) return false;
