@@ -14,7 +14,8 @@
 // Launched with programmatic stream serialization: a launch follows the one before it without the drain-and-refill gap, and
 // costs the host 0.45 us less.  Calls in a stream, residual form, before and after: 8192 x 4096 BF16 43.4 -> 41.7 us (6.4
 // TB/s), 4741 x 12224 BF16 110 -> 72 us (the row held as floats spilled), 4000 x 3185 BF16 64 -> 25 us (element-wise before),
-// 4775 x 128 FP32 6.1 -> 3.2 us, 16 x 4096 BF16 4.8 -> 3.1 us (bound by the launch; most of it the host, see python_calls.cpp).
+// 4775 x 128 FP32 6.1 -> 3.2 us, 16 x 4096 BF16 4.8 -> 3.1 us (bound by the launch: most of it the host's, see
+// python_calls.cpp).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <stdint.h>
