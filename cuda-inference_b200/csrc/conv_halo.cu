@@ -55,9 +55,10 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_consta
   constexpr uint32_t TMEM_COLS = 2 * BN < 32 ? 32 : 2 * BN;
   constexpr int EG = NW / 4;                  // worker warps per TMEM lane quarter
 
-  // (aligned here, not by the declaration as in conv_tc_kernel: with that the compiler lays the kernel out for 1 % more time)
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = smem_raw + ((1024u - (ptx::smem_u32(smem_raw) & 1023u)) & 1023u);
+  // (Pairs take the alignment of the declaration; single CTAs round up by hand: what the compiler makes of either is 1 % faster
+  // there, 3x3 14x14 b32 15.1 and 15.35 us, 70 -> 64 at 65x65, 76 images 97.2 and 96.2.)
+  extern __shared__ __align__(PAIR ? 1024 : 16) uint8_t smem_raw[];
+  uint8_t* smem = PAIR ? smem_raw : smem_raw + ((1024u - (ptx::smem_u32(smem_raw) & 1023u)) & 1023u);
   float* bias_s = reinterpret_cast<float*>(smem);  // [NW][32]
   uint64_t* b_full = reinterpret_cast<uint64_t*>(smem + 2048);
   uint64_t* b_empty = b_full + kMaxStages;
