@@ -142,9 +142,10 @@ int channel_units(const gieb_conv_desc& d) {
 bool padding_pays(int units, int percent) { return round_up(units, 64) * 100LL <= int64_t(round_up(units, 16)) * percent; }
 
 // Slab width for a channel count in 2-byte units: the narrowest of 16, 32 and 64 that holds all of it, else 64.  Where whole slabs
-// would pad too much (see resolve()) channels are padded to multiples of 16 only: the last slab of a tap reads on into the next
-// tap's columns and the MMA steps over them are left out, so a layer of 144 channels takes 3 slabs per tap (of 4 + 4 + 1 steps) instead of 9 of one step each, every one
-// of which costs the producers and the issuer the same (6 x 35 x 45, 144 -> 200 channels, 3x3: 22.0 -> 12.8 us).
+// would pad too much, or a tensor is read in place (see resolve()), channels are padded to multiples of 16 only: the last slab of a
+// tap reads on into the next tap's columns and the MMA steps over them are left out, so a layer of 144 channels takes 3 slabs per
+// tap (of 4 + 4 + 1 steps) instead of 9 of one step each, every one of which costs the producers and the issuer the same
+// (channel-contiguous, 6 x 35 x 45, 144 -> 200 channels, 3x3: 22.0 -> 12.8 us).
 int pick_tile_k(int units) { return units <= 16 ? 16 : (units <= 32 ? 32 : 64); }
 
 // Measured on B200: with every SM pulling, one SM receives about 74 B/clk of operands from L2 through TMA, well below
@@ -434,12 +435,12 @@ bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, const gieb_conv_cf
     }
   }
   // What the ratio of the two estimates has to stay below, by the times of both kernels on 330 layers (sizes, types and layouts
-  // spread over what networks have): with these lines 104 layers take this kernel, at 0.922 of the slab kernels' time on average, and
-  // ten of them lose more than 2 %.  One wave of single CTAs gains up to 0.945, one of pairs up to 0.90 (four of seven between
-  // that and 0.95 lose by 4 to 15 %), two waves only well below (0.89 to 0.96: four of five lose); clusters gain at par, most of all against
-  // slices that the slab kernels sum in a launch of their own.  With many waves of tiles of at most 64 channels the slab model is
-  // too short (co-resident CTAs do not double the issue rate there), except for FP8; TF32 layers rarely gain (13 of the 15
-  // between 0.85 and 1.05 lose).
+  // spread over what networks have): with these lines 104 layers take this kernel, at 0.922 of the slab kernels' time on
+  // average, and ten of them lose more than 2 %.  One wave of single CTAs gains up to 0.945, one of pairs up to 0.90 (four of
+  // seven between that and 0.95 lose by 4 to 15 %), two waves only well below (0.89 to 0.96: four of five lose); clusters gain at
+  // par, most of all against slices that the slab kernels sum in a launch of their own.  With many waves of tiles of at most 64
+  // channels the slab model is too short (co-resident CTAs do not double the issue rate there), except for FP8; TF32 layers
+  // rarely gain (13 of the 15 between 0.85 and 1.05 lose).
   double margin = best_load >= 2 ? 0.85 : (b.pair ? 0.90 : 0.945);
   if (b.split_k > 1) margin = 1.0;
   if (best_load >= 3) margin = (b.tile_n <= 64 && ph * pw == 1 && d.precision != GIEB_FP8_E4M3) ? 1.2 : 1.0;
