@@ -112,7 +112,11 @@ struct Resolved {
   // position) and the im2col tensor map reads it with a pixel stride of one position, so that the windows of adjacent
   // output columns overlap in memory instead of being stored twice.  gp_t positions (8 values each) per window.
   int gather_pairs, gp_positions, gp_left, gp_t, gp_shift;
-  int strip;  // the pair layout read as one position strip per (output row, filter row): see resolve()
+  // The same layer straight from the NCHW tensor (conv_image.cu); `strip`: its rows are counted in 128-row tiles per output row
+  // (tile counts, which a query reports).
+  int image, strip;
+  int im_group_rows, im_in_rows, im_rows_per_phase;
+  size_t im_stage_bytes, im_smem;
   double est_cycles;  // the cost model's estimate for the chosen configuration (SM cycles; 0 on the FP32 path)
   int tma_epilogue;  // channel-contiguous output staged in shared memory and written by TMA stores
   int row_epilogue;  // the same staging for channel counts that TMA cannot address, written row by row
@@ -303,14 +307,6 @@ bool pdl_enabled() {
   }();
   return on;
 }
-// GIEB_GATHER_STRIPS=0 reads the pair layout through im2col-mode loads of whole windows (a debugging aid).
-bool strips_enabled() {
-  static const bool on = [] {
-    const char* e = getenv("GIEB_GATHER_STRIPS");
-    return !(e && e[0] == '0');
-  }();
-  return on;
-}
 // GIEB_GATHER_PAIRS=0 keeps the row-gather route on its one-window-per-pixel layout (a debugging aid).
 bool pairs_enabled() {
   static const bool on = [] {
@@ -470,6 +466,46 @@ bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, const gieb_conv_cf
   return true;
 }
 
+// Groups of the image kernel (conv_image.cu): how many output rows a CTA takes at a time.  False: no group fits shared memory.
+bool resolve_image(const gieb_conv_desc& d, const Geometry& g, Resolved* r) {
+  const int pitch = g.out_w + r->gp_t - 1, tiles_n = ceil_div(d.out_channels, 64);
+  const bool staging = (d.flags & GIEB_FLAG_OUTPUT_NHWC) != 0;
+  double best = 1e300;
+  for (int ctas = 2; ctas >= 1 && best >= 1e299; --ctas) {
+    for (int rows = 1; rows <= g.out_h && rows <= 16; ++rows) {
+      const int in_rows = (rows - 1) * d.stride_h + d.kernel_h, per_phase = ceil_div(in_rows, d.stride_h);
+      const int tiles = ceil_div(int64_t(rows - 1) * pitch + g.out_w, kTileM);
+      // (a tile's last rows may lie beyond the strips: they are read, but no output pixel depends on them)
+      int64_t last = 0;
+      for (int k = 0; k < d.kernel_h; ++k) {
+        const int64_t first = int64_t(k % d.stride_h * per_phase + k / d.stride_h) * pitch;
+        if (first > last) last = first;
+      }
+      int64_t positions = last + int64_t(tiles) * kTileM + r->gp_t;
+      if (positions < int64_t(d.stride_h) * per_phase * pitch) positions = int64_t(d.stride_h) * per_phase * pitch;
+      const size_t stage = (size_t(positions) * 16 + 127) / 128 * 128;
+      if (stage > kMaxDynamicSmem) break;
+      const size_t smem = conv_image_smem_bytes(d.kernel_h, r->gp_t, stage, staging);
+      if (smem > (ctas == 2 ? kSmSmem / 2 - 1024 : kMaxDynamicSmem)) break;
+      // cycles: instructions of a run of 32 positions and of a tile on an SM that two CTAs share; a group's loads take at least a
+      // round trip per 32 runs
+      const int64_t groups = int64_t(d.batch) * ceil_div(g.out_h, rows);
+      const double waves = double(ceil_div(groups * tiles_n, kNumSms * ctas)), runs = double(in_rows) * ceil_div(pitch, 32);
+      const double busy = ctas * (12.0 * runs + 500.0 * tiles), load = 900.0 * std::ceil(runs / 32.0);
+      const double t = load + waves * fmax(load, busy) + 700.0 * tiles;
+      if (t < best) {
+        best = t;
+        r->im_group_rows = rows;
+        r->im_in_rows = in_rows;
+        r->im_rows_per_phase = per_phase;
+        r->im_stage_bytes = stage;
+        r->im_smem = smem;
+      }
+    }
+  }
+  return best < 1e299;
+}
+
 int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, char* why, size_t why_len) {
   auto no = [&](const char* m) { snprintf(why, why_len, "%s", m); return GIEB_UNSUPPORTED; };
   memset(r, 0, sizeof(*r));
@@ -538,11 +574,9 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
       r->gp_positions = d.in_w / 2 + left + right;
     }
   }
-  // The pair layout read as STRIPS: one 128-row tile per output row, whose operand for filter row r is the strip of positions
-  // of ONE input row (a single 2 KiB box instead of 128 pixels x 64 bytes), multiplied as overlapping windows through an
-  // unswizzled descriptor.  Needs out_w <= 128 and a CTA that finishes its tiles alone.
-  r->strip = (r->gather_pairs && g.out_w <= 128 && c.split_k <= 1 && c.reduce == 0 && c.cta_pair != 2 && (c.tile_k == 0 || c.tile_k == r->gp_t * 8) &&
-              strips_enabled()) ? 1 : 0;   // (one slab per filter row: the strip is loaded once per slab)
+  // Read straight from the image (conv_image.cu) unless the reduction is asked to be split or spread over a pair.
+  const bool image_fits = r->gather_pairs && resolve_image(d, g, r);
+  r->strip = (image_fits && g.out_w <= 128 && c.split_k <= 1 && c.reduce == 0 && c.cta_pair != 2 && (c.tile_k == 0 || c.tile_k == r->gp_t * 8)) ? 1 : 0;
   const int64_t rows = r->strip ? int64_t(d.batch) * g.out_h * 128 : (r->variant == 2 ? int64_t(d.batch) * r->boxes_per_image * 64 : g.pixels);
 
   // hardware limits of the im2col-mode tensor map (rank 4): traversal strides 1..8, corners and offsets 8-bit
@@ -767,6 +801,7 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
   r->ws_part = r->split_k > 1 && r->reduce == 1 ? align256(size_t(r->split_k) * size_t((g.y_elems + 3) & ~int64_t(3)) * 4) : 0;
   r->ws_total = r->ws_x + r->ws_w + r->ws_part;
   if (r->ws_total > (size_t(180) << 30) / 4) return no("workspace exceeds a quarter of device memory");
+  r->image = image_fits && r->split_k == 1 && !r->pair && r->tile_k == r->gp_t * 8;
   return GIEB_OK;
 }
 
@@ -798,7 +833,7 @@ void fill_info(const gieb_conv_desc& d, const Resolved& r, gieb_conv_info* out) 
     const bool x_in_place = r.variant == 2 || (d.flags & GIEB_FLAG_INPUT_NHWC);
     const bool w_in_place = (d.flags & GIEB_FLAG_WEIGHTS_PREPACKED) != 0 ||
                             (x_in_place && d.precision != GIEB_TF32 && d.kernel_h * d.kernel_w == 1 && r.c_padded == d.in_channels);  // 16-byte aligned w assumed
-    out->launches = (x_in_place && w_in_place ? 0 : 1) + 1 + (r.reduce == 1 ? 1 : 0);
+    out->launches = r.image ? 1 : (x_in_place && w_in_place ? 0 : 1) + 1 + (r.reduce == 1 ? 1 : 0);
   }
 }
 
@@ -873,15 +908,6 @@ int encode_maps(const gieb_conv_plan* pl, int mode, const void* xn, const void* 
                                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (res != CUDA_SUCCESS) return fail(GIEB_CUDA_ERROR, "cuTensorMapEncodeTiled (NCHW activations) failed with CUresult %d", int(res));
     small_tensor_fixup(tm_act, size_t(hw) * d.in_channels * d.batch * 2);
-  } else if (mode == 3) {  // the pair layout {8 values, positions, H, N}: one box = the strip of 128 + T - 1 positions of one input row
-    const cuuint64_t dims[4] = {8, cuuint64_t(r.gp_positions), cuuint64_t(d.in_h), cuuint64_t(d.batch)};
-    const cuuint64_t strides[3] = {16, cuuint64_t(r.gp_positions) * 16, cuuint64_t(d.in_h) * r.gp_positions * 16};
-    const cuuint32_t box[4] = {8, cuuint32_t(128 + r.gp_t - 1), 1, 1};
-    const cuuint32_t estr[4] = {1, 1, 1, 1};
-    const CUresult res = g_encode_tiled(tm_act, dt, 4, const_cast<void*>(xn), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (res != CUDA_SUCCESS) return fail(GIEB_CUDA_ERROR, "cuTensorMapEncodeTiled (position strips) failed with CUresult %d", int(res));
-    small_tensor_fixup(tm_act, size_t(d.batch) * d.in_h * r.gp_positions * 16);
   } else if (mode == 1) {  // 1x1 / stride 1 / pad 0: the NHWC copy is the GEMM operand [pixels][Cp] itself
     const cuuint64_t plane = r.subsampled ? cuuint64_t(pl->g.out_h) * pl->g.out_w : cuuint64_t(d.in_h) * d.in_w;
     const cuuint64_t dims[2] = {cuuint64_t(el(r.c_padded)), cuuint64_t(d.batch) * plane};
@@ -1030,6 +1056,50 @@ int launch_halo(const gieb_conv_plan* pl, const CUtensorMap& tm_act, const CUten
   return GIEB_OK;
 }
 
+// The one launch of a plan on the image kernel; the arguments have been checked.
+int launch_image(const gieb_conv_plan* pl, const void* x, const void* w, const void* bias, const void* residual, void* y, cudaStream_t st,
+                 cudaEvent_t* ev, unsigned stage_mask) {
+  const gieb_conv_desc& d = pl->desc;
+  const Resolved& r = pl->r;
+  ConvImageParams p;
+  memset(&p, 0, sizeof(p));
+  p.x = x; p.w = w; p.bias = bias; p.residual = residual; p.y = y;
+  p.status = pl->d_status;
+  p.wait_limit = pl->wait_limit;
+  p.debug_skip = pl->debug_skip;
+  p.channels = d.in_channels; p.in_h = d.in_h; p.in_w = d.in_w;
+  p.out_channels = d.out_channels; p.out_h = pl->g.out_h; p.out_w = pl->g.out_w; p.pq = pl->g.pq;
+  p.kernel_h = d.kernel_h; p.kernel_w = d.kernel_w; p.stride_h = d.stride_h; p.pad_h = d.pad_h;
+  p.left = r.gp_left; p.shift = r.gp_shift;
+  p.pitch = pl->g.out_w + r.gp_t - 1;
+  p.segments = ceil_div(p.pitch, 32);
+  p.group_rows = r.im_group_rows; p.group_in_rows = r.im_in_rows; p.rows_per_phase = r.im_rows_per_phase;
+  p.groups_per_image = ceil_div(p.out_h, p.group_rows);
+  p.groups = d.batch * p.groups_per_image;  // (at most the number of output rows)
+  p.strip_stage_bytes = uint32_t(r.im_stage_bytes);
+  p.words = reinterpret_cast<uintptr_t>(x) % 4 == 0;
+  p.prepacked = (d.flags & GIEB_FLAG_WEIGHTS_PREPACKED) != 0;
+  p.is_bf16 = d.precision == GIEB_BF16;
+  p.bias_fp32 = (d.flags & GIEB_FLAG_BIAS_FP32) != 0;
+  p.relu = d.relu;
+  p.out_nhwc = (d.flags & GIEB_FLAG_OUTPUT_NHWC) != 0;
+  p.out_cells = p.out_nhwc && (reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(residual)) % 16 == 0 && d.out_channels % 8 == 0;
+  p.idesc = ptx::make_idesc_f16(kTileM, 64, p.is_bf16, false, false);
+  p.fd_groups_per_image = FastDiv::make(p.groups_per_image);
+  p.fd_pitch = FastDiv::make(p.pitch);
+  p.fd_stride_h = FastDiv::make(p.stride_h);
+  p.fd_segments = FastDiv::make(p.segments);
+  p.fd_cells = FastDiv::make(p.kernel_h * r.gp_t);
+  const int tiles_n = ceil_div(d.out_channels, 64);
+  int ctas = kNumSms * (r.im_smem <= kSmSmem / 2 - 1024 ? 2 : 1) / tiles_n;  // persistent CTAs for each tile of channels
+  if (ctas < 1) ctas = 1;
+  const dim3 grid(unsigned(p.groups < ctas ? p.groups : ctas), unsigned(tiles_n));
+  if (ev) for (int k = 0; k < 2; ++k) GIEB_CUDA(cudaEventRecord(ev[k], st));
+  if (stage_mask & 2u) GIEB_CUDA(conv_image_launch(r.gp_t, p, grid, r.im_smem, st));
+  if (ev) for (int k = 2; k < 4; ++k) GIEB_CUDA(cudaEventRecord(ev[k], st));
+  return GIEB_OK;
+}
+
 // `ev`, when given, receives four stage marks: before the repack, before the convolution kernel, after it, and
 // after the split-K reduction (LaunchArgs::stage_events analogue, include/gpu_inference/kernel_registry.h:38-40).
 int launch_impl(const gieb_conv_plan* pl, const void* x, const void* w, const void* bias, void* y, void* ws, size_t ws_bytes,
@@ -1062,6 +1132,12 @@ int launch_impl(const gieb_conv_plan* pl, const void* x, const void* w, const vo
     return GIEB_OK;
   }
 
+  if (r.image) {
+    if ((d.flags & GIEB_FLAG_WEIGHTS_PREPACKED) && reinterpret_cast<uintptr_t>(w) % 16 != 0)
+      return fail(GIEB_INVALID_ARGUMENT, "prepacked weights must be 16-byte aligned");
+    return launch_image(pl, x, w, bias, residual, y, st, ev, stage_mask);
+  }
+
   std::call_once(g_driver_once, load_driver_entry_points);
   if (g_driver_err != cudaSuccess) return fail_cuda(g_driver_err, "resolving cuTensorMapEncode* driver entry points");
 
@@ -1073,14 +1149,14 @@ int launch_impl(const gieb_conv_plan* pl, const void* x, const void* w, const vo
   float* part = r.reduce == 1 ? reinterpret_cast<float*>(wsb + r.ws_x + r.ws_w) : nullptr;
 
   // A direct-NCHW plan needs a 16-byte aligned x (TMA base address rule); otherwise this call takes the repack route.
-  int mode = r.strip ? 3 : ((r.variant == 1 || r.variant == 5) ? 0 : (r.variant == 4 ? 1 : 2));
+  int mode = (r.variant == 1 || r.variant == 5) ? 0 : (r.variant == 4 ? 1 : 2);
   if (mode == 2 && reinterpret_cast<uintptr_t>(x) % 16 != 0) mode = 1;
   const bool in_nhwc = (d.flags & GIEB_FLAG_INPUT_NHWC) != 0;
   if (in_nhwc) {  // read in place
     if (reinterpret_cast<uintptr_t>(x) % 16 != 0) return fail(GIEB_INVALID_ARGUMENT, "a channel-contiguous input must be 16-byte aligned");
     xn = const_cast<void*>(x);
   }
-  const int64_t rows = mode == 3 ? int64_t(d.batch) * pl->g.out_h * 128 : (mode == 2 ? int64_t(d.batch) * r.boxes_per_image * 64 : pl->g.pixels);
+  const int64_t rows = mode == 2 ? int64_t(d.batch) * r.boxes_per_image * 64 : pl->g.pixels;
   // 1x1 filters over unpadded channels: OIHW *is* the [O][RS][C] layout, so when no activation repack would share the
   // launch the weights are read where they lie and the step is the convolution kernel alone (measured on 512 -> 128
   // channels at 28x28: 16.4 instead of 17.5 us per step).
@@ -1170,8 +1246,6 @@ int launch_impl(const gieb_conv_plan* pl, const void* x, const void* w, const vo
   p.fd_kb_per_tap = FastDiv::make(p.kb_per_tap);
   p.fd_kernel_w = FastDiv::make(p.kernel_w);
   p.fd_boxes = FastDiv::make(p.boxes_per_image > 0 ? p.boxes_per_image : 1);
-  p.fd_out_h = FastDiv::make(p.out_h > 0 ? p.out_h : 1);
-  p.strip_bytes = r.strip ? (128 + r.gp_t - 1) * 16 : 0;
   // persistent CTAs: as many as can be resident at once, each walking the tile list
   const int64_t resident = r.pair ? kNumSmPairs : int64_t(kNumSms) * resident_ctas(r.tile_m, r.tile_n, r.smem);
   // cluster mode: one tile per CTA, blockIdx.x = tile * split + slice (the grid is a multiple of the cluster size);
@@ -1230,6 +1304,7 @@ int launch_impl(const gieb_conv_plan* pl, const void* x, const void* w, const vo
 // Opts every kernel that launches of this configuration may take in to large dynamic shared memory.
 cudaError_t prepare_kernels(const Resolved& r) {
   if (r.variant == 3) return cudaSuccess;
+  if (r.image) return conv_image_prepare(r.gp_t, r.im_smem);
   if (r.halo) return conv_halo_prepare(r.tile_n, r.epi_warps, r.pair != 0, kMaxDynamicSmem);
   // The general kernel: a partial last slab, or rows that TMA cannot store (which tensors off their alignment are as well).
   const bool tail = r.tile_k == 64 && r.c_padded % 64 != 0;

@@ -125,8 +125,6 @@ struct ConvTcParams {
   //      numbered in 64-pixel boxes that never straddle an image: m_total = batch * boxes_per_image * 64.
   int a_mode;
   int boxes_per_image;  // mode 2: ceil(H*W / 64)
-  int strip_bytes;      // mode 3: bytes of one position strip (one TMA box); rows are numbered in 128-row boxes per output row
-  FastDiv fd_out_h;     // mode 3: reciprocal of out_h
   uint32_t idesc;
   // > 1: split-K slices of one tile form a thread-block cluster (cluster rank = slice) and are summed through
   // distributed shared memory; blockIdx.x = tile * cluster_split + slice, one tile per CTA, `partial` unused.
@@ -185,6 +183,34 @@ size_t conv_halo_smem_bytes(int tile_n, bool pair, int workers, int taps_per_loa
 cudaError_t conv_halo_prepare(int tile_n, int workers, bool pair, size_t smem);
 cudaError_t conv_halo_launch(int tile_n, int workers, bool pair, const CUtensorMap& tm_act, const CUtensorMap& tm_wgt,
                              const ConvHaloParams& p, dim3 grid, size_t smem, cudaStream_t stream);
+
+// Everything conv_image_kernel needs (see conv_image.cu for strips, positions and groups).
+struct ConvImageParams {
+  const void* x;         // NCHW, 16-bit
+  const void* w;         // OIHW, or [O][R][T * 8] as the plan converts them (prepacked, 16-byte aligned)
+  const void* bias;      // or null
+  const void* residual;  // or null; shape and layout of y
+  void* y;
+  uint32_t* status;
+  long long wait_limit;
+  int channels, in_h, in_w;
+  int out_channels, out_h, out_w, pq;
+  int kernel_h, kernel_w, stride_h, pad_h;
+  int left, shift;                        // positions left of column 0, first tap within the window
+  int pitch, segments;                    // positions per strip, in runs of 32
+  int group_rows, group_in_rows, rows_per_phase;  // output rows of a group, input rows they read, ceil(group_in_rows / stride_h)
+  int groups_per_image, groups;
+  uint32_t strip_stage_bytes;
+  int words;                              // x may be read as aligned 32-bit column pairs
+  int prepacked, is_bf16, bias_fp32, relu;
+  int out_nhwc, out_cells;                // channel-contiguous output; in aligned 16-byte cells
+  uint32_t idesc, debug_skip;
+  FastDiv fd_groups_per_image, fd_pitch, fd_stride_h, fd_segments, fd_cells;  // fd_cells: kernel_h * T
+};
+// t_positions: positions per window, 2, 4 or 8
+size_t conv_image_smem_bytes(int kernel_h, int t_positions, size_t strip_stage_bytes, bool staging);
+cudaError_t conv_image_prepare(int t_positions, size_t smem);
+cudaError_t conv_image_launch(int t_positions, const ConvImageParams& p, dim3 grid, size_t smem, cudaStream_t stream);
 
 // tile_m is 128 or 256 output pixels per CTA (one or two TMEM accumulators sharing each weight tile).
 // pair: the tile belongs to a CTA pair (tile_m = 256), each CTA stages 128 activation rows and tile_n / 2 weight rows.

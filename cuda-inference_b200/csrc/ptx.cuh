@@ -231,6 +231,14 @@ __device__ __forceinline__ void tmem_relinquish() {
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
+// The allocation of a kernel's allocating warp, its permit given up, and only then the signal that lets the next kernel of the
+// stream start: a CTA of that kernel beside this one while it still waited for columns could take them first, and would then hold
+// them until this kernel has ended, which it could not without them.
+__device__ __forceinline__ void tmem_alloc_then_signal(uint32_t* smem_result, uint32_t cols) {
+  tmem_alloc(smem_result, cols);
+  tmem_relinquish();
+  grid_dep_launch();
+}
 // The same for a CTA pair (cta_group::2): one warp of EACH CTA of the pair executes the instruction, the same warp index
 // in both, with the same shared-memory offset for the result; the columns are reserved in both CTAs' tensor memory at
 // the same address.
