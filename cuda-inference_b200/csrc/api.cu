@@ -525,8 +525,9 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
     if (d.flags & (GIEB_FLAG_WEIGHTS_PREPACKED | GIEB_FLAG_INPUT_NHWC | GIEB_FLAG_OUTPUT_NHWC | GIEB_FLAG_RESIDUAL))
       return no("prepacked weights, channel-contiguous tensors and the fused residual apply to the 16-bit tensor path only");
     r->variant = 3;
-    r->tile_m = conv_fp32_tile_pixels(d.out_channels);
-    r->tile_n = conv_fp32_tile_channels(d.out_channels);
+    const Fp32Choice choice = conv_fp32_choose(g.pixels, d.in_channels, d.kernel_h, d.kernel_w, d.out_channels);
+    r->tile_m = choice.tile_p;
+    r->tile_n = choice.tile_o;
     r->tile_k = 16;
     r->stages = 2;
     r->split_k = 1;
@@ -823,7 +824,7 @@ void fill_info(const gieb_conv_desc& d, const Resolved& r, gieb_conv_info* out) 
   if (r.variant == 3) {
     out->dynamic_smem_bytes = 0;
     out->threads_per_block = 128;
-    out->num_blocks = conv_fp32_num_blocks(g.pixels, d.out_channels);
+    out->num_blocks = int64_t(ceil_div(g.pixels, r.tile_m)) * ceil_div(d.out_channels, r.tile_n);
     out->launches = 1;
   } else {
     out->dynamic_smem_bytes = uint32_t(r.smem);

@@ -326,33 +326,60 @@ conv_fp32_kernel(const Fp32Args a) {
 int tile_o(int o) { return o <= 32 ? 32 : 64; }
 int tile_p(int o) { return o <= 32 ? 128 : 64; }
 
-// CTAs that share one output tile.  The CTAs that an SM holds together hide each other's latencies: a slab costs ~1600 cycles
-// of a CTA alone on its SM, ~1100 per CTA of two and ~1030 of more; a CTA's prologue and epilogue cost ~1500 cycles, a
-// cluster's exchange ~2000 more, and up to five CTAs share an SM.
-int pick_slices(int64_t tiles, int slabs) {
-  int best = 1;
+constexpr int kMaxWideTaps = 31;  // filter taps in a pixel's bit mask (conv_fp32_wide.cu)
+
+}  // namespace
+
+// The choice by SM cycles.
+// This kernel: the CTAs that an SM holds together hide each other's latencies: a slab costs ~1600 cycles of a CTA alone on its SM,
+// ~1100 per CTA of two and ~1030 of more; a CTA's prologue and epilogue cost ~1500 cycles, a cluster's exchange ~2000 more, and up to
+// five CTAs share an SM.  Without the decode table (reductions of more than kLutMax terms per slice) everything takes twice as long.
+// The wide tiles (fitted to 230 timings of 18 layers, 7 % off on average): 16 terms of a CTA's tiles are 2048 cycles of FMA issue and
+// cost 3510 cycles of a CTA alone on its SM, 3075 each of two; ~6900 per wave of CTAs, and ~12,100 to exchange partial tiles.
+// So they are taken for long reductions and many tiles: 17 x 64 -> 109 at 69 x 38, 5x5 474 -> 402 us; 2 x 762 -> 256 at 18 x 18,
+// 3x3/2 48.3 -> 40.6; 2 x 976 -> 80 at 37 x 37, 5x5 885 -> 433; not for 64 -> 64 at 56 x 56, 3x3, one image (16.1 us; 19.9 wide).
+Fp32Choice conv_fp32_choose(int64_t pixels, int c, int r, int s, int o) {
+  const int slabs = int((int64_t(c) * r * s + kBK - 1) / kBK);
+  Fp32Choice best{0, tile_p(o), tile_o(o), 1};
   double best_t = 1e300;
-  for (int s = 1; s <= 8 && s <= slabs; ++s) {
-    const int per = (slabs + s - 1) / s;
-    if ((slabs + per - 1) / per != s) continue;  // (an empty slice)
-    const double load = double((tiles * s + kNumSms - 1) / kNumSms);
-    const double slab = load <= 1 ? 1600.0 : (load <= 2 ? 1100.0 : 1030.0);
-    const double t = load * per * slab + std::ceil(load / 5.0) * (1500.0 + (s > 1 ? 2000.0 : 0.0));
-    if (t < best_t * 0.98) { best_t = t; best = s; }
+  {
+    const int64_t tiles = ((pixels + best.tile_p - 1) / best.tile_p) * ((o + best.tile_o - 1) / best.tile_o);
+    for (int sl = 1; sl <= 8 && sl <= slabs; ++sl) {
+      const int per = (slabs + sl - 1) / sl;
+      if ((slabs + per - 1) / per != sl) continue;  // (an empty slice)
+      const double load = double((tiles * sl + kNumSms - 1) / kNumSms);
+      const double slab = load <= 1 ? 1600.0 : (load <= 2 ? 1100.0 : 1030.0);
+      const double t = load * per * slab + std::ceil(load / 5.0) * (1500.0 + (sl > 1 ? 2000.0 : 0.0));
+      if (t < best_t * 0.98) { best_t = t; best.slices = sl; }
+    }
+  }
+  if (r * s > kMaxWideTaps) return best;
+  const bool table = int64_t((slabs + best.slices - 1) / best.slices) * kBK <= kLutMax;
+  const double other = best_t * (table ? 1.0 : 2.0) + 7600.0;
+  double limit = 1e300;
+  for (int tp = 128; tp >= 64; tp /= 2) {
+    const int groups = 256 / tp;
+    const int64_t tiles = ((pixels + tp - 1) / tp) * ((o + 63) / 64);
+    for (int sl = 1; sl <= 8 && sl * groups <= slabs; ++sl) {
+      const int members = sl * groups, per = (slabs + members - 1) / members;
+      const int64_t ctas = tiles * sl, rest = ctas % (2 * kNumSms);
+      if (tiles * (sl - 1) > 6 * kNumSms) break;  // (clusters of many waves of CTAs: not measured, and splitting gains nothing)
+      const double pair = 2.0 * per * 3075.0 + 6900.0;
+      double t = double(ctas / (2 * kNumSms)) * pair + (rest > kNumSms ? pair : (rest > 0 ? per * 3510.0 + 6900.0 : 0.0));
+      if (members > 1) t += 12100.0 * double((ctas + 2 * kNumSms - 1) / (2 * kNumSms));
+      // (margins: over 24 layers seven gained 2 to 62 % and one lost 2 % with them, of 16 before four had lost 2 to 13 %)
+      if (t < limit && t < (tp == 128 ? 0.88 : 0.85) * other - 3200.0) { limit = t; best = Fp32Choice{1, tp, 64, sl}; }
+    }
   }
   return best;
 }
 
-}  // namespace
-
-int conv_fp32_tile_pixels(int o) { return tile_p(o); }
-int conv_fp32_tile_channels(int o) { return tile_o(o); }
-
-int64_t conv_fp32_num_blocks(int64_t pixels, int o) { return ((pixels + tile_p(o) - 1) / tile_p(o)) * ((o + tile_o(o) - 1) / tile_o(o)); }
-
 cudaError_t conv_fp32_launch(const void* x, const void* w, const void* bias, void* y, int batch, int c, int h, int wd, int o,
                              int r, int s, int stride_h, int stride_w, int pad_h, int pad_w, int out_h, int out_w, int relu,
                              cudaStream_t stream) {
+  const Fp32Choice choice = conv_fp32_choose(int64_t(batch) * out_h * out_w, c, r, s, o);
+  if (choice.wide)
+    return conv_fp32_wide_launch(choice, x, w, bias, y, batch, c, h, wd, o, r, s, stride_h, stride_w, pad_h, pad_w, out_h, out_w, relu, stream);
   Fp32Args a;
   a.x = static_cast<const float*>(x);
   a.w = static_cast<const float*>(w);
@@ -367,10 +394,10 @@ cudaError_t conv_fp32_launch(const void* x, const void* w, const void* bias, voi
   a.fd_s = FastDiv::make(s);
   a.fd_pq = FastDiv::make(out_h * out_w);
   a.fd_out_w = FastDiv::make(out_w);
-  const int tp = tile_p(o), to = tile_o(o);
+  const int tp = choice.tile_p, to = choice.tile_o;
   const int64_t tiles_p = (int64_t(a.pixels) + tp - 1) / tp, tiles_o = (o + to - 1) / to;
   const int slabs = (a.k + kBK - 1) / kBK;
-  a.slices = pick_slices(tiles_p * tiles_o, slabs);
+  a.slices = choice.slices;
   a.slabs_per_slice = (slabs + a.slices - 1) / a.slices;
   const bool xvec = r == 1 && s == 1 && stride_h == 1 && stride_w == 1 && pad_h == 0 && pad_w == 0 && (out_h * out_w) % 4 == 0 &&
                     (reinterpret_cast<uintptr_t>(x) & 15u) == 0;

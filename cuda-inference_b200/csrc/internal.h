@@ -282,14 +282,19 @@ cudaError_t repack_pair_launch(const void* src_a, void* dst_a, int batch_a, int 
 cudaError_t gather_rows_launch(const void* x, void* x2, int batch, int channels, int h, int w, int q, int kernel_w, int stride_w,
                                int pad_w, int c2, const void* wsrc, void* w2, int out_channels, int kernel_h, cudaStream_t stream);
 
-// FP32 SIMT implicit GEMM straight from NCHW.
+// FP32 SIMT implicit GEMM straight from NCHW.  The kernel, the tile and the CTAs of a cluster that split the reduction of a tile:
+struct Fp32Choice {
+  int wide;            // 1: conv_fp32_wide.cu (thread tiles of 16 x 8)
+  int tile_p, tile_o;  // output pixels and channels of a tile
+  int slices;
+};
+Fp32Choice conv_fp32_choose(int64_t pixels, int c, int r, int s, int o);
+cudaError_t conv_fp32_wide_launch(const Fp32Choice& ch, const void* x, const void* w, const void* bias, void* y, int batch, int c, int h, int wd,
+                                  int o, int r, int s, int stride_h, int stride_w, int pad_h, int pad_w, int out_h, int out_w, int relu,
+                                  cudaStream_t stream);
 cudaError_t conv_fp32_launch(const void* x, const void* w, const void* bias, void* y, int batch, int c, int h, int wd,
                              int o, int r, int s, int stride_h, int stride_w, int pad_h, int pad_w, int out_h, int out_w,
                              int relu, cudaStream_t stream);
-int conv_fp32_tile_pixels(int o);    // output pixels ..
-int conv_fp32_tile_channels(int o);  // .. and channels of the tile a CTA (or a cluster that splits the reduction) computes
-int64_t conv_fp32_num_blocks(int64_t pixels, int o);  // output tiles
-
 cudaError_t rmsnorm_launch(int rows, int hidden, float eps, int dtype, int gamma_fp32, const void* x, const void* gamma,
                            void* y, const void* res_in, void* res_out, cudaStream_t stream);
 
