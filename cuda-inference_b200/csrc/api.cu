@@ -677,6 +677,26 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
       if (t < best) { best = t; best_m = 2 * kTileM; best_n = tn; best_s = s; best_mode = s > 1 ? 1 : 0; best_pair = 1; }
     }
   }
+  // Tiles of the direct-NCHW route, left to the library: the narrowest of 32, 64 and 128 channels whose tiles all have an SM of
+  // their own.  Re-reading the activations costs less than the epilogue of a wide tile on few SMs (the channel tiles of the same
+  // pixels read them from L2 at the same time): 512 -> 256 channels at 28 x 28 takes 8.63 us in one tile of 256 channels, 5.18 in
+  // eight of 32 (1 image), 9.04 and 5.48 in four of 64 (4 images), 9.20 and 6.41 in two of 128 (8 images).
+  // With more tiles than SMs: 128 channels with two CTAs per SM, which hide each other's epilogues, for one or two slabs (64 -> 256
+  // at 56 x 56, 32 images 17.5 us in tiles of 256, 14.8 in tiles of 128); for longer reductions, where a CTA of 128 columns takes the
+  // SM for a deep ring (see stages_for), where it walks fewer half-width tiles (320 -> 256 at 28 x 28, 32 images 11.1 and 9.8; with
+  // as many 256 columns are up to 10 % faster) or 256 columns give a CTA a single tile (320 -> 256, 16 images 8.0 and 7.1).
+  int direct_n = 0;
+  if (r->variant == 2 && !r->tile_n && c.tile_m == 0 && c.stages == 0 && c.split_k <= 1 && c.reduce == 0 && c.cta_pair != 2) {
+    const int64_t tiles_m = ceil_div(rows, kTileM);
+    auto walks = [&](int tn) { return (tiles_m * ceil_div(d.out_channels, tn) + kNumSms - 1) / kNumSms; };  // tiles of an SM
+    for (int tn = 128; tn >= 32; tn /= 2) {
+      if (tn > 32 && tn / 2 >= d.out_channels) continue;
+      if (direct_n == 0 || walks(tn) == 1) direct_n = tn;
+    }
+    // (a residual lengthens the epilogue that a CTA alone on its SM does not hide: 224 -> 640 at 16 x 37, 25 images 22.8 us with 256, 28.2 with 128)
+    const bool fewer = walks(256) == 1 || walks(128) * 8 <= walks(256) * 14, exposed = (d.flags & GIEB_FLAG_RESIDUAL) != 0 && r->total_kb < 8;
+    if (d.out_channels > 128 && direct_n == 128 && walks(128) > 1 && r->total_kb > 2 && (exposed || !fewer)) direct_n = 256;
+  }
   for (int tm = 128; tm <= 256 && c.cta_pair != 2 && !(pair_unasked && best_pair); tm += 128) {
     if (c.tile_m && tm != c.tile_m) continue;
     if (!c.tile_m && tm == 256 && int64_t(ceil_div(g.pixels, 256)) * ceil_div(d.out_channels, 128) < 4 * kNumSms) continue;  // big tiles only where wave quantisation is negligible
@@ -684,7 +704,8 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
       const int tn = n_opts[ni];
       if (r->tile_n && tn != r->tile_n) continue;
       if (!r->tile_n && tn > 32 && tn / 2 >= d.out_channels) continue;  // never pad channels by 2x or more
-      for (int s = 1; s <= (r->strip ? 1 : 16); ++s) {   // (position strips: a CTA finishes its tiles alone)
+      if (direct_n && tn != direct_n) continue;
+      for (int s = 1; s <= (r->strip ? 1 : 16); ++s) {   // (the image kernel finishes its tiles alone)
         if (c.split_k && s != c.split_k) continue;
         if (s > 1 && r->total_kb < 2 * s) break;  // reduction too short (src/kernels/tensor_core_mma.cu:292 rule)
         const int kbs = ceil_div(r->total_kb, s);
@@ -703,7 +724,7 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
           const bool can_swap = swap_ok && s == 1 && tn >= 128;
           for (int sw = (can_swap && swap_forced ? 1 : 0); sw <= (can_swap ? 1 : 0); ++sw) {
             const double t = estimate_cycles(d, g, tm, tn, r->tile_k, s, mode, r->total_kb, sw != 0) +
-                             (r->variant == 2 && tn < d.out_channels && tn < 256 ? 1e6 : 0.0);
+                             (r->variant == 2 && !direct_n && tn < d.out_channels && tn < 256 ? 1e6 : 0.0);
             if (t < best) { best = t; best_m = tm; best_n = tn; best_s = s; best_mode = mode; best_pair = 0; best_swap = sw; }
           }
         }
@@ -738,8 +759,10 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
              : r->pair ? pick_pair_stages(r->tile_n, r->tile_k, r->kb_per_split, epi_smem)
                        : pick_stages(r->tile_m, r->tile_n, r->tile_k, r->kb_per_split, total_tiles, epi_smem);
     // Activations streamed once from DRAM (direct-NCHW route) with a long reduction: one CTA per SM with a deep ring
-    // keeps more loads in flight than two shallow ones (measured on 512 -> 128 channels at 28x28: 17.5 vs 18.4 us).
-    if (!c.stages && !r->pair && r->variant == 2 && r->kb_per_split >= 8) {
+    // keeps more loads in flight than two shallow ones (measured on 512 -> 128 channels at 28x28: 17.5 vs 18.4 us).  Two CTAs of
+    // 128 x 128 tiles hold two slabs each beside their staging: from four slabs on they are slower too (320 -> 256 at 28 x 28, 32
+    // images 13.95 us, 9.84 with one CTA and six slabs; 256 -> 512, 16 images 10.3 and 8.6).
+    if (!c.stages && !r->pair && r->variant == 2 && (r->kb_per_split >= 8 || (r->kb_per_split >= 4 && r->tile_n == 128 && r->tile_m == kTileM && !(d.flags & GIEB_FLAG_RESIDUAL)))) {
       const size_t sb = stage_bytes_of(r->tile_m, r->tile_n, r->tile_k);
       if (3072 + 6 * sb + epi_smem <= kMaxDynamicSmem) st = 6;
     }

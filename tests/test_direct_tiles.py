@@ -1,0 +1,31 @@
+"""CPU test of the tiles that the direct-NCHW route takes when they are left to the library: the narrowest of 32, 64 and 128 channels
+with at most one tile per SM; where there is none, 128 (64 or 32 where a layer has no more channels), or 256 for reductions of more
+than two slabs whose tiles of 128 channels take an SM more than 7/8 of the time that those of 256 do.  What is asked for stays."""
+SMS = 148
+
+
+def test_direct_tiles_by_the_number_of_tiles(pkg):
+    seen = set()
+    for b in (1, 2, 4, 8, 16, 64):
+        for c in (16, 64, 191, 512):
+            for h, w in ((8, 8), (24, 13), (28, 28), (56, 56)):
+                for o in (21, 37, 64, 128, 200, 256, 768):
+                    def query(**kw):
+                        return pkg.query(pkg.ConvProblem(b, c, h, w, o, 1, 1, precision=pkg.BF16, has_bias=True, relu=True), pkg.make_cfg(**kw) if kw else None)
+                    auto = query()
+                    assert auto.variant == 2 and auto.cfg.cta_pair == 1
+                    tiles_m = -(-(b * -(-(h * w) // 64)) // 2)   # 128 rows: two boxes of 64 pixels of an image
+                    widths = [n for n in (32, 64, 128) if n == 32 or n // 2 < o]
+                    walks = {n: -(-tiles_m * -(-o // n) // SMS) for n in (32, 64, 128, 256)}
+                    fitting = [n for n in widths if walks[n] == 1]
+                    want = fitting[0] if fitting else widths[-1]
+                    if not fitting and o > 128 and c > 128 and walks[256] > 1 and 8 * walks[128] > 7 * 2 * walks[256]:
+                        want = 256
+                    assert auto.cfg.tile_n == want, (b, c, h, w, o)
+                    seen.add(want)
+                    for n in (32, 64, 128, 256):
+                        asked = query(tile_n=n)
+                        assert asked.supported and asked.cfg.tile_n == n
+                    if c == 512 and o >= 64:   # (a split in clusters needs tiles of 64 channels or more: its search keeps every width)
+                        assert query(split_k=2, reduce=2).supported
+    assert seen == {32, 64, 128, 256}
