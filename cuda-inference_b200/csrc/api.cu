@@ -352,8 +352,11 @@ bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, const gieb_conv_cf
   auto taps_per_load = [&](int b_rows) { return size_t(d.kernel_w) * b_rows * 128 <= 48 * 1024 ? d.kernel_w : 1; };
   // shared memory: halo tiles, weight stages
   struct Fit { int a, b, resident; size_t smem; };
-  auto fit = [&](int bn, bool pair, int workers, size_t stage, int tpl, int loads, bool one_n, size_t budget, Fit* f) {
-    const bool staging = (d.flags & GIEB_FLAG_OUTPUT_NHWC) != 0;
+  // (The slices of a cluster store their columns directly: the staging they do not need would keep the next launch's clusters off
+  // the SMs.  512 -> 512, 7 x 7, 3x3, channel-contiguous 12.0 us with it and 8.2 without for one image, 12.4 and 8.5 for two.  Of
+  // launches that fit the machine side by side the next one is better kept off: 256 -> 256, 64 CTAs 6.24 and 6.55.)
+  auto fit = [&](int bn, bool pair, int workers, size_t stage, int tpl, int loads, bool direct, bool one_n, size_t budget, Fit* f) {
+    const bool staging = (d.flags & GIEB_FLAG_OUTPUT_NHWC) != 0 && !direct;
     for (int a = 2; a >= 1; --a) {
       const size_t fixed = conv_halo_smem_bytes(bn, pair, workers, tpl, a, stage, 0, staging);
       if (fixed >= budget) continue;
@@ -397,7 +400,7 @@ bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, const gieb_conv_cf
         // to 148 such CTAs took 1.3 (four) and 1.8 (eight) times the estimate)
         if (s >= 4 && tiles * s > 128 && !c.split_k) continue;
         Fit f;
-        if (!fit(bn, pair != 0, workers, stage, tpl, per, s == 1 && tiles_n == 1, kMaxDynamicSmem, &f)) continue;
+        if (!fit(bn, pair != 0, workers, stage, tpl, per, s > 1 && 2 * tiles * s > kNumSms, s == 1 && tiles_n == 1, kMaxDynamicSmem, &f)) continue;
         const double load = double((tiles * s + sms - 1) / sms);
         // Cycles, in the terms of estimate_cycles(), fitted to clock stamps and to the times of ~90 layers: an instruction of
         // 32 bytes along K takes `step` cycles (shared-memory reads of shifted rows), a round of up to two weight loads ~230
