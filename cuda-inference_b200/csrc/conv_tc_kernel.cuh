@@ -112,25 +112,40 @@ __device__ __forceinline__ void store_chunk_tail(const uint32_t (&v)[32], const 
   }
 }
 
-// A chunk with a residual in the output's own layout.  Nothing proves to the compiler that the residual and the output do not
-// overlap, so written as one loop every load would wait for the store before it: the loads of eight channels are issued as a
-// group, then their eight stores.  In a partial chunk (FULL false) the channels beyond it read the last valid one: guarded one by
-// one, its loads took a round trip each (64 -> 44 channels at 29 x 29, 119 images, 3x3: 52.5 us, 30.3 so).
-template <typename T, bool RELU, bool FULL>
-__device__ __forceinline__ void store_chunk_res(const uint32_t (&v)[32], const float* __restrict__ bias, T* dst, const T* res, int64_t stride,
-                                                int nvalid) {
+// A full chunk with a residual in the output's own layout.  Nothing proves to the compiler that the residual and the output
+// do not overlap, so written as one loop every load would wait for the store before it: the loads of eight channels are
+// issued as a group, then their eight stores.
+template <typename T, bool RELU>
+__device__ __forceinline__ void store_chunk_full_res(const uint32_t (&v)[32], const float* __restrict__ bias, T* dst, const T* res,
+                                                     int64_t stride) {
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
-    if (!FULL && g * 8 >= nvalid) break;
     float r[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) r[j] = load_as_float(res + int64_t(FULL ? g * 8 + j : min(g * 8 + j, nvalid - 1)) * stride);
+    for (int j = 0; j < 8; ++j) r[j] = load_as_float(res + int64_t(g * 8 + j) * stride);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       float a = __uint_as_float(v[g * 8 + j]) + bias[g * 8 + j] + r[j];
       if (RELU) a = fmaxf(a, 0.f);
-      if (FULL || g * 8 + j < nvalid) dst[int64_t(g * 8 + j) * stride] = round_to<T>(a);
+      dst[int64_t(g * 8 + j) * stride] = round_to<T>(a);
     }
+  }
+}
+
+// The residual of a partial chunk, added to its sums ahead of the stores: channels beyond the chunk read the last valid one, so that
+// the loads of eight go out together.  (Read one by one between the stores they took a round trip each: 64 -> 44 channels at 29 x 29,
+// 119 images, 3x3 52.5 us, 30 so.  In the stores' own loop, once more for either activation, the code made halo layers without a
+// residual 1 to 3 % slower.)
+template <typename T>
+__device__ __forceinline__ void add_residual_tail(uint32_t (&v)[32], const T* res, int64_t stride, int nvalid) {
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    if (g * 8 >= nvalid) break;
+    float r[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) r[j] = load_as_float(res + int64_t(min(g * 8 + j, nvalid - 1)) * stride);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[g * 8 + j] = __float_as_uint(__uint_as_float(v[g * 8 + j]) + r[j]);
   }
 }
 
@@ -263,7 +278,7 @@ __device__ __forceinline__ void row_to_staging(const uint32_t (&v)[32], float bi
 // dst / res point at the first element of the chunk for this row; consecutive channels are `stride` elements apart
 // (P*Q for NCHW, 1 for channel-contiguous output).
 template <typename T>
-__device__ __forceinline__ void store_chunk(const uint32_t (&v)[32], const float* bias, T* dst, const T* res, int64_t stride,
+__device__ __forceinline__ void store_chunk(uint32_t (&v)[32], const float* bias, T* dst, const T* res, int64_t stride,
                                             int nvalid, int relu) {
   if constexpr (sizeof(T) == 2) {
     if (nvalid == 32 && stride == 1 && ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(res)) & 15u) == 0) {
@@ -277,18 +292,14 @@ __device__ __forceinline__ void store_chunk(const uint32_t (&v)[32], const float
       return;
     }
   }
-  if (res != nullptr) {
-    if (nvalid == 32) {
-      if (relu) store_chunk_res<T, true, true>(v, bias, dst, res, stride, nvalid);
-      else store_chunk_res<T, false, true>(v, bias, dst, res, stride, nvalid);
-    } else {
-      if (relu) store_chunk_res<T, true, false>(v, bias, dst, res, stride, nvalid);
-      else store_chunk_res<T, false, false>(v, bias, dst, res, stride, nvalid);
-    }
-  } else if (nvalid == 32) {
+  if (nvalid == 32 && res == nullptr) {
     if (relu) store_chunk_full<T, true>(v, bias, dst, stride);
     else store_chunk_full<T, false>(v, bias, dst, stride);
+  } else if (nvalid == 32) {
+    if (relu) store_chunk_full_res<T, true>(v, bias, dst, res, stride);
+    else store_chunk_full_res<T, false>(v, bias, dst, res, stride);
   } else {
+    if (res != nullptr) add_residual_tail(v, res, stride, nvalid);
     if (relu) store_chunk_tail<T, true>(v, bias, dst, stride, nvalid);
     else store_chunk_tail<T, false>(v, bias, dst, stride, nvalid);
   }
