@@ -697,8 +697,9 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
       if (direct_n == 0 || walks(tn) == 1) direct_n = tn;
     }
     // (a residual lengthens the epilogue that a CTA alone on its SM does not hide: 224 -> 640 at 16 x 37, 25 images 22.8 us with 256, 28.2 with 128)
+    // (up to 192 channels the second tile of 128 is at least half empty: 64 -> 160 at 60 x 60, 141 images, residual 162 and 180 us)
     const bool fewer = walks(256) == 1 || walks(128) * 8 <= walks(256) * 14, exposed = (d.flags & GIEB_FLAG_RESIDUAL) != 0 && r->total_kb < 8;
-    if (d.out_channels > 128 && direct_n == 128 && walks(128) > 1 && r->total_kb > 2 && (exposed || !fewer)) direct_n = 256;
+    if (d.out_channels > 128 && direct_n == 128 && walks(128) > 1 && (r->total_kb > 2 ? exposed || !fewer : d.out_channels <= 192)) direct_n = 256;
   }
   for (int tm = 128; tm <= 256 && c.cta_pair != 2 && !(pair_unasked && best_pair); tm += 128) {
     if (c.tile_m && tm != c.tile_m) continue;
