@@ -8,8 +8,8 @@
 // load and a store, and a decoded (c, r, s) entry serves two pixels; weights are stored [k][channel], so eight of them are two reads.
 // In the end the loop takes 1.5 times its FMA issue (3075 cycles per 2048, two CTAs per SM; 8 x 4 tiles take 2.0 times), and a CTA's
 // first loads and last stores ~6900 cycles: see conv_fp32_choose() for where it is taken and what it gains.
-// A CTA has 128 threads in KG groups, which compute the same TP x 64 tile over slices of the reduction of their own (KG * TP = 256: two of 128 pixels, or four of 64);
-// a cluster of `slices` CTAs splits it further.  The partial tiles are added in slice order: results are run-to-run identical.
+// A CTA has 128 threads in KG groups, which compute the same TP x 64 tile over slices of the reduction of their own (KG * TP = 256: two
+// groups and 128 pixels, or four and 64); a cluster of `slices` CTAs splits it further.  The partial tiles are added in slice order: results are run-to-run identical.
 #include <stdint.h>
 
 #include <type_traits>
