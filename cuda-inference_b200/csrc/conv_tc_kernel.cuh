@@ -134,7 +134,7 @@ __device__ __forceinline__ void store_chunk_full_res(const uint32_t (&v)[32], co
 
 // The residual of a partial chunk, added to its sums ahead of the stores: channels beyond the chunk read the last valid one, so that
 // the loads of eight go out together.  (Read one by one between the stores they took a round trip each: 64 -> 44 channels at 29 x 29,
-// 119 images, 3x3 52.5 us, 30 so.  In the stores' own loop, once more for either activation, the code made halo layers without a
+// 119 images, 3x3 53.5 us, 34.6 so.  In the stores' own loop, once more for either activation, the code made halo layers without a
 // residual 1 to 3 % slower.)
 template <typename T>
 __device__ __forceinline__ void add_residual_tail(uint32_t (&v)[32], const T* res, int64_t stride, int nvalid) {
