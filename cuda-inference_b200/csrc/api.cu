@@ -701,6 +701,14 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
     const bool fewer = walks(256) == 1 || walks(128) * 8 <= walks(256) * 14, exposed = (d.flags & GIEB_FLAG_RESIDUAL) != 0 && r->total_kb < 8;
     if (d.out_channels > 128 && direct_n == 128 && walks(128) > 1 && (r->total_kb > 2 ? exposed || !fewer : d.out_channels <= 192)) direct_n = 256;
   }
+  // 1x1 layers of one or two slabs over a channel-contiguous tensor (or its copy), left to the library: with more than two tiles of
+  // 32 channels per SM those of 64 are faster (9 x 16 -> 895 at 10 x 19 10.3 and 6.8 us, 2 x 16 -> 448 at 82 x 82 13.1 and 9.2,
+  // 68 x 64 -> 64 at 26 x 26 6.3 and 5.2, 54 x 124 -> 640 at 7 x 7 9.1 and 7.7; with fewer, 32 are as fast or faster).  Tiles of 256
+  // pixels and 128 channels fill tensor memory with the accumulators of one CTA per SM and lose to 128 pixels where the reduction is
+  // this short (58 x 64 -> 640 at 61 x 61 103 and 72 us).
+  const bool short_pointwise = r->variant == 4 && r->total_kb <= 2 && !r->tile_n && c.tile_m == 0 && c.stages == 0 && c.split_k <= 1 && c.reduce == 0 &&
+                               c.cta_pair != 2;
+  const bool no_32 = short_pointwise && d.out_channels > 32 && int64_t(ceil_div(rows, kTileM)) * ceil_div(d.out_channels, 32) > 2 * kNumSms;
   for (int tm = 128; tm <= 256 && c.cta_pair != 2 && !(pair_unasked && best_pair); tm += 128) {
     if (c.tile_m && tm != c.tile_m) continue;
     if (!c.tile_m && tm == 256 && int64_t(ceil_div(g.pixels, 256)) * ceil_div(d.out_channels, 128) < 4 * kNumSms) continue;  // big tiles only where wave quantisation is negligible
@@ -709,6 +717,7 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
       if (r->tile_n && tn != r->tile_n) continue;
       if (!r->tile_n && tn > 32 && tn / 2 >= d.out_channels) continue;  // never pad channels by 2x or more
       if (direct_n && tn != direct_n) continue;
+      if ((no_32 && tn == 32) || (short_pointwise && tm == 256 && tn == 128)) continue;
       for (int s = 1; s <= (r->strip ? 1 : 16); ++s) {   // (the image kernel finishes its tiles alone)
         if (c.split_k && s != c.split_k) continue;
         if (s > 1 && r->total_kb < 2 * s) break;  // reduction too short (src/kernels/tensor_core_mma.cu:292 rule)

@@ -30,3 +30,25 @@ def test_direct_tiles_by_the_number_of_tiles(pkg):
                     if c == 512 and o >= 64:   # (a split in clusters needs tiles of 64 channels or more: its search keeps every width)
                         assert query(split_k=2, reduce=2).supported
     assert seen == {32, 64, 128, 256}
+
+
+def test_short_pointwise_tiles(pkg):
+    """1x1 layers of one or two slabs over channel-contiguous tensors: no tiles of 32 channels beyond two of them per SM, none of 256
+    pixels and 128 channels; what is asked for stays."""
+    seen = set()
+    for b in (1, 3, 9, 30, 58, 128):
+        for c in (16, 64, 128):
+            for h, w in ((7, 7), (10, 19), (33, 33), (61, 61)):
+                for o in (24, 64, 192, 640, 896):
+                    def query(**kw):
+                        return pkg.query(pkg.ConvProblem(b, c, h, w, o, 1, 1, precision=pkg.FP16, has_bias=True, relu=True, flags=pkg.FLAG_INPUT_NHWC | pkg.FLAG_OUTPUT_NHWC),
+                                         pkg.make_cfg(**kw) if kw else None)
+                    cfg = query().cfg
+                    if cfg.cta_pair == 2:
+                        continue
+                    if o > 32 and -(-(b * h * w) // 128) * -(-o // 32) > 2 * SMS:
+                        assert cfg.tile_n != 32, (b, c, h, w, o)
+                    assert (cfg.tile_m, cfg.tile_n) != (256, 128), (b, c, h, w, o)
+                    assert query(tile_n=32).cfg.tile_n == 32 and query(tile_m=256, tile_n=128).cfg.tile_m == 256
+                    seen.add((cfg.tile_m, cfg.tile_n))
+    assert {(128, 32), (128, 64), (128, 128)} <= seen
