@@ -1341,7 +1341,7 @@ int launch_impl(const gieb_conv_plan* pl, const void* x, const void* w, const vo
 // Opts every kernel that launches of this configuration may take in to large dynamic shared memory.
 cudaError_t prepare_kernels(const Resolved& r) {
   if (r.variant == 3) return cudaSuccess;
-  if (r.image) return conv_image_prepare(r.gp_t, r.im_smem);
+  if (r.image) return conv_image_prepare(r.gp_t);
   if (r.halo) return conv_halo_prepare(r.tile_n, r.epi_warps, r.pair != 0, kMaxDynamicSmem);
   // The general kernel: a partial last slab, or rows that TMA cannot store (which tensors off their alignment are as well).
   const bool tail = r.tile_k == 64 && r.c_padded % 64 != 0;

@@ -329,8 +329,9 @@ size_t conv_image_smem_bytes(int kernel_h, int t_positions, size_t strip_stage_b
   return kImageCtrl + size_t(kernel_h) * t_positions * (kImageCols * 16) + 2 * strip_stage_bytes + (staging ? size_t(kImageWorkers) * 4096 : 0);
 }
 
-cudaError_t conv_image_prepare(int t_positions, size_t smem) {
-  const auto set = [&](auto kernel) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)); };
+cudaError_t conv_image_prepare(int t_positions) {
+  // (the limit belongs to the function and is replaced by each call: every plan sets the same one, so that none lowers another's)
+  const auto set = [&](auto kernel) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kCtaSmemLimit)); };
   return t_positions == 2 ? set(conv_image_kernel<2>) : (t_positions == 4 ? set(conv_image_kernel<4>) : set(conv_image_kernel<8>));
 }
 

@@ -209,7 +209,7 @@ struct ConvImageParams {
 };
 // t_positions: positions per window, 2, 4 or 8
 size_t conv_image_smem_bytes(int kernel_h, int t_positions, size_t strip_stage_bytes, bool staging);
-cudaError_t conv_image_prepare(int t_positions, size_t smem);
+cudaError_t conv_image_prepare(int t_positions);
 cudaError_t conv_image_launch(int t_positions, const ConvImageParams& p, dim3 grid, size_t smem, cudaStream_t stream);
 
 // tile_m is 128 or 256 output pixels per CTA (one or two TMEM accumulators sharing each weight tile).

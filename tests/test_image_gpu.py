@@ -83,3 +83,30 @@ def test_expired_waits_are_reported(pkg, orc, oracle, roles):
     got, _, _ = gu.run_conv(pkg, oracle, p, x, w, b, plan=pkg.ConvPlan(gu.pkg_problem(pkg, p)))
     m = oracle.compare(p, got, ref, scale)
     assert m.passed(), m.summary()
+
+
+def test_plans_of_other_sizes_leave_a_plan_alone(pkg, orc, oracle):
+    """A plan keeps working when plans and allocation-free calls of the same window width that ask for less shared memory come after it
+    (600 columns: 107,264 bytes; 64: 40,704)."""
+    def problem(args, seed):
+        p = orc.Problem.P(*args, precision=orc.FP16, bias=True, relu=True)
+        x, w, b = oracle.make_conv_data(p, seed, 1)
+        return p, x, w, b, oracle.conv2d(p, x, w, b)
+    large = problem((1, 3, 23, 600, 40, 7, 7, 2, 2, 3, 3), 7300)
+    small = problem((1, 3, 64, 64, 64, 7, 7, 2, 2, 3, 3), 7301)
+    plans = [pkg.ConvPlan(gu.pkg_problem(pkg, large[0])), pkg.ConvPlan(gu.pkg_problem(pkg, small[0]))]
+
+    def check(plan, data):
+        p, x, w, b, (ref, scale) = data
+        got, _, _ = gu.run_conv(pkg, oracle, p, x, w, b, plan=plan)
+        m = oracle.compare(p, got, ref, scale)
+        assert m.passed(), m.summary()
+    check(plans[0], large)
+    check(plans[1], small)
+    check(plans[0], large)
+    p, x, w, b, _ = small
+    bufs = [gu.to_device_storage(oracle, p.precision, a) for a in (x, w, b)]
+    out = gu.OutBuf(p.precision, int(np.prod(p.y_shape)))
+    pkg.conv_forward_static(gu.pkg_problem(pkg, p), bufs[0][1], bufs[1][1], bufs[2][1], out.ptr, 0)
+    assert pkg.conv_static_status(0) == 0
+    check(plans[0], large)
