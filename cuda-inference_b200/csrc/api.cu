@@ -528,7 +528,7 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
     if (d.flags & (GIEB_FLAG_WEIGHTS_PREPACKED | GIEB_FLAG_INPUT_NHWC | GIEB_FLAG_OUTPUT_NHWC | GIEB_FLAG_RESIDUAL))
       return no("prepacked weights, channel-contiguous tensors and the fused residual apply to the 16-bit tensor path only");
     r->variant = 3;
-    const Fp32Choice choice = conv_fp32_choose(g.pixels, d.in_channels, d.kernel_h, d.kernel_w, d.out_channels);
+    const Fp32Choice choice = conv_fp32_choose(g.pixels, d.in_channels, d.in_h, d.in_w, d.kernel_h, d.kernel_w, d.out_channels);
     r->tile_m = choice.tile_p;
     r->tile_n = choice.tile_o;
     r->tile_k = 16;

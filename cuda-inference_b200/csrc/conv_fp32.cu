@@ -338,7 +338,7 @@ constexpr int kMaxWideTaps = 31;  // filter taps in a pixel's bit mask (conv_fp3
 // cost 3510 cycles of a CTA alone on its SM, 3075 each of two; ~6900 per wave of CTAs, and ~12,100 to exchange partial tiles.
 // So they are taken for long reductions and many tiles: 17 x 64 -> 109 at 69 x 38, 5x5 474 -> 402 us; 2 x 762 -> 256 at 18 x 18,
 // 3x3/2 48.3 -> 40.6; 2 x 976 -> 80 at 37 x 37, 5x5 885 -> 433; not for 64 -> 64 at 56 x 56, 3x3, one image (16.1 us; 19.9 wide).
-Fp32Choice conv_fp32_choose(int64_t pixels, int c, int r, int s, int o) {
+Fp32Choice conv_fp32_choose(int64_t pixels, int c, int h, int w, int r, int s, int o) {
   const int slabs = int((int64_t(c) * r * s + kBK - 1) / kBK);
   Fp32Choice best{0, tile_p(o), tile_o(o), 1};
   double best_t = 1e300;
@@ -353,7 +353,7 @@ Fp32Choice conv_fp32_choose(int64_t pixels, int c, int r, int s, int o) {
       if (t < best_t * 0.98) { best_t = t; best.slices = sl; }
     }
   }
-  if (r * s > kMaxWideTaps) return best;
+  if (r * s > kMaxWideTaps || !conv_fp32_wide_offsets_fit(c, h, w, r, s)) return best;
   const bool table = int64_t((slabs + best.slices - 1) / best.slices) * kBK <= kLutMax;
   const double other = best_t * (table ? 1.0 : 2.0) + 7600.0;
   double limit = 1e300;
@@ -377,7 +377,7 @@ Fp32Choice conv_fp32_choose(int64_t pixels, int c, int r, int s, int o) {
 cudaError_t conv_fp32_launch(const void* x, const void* w, const void* bias, void* y, int batch, int c, int h, int wd, int o,
                              int r, int s, int stride_h, int stride_w, int pad_h, int pad_w, int out_h, int out_w, int relu,
                              cudaStream_t stream) {
-  const Fp32Choice choice = conv_fp32_choose(int64_t(batch) * out_h * out_w, c, r, s, o);
+  const Fp32Choice choice = conv_fp32_choose(int64_t(batch) * out_h * out_w, c, h, wd, r, s, o);
   if (choice.wide)
     return conv_fp32_wide_launch(choice, x, w, bias, y, batch, c, h, wd, o, r, s, stride_h, stride_w, pad_h, pad_w, out_h, out_w, relu, stream);
   Fp32Args a;

@@ -1,5 +1,5 @@
-// When the strict-FP32 kernel may decode its reduction indices through a table (conv_fp32.cu).  Host code only: the rule is
-// compiled by itself in the CPU tests.
+// When the strict-FP32 kernels may decode their reduction indices through tables (conv_fp32.cu, conv_fp32_wide.cu).  Host code only:
+// the rules are compiled by themselves in the CPU tests.
 #ifndef GIEB_CONV_FP32_TABLE_H_
 #define GIEB_CONV_FP32_TABLE_H_
 
@@ -15,6 +15,12 @@ constexpr int kNoRow = 0x7fff;   // filter row of a table entry beyond the reduc
 // topmost output row it is kNoRow - pad_h, which lies below the image as long as h + pad_h <= kNoRow.
 inline bool conv_fp32_table_fits(int64_t terms, int c, int h, int w, int r, int s, int pad_h) {
   return terms <= kLutMax && int64_t(c) * h * w < (int64_t(1) << 31) && r < kNoRow && s <= 0xffff && int64_t(h) + pad_h <= kNoRow;
+}
+
+// Whether the wide kernel (conv_fp32_wide.cu) may hold the offsets of its terms in 32 bits: an entry is the offset of (c, r, s) from
+// the window's corner, which may lie in the padding, so the largest exceeds the image's own size by up to r rows and s columns.
+inline bool conv_fp32_wide_offsets_fit(int c, int h, int w, int r, int s) {
+  return ((int64_t(c) - 1) * h + r - 1) * w + s - 1 < (int64_t(1) << 31);
 }
 
 }  // namespace gieb

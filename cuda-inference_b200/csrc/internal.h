@@ -288,7 +288,7 @@ struct Fp32Choice {
   int tile_p, tile_o;  // output pixels and channels of a tile
   int slices;
 };
-Fp32Choice conv_fp32_choose(int64_t pixels, int c, int r, int s, int o);
+Fp32Choice conv_fp32_choose(int64_t pixels, int c, int h, int w, int r, int s, int o);
 cudaError_t conv_fp32_wide_launch(const Fp32Choice& ch, const void* x, const void* w, const void* bias, void* y, int batch, int c, int h, int wd,
                                   int o, int r, int s, int stride_h, int stride_w, int pad_h, int pad_w, int out_h, int out_w, int relu,
                                   cudaStream_t stream);

@@ -41,3 +41,44 @@ def test_entries_beyond_the_reduction_never_read(tmp_path):
     subprocess.check_call(["g++", "-std=c++17", "-Wall", "-Werror", "-I" + os.path.join(ROOT, "cuda-inference_b200", "csrc"), str(src), "-o", str(exe)])
     r = subprocess.run([str(exe)], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout
+
+
+WIDE_PROGRAM = r"""
+#include "conv_fp32_table.h"
+#include <cstdio>
+using namespace gieb;
+int main() {
+  // {c, h, w, r, s}: images of up to 2^31 - 1 values, windows that reach into the padding
+  const int shapes[][5] = {{64, 56, 56, 3, 3}, {3243932, 2, 331, 3, 3}, {3243933, 2, 331, 3, 3}, {1, 1, 2147483646, 3, 3}, {1, 1, 2147483646, 1, 1}, {2147483647, 1, 1, 1, 1},
+                           {64, 5792, 5792, 5, 5}, {1, 1, 200000000, 31, 1}, {1, 46340, 46341, 1, 31}, {16777215, 128, 1, 3, 3}, {2097152, 1, 1023, 3, 5}};
+  int accepted = 0, refused = 0, bad = 0;
+  for (const auto& d : shapes) {
+    long long most = 0;
+    for (int r = 0; r < d[3]; ++r)
+      for (int s = 0; s < d[4]; ++s) {
+        const long long offset = ((d[0] - 1LL) * d[1] + r) * d[2] + s;  // the last channel's
+        if (offset > most) most = offset;
+      }
+    const bool fits = conv_fp32_wide_offsets_fit(d[0], d[1], d[2], d[3], d[4]);
+    ++(fits ? accepted : refused);
+    if (fits != (most <= 2147483647LL)) { ++bad; std::printf("c %d h %d w %d r %d s %d: largest offset %lld\n", d[0], d[1], d[2], d[3], d[4], most); }
+  }
+  std::printf("%d accepted, %d refused, %d bad\n", accepted, refused, bad);
+  return bad != 0 || accepted < 3 || refused < 3;
+}
+"""
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+def test_offsets_of_the_wide_kernel_fit_32_bits(tmp_path):
+    src, exe = tmp_path / "wide.cpp", tmp_path / "wide"
+    src.write_text(WIDE_PROGRAM)
+    subprocess.check_call(["g++", "-std=c++17", "-Wall", "-Werror", "-I" + os.path.join(ROOT, "cuda-inference_b200", "csrc"), str(src), "-o", str(exe)])
+    r = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
+
+
+def test_wide_tiles_leave_images_whose_offsets_do_not_fit(pkg):
+    """One channel more than fits, and the kernel that indexes in 64 bits takes the layer (tiles of 64 pixels instead of 128)."""
+    tiles = [pkg.query(pkg.ConvProblem(8, c, 2, 331, 64, 3, 3, 1, 1, 1, 1, precision=pkg.FP32)).cfg.tile_m for c in (3243932, 3243933)]
+    assert tiles == [128, 64]
