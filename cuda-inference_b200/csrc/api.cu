@@ -352,9 +352,13 @@ bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, const gieb_conv_cf
   auto taps_per_load = [&](int b_rows) { return size_t(d.kernel_w) * b_rows * 128 <= 48 * 1024 ? d.kernel_w : 1; };
   // shared memory: halo tiles, weight stages
   struct Fit { int a, b, resident; size_t smem; };
-  // (The slices of a cluster store their columns directly: the staging they do not need would keep the next launch's clusters off
-  // the SMs.  512 -> 512, 7 x 7, 3x3, channel-contiguous 12.0 us with it and 8.2 without for one image, 12.4 and 8.5 for two.  Of
-  // launches that fit the machine side by side the next one is better kept off: 256 -> 256, 64 CTAs 6.24 and 6.55.)
+  // (The slices of a cluster store their columns directly and never touch the staging.  With it a CTA of a narrow tile asks for more
+  // than half of an SM, which keeps the CTAs of a launch apart; without it two lie on one SM while others have none.  FP16, 3x3,
+  // channel-contiguous, launches in a row and, in brackets, with another kernel between them: 2 x 256 -> 256 at 14 x 14, 32 clusters
+  // of four 7.1 us with and 9.7 without (11.0, 12.5), 5 x 768 -> 64 at 10 x 10, ten of eight 7.9 and 10.1 (11.7, 13.5).  But of
+  // clusters of eight, 15 fit the machine with one CTA per SM, of four 33, of two 74 (cudaOccupancyMaxActiveClusters): the rest wait
+  // for a second wave unless two CTAs share an SM, 3 x 512 -> 64 at 17 x 17, 16 of eight 12.0 and 8.6 (15.0, 11.8).  So `direct`,
+  // without staging, is for more clusters than that.)
   auto fit = [&](int bn, bool pair, int workers, size_t stage, int tpl, int loads, bool direct, bool one_n, size_t budget, Fit* f) {
     const bool staging = (d.flags & GIEB_FLAG_OUTPUT_NHWC) != 0 && !direct;
     for (int a = 2; a >= 1; --a) {
@@ -399,8 +403,9 @@ bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, const gieb_conv_cf
         // (a GPC holds two clusters of eight or four of four: beyond 128 CTAs the rest wait for a second wave, and layers of 129
         // to 148 such CTAs took 1.3 (four) and 1.8 (eight) times the estimate)
         if (s >= 4 && tiles * s > 128 && !c.split_k) continue;
+        const bool direct = s > 1 && tiles > (s == 8 ? 15 : (s == 4 ? 33 : 74));
         Fit f;
-        if (!fit(bn, pair != 0, workers, stage, tpl, per, s > 1 && 2 * tiles * s > kNumSms, s == 1 && tiles_n == 1, kMaxDynamicSmem, &f)) continue;
+        if (!fit(bn, pair != 0, workers, stage, tpl, per, direct, s == 1 && tiles_n == 1, kMaxDynamicSmem, &f)) continue;
         const double load = double((tiles * s + sms - 1) / sms);
         // Cycles, in the terms of estimate_cycles(), fitted to clock stamps and to the times of ~90 layers: an instruction of
         // 32 bytes along K takes `step` cycles (shared-memory reads of shifted rows), a round of up to two weight loads ~230
