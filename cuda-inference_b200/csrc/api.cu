@@ -135,7 +135,13 @@ struct Resolved {
   int h_box_h, h_boxes;                          // padded rows per TMA box, boxes per phase
   int h_a_stages, h_taps_per_load, h_tap_groups, h_total_loads, h_loads_per_split, h_last_ksteps, h_resident;
   size_t h_stage_bytes;
+  Fp32Choice fp32;  // variant 3
 };
+
+Fp32Shape fp32_shape(const gieb_conv_desc& d, const Geometry& g) {
+  return Fp32Shape{d.batch,    d.in_channels, d.in_h,     d.in_w,  d.out_channels, d.kernel_h, d.kernel_w,
+                   d.stride_h, d.stride_w,    d.pad_h, d.pad_w, g.out_h,        g.out_w};
+}
 
 // Input channels in 2-byte units (FP8 values count half, TF32 values twice).
 int channel_units(const gieb_conv_desc& d) {
@@ -533,9 +539,9 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
     if (d.flags & (GIEB_FLAG_WEIGHTS_PREPACKED | GIEB_FLAG_INPUT_NHWC | GIEB_FLAG_OUTPUT_NHWC | GIEB_FLAG_RESIDUAL))
       return no("prepacked weights, channel-contiguous tensors and the fused residual apply to the 16-bit tensor path only");
     r->variant = 3;
-    const Fp32Choice choice = conv_fp32_choose(g.pixels, d.in_channels, d.in_h, d.in_w, d.kernel_h, d.kernel_w, d.out_channels);
-    r->tile_m = choice.tile_p;
-    r->tile_n = choice.tile_o;
+    r->fp32 = conv_fp32_choose(fp32_shape(d, g));
+    r->tile_m = r->fp32.tile_p;
+    r->tile_n = r->fp32.tile_o;
     r->tile_k = 16;
     r->stages = 2;
     r->split_k = 1;
@@ -863,9 +869,9 @@ void fill_info(const gieb_conv_desc& d, const Resolved& r, gieb_conv_info* out) 
   out->persistent_bytes = sizeof(uint32_t);
   out->padded_channels = d.precision == GIEB_TF32 ? r.c_padded / 2 : (d.precision == GIEB_FP8_E4M3 ? r.c_padded * 2 : r.c_padded);
   if (r.variant == 3) {
-    out->dynamic_smem_bytes = 0;
+    out->dynamic_smem_bytes = uint32_t(conv_fp32_smem_bytes(r.fp32, fp32_shape(d, g)));
     out->threads_per_block = 128;
-    out->num_blocks = int64_t(ceil_div(g.pixels, r.tile_m)) * ceil_div(d.out_channels, r.tile_n);
+    out->num_blocks = int64_t(ceil_div(g.pixels, r.tile_m)) * ceil_div(d.out_channels, r.tile_n) * r.fp32.slices;
     out->launches = 1;
   } else {
     out->dynamic_smem_bytes = uint32_t(r.smem);
@@ -1168,8 +1174,7 @@ int launch_impl(const gieb_conv_plan* pl, const void* x, const void* w, const vo
 
   if (r.variant == 3) {
     if (ev) { GIEB_CUDA(cudaEventRecord(ev[0], st)); GIEB_CUDA(cudaEventRecord(ev[1], st)); }
-    GIEB_CUDA(conv_fp32_launch(x, w, bias, y, d.batch, d.in_channels, d.in_h, d.in_w, d.out_channels, d.kernel_h, d.kernel_w,
-                               d.stride_h, d.stride_w, d.pad_h, d.pad_w, pl->g.out_h, pl->g.out_w, d.relu, st));
+    GIEB_CUDA(conv_fp32_launch(r.fp32, fp32_shape(d, pl->g), x, w, bias, y, d.relu, st));
     if (ev) { GIEB_CUDA(cudaEventRecord(ev[2], st)); GIEB_CUDA(cudaEventRecord(ev[3], st)); }
     return GIEB_OK;
   }
@@ -1345,7 +1350,7 @@ int launch_impl(const gieb_conv_plan* pl, const void* x, const void* w, const vo
 
 // Opts every kernel that launches of this configuration may take in to large dynamic shared memory.
 cudaError_t prepare_kernels(const Resolved& r) {
-  if (r.variant == 3) return cudaSuccess;
+  if (r.variant == 3) return r.fp32.wide ? conv_fp32_wide_prepare(r.fp32.tile_p) : cudaSuccess;
   if (r.image) return conv_image_prepare(r.gp_t);
   if (r.halo) return conv_halo_prepare(r.tile_n, r.epi_warps, r.pair != 0, kMaxDynamicSmem);
   // The general kernel: a partial last slab, or rows that TMA cannot store (which tensors off their alignment are as well).

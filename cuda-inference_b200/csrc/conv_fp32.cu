@@ -22,6 +22,7 @@
 #include <type_traits>
 #include <utility>
 
+#include "conv_fp32_device.cuh"
 #include "conv_fp32_table.h"
 #include "internal.h"
 #include "ptx.cuh"
@@ -45,14 +46,9 @@ struct Fp32Args {
   FastDiv fd_rs, fd_s, fd_pq, fd_out_w;  // multiply-high reciprocals of r*s, s, out_h*out_w, out_w
 };
 
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 // 4-byte asynchronous copy global -> shared; `valid` false writes zero (nothing is read: the source size is 0).
 __device__ __forceinline__ void cp_async4(void* dst, const float* src, bool valid) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(valid ? 4 : 0) : "memory");
-}
-// 16-byte asynchronous copy (both addresses 16-byte aligned); `bytes` of the source are read, the rest is zero-filled.
-__device__ __forceinline__ void cp_async16(void* dst, const float* src, int bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(bytes) : "memory");
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(ptx::smem_u32(dst)), "l"(src), "r"(valid ? 4 : 0) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -61,19 +57,6 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 constexpr int kWPitch = kBK + 4;  // floats per weight row in shared memory: 16-byte aligned rows, conflict-free 128-bit reads
 constexpr int kThreads = 128;
 constexpr int kRing = 4;          // slabs in shared memory
-
-// Two FP32 values in one 64-bit register: the operands of fma.rn.f32x2.
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ float2 unpack2(uint64_t v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
 
 // X slab [kBK][TP]: gathered from NCHW element by element with zeros for padding (pixels contiguous), or, for unpadded 1x1
 //   kernels of stride 1 whose planes are multiples of 4 pixels (XVEC), 16-byte asynchronous copies along the pixels;
@@ -338,8 +321,10 @@ constexpr int kMaxWideTaps = 31;  // filter taps in a pixel's bit mask (conv_fp3
 // cost 3510 cycles of a CTA alone on its SM, 3075 each of two; ~6900 per wave of CTAs, and ~12,100 to exchange partial tiles.
 // So they are taken for long reductions and many tiles: 17 x 64 -> 109 at 69 x 38, 5x5 474 -> 402 us; 2 x 762 -> 256 at 18 x 18,
 // 3x3/2 48.3 -> 40.6; 2 x 976 -> 80 at 37 x 37, 5x5 885 -> 433; not for 64 -> 64 at 56 x 56, 3x3, one image (16.1 us; 19.9 wide).
-Fp32Choice conv_fp32_choose(int64_t pixels, int c, int h, int w, int r, int s, int o) {
-  const int slabs = int((int64_t(c) * r * s + kBK - 1) / kBK);
+Fp32Choice conv_fp32_choose(const Fp32Shape& g) {
+  const int o = g.o;
+  const int64_t pixels = int64_t(g.batch) * g.out_h * g.out_w;
+  const int slabs = int((int64_t(g.c) * g.r * g.s + kBK - 1) / kBK);
   Fp32Choice best{0, tile_p(o), tile_o(o), 1};
   double best_t = 1e300;
   {
@@ -353,7 +338,7 @@ Fp32Choice conv_fp32_choose(int64_t pixels, int c, int h, int w, int r, int s, i
       if (t < best_t * 0.98) { best_t = t; best.slices = sl; }
     }
   }
-  if (r * s > kMaxWideTaps || !conv_fp32_wide_offsets_fit(c, h, w, r, s)) return best;
+  if (g.r * g.s > kMaxWideTaps || !conv_fp32_wide_offsets_fit(g.c, g.h, g.w, g.r, g.s)) return best;
   const bool table = int64_t((slabs + best.slices - 1) / best.slices) * kBK <= kLutMax;
   const double other = best_t * (table ? 1.0 : 2.0) + 7600.0;
   double limit = 1e300;
@@ -374,36 +359,54 @@ Fp32Choice conv_fp32_choose(int64_t pixels, int c, int h, int w, int r, int s, i
   return best;
 }
 
-cudaError_t conv_fp32_launch(const void* x, const void* w, const void* bias, void* y, int batch, int c, int h, int wd, int o,
-                             int r, int s, int stride_h, int stride_w, int pad_h, int pad_w, int out_h, int out_w, int relu,
+namespace {
+
+// How conv_fp32_kernel is launched for a choice: the instance, the slabs of a CTA and its shared memory.
+struct Form {
+  bool xvec, lut;
+  int slabs_per_slice;
+  size_t smem;
+};
+Form form_of(const Fp32Choice& ch, const Fp32Shape& g, bool x_aligned) {
+  Form f;
+  const int slabs = (g.c * g.r * g.s + kBK - 1) / kBK;
+  f.slabs_per_slice = (slabs + ch.slices - 1) / ch.slices;
+  f.xvec = x_aligned && g.r == 1 && g.s == 1 && g.stride_h == 1 && g.stride_w == 1 && g.pad_h == 0 && g.pad_w == 0 && (g.out_h * g.out_w) % 4 == 0;
+  f.lut = !f.xvec && conv_fp32_table_fits(int64_t(f.slabs_per_slice) * kBK, g.c, g.h, g.w, g.r, g.s, g.pad_h);
+  f.smem = size_t(kRing) * (kBK * ch.tile_p + ch.tile_o * kWPitch) * sizeof(float) + (f.lut ? size_t(f.slabs_per_slice) * kBK * sizeof(int2) : 0);
+  return f;
+}
+
+}  // namespace
+
+size_t conv_fp32_smem_bytes(const Fp32Choice& ch, const Fp32Shape& g) {
+  return ch.wide ? conv_fp32_wide_smem_bytes(ch.tile_p) : form_of(ch, g, true).smem;
+}
+
+cudaError_t conv_fp32_launch(const Fp32Choice& ch, const Fp32Shape& g, const void* x, const void* w, const void* bias, void* y, int relu,
                              cudaStream_t stream) {
-  const Fp32Choice choice = conv_fp32_choose(int64_t(batch) * out_h * out_w, c, h, wd, r, s, o);
-  if (choice.wide)
-    return conv_fp32_wide_launch(choice, x, w, bias, y, batch, c, h, wd, o, r, s, stride_h, stride_w, pad_h, pad_w, out_h, out_w, relu, stream);
+  if (ch.wide) return conv_fp32_wide_launch(ch, g, x, w, bias, y, relu, stream);
   Fp32Args a;
   a.x = static_cast<const float*>(x);
   a.w = static_cast<const float*>(w);
   a.bias = static_cast<const float*>(bias);
   a.y = static_cast<float*>(y);
-  a.batch = batch; a.c = c; a.h = h; a.wd = wd; a.o = o; a.r = r; a.s = s;
-  a.stride_h = stride_h; a.stride_w = stride_w; a.pad_h = pad_h; a.pad_w = pad_w;
-  a.out_h = out_h; a.out_w = out_w; a.relu = relu;
-  a.pixels = batch * out_h * out_w;
-  a.k = c * r * s;
-  a.fd_rs = FastDiv::make(r * s);
-  a.fd_s = FastDiv::make(s);
-  a.fd_pq = FastDiv::make(out_h * out_w);
-  a.fd_out_w = FastDiv::make(out_w);
-  const int tp = choice.tile_p, to = choice.tile_o;
-  const int64_t tiles_p = (int64_t(a.pixels) + tp - 1) / tp, tiles_o = (o + to - 1) / to;
-  const int slabs = (a.k + kBK - 1) / kBK;
-  a.slices = choice.slices;
-  a.slabs_per_slice = (slabs + a.slices - 1) / a.slices;
-  const bool xvec = r == 1 && s == 1 && stride_h == 1 && stride_w == 1 && pad_h == 0 && pad_w == 0 && (out_h * out_w) % 4 == 0 &&
-                    (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
-  const bool lut = !xvec && conv_fp32_table_fits(int64_t(a.slabs_per_slice) * kBK, c, h, wd, r, s, pad_h);
+  a.batch = g.batch; a.c = g.c; a.h = g.h; a.wd = g.w; a.o = g.o; a.r = g.r; a.s = g.s;
+  a.stride_h = g.stride_h; a.stride_w = g.stride_w; a.pad_h = g.pad_h; a.pad_w = g.pad_w;
+  a.out_h = g.out_h; a.out_w = g.out_w; a.relu = relu;
+  a.pixels = g.batch * g.out_h * g.out_w;
+  a.k = g.c * g.r * g.s;
+  a.fd_rs = FastDiv::make(g.r * g.s);
+  a.fd_s = FastDiv::make(g.s);
+  a.fd_pq = FastDiv::make(g.out_h * g.out_w);
+  a.fd_out_w = FastDiv::make(g.out_w);
+  const int tp = ch.tile_p, to = ch.tile_o;
+  const int64_t tiles_p = (int64_t(a.pixels) + tp - 1) / tp, tiles_o = (g.o + to - 1) / to;
+  const Form f = form_of(ch, g, (reinterpret_cast<uintptr_t>(x) & 15u) == 0);
+  a.slices = ch.slices;
+  a.slabs_per_slice = f.slabs_per_slice;
   const bool w16 = a.k % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15u) == 0;  // 128-bit copies along k
-  const size_t smem = size_t(kRing) * (kBK * tp + to * kWPitch) * sizeof(float) + (lut ? size_t(a.slabs_per_slice) * kBK * sizeof(int2) : 0);
+  const size_t smem = f.smem;
   const dim3 grid(unsigned(tiles_p * a.slices), unsigned(tiles_o));
   auto go = [&](auto kernel) -> cudaError_t {
     // the opt-in to more than 48 KiB of dynamic shared memory is per function and device: done once each, under a mutex
@@ -426,8 +429,8 @@ cudaError_t conv_fp32_launch(const void* x, const void* w, const void* bias, voi
   };
   auto pick = [&](auto tpc, auto toc) {
     constexpr int TP = decltype(tpc)::value, TO = decltype(toc)::value;
-    if (xvec) return w16 ? go(conv_fp32_kernel<TP, TO, false, true, true>) : go(conv_fp32_kernel<TP, TO, false, false, true>);
-    if (lut) return w16 ? go(conv_fp32_kernel<TP, TO, true, true, false>) : go(conv_fp32_kernel<TP, TO, true, false, false>);
+    if (f.xvec) return w16 ? go(conv_fp32_kernel<TP, TO, false, true, true>) : go(conv_fp32_kernel<TP, TO, false, false, true>);
+    if (f.lut) return w16 ? go(conv_fp32_kernel<TP, TO, true, true, false>) : go(conv_fp32_kernel<TP, TO, true, false, false>);
     return w16 ? go(conv_fp32_kernel<TP, TO, false, true, false>) : go(conv_fp32_kernel<TP, TO, false, false, false>);
   };
   return to == 32 ? pick(std::integral_constant<int, 128>{}, std::integral_constant<int, 32>{})

@@ -14,8 +14,8 @@
 
 #include <type_traits>
 
+#include "conv_fp32_device.cuh"
 #include "internal.h"
-#include "ptx.cuh"
 
 namespace gieb {
 namespace {
@@ -38,22 +38,6 @@ struct Fp32WideArgs {
   int slices, slabs_per_group;
   FastDiv fd_rs, fd_s, fd_pq, fd_out_w, fd_slices;
 };
-
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ float2 unpack2(uint64_t v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
-// 16-byte asynchronous copy; `valid` false writes zeros (nothing is read).
-__device__ __forceinline__ void cp_async16(void* dst, const float* src, bool valid) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ptx::smem_u32(dst)), "l"(src), "r"(valid ? 16 : 0) : "memory");
-}
 
 // XVEC: unpadded 1x1 of stride 1 whose planes are multiples of 4 pixels, x 16-byte aligned: 16-byte copies along the pixels.
 // W16: rows of w are multiples of 4 terms and 16-byte aligned.
@@ -160,7 +144,7 @@ __global__ void __launch_bounds__(kThreads, 2) conv_fp32_wide_kernel(const __gri
         for (int i = 0; i < kBK; i += VROWS) {
           const int kk = i + t / VG, k = kbase + sl * kBK + kk;
           const bool ok = v_ok && k < a.k;
-          cp_async16(xs + kk * TP, ok ? vb + size_t(k) * a.pq : a.x, ok);
+          cp_async16(xs + kk * TP, ok ? vb + size_t(k) * a.pq : a.x, ok ? 16 : 0);
         }
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
@@ -340,48 +324,60 @@ __global__ void __launch_bounds__(kThreads, 2) conv_fp32_wide_kernel(const __gri
   if (a.slices > 1) ptx::cluster_sync_all();  // nobody leaves while a peer still reads its tile
 }
 
-size_t smem_of(int tp) {
-  const size_t group = size_t(kXRing) * kBK * tp + 2 * kBK * kWRow + 2 * 3 * kBK;
-  const size_t loop = group * (256 / tp) * sizeof(float), exchange = size_t(32) * kThreads * 16;
+}  // namespace
+
+size_t conv_fp32_wide_smem_bytes(int tile_p) {
+  const size_t group = size_t(kXRing) * kBK * tile_p + 2 * kBK * kWRow + 2 * 3 * kBK;
+  const size_t loop = group * (256 / tile_p) * sizeof(float), exchange = size_t(32) * kThreads * 16;
   return loop > exchange ? loop : exchange;
+}
+
+namespace {
+
+template <int TP>
+cudaError_t prepare_all() {
+  const int smem = int(conv_fp32_wide_smem_bytes(TP));
+  cudaError_t e = cudaSuccess;
+  for (auto kernel : {conv_fp32_wide_kernel<TP, true, true>, conv_fp32_wide_kernel<TP, true, false>, conv_fp32_wide_kernel<TP, false, true>,
+                      conv_fp32_wide_kernel<TP, false, false>})
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  return e;
 }
 
 template <int TP, bool XVEC, bool W16>
 cudaError_t go(const Fp32WideArgs& a, dim3 grid, cudaStream_t st) {
-  // (an attribute of the function and device, set on each launch: a call of some 100 ns that keeps no state here)
-  const size_t smem = smem_of(TP);
-  const cudaError_t e = cudaFuncSetAttribute(conv_fp32_wide_kernel<TP, XVEC, W16>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-  if (e != cudaSuccess) return e;
-  return launch_pdl_cluster(conv_fp32_wide_kernel<TP, XVEC, W16>, grid, dim3(kThreads), smem, st, unsigned(a.slices), a);
+  return launch_pdl_cluster(conv_fp32_wide_kernel<TP, XVEC, W16>, grid, dim3(kThreads), conv_fp32_wide_smem_bytes(TP), st, unsigned(a.slices), a);
 }
 
 }  // namespace
 
-cudaError_t conv_fp32_wide_launch(const Fp32Choice& ch, const void* x, const void* w, const void* bias, void* y, int batch, int c, int h, int wd,
-                                  int o, int r, int s, int stride_h, int stride_w, int pad_h, int pad_w, int out_h, int out_w, int relu,
+// (which instance a call takes depends on its pointers: all of the tile width)
+cudaError_t conv_fp32_wide_prepare(int tile_p) { return tile_p == 128 ? prepare_all<128>() : prepare_all<64>(); }
+
+cudaError_t conv_fp32_wide_launch(const Fp32Choice& ch, const Fp32Shape& g, const void* x, const void* w, const void* bias, void* y, int relu,
                                   cudaStream_t stream) {
   Fp32WideArgs a;
   a.x = static_cast<const float*>(x);
   a.w = static_cast<const float*>(w);
   a.bias = static_cast<const float*>(bias);
   a.y = static_cast<float*>(y);
-  a.c = c; a.h = h; a.wd = wd; a.o = o; a.s = s; a.taps = r * s;
-  a.stride_h = stride_h; a.stride_w = stride_w; a.pad_h = pad_h; a.pad_w = pad_w;
-  a.out_w = out_w; a.pq = out_h * out_w; a.relu = relu;
-  a.pixels = batch * out_h * out_w;
-  a.k = c * r * s;
+  a.c = g.c; a.h = g.h; a.wd = g.w; a.o = g.o; a.s = g.s; a.taps = g.r * g.s;
+  a.stride_h = g.stride_h; a.stride_w = g.stride_w; a.pad_h = g.pad_h; a.pad_w = g.pad_w;
+  a.out_w = g.out_w; a.pq = g.out_h * g.out_w; a.relu = relu;
+  a.pixels = g.batch * g.out_h * g.out_w;
+  a.k = g.c * g.r * g.s;
   a.slices = ch.slices;
   const int slabs = (a.k + kBK - 1) / kBK, members = ch.slices * (256 / ch.tile_p);
   a.slabs_per_group = (slabs + members - 1) / members;
   a.fd_rs = FastDiv::make(a.taps);
-  a.fd_s = FastDiv::make(s);
+  a.fd_s = FastDiv::make(g.s);
   a.fd_pq = FastDiv::make(a.pq);
-  a.fd_out_w = FastDiv::make(out_w);
+  a.fd_out_w = FastDiv::make(g.out_w);
   a.fd_slices = FastDiv::make(a.slices);
-  const bool xvec = r == 1 && s == 1 && stride_h == 1 && stride_w == 1 && pad_h == 0 && pad_w == 0 && a.pq % 4 == 0 &&
+  const bool xvec = g.r == 1 && g.s == 1 && g.stride_h == 1 && g.stride_w == 1 && g.pad_h == 0 && g.pad_w == 0 && a.pq % 4 == 0 &&
                     (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
   const bool w16 = a.k % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15u) == 0;
-  const dim3 grid(unsigned((int64_t(a.pixels) + ch.tile_p - 1) / ch.tile_p * ch.slices), unsigned((o + kTO - 1) / kTO));
+  const dim3 grid(unsigned((int64_t(a.pixels) + ch.tile_p - 1) / ch.tile_p * ch.slices), unsigned((g.o + kTO - 1) / kTO));
   auto pick = [&](auto tp) {
     constexpr int TP = decltype(tp)::value;
     if (xvec) return w16 ? go<TP, true, true>(a, grid, stream) : go<TP, true, false>(a, grid, stream);

@@ -282,19 +282,24 @@ cudaError_t repack_pair_launch(const void* src_a, void* dst_a, int batch_a, int 
 cudaError_t gather_rows_launch(const void* x, void* x2, int batch, int channels, int h, int w, int q, int kernel_w, int stride_w,
                                int pad_w, int c2, const void* wsrc, void* w2, int out_channels, int kernel_h, cudaStream_t stream);
 
-// FP32 SIMT implicit GEMM straight from NCHW.  The kernel, the tile and the CTAs of a cluster that split the reduction of a tile:
+// FP32 SIMT implicit GEMM straight from NCHW.
+struct Fp32Shape {
+  int batch, c, h, w, o, r, s, stride_h, stride_w, pad_h, pad_w, out_h, out_w;
+};
+// The kernel, the tile and the CTAs of a cluster that split the reduction of a tile:
 struct Fp32Choice {
   int wide;            // 1: conv_fp32_wide.cu (thread tiles of 16 x 8)
   int tile_p, tile_o;  // output pixels and channels of a tile
   int slices;
 };
-Fp32Choice conv_fp32_choose(int64_t pixels, int c, int h, int w, int r, int s, int o);
-cudaError_t conv_fp32_wide_launch(const Fp32Choice& ch, const void* x, const void* w, const void* bias, void* y, int batch, int c, int h, int wd,
-                                  int o, int r, int s, int stride_h, int stride_w, int pad_h, int pad_w, int out_h, int out_w, int relu,
+Fp32Choice conv_fp32_choose(const Fp32Shape& g);
+size_t conv_fp32_smem_bytes(const Fp32Choice& ch, const Fp32Shape& g);  // dynamic, for tensors on 16-byte boundaries
+size_t conv_fp32_wide_smem_bytes(int tile_p);
+cudaError_t conv_fp32_wide_prepare(int tile_p);
+cudaError_t conv_fp32_launch(const Fp32Choice& ch, const Fp32Shape& g, const void* x, const void* w, const void* bias, void* y, int relu,
+                             cudaStream_t stream);
+cudaError_t conv_fp32_wide_launch(const Fp32Choice& ch, const Fp32Shape& g, const void* x, const void* w, const void* bias, void* y, int relu,
                                   cudaStream_t stream);
-cudaError_t conv_fp32_launch(const void* x, const void* w, const void* bias, void* y, int batch, int c, int h, int wd,
-                             int o, int r, int s, int stride_h, int stride_w, int pad_h, int pad_w, int out_h, int out_w,
-                             int relu, cudaStream_t stream);
 cudaError_t rmsnorm_launch(int rows, int hidden, float eps, int dtype, int gamma_fp32, const void* x, const void* gamma,
                            void* y, const void* res_in, void* res_out, cudaStream_t stream);
 
