@@ -834,11 +834,12 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
   // asks for more than half of an SM's shared memory.
   if (r->pair && r->smem < kMaxDynamicSmem / 2 + 2048) r->smem = kMaxDynamicSmem / 2 + 2048;
 
+  r->image = image_fits && r->split_k == 1 && !r->pair && r->tile_k == r->gp_t * 8;
   // workspace: channel-padded NHWC activations, prepacked weights, split-K partials (ws_layout analogue,
   // src/kernels/tensor_core_mma.cu:265-278)
   r->ws_x = in_nhwc ? 0 : align256(size_t(d.batch) * (r->subsampled ? size_t(g.out_h) * g.out_w : size_t(d.in_h) * r->eff_in_w) * r->c_padded * 2);
-  if (r->gather_pairs) r->ws_x = align256(size_t(d.batch) * d.in_h * r->gp_positions * 16);
-  r->ws_w = (d.flags & GIEB_FLAG_WEIGHTS_PREPACKED) ? 0 : align256(size_t(d.out_channels) * d.kernel_h * r->eff_kernel_w * r->c_padded * 2);
+  if (r->gather_pairs) r->ws_x = r->image ? 0 : align256(size_t(d.batch) * d.in_h * r->gp_positions * 16);
+  r->ws_w = (d.flags & GIEB_FLAG_WEIGHTS_PREPACKED) || r->image ? 0 : align256(size_t(d.out_channels) * d.kernel_h * r->eff_kernel_w * r->c_padded * 2);
   // how the split-K slices are summed
   if (c.reduce < 0 || c.reduce > 2) return no("reduce must be 0 (auto), 1 (workspace) or 2 (cluster)");
   r->reduce = r->split_k > 1 ? best_mode : 0;
@@ -849,7 +850,6 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
   r->ws_part = r->split_k > 1 && r->reduce == 1 ? align256(size_t(r->split_k) * size_t((g.y_elems + 3) & ~int64_t(3)) * 4) : 0;
   r->ws_total = r->ws_x + r->ws_w + r->ws_part;
   if (r->ws_total > (size_t(180) << 30) / 4) return no("workspace exceeds a quarter of device memory");
-  r->image = image_fits && r->split_k == 1 && !r->pair && r->tile_k == r->gp_t * 8;
   return GIEB_OK;
 }
 

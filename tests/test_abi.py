@@ -131,9 +131,11 @@ def test_workspace_layout_and_padding(pkg):
     assert pkg.query(stem, pkg.make_cfg(variant=1)).padded_channels == 16
     auto = pkg.query(stem)  # few channels: the 7 taps of a filter row become 7 * 3 -> 32 channels of a 7 x 1 convolution
     assert auto.variant == 5 and auto.padded_channels == 32
-    # stride 2, 3 channels: column pairs are stored once (115 positions of 16 bytes per input row: 2 of padding on the left,
-    # 112 pairs, 1 on the right) and adjacent windows overlap in memory
-    assert auto.workspace_bytes == a256(1 * 224 * 115 * 16) + a256(64 * 7 * 32 * 2)
+    # stride 2, 3 channels: the image is read in place, without scratch; where the layer is gathered first, column pairs are stored
+    # once (115 positions of 16 bytes per input row: 2 of padding on the left, 112 pairs, 1 on the right) and adjacent windows overlap
+    # in memory
+    assert auto.workspace_bytes == 0
+    assert pkg.query(stem, pkg.make_cfg(cta_pair=2)).workspace_bytes == a256(1 * 224 * 115 * 16) + a256(64 * 7 * 32 * 2)
     assert pkg.query(P(pkg, 1, 96, 27, 27, 192, 5, 5, 1, 1, 2, 2, precision=pkg.FP16)).padded_channels == 96
 
 

@@ -110,3 +110,26 @@ def test_plans_of_other_sizes_leave_a_plan_alone(pkg, orc, oracle):
     pkg.conv_forward_static(gu.pkg_problem(pkg, p), bufs[0][1], bufs[1][1], bufs[2][1], out.ptr, 0)
     assert pkg.conv_static_status(0) == 0
     check(plans[0], large)
+
+
+@pytest.mark.parametrize("static", [False, True])
+def test_no_workspace(pkg, orc, oracle, static):
+    """The image is read in place: no scratch, so the allocation-free call takes layers whose gathered copy (32 MB here) would not fit
+    its own."""
+    import torch
+    p = orc.Problem.P(1, 1, 4000, 1000, 2, 3, 3, 2, 2, 1, 1, precision=orc.FP16, bias=True, relu=True)
+    x, w, b = oracle.make_conv_data(p, 7400, 1)
+    ref, scale = oracle.conv2d(p, x, w, b)
+    plan = pkg.ConvPlan(gu.pkg_problem(pkg, p))
+    assert plan.workspace_bytes == 0
+    bufs = [gu.to_device_storage(oracle, p.precision, a) for a in (x, w, b)]
+    out = gu.OutBuf(p.precision, int(np.prod(p.y_shape)))
+    if static:
+        pkg.conv_forward_static(gu.pkg_problem(pkg, p), bufs[0][1], bufs[1][1], bufs[2][1], out.ptr, 0)
+        assert pkg.conv_static_status(0) == 0
+    else:
+        plan.launch(bufs[0][1], bufs[1][1], bufs[2][1], out.ptr, None, 0, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert plan.device_status() == 0
+    m = oracle.compare(p, out.read(oracle).reshape(p.y_shape), ref, scale)
+    assert m.passed(), m.summary()
