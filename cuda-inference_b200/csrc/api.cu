@@ -112,9 +112,8 @@ struct Resolved {
   // position) and the im2col tensor map reads it with a pixel stride of one position, so that the windows of adjacent
   // output columns overlap in memory instead of being stored twice.  gp_t positions (8 values each) per window.
   int gather_pairs, gp_positions, gp_left, gp_t, gp_shift;
-  // The same layer straight from the NCHW tensor (conv_image.cu); `strip`: its rows are counted in 128-row tiles per output row
-  // (tile counts, which a query reports).
-  int image, strip;
+  // The same layer straight from the NCHW tensor (conv_image.cu): tiles of 128 pixels x kImageTileN channels, `stages` 2.
+  int image;
   int im_group_rows, im_in_rows, im_rows_per_phase;
   size_t im_stage_bytes, im_smem;
   double est_cycles;  // the cost model's estimate for the chosen configuration (SM cycles; 0 on the FP32 path)
@@ -480,9 +479,9 @@ bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, const gieb_conv_cf
   return true;
 }
 
-// Groups of the image kernel (conv_image.cu): how many output rows a CTA takes at a time.  False: no group fits shared memory.
+// The plan on the image kernel (conv_image.cu): how many output rows a CTA takes at a time.  False: no group fits shared memory.
 bool resolve_image(const gieb_conv_desc& d, const Geometry& g, Resolved* r) {
-  const int pitch = g.out_w + r->gp_t - 1, tiles_n = ceil_div(d.out_channels, 64);
+  const int pitch = g.out_w + r->gp_t - 1, tiles_n = ceil_div(d.out_channels, kImageTileN);
   const bool staging = (d.flags & GIEB_FLAG_OUTPUT_NHWC) != 0;
   double best = 1e300;
   for (int ctas = 2; ctas >= 1 && best >= 1e299; --ctas) {
@@ -517,7 +516,27 @@ bool resolve_image(const gieb_conv_desc& d, const Geometry& g, Resolved* r) {
       }
     }
   }
-  return best < 1e299;
+  if (best >= 1e299) return false;
+  r->image = 1;
+  r->tile_m = kTileM;
+  r->tile_n = kImageTileN;
+  r->stages = 2;
+  r->split_k = 1;
+  r->kb_per_split = r->total_kb;
+  r->tiles_n = tiles_n;
+  r->smem = r->im_smem;
+  // (what a query estimates: bound by its tensors, ~1370 bytes per cycle, which fits 5.8, 9.2, 22.6, 33.3 and 101 us for 1 x 64 x 64,
+  // 4 x 224 x 224, 57 x 144 x 144, 32 and 128 x 224 x 224, 7x7/2, 3 -> 64 channels within 13 %)
+  r->est_cycles = 4750.0 + 2.0 * double(g.x_elems + g.y_elems * ((d.flags & GIEB_FLAG_RESIDUAL) ? 2 : 1)) / 1370.0;
+  return true;
+}
+
+// CTAs of the image kernel for each tile of channels: persistent, as many as fit the machine.
+int64_t image_ctas(const gieb_conv_desc& d, const Geometry& g, const Resolved& r) {
+  const int64_t groups = int64_t(d.batch) * ceil_div(g.out_h, r.im_group_rows);
+  int64_t ctas = kNumSms * (r.im_smem <= kSmSmem / 2 - 1024 ? 2 : 1) / r.tiles_n;
+  if (ctas < 1) ctas = 1;
+  return groups < ctas ? groups : ctas;
 }
 
 int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, char* why, size_t why_len) {
@@ -589,10 +608,7 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
       r->gp_positions = d.in_w / 2 + left + right;
     }
   }
-  // Read straight from the image (conv_image.cu) unless the reduction is asked to be split or spread over a pair.
-  const bool image_fits = r->gather_pairs && resolve_image(d, g, r);
-  r->strip = (image_fits && g.out_w <= 128 && c.split_k <= 1 && c.reduce == 0 && c.cta_pair != 2 && (c.tile_k == 0 || c.tile_k == r->gp_t * 8)) ? 1 : 0;
-  const int64_t rows = r->strip ? int64_t(d.batch) * g.out_h * 128 : (r->variant == 2 ? int64_t(d.batch) * r->boxes_per_image * 64 : g.pixels);
+  const int64_t rows = r->variant == 2 ? int64_t(d.batch) * r->boxes_per_image * 64 : g.pixels;
 
   // hardware limits of the im2col-mode tensor map (rank 4): traversal strides 1..8, corners and offsets 8-bit
   if (d.stride_h > 8 || d.stride_w > 8) return no("stride > 8 cannot be expressed by the TMA im2col traversal stride");
@@ -656,6 +672,10 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
     if (c.tile_n != 0 && c.tile_n < 64) return no("CTA-pair tiles are 64, 128 or 256 output channels wide");
     if (c.reduce == 2) return no("a CTA pair is a cluster already: its split-K slices are summed through the workspace (reduce 0 or 1)");
   }
+  // Read straight from the image (conv_image.cu), unless something is asked for that this kernel is not.
+  if (r->gather_pairs && (c.tile_m == 0 || c.tile_m == kTileM) && (c.tile_n == 0 || c.tile_n == kImageTileN) && r->tile_k == r->gp_t * 8 &&
+      (c.stages == 0 || c.stages == 2) && c.split_k <= 1 && c.reduce == 0 && c.cta_pair != 2 && resolve_image(d, g, r))
+    return GIEB_OK;
   if (halo) {
     if (c.stages != 0 && (c.stages < 2 || c.stages > kMaxStages)) return no("stages must be in [2, 8]");
     if (c.reduce < 0 || c.reduce > 2) return no("reduce must be 0 (auto), 1 (workspace) or 2 (cluster)");
@@ -676,7 +696,7 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
   int best_m = 0, best_n = 0, best_s = 0, best_mode = 0, best_pair = 0, best_swap = 0;
   const int n_opts[4] = {32, 64, 128, 256};
   // 256-pixel tiles of CTA pairs: only the workspace reduction for split-K
-  const bool pair_unasked = c.cta_pair == 0 && !r->strip && d.precision != GIEB_TF32 && c.tile_m == 0 && c.split_k <= 1 && c.reduce == 0 && c.variant != 2 &&
+  const bool pair_unasked = c.cta_pair == 0 && d.precision != GIEB_TF32 && c.tile_m == 0 && c.split_k <= 1 && c.reduce == 0 && c.variant != 2 &&
                             auto_pair(d, rows, r->total_kb, r->tile_k);
   for (int ni = 1; ni < 4 && d.precision != GIEB_TF32 && (c.cta_pair == 2 || pair_unasked) && (c.tile_m == 0 || c.tile_m == 256) && c.reduce != 2; ++ni) {
     const int tn = n_opts[ni];
@@ -729,7 +749,7 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
       if (!r->tile_n && tn > 32 && tn / 2 >= d.out_channels) continue;  // never pad channels by 2x or more
       if (direct_n && tn != direct_n) continue;
       if ((no_32 && tn == 32) || (short_pointwise && tm == 256 && tn == 128)) continue;
-      for (int s = 1; s <= (r->strip ? 1 : 16); ++s) {   // (the image kernel finishes its tiles alone)
+      for (int s = 1; s <= 16; ++s) {
         if (c.split_k && s != c.split_k) continue;
         if (s > 1 && r->total_kb < 2 * s) break;  // reduction too short (src/kernels/tensor_core_mma.cu:292 rule)
         const int kbs = ceil_div(r->total_kb, s);
@@ -774,9 +794,9 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
 
   // Channel-contiguous output goes through shared-memory boxes and TMA stores when the rows of the [pixels][O] matrix
   // are 16-byte multiples, rows are numbered by pixel (not the direct-NCHW route) and each CTA finishes its tiles alone.
-  r->tma_epilogue = (d.flags & GIEB_FLAG_OUTPUT_NHWC) && d.out_channels % 8 == 0 && r->variant != 2 && !r->strip && r->split_k == 1;
+  r->tma_epilogue = (d.flags & GIEB_FLAG_OUTPUT_NHWC) && d.out_channels % 8 == 0 && r->variant != 2 && r->split_k == 1;
   r->row_epilogue = (d.flags & GIEB_FLAG_OUTPUT_NHWC) && d.out_channels % 8 != 0 && r->split_k == 1;
-  bool swap = best_swap != 0 && !r->pair && !r->strip && r->split_k == 1;  // 2 KiB of staging per epilogue warp
+  bool swap = best_swap != 0 && !r->pair && r->split_k == 1;  // 2 KiB of staging per epilogue warp
   const int64_t total_tiles = int64_t(r->tiles_m) * r->tiles_n * r->split_k;
   auto stages_for = [&](size_t epi_smem) {
     int st = c.stages ? c.stages
@@ -834,12 +854,11 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
   // asks for more than half of an SM's shared memory.
   if (r->pair && r->smem < kMaxDynamicSmem / 2 + 2048) r->smem = kMaxDynamicSmem / 2 + 2048;
 
-  r->image = image_fits && r->split_k == 1 && !r->pair && r->tile_k == r->gp_t * 8;
   // workspace: channel-padded NHWC activations, prepacked weights, split-K partials (ws_layout analogue,
   // src/kernels/tensor_core_mma.cu:265-278)
   r->ws_x = in_nhwc ? 0 : align256(size_t(d.batch) * (r->subsampled ? size_t(g.out_h) * g.out_w : size_t(d.in_h) * r->eff_in_w) * r->c_padded * 2);
-  if (r->gather_pairs) r->ws_x = r->image ? 0 : align256(size_t(d.batch) * d.in_h * r->gp_positions * 16);
-  r->ws_w = (d.flags & GIEB_FLAG_WEIGHTS_PREPACKED) || r->image ? 0 : align256(size_t(d.out_channels) * d.kernel_h * r->eff_kernel_w * r->c_padded * 2);
+  if (r->gather_pairs) r->ws_x = align256(size_t(d.batch) * d.in_h * r->gp_positions * 16);
+  r->ws_w = (d.flags & GIEB_FLAG_WEIGHTS_PREPACKED) ? 0 : align256(size_t(d.out_channels) * d.kernel_h * r->eff_kernel_w * r->c_padded * 2);
   // how the split-K slices are summed
   if (c.reduce < 0 || c.reduce > 2) return no("reduce must be 0 (auto), 1 (workspace) or 2 (cluster)");
   r->reduce = r->split_k > 1 ? best_mode : 0;
@@ -873,6 +892,11 @@ void fill_info(const gieb_conv_desc& d, const Resolved& r, gieb_conv_info* out) 
     out->threads_per_block = 128;
     out->num_blocks = int64_t(ceil_div(g.pixels, r.tile_m)) * ceil_div(d.out_channels, r.tile_n) * r.fp32.slices;
     out->launches = 1;
+  } else if (r.image) {
+    out->dynamic_smem_bytes = uint32_t(r.smem);
+    out->threads_per_block = kImageThreads;
+    out->num_blocks = image_ctas(d, g, r) * r.tiles_n;
+    out->launches = 1;
   } else {
     out->dynamic_smem_bytes = uint32_t(r.smem);
     out->threads_per_block = conv_tc_threads(r.epi_warps);
@@ -881,7 +905,7 @@ void fill_info(const gieb_conv_desc& d, const Resolved& r, gieb_conv_info* out) 
     const bool x_in_place = r.variant == 2 || (d.flags & GIEB_FLAG_INPUT_NHWC);
     const bool w_in_place = (d.flags & GIEB_FLAG_WEIGHTS_PREPACKED) != 0 ||
                             (x_in_place && d.precision != GIEB_TF32 && d.kernel_h * d.kernel_w == 1 && r.c_padded == d.in_channels);  // 16-byte aligned w assumed
-    out->launches = r.image ? 1 : (x_in_place && w_in_place ? 0 : 1) + 1 + (r.reduce == 1 ? 1 : 0);
+    out->launches = (x_in_place && w_in_place ? 0 : 1) + 1 + (r.reduce == 1 ? 1 : 0);
   }
 }
 
@@ -1132,16 +1156,13 @@ int launch_image(const gieb_conv_plan* pl, const void* x, const void* w, const v
   p.relu = d.relu;
   p.out_nhwc = (d.flags & GIEB_FLAG_OUTPUT_NHWC) != 0;
   p.out_cells = p.out_nhwc && (reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(residual)) % 16 == 0 && d.out_channels % 8 == 0;
-  p.idesc = ptx::make_idesc_f16(kTileM, 64, p.is_bf16, false, false);
+  p.idesc = ptx::make_idesc_f16(kTileM, kImageTileN, p.is_bf16, false, false);
   p.fd_groups_per_image = FastDiv::make(p.groups_per_image);
   p.fd_pitch = FastDiv::make(p.pitch);
   p.fd_stride_h = FastDiv::make(p.stride_h);
   p.fd_segments = FastDiv::make(p.segments);
   p.fd_cells = FastDiv::make(p.kernel_h * r.gp_t);
-  const int tiles_n = ceil_div(d.out_channels, 64);
-  int ctas = kNumSms * (r.im_smem <= kSmSmem / 2 - 1024 ? 2 : 1) / tiles_n;  // persistent CTAs for each tile of channels
-  if (ctas < 1) ctas = 1;
-  const dim3 grid(unsigned(p.groups < ctas ? p.groups : ctas), unsigned(tiles_n));
+  const dim3 grid(unsigned(image_ctas(d, pl->g, r)), unsigned(r.tiles_n));
   if (ev) for (int k = 0; k < 2; ++k) GIEB_CUDA(cudaEventRecord(ev[k], st));
   if (stage_mask & 2u) GIEB_CUDA(conv_image_launch(r.gp_t, p, grid, r.im_smem, st));
   if (ev) for (int k = 2; k < 4; ++k) GIEB_CUDA(cudaEventRecord(ev[k], st));

@@ -24,10 +24,10 @@ namespace gieb {
 namespace {
 
 constexpr int kGatherWarps = 4, kImageWorkers = 8;
-constexpr int kImageThreads = 32 * (kGatherWarps + 1 + kImageWorkers);
+static_assert(kImageThreads == 32 * (kGatherWarps + 1 + kImageWorkers), "warps of a CTA");
 constexpr int kImageSlots = 4;                       // accumulators of 64 columns
 constexpr uint32_t kImageCtrl = 1024;                // 64 bias values, barriers, TMEM address slot
-constexpr int kImageCols = 64;
+constexpr int kImageCols = kImageTileN;
 
 // The words of C channels at one column pair (low half: even column) as the 8 values of a position: the channels of the even
 // column, those of the odd one, zeros.

@@ -207,6 +207,8 @@ struct ConvImageParams {
   uint32_t idesc, debug_skip;
   FastDiv fd_groups_per_image, fd_pitch, fd_stride_h, fd_segments, fd_cells;  // fd_cells: kernel_h * T
 };
+constexpr int kImageTileN = 64;                  // output channels of a tile
+constexpr int kImageThreads = 32 * (4 + 1 + 8);  // warps that load the image, issue the MMAs, drain the accumulators
 // t_positions: positions per window, 2, 4 or 8
 size_t conv_image_smem_bytes(int kernel_h, int t_positions, size_t strip_stage_bytes, bool staging);
 cudaError_t conv_image_prepare(int t_positions);

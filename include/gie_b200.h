@@ -97,9 +97,9 @@ typedef struct gieb_conv_cfg {
                        5 = tensor path over row-gathered activations for inputs with few channels (NCHW input,
                            kernel_w > 1, kernel_w * C <= 64): the S taps of a filter row become channels, so a 7x7
                            stem over 3 channels reduces over 7 x 32 values instead of 49 x 16 padded ones.  With at most 4
-                           channels, stride_w 2 and an even width the image is read in place, in one launch, unless the
-                           reduction is split or spread over a pair (tile_m, tile_n and stages then describe the form
-                           that gathers first);
+                           channels, stride_w 2 and an even width the image is read in place, in one launch without workspace, by
+                           tiles of 128 pixels and 64 channels with two stages: other tiles, stages, slabs or
+                           reductions that are asked for get the form that gathers first;
                        6 = tensor path whose tiles hold every activation once for all filter taps (kernels of 2 to 64
                            taps, strides 1 or 2, padding below the kernel's extents, 16 output pixels or more);
                            tile_m 128, or 256 with cta_pair 2; tile_n 128 or 256 in pairs; split_k 1, 2, 4 or 8, summed

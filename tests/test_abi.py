@@ -154,10 +154,11 @@ def test_selection_is_deterministic_and_fills_the_machine(pkg):
         assert 2 <= c.stages <= 8 and i1.dynamic_smem_bytes <= 232448
         total_kb = a[5] * a[6] * (i1.padded_channels // c.tile_k)
         assert 1 <= c.split_k <= max(1, total_kb // 2)
+        if i1.variant == 5:   # straight from the image: persistent CTAs, at most two per SM
+            assert i1.launches == 1 and i1.num_blocks == 2 * 148
+            continue
         pixels = a[0] * p.out_h * p.out_w
         rows = a[0] * -(-(a[2] * a[3]) // 64) * 64 if i1.variant == 2 else pixels   # direct NCHW route counts 64-pixel boxes
-        if i1.variant == 5 and a[8] == 2 and a[1] <= 4 and p.out_w <= 128:
-            rows = a[0] * p.out_h * 128   # position strips: one 128-row box per output row
         if c.variant == 6:                # halo tiles cover the padded grid; at stride 1 neighbours share their padding
             assert (a[7], a[8]) == (1, 1)
             rows = a[0] * (a[2] + a[9]) * (a[3] + a[10])

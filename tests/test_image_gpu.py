@@ -133,3 +133,22 @@ def test_no_workspace(pkg, orc, oracle, static):
     assert plan.device_status() == 0
     m = oracle.compare(p, out.read(oracle).reshape(p.y_shape), ref, scale)
     assert m.passed(), m.summary()
+
+
+@pytest.mark.parametrize("cfg", [dict(tile_n=32), dict(tile_n=128), dict(tile_n=256), dict(tile_m=256, tile_n=64), dict(tile_n=64, stages=4), dict(tile_k=16)])
+@pytest.mark.parametrize("args", [(2, 3, 64, 64, 64, 7, 7, 2, 2, 3, 3), (1, 3, 30, 258, 72, 7, 7, 2, 2, 3, 3)])
+@pytest.mark.parametrize("nhwc", [False, True])
+def test_forms_that_gather_first(pkg, orc, oracle, cfg, args, nhwc):
+    """Tiles, stages and slabs other than the image kernel's, asked for: overlapping windows read from the copy of the image."""
+    p = orc.Problem.P(*args, precision=orc.BF16, bias=True, relu=True)
+    x, w, b = oracle.make_conv_data(p, 7500, 2)
+    ref, scale = oracle.conv2d(p, x, w, b)
+    flags = pkg.FLAG_OUTPUT_NHWC if nhwc else 0
+    plan = pkg.ConvPlan(gu.pkg_problem(pkg, p, flags), pkg.make_cfg(**cfg))
+    assert plan.info.launches == 2 and all(getattr(plan.info.cfg, k) == v for k, v in cfg.items())
+    got, _, _ = gu.run_conv(pkg, oracle, p, x, w, b, flags=flags, plan=plan)
+    if nhwc:
+        B, O, P, Q = p.y_shape
+        got = np.ascontiguousarray(got.reshape(B, P, Q, O).transpose(0, 3, 1, 2))
+    m = oracle.compare(p, got, ref, scale)
+    assert m.passed(), m.summary()
