@@ -313,12 +313,20 @@ constexpr int kMaxWideTaps = 31;  // filter taps in a pixel's bit mask (conv_fp3
 
 }  // namespace
 
+// Clusters of 1 to 8 CTAs that the machine holds at a time, with at most 1 to 5 CTAs per SM (cudaOccupancyMaxActiveClusters).
+constexpr int kClusters[5][8] = {{148, 74, 45, 33, 26, 22, 15, 15}, {296, 148, 93, 71, 56, 45, 37, 33}, {444, 222, 142, 104, 82, 71, 56, 48},
+                                 {592, 296, 187, 142, 112, 93, 78, 71}, {740, 370, 235, 175, 142, 116, 97, 86}};
+// As many clusters are spread with one CTA per SM although two would fit.  (Wide tiles of clusters of eight: 15 take the time of CTAs
+// alone on their SMs, 16 that of pairs; of five 21 and 25; of six 14, with 16 to 19 between the two; three and four not measured.)
+constexpr int kSpread[8] = {148, 74, 41, 30, 22, 15, 15, 15};
+
 // The choice by SM cycles.
 // This kernel: the CTAs that an SM holds together hide each other's latencies: a slab costs ~1600 cycles of a CTA alone on its SM,
 // ~1100 per CTA of two and ~1030 of more; a CTA's prologue and epilogue cost ~1500 cycles, a cluster's exchange ~2000 more, and up to
 // five CTAs share an SM.  Without the decode table (reductions of more than kLutMax terms per slice) everything takes twice as long.
 // The wide tiles (fitted to 230 timings of 18 layers, 7 % off on average): 16 terms of a CTA's tiles are 2048 cycles of FMA issue and
 // cost 3510 cycles of a CTA alone on its SM, 3075 each of two; ~6900 per wave of CTAs, and ~12,100 to exchange partial tiles.
+// Both run in waves of what kClusters says: a wave of more clusters than that, as of more CTAs than SMs, takes as long as two.
 // So they are taken for long reductions and many tiles: 17 x 64 -> 109 at 69 x 38, 5x5 474 -> 402 us; 2 x 762 -> 256 at 18 x 18,
 // 3x3/2 48.3 -> 40.6; 2 x 976 -> 80 at 37 x 37, 5x5 885 -> 433; not for 64 -> 64 at 56 x 56, 3x3, one image (16.1 us; 19.9 wide).
 Fp32Choice conv_fp32_choose(const Fp32Shape& g) {
@@ -326,32 +334,35 @@ Fp32Choice conv_fp32_choose(const Fp32Shape& g) {
   const int64_t pixels = int64_t(g.batch) * g.out_h * g.out_w;
   const int slabs = int((int64_t(g.c) * g.r * g.s + kBK - 1) / kBK);
   Fp32Choice best{0, tile_p(o), tile_o(o), 1};
+  const int64_t tiles = ((pixels + best.tile_p - 1) / best.tile_p) * ((o + best.tile_o - 1) / best.tile_o);
+  auto narrow = [&](int sl, double load) {
+    const double slab = load <= 1 ? 1600.0 : (load <= 2 ? 1100.0 : 1030.0);
+    return load * ((slabs + sl - 1) / sl) * slab + std::ceil(load / 5.0) * (1500.0 + (sl > 1 ? 2000.0 : 0.0));
+  };
   double best_t = 1e300;
-  {
-    const int64_t tiles = ((pixels + best.tile_p - 1) / best.tile_p) * ((o + best.tile_o - 1) / best.tile_o);
-    for (int sl = 1; sl <= 8 && sl <= slabs; ++sl) {
-      const int per = (slabs + sl - 1) / sl;
-      if ((slabs + per - 1) / per != sl) continue;  // (an empty slice)
-      const double load = double((tiles * sl + kNumSms - 1) / kNumSms);
-      const double slab = load <= 1 ? 1600.0 : (load <= 2 ? 1100.0 : 1030.0);
-      const double t = load * per * slab + std::ceil(load / 5.0) * (1500.0 + (sl > 1 ? 2000.0 : 0.0));
-      if (t < best_t * 0.98) { best_t = t; best.slices = sl; }
-    }
+  for (int sl = 1; sl <= 8 && sl <= slabs; ++sl) {
+    const int per = (slabs + sl - 1) / sl;
+    if ((slabs + per - 1) / per != sl) continue;  // (an empty slice)
+    const double t = narrow(sl, double((tiles * sl + kNumSms - 1) / kNumSms));
+    if (t < best_t * 0.98) { best_t = t; best.slices = sl; }
   }
   if (g.r * g.s > kMaxWideTaps || !conv_fp32_wide_offsets_fit(g.c, g.h, g.w, g.r, g.s)) return best;
+  const int64_t five = kClusters[4][best.slices - 1], left = tiles % five;
+  int level = 0;
+  while (level < 5 && left > (level ? kClusters[level - 1][best.slices - 1] : 0)) ++level;
   const bool table = int64_t((slabs + best.slices - 1) / best.slices) * kBK <= kLutMax;
-  const double other = best_t * (table ? 1.0 : 2.0) + 7600.0;
+  const double other = narrow(best.slices, double(5 * (tiles / five) + level)) * (table ? 1.0 : 2.0) + 7600.0;
   double limit = 1e300;
   for (int tp = 128; tp >= 64; tp /= 2) {
     const int groups = 256 / tp;
-    const int64_t tiles = ((pixels + tp - 1) / tp) * ((o + 63) / 64);
+    const int64_t clusters = ((pixels + tp - 1) / tp) * ((o + 63) / 64);
     for (int sl = 1; sl <= 8 && sl * groups <= slabs; ++sl) {
       const int members = sl * groups, per = (slabs + members - 1) / members;
-      const int64_t ctas = tiles * sl, rest = ctas % (2 * kNumSms);
-      if (tiles * (sl - 1) > 6 * kNumSms) break;  // (clusters of many waves of CTAs: not measured, and splitting gains nothing)
+      if (clusters * (sl - 1) > 6 * kNumSms) break;  // (clusters of many waves of CTAs: not measured, and splitting gains nothing)
+      const int64_t wave = kClusters[1][sl - 1], rest = clusters % wave;
       const double pair = 2.0 * per * 3075.0 + 6900.0;
-      double t = double(ctas / (2 * kNumSms)) * pair + (rest > kNumSms ? pair : (rest > 0 ? per * 3510.0 + 6900.0 : 0.0));
-      if (members > 1) t += 12100.0 * double((ctas + 2 * kNumSms - 1) / (2 * kNumSms));
+      double t = double(clusters / wave) * pair + (rest == 0 ? 0.0 : (rest <= kSpread[sl - 1] ? per * 3510.0 + 6900.0 : pair));
+      if (members > 1) t += 12100.0 * double((clusters + wave - 1) / wave);
       // (margins: over 24 layers seven gained 2 to 62 % and one lost 2 % with them, of 16 before four had lost 2 to 13 %)
       if (t < limit && t < (tp == 128 ? 0.88 : 0.85) * other - 3200.0) { limit = t; best = Fp32Choice{1, tp, 64, sl}; }
     }
