@@ -99,13 +99,13 @@ __device__ __forceinline__ void store_chunk_full(const uint32_t (&v)[32], const 
   }
 }
 
-// Partial chunks, any element stride.
+// Partial chunks, any element stride; v holds the sums with their bias (and residual).
 template <typename T, bool RELU>
-__device__ __forceinline__ void store_chunk_tail(const uint32_t (&v)[32], const float* __restrict__ bias, T* dst, int64_t stride, int nvalid) {
+__device__ __forceinline__ void store_chunk_tail(const uint32_t (&v)[32], T* dst, int64_t stride, int nvalid) {
 #pragma unroll
   for (int j = 0; j < 32; ++j) {
     if (j < nvalid) {
-      float a = __uint_as_float(v[j]) + bias[j];
+      float a = __uint_as_float(v[j]);
       if (RELU) a = fmaxf(a, 0.f);
       dst[int64_t(j) * stride] = round_to<T>(a);
     }
@@ -130,6 +130,12 @@ __device__ __forceinline__ void store_chunk_full_res(const uint32_t (&v)[32], co
       dst[int64_t(g * 8 + j) * stride] = round_to<T>(a);
     }
   }
+}
+
+// The bias of a partial chunk (the tile's array covers whole chunks).  Ahead of the residual, as in whole chunks: (sum + bias) + residual.
+__device__ __forceinline__ void add_bias_tail(uint32_t (&v)[32], const float* __restrict__ bias) {
+#pragma unroll
+  for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + bias[j]);
 }
 
 // The residual of a partial chunk, added to its sums ahead of the stores: channels beyond the chunk read the last valid one, so that
@@ -299,9 +305,10 @@ __device__ __forceinline__ void store_chunk(uint32_t (&v)[32], const float* bias
     if (relu) store_chunk_full_res<T, true>(v, bias, dst, res, stride);
     else store_chunk_full_res<T, false>(v, bias, dst, res, stride);
   } else {
+    add_bias_tail(v, bias);
     if (res != nullptr) add_residual_tail(v, res, stride, nvalid);
-    if (relu) store_chunk_tail<T, true>(v, bias, dst, stride, nvalid);
-    else store_chunk_tail<T, false>(v, bias, dst, stride, nvalid);
+    if (relu) store_chunk_tail<T, true>(v, dst, stride, nvalid);
+    else store_chunk_tail<T, false>(v, dst, stride, nvalid);
   }
 }
 
