@@ -32,6 +32,30 @@ def test_direct_tiles_by_the_number_of_tiles(pkg):
     assert seen == {32, 64, 128, 256}
 
 
+def test_direct_tiles_and_rings_with_a_residual(pkg):
+    """More tiles of 128 channels than SMs: a residual takes 256 channels for three to seven slabs; without one, tiles of 128 have six
+    stages from four slabs on."""
+    seen = set()
+    for residual in (False, True):
+        for c, slabs in ((191, 3), (256, 4), (320, 5), (512, 8)):
+            for b in (1, 16, 32, 64):
+                for o in (128, 200, 256, 768):
+                    p = pkg.ConvProblem(b, c, 28, 28, o, 1, 1, precision=pkg.BF16, has_bias=True, relu=True, flags=pkg.FLAG_RESIDUAL if residual else 0)
+                    cfg = pkg.query(p).cfg
+                    tiles_m = -(-(b * -(-784 // 64)) // 2)
+                    walks = {n: -(-tiles_m * -(-o // n) // SMS) for n in (32, 64, 128, 256)}
+                    fitting = [n for n in (32, 64, 128) if walks[n] == 1]
+                    want = fitting[0] if fitting else 128
+                    if not fitting and o > 128 and ((residual and slabs < 8) or (walks[256] > 1 and 8 * walks[128] > 7 * 2 * walks[256])):
+                        want = 256
+                    assert cfg.tile_n == want, (residual, c, b, o)
+                    if want == 128 and cfg.tile_m == 128:
+                        six = slabs >= 8 or (slabs >= 4 and not residual)
+                        assert (cfg.stages == 6) == six, (residual, c, b, o, cfg.stages)
+                    seen.add((residual, slabs, want))
+    assert {(True, 4, 256), (False, 4, 128), (False, 3, 128), (True, 3, 256), (True, 5, 128), (True, 8, 128)} <= seen, seen
+
+
 def test_short_pointwise_tiles(pkg):
     """1x1 layers of one or two slabs over channel-contiguous tensors: no tiles of 32 channels beyond two of them per SM, none of 256
     pixels and 128 channels; what is asked for stays."""

@@ -18,7 +18,10 @@ CASES = [
     ((5, 762, 60, 30, 70, 1, 1, 1, 1, 0, 0), 128, 1),       # the same off its alignment: gathered
     ((2, 762, 18, 18, 256, 3, 3, 2, 2, 1, 1), 64, 0),       # 429 slabs over few pixels
     ((1, 1030, 12, 12, 40, 3, 3, 1, 1, 1, 1), 64, 1),
+    ((1, 4090, 16, 16, 70, 1, 1, 1, 1, 0, 0), 64, 0),       # 1x1 in four groups: 16-byte copies, 4090 terms, a channel tail
+    ((1, 4094, 12, 17, 40, 1, 1, 1, 1, 0, 0), 64, 1),       # the same off its alignment, a last tile of 12 pixels
 ]
+SHARED_MEMORY = {128: 67328, 64: 85504}  # of this kernel's CTAs (the other kernel has tiles of 64 pixels too)
 
 
 @pytest.mark.parametrize("case", range(len(CASES)))
@@ -28,7 +31,7 @@ def test_fp32_wide_tiles(pkg, orc, oracle, case):
     x, w, b = oracle.make_conv_data(p, 600 + case, case % 4)
     ref, scale = oracle.conv2d(p, x, w, b if p.has_bias else None)
     got, plan, out = gu.run_conv(pkg, oracle, p, x, w, b if p.has_bias else None, offsets=(off, off, off))
-    assert plan.info.cfg.tile_m == tile
+    assert plan.info.cfg.tile_m == tile and plan.info.dynamic_smem_bytes == SHARED_MEMORY[tile]
     m = oracle.compare(p, got, ref, scale)   # the reference's FP32 policy: the rounding of FP32 sums of this length
     assert m.passed(), f"fp32 case {case}: {m.summary()}"
     again, _, out2 = gu.run_conv(pkg, oracle, p, x, w, b if p.has_bias else None, plan=plan, offsets=(off, off, off))
