@@ -483,6 +483,7 @@ bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, const gieb_conv_cf
 bool resolve_image(const gieb_conv_desc& d, const Geometry& g, Resolved* r) {
   const int pitch = g.out_w + r->gp_t - 1, tiles_n = ceil_div(d.out_channels, kImageTileN);
   const bool staging = (d.flags & GIEB_FLAG_OUTPUT_NHWC) != 0;
+  if (tiles_n > 65535) return false;  // (the grid's second dimension)
   double best = 1e300;
   for (int ctas = 2; ctas >= 1 && best >= 1e299; --ctas) {
     for (int rows = 1; rows <= g.out_h && rows <= 16; ++rows) {

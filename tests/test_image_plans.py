@@ -42,3 +42,10 @@ def test_what_is_asked_for_runs(pkg, args, nhwc, smem, ctas):
         if i.cfg.reduce != 1:
             assert gathered in (None, i.workspace_bytes) and i.workspace_bytes > 0
             gathered = i.workspace_bytes
+
+
+def test_more_channels_than_the_grid_takes(pkg):
+    """Tiles of channels are the grid's second dimension: 65535 of 64.  Beyond, the form that gathers first takes the layer."""
+    for filters, launches in ((65535 * 64, 1), (65535 * 64 + 1, 2)):
+        i = query(pkg, (1, 1, 4, 4, filters, 3, 3, 2, 2, 1, 1))
+        assert i.supported and i.variant == 5 and i.launches == launches, filters
