@@ -30,7 +30,7 @@
 namespace gieb {
 namespace {
 
-constexpr int kBK = 16;
+constexpr int kBK = kFp32Slab;
 constexpr int kMaxSmem = 96 * 1024;
 
 struct Fp32Args {
@@ -82,7 +82,7 @@ conv_fp32_kernel(const Fp32Args a) {
   const int pix0 = int(blockIdx.x / unsigned(a.slices)) * TP, oc0 = blockIdx.y * TO;
   const int rs = a.r * a.s;
   const int pq = a.out_h * a.out_w;
-  const int slabs_all = (a.k + kBK - 1) / kBK;
+  const int slabs_all = fp32_slabs(a.k);
   const int slab0 = slice * a.slabs_per_slice;
   const int slabs = max(0, min(a.slabs_per_slice, slabs_all - slab0));
   const int kbase = slab0 * kBK;
@@ -332,7 +332,7 @@ constexpr int kSpread[8] = {148, 74, 41, 30, 22, 15, 15, 15};
 Fp32Choice conv_fp32_choose(const Fp32Shape& g) {
   const int o = g.o;
   const int64_t pixels = int64_t(g.batch) * g.out_h * g.out_w;
-  const int slabs = int((int64_t(g.c) * g.r * g.s + kBK - 1) / kBK);
+  const int slabs = fp32_slabs(g.c * g.r * g.s);
   Fp32Choice best{0, tile_p(o), tile_o(o), 1};
   const int64_t tiles = ((pixels + best.tile_p - 1) / best.tile_p) * ((o + best.tile_o - 1) / best.tile_o);
   auto narrow = [&](int sl, double load) {
@@ -380,7 +380,7 @@ struct Form {
 };
 Form form_of(const Fp32Choice& ch, const Fp32Shape& g, bool x_aligned) {
   Form f;
-  const int slabs = (g.c * g.r * g.s + kBK - 1) / kBK;
+  const int slabs = fp32_slabs(g.c * g.r * g.s);
   f.slabs_per_slice = (slabs + ch.slices - 1) / ch.slices;
   f.xvec = x_aligned && g.r == 1 && g.s == 1 && g.stride_h == 1 && g.stride_w == 1 && g.pad_h == 0 && g.pad_w == 0 && (g.out_h * g.out_w) % 4 == 0;
   f.lut = !f.xvec && conv_fp32_table_fits(int64_t(f.slabs_per_slice) * kBK, g.c, g.h, g.w, g.r, g.s, g.pad_h);

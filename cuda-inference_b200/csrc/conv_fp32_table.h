@@ -10,6 +10,13 @@ namespace gieb {
 constexpr int kLutMax = 4096;    // reduction length of a CTA up to which the (c, r, s) decode of k is tabulated in shared memory
 constexpr int kNoRow = 0x7fff;   // filter row of a table entry beyond the reduction: no image has the row it leads to
 
+constexpr int kFp32Slab = 16;
+// Slabs that a reduction of k terms has, rounded up; k may be any positive 32-bit value.
+#if defined(__CUDACC__)
+__host__ __device__
+#endif
+constexpr int fp32_slabs(int k) { return (k - 1) / kFp32Slab + 1; }
+
 // `terms`: table entries of a CTA.  An entry is the offset of (c, r, s) inside one image and (r << 16) | s, so offsets have 31
 // bits, r 15 and s 16.  The kernel reads input row oh * stride - pad_h + r when that lies in [0, h): for r = kNoRow and the
 // topmost output row it is kNoRow - pad_h, which lies below the image as long as h + pad_h <= kNoRow.

@@ -15,12 +15,13 @@
 #include <type_traits>
 
 #include "conv_fp32_device.cuh"
+#include "conv_fp32_table.h"
 #include "internal.h"
 
 namespace gieb {
 namespace {
 
-constexpr int kBK = 16;         // terms of a slab
+constexpr int kBK = kFp32Slab;         // terms of a slab
 constexpr int kHalf = kBK / 2;  // gathered elements pass through registers half a slab at a time
 constexpr int kThreads = 128;
 constexpr int kTO = 64;
@@ -58,7 +59,7 @@ __global__ void __launch_bounds__(kThreads, 2) conv_fp32_wide_kernel(const __gri
 
   const int tile = a.fd_slices.div(int(blockIdx.x)), slice = int(blockIdx.x) - tile * a.slices;
   const int pix0 = tile * TP, oc0 = int(blockIdx.y) * kTO;
-  const int slabs_all = (a.k + kBK - 1) / kBK;
+  const int slabs_all = fp32_slabs(a.k);
   const int slab0 = (slice * KG + grp) * a.slabs_per_group;
   const int slabs = max(0, min(a.slabs_per_group, slabs_all - slab0));
   const int kbase = slab0 * kBK;
@@ -367,7 +368,7 @@ cudaError_t conv_fp32_wide_launch(const Fp32Choice& ch, const Fp32Shape& g, cons
   a.pixels = g.batch * g.out_h * g.out_w;
   a.k = g.c * g.r * g.s;
   a.slices = ch.slices;
-  const int slabs = (a.k + kBK - 1) / kBK, members = ch.slices * (256 / ch.tile_p);
+  const int slabs = fp32_slabs(a.k), members = ch.slices * (256 / ch.tile_p);
   a.slabs_per_group = (slabs + members - 1) / members;
   a.fd_rs = FastDiv::make(a.taps);
   a.fd_s = FastDiv::make(g.s);

@@ -82,3 +82,21 @@ def test_wide_tiles_leave_images_whose_offsets_do_not_fit(pkg):
     """One channel more than fits, and the kernel that indexes in 64 bits takes the layer (tiles of 64 pixels instead of 128)."""
     tiles = [pkg.query(pkg.ConvProblem(8, c, 2, 331, 64, 3, 3, 1, 1, 1, 1, precision=pkg.FP32)).cfg.tile_m for c in (3243932, 3243933)]
     assert tiles == [128, 64]
+
+
+SLABS_PROGRAM = r"""
+#include "conv_fp32_table.h"
+int main() {
+  const int ks[] = {1, 15, 16, 17, 576, 2147483631, 2147483632, 2147483633, 2147483647};
+  for (int k : ks) if (gieb::fp32_slabs(k) != int((k + 15LL) / 16)) return 1;
+  return 0;
+}
+"""
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+def test_slabs_of_the_longest_reductions(tmp_path):
+    src, exe = tmp_path / "slabs.cpp", tmp_path / "slabs"
+    src.write_text(SLABS_PROGRAM)
+    subprocess.check_call(["g++", "-std=c++17", "-Wall", "-Werror", "-I" + os.path.join(ROOT, "cuda-inference_b200", "csrc"), str(src), "-o", str(exe)])
+    assert subprocess.run([str(exe)]).returncode == 0
