@@ -720,6 +720,8 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
   // at 56 x 56, 32 images 17.5 us in tiles of 256, 14.8 in tiles of 128); for longer reductions, where a CTA of 128 columns takes the
   // SM for a deep ring (see stages_for), where it walks fewer half-width tiles (320 -> 256 at 28 x 28, 32 images 11.1 and 9.8; with
   // as many 256 columns are up to 10 % faster) or 256 columns give a CTA a single tile (320 -> 256, 16 images 8.0 and 7.1).
+  // Over layers of random sizes whose tiles the rule changed: 53 with NCHW outputs 1.29 times as fast as in tiles of 256 (none
+  // slower), 38 with channel-contiguous outputs 1.21 (four 2 to 4 % slower, two of them also with another kernel between the calls).
   int direct_n = 0;
   if (r->variant == 2 && !r->tile_n && c.tile_m == 0 && c.stages == 0 && c.split_k <= 1 && c.reduce == 0 && c.cta_pair != 2) {
     const int64_t tiles_m = ceil_div(rows, kTileM);
@@ -728,8 +730,10 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
       if (tn > 32 && tn / 2 >= d.out_channels) continue;
       if (direct_n == 0 || walks(tn) == 1) direct_n = tn;
     }
-    // (a residual lengthens the epilogue that a CTA alone on its SM does not hide: 224 -> 640 at 16 x 37, 25 images 22.8 us with 256, 28.2 with 128)
-    // (up to 192 channels the second tile of 128 is at least half empty: 64 -> 160 at 60 x 60, 141 images, residual 162 and 180 us)
+    // 256 as well with a residual of three to seven slabs, which lengthens the epilogue that a CTA alone on its SM does not hide, and
+    // for one or two slabs of 129 to 192 channels, whose second tile of 128 is at least half empty.  Both are right for
+    // channel-contiguous outputs (14 layers each: tiles of 128 take 1.11 and 1.18 of the time); of NCHW outputs most layers would be
+    // faster in tiles of 128 (0.90 and 0.84 over 14 layers each, three and one of them slower).
     const bool fewer = walks(256) == 1 || walks(128) * 8 <= walks(256) * 14, exposed = (d.flags & GIEB_FLAG_RESIDUAL) != 0 && r->total_kb < 8;
     if (d.out_channels > 128 && direct_n == 128 && walks(128) > 1 && (r->total_kb > 2 ? exposed || !fewer : d.out_channels <= 192)) direct_n = 256;
   }
@@ -737,7 +741,8 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
   // 32 channels per SM those of 64 are faster (9 x 16 -> 895 at 10 x 19 10.3 and 6.8 us, 2 x 16 -> 448 at 82 x 82 13.1 and 9.2,
   // 68 x 64 -> 64 at 26 x 26 6.3 and 5.2, 54 x 124 -> 640 at 7 x 7 9.1 and 7.7; with fewer, 32 are as fast or faster).  Tiles of 256
   // pixels and 128 channels fill tensor memory with the accumulators of one CTA per SM and lose to 128 pixels where the reduction is
-  // this short (58 x 64 -> 640 at 61 x 61 103 and 72 us).
+  // this short (58 x 64 -> 640 at 61 x 61 103 and 72 us).  For every type: over random layers whose tiles it changed 12 of FP16 1.4
+  // times as fast, 11 of FP8 1.14, 6 of TF32 1.17, none slower.
   const bool short_pointwise = r->variant == 4 && r->total_kb <= 2 && !r->tile_n && c.tile_m == 0 && c.stages == 0 && c.split_k <= 1 && c.reduce == 0 &&
                                c.cta_pair != 2;
   const bool no_32 = short_pointwise && d.out_channels > 32 && int64_t(ceil_div(rows, kTileM)) * ceil_div(d.out_channels, 32) > 2 * kNumSms;
