@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(kImageThreads, 2) conv_image_kernel(const __gr
             if (m_ok) {
               const int nvalid = min(32, p.out_channels - (n0 + chunk * 32));
               const int64_t off = base + int64_t(chunk * 32) * cstride;
-              with_type([&](auto* yp, auto* rp) { store_chunk(v, bias_s + chunk * 32, yp + off, rp != nullptr ? rp + off : nullptr, cstride, nvalid, p.relu); });
+              with_type([&](auto* yp, auto* rp) { store_chunk<true>(v, bias_s + chunk * 32, yp + off, rp != nullptr ? rp + off : nullptr, cstride, nvalid, p.relu); });
             }
           }
         }

@@ -99,13 +99,13 @@ __device__ __forceinline__ void store_chunk_full(const uint32_t (&v)[32], const 
   }
 }
 
-// Partial chunks, any element stride; v holds the sums with their bias (and residual).
+// Partial chunks, any element stride.  `biased`: v holds the sums with their bias (and residual).
 template <typename T, bool RELU>
-__device__ __forceinline__ void store_chunk_tail(const uint32_t (&v)[32], T* dst, int64_t stride, int nvalid) {
+__device__ __forceinline__ void store_chunk_tail(const uint32_t (&v)[32], const float* __restrict__ bias, bool biased, T* dst, int64_t stride, int nvalid) {
 #pragma unroll
   for (int j = 0; j < 32; ++j) {
     if (j < nvalid) {
-      float a = __uint_as_float(v[j]);
+      float a = __uint_as_float(v[j]) + (biased ? -0.f : bias[j]);
       if (RELU) a = fmaxf(a, 0.f);
       dst[int64_t(j) * stride] = round_to<T>(a);
     }
@@ -142,8 +142,8 @@ __device__ __forceinline__ void add_bias_tail(uint32_t (&v)[32], const float* __
 // the loads of eight go out together.  (Read one by one between the stores they took a round trip each: 64 -> 44 channels at 29 x 29,
 // 119 images, 3x3 53.5 us, 34.6 so.  In the stores' own loop, once more for either activation, the code made halo layers without a
 // residual 1 to 3 % slower.)
-template <typename T>
-__device__ __forceinline__ void add_residual_tail(uint32_t (&v)[32], const T* res, int64_t stride, int nvalid) {
+template <bool BIAS, typename T>
+__device__ __forceinline__ void add_residual_tail(uint32_t (&v)[32], const float* __restrict__ bias, const T* res, int64_t stride, int nvalid) {
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
     if (g * 8 >= nvalid) break;
@@ -151,7 +151,7 @@ __device__ __forceinline__ void add_residual_tail(uint32_t (&v)[32], const T* re
 #pragma unroll
     for (int j = 0; j < 8; ++j) r[j] = load_as_float(res + int64_t(min(g * 8 + j, nvalid - 1)) * stride);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[g * 8 + j] = __float_as_uint(__uint_as_float(v[g * 8 + j]) + r[j]);
+    for (int j = 0; j < 8; ++j) v[g * 8 + j] = __float_as_uint(__uint_as_float(v[g * 8 + j]) + (BIAS ? bias[g * 8 + j] : -0.f) + r[j]);
   }
 }
 
@@ -283,7 +283,9 @@ __device__ __forceinline__ void row_to_staging(const uint32_t (&v)[32], float bi
 
 // dst / res point at the first element of the chunk for this row; consecutive channels are `stride` elements apart
 // (P*Q for NCHW, 1 for channel-contiguous output).
-template <typename T>
+// LATE_BIAS: the bias of a partial chunk is added between its stores.  Added ahead of them the slab and halo kernels' partial chunks are
+// 1 to 5 % faster; the image kernel, at its cap of registers, slows down, whole chunks and all (128 x 224 x 224, NCHW 98 and 112 us).
+template <bool LATE_BIAS = false, typename T>
 __device__ __forceinline__ void store_chunk(uint32_t (&v)[32], const float* bias, T* dst, const T* res, int64_t stride,
                                             int nvalid, int relu) {
   if constexpr (sizeof(T) == 2) {
@@ -305,10 +307,11 @@ __device__ __forceinline__ void store_chunk(uint32_t (&v)[32], const float* bias
     if (relu) store_chunk_full_res<T, true>(v, bias, dst, res, stride);
     else store_chunk_full_res<T, false>(v, bias, dst, res, stride);
   } else {
-    add_bias_tail(v, bias);
-    if (res != nullptr) add_residual_tail(v, res, stride, nvalid);
-    if (relu) store_chunk_tail<T, true>(v, dst, stride, nvalid);
-    else store_chunk_tail<T, false>(v, dst, stride, nvalid);
+    if constexpr (!LATE_BIAS) add_bias_tail(v, bias);
+    if (res != nullptr) add_residual_tail<LATE_BIAS>(v, bias, res, stride, nvalid);
+    const bool biased = !LATE_BIAS || res != nullptr;
+    if (relu) store_chunk_tail<T, true>(v, bias, biased, dst, stride, nvalid);
+    else store_chunk_tail<T, false>(v, bias, biased, dst, stride, nvalid);
   }
 }
 
