@@ -1376,8 +1376,8 @@ int launch_impl(const gieb_conv_plan* pl, const void* x, const void* w, const vo
 }
 
 // Opts every kernel that launches of this configuration may take in to large dynamic shared memory.
-cudaError_t prepare_kernels(const Resolved& r) {
-  if (r.variant == 3) return r.fp32.wide ? conv_fp32_wide_prepare(r.fp32.tile_p) : cudaSuccess;
+cudaError_t prepare_kernels(const gieb_conv_desc& d, const Geometry& g, const Resolved& r) {
+  if (r.variant == 3) return r.fp32.wide ? conv_fp32_wide_prepare(r.fp32, fp32_shape(d, g)) : cudaSuccess;
   if (r.image) return conv_image_prepare(r.gp_t);
   if (r.halo) return conv_halo_prepare(r.tile_n, r.epi_warps, r.pair != 0, kMaxDynamicSmem);
   // The general kernel: a partial last slab, or rows that TMA cannot store (which tensors off their alignment are as well).
@@ -1459,7 +1459,7 @@ int gieb_conv_plan_create(const gieb_conv_desc* desc, const gieb_conv_cfg* cfg, 
       cudaStreamDestroy(s);
     }
   }
-  if (e == cudaSuccess) e = prepare_kernels(r);
+  if (e == cudaSuccess) e = prepare_kernels(pl->desc, pl->g, r);
   if (e != cudaSuccess) {
     if (pl->d_status) cudaFree(pl->d_status);
     delete pl;
@@ -1608,7 +1608,7 @@ int gieb_conv_forward_static(const gieb_conv_desc* desc, const gieb_conv_cfg* cf
   if (cc_major != 10) return fail(GIEB_UNSUPPORTED, "this library contains sm_100a code only; device %d has compute capability %d.x", pl.device, cc_major);
   pl.d_status = reinterpret_cast<uint32_t*>(base);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  GIEB_CUDA(prepare_kernels(pl.r));
+  GIEB_CUDA(prepare_kernels(pl.desc, pl.g, pl.r));
   // The array keeps whatever the previous call left: the status word must start at zero.  Everything else in the
   // scratch is fully rewritten by the repack kernels (padding channels included) and the split-K slices before use.
   GIEB_CUDA(cudaMemsetAsync(base, 0, kStaticScratchHeader, s));

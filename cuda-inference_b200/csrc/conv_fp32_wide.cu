@@ -335,13 +335,23 @@ size_t conv_fp32_wide_smem_bytes(int tile_p) {
 
 namespace {
 
+// 16-byte copies along the pixels, and of rows of w, for tensors on 16-byte boundaries.
+bool copies_x(const Fp32Shape& g) {
+  return g.r == 1 && g.s == 1 && g.stride_h == 1 && g.stride_w == 1 && g.pad_h == 0 && g.pad_w == 0 && g.out_h * g.out_w % 4 == 0;
+}
+bool copies_w(const Fp32Shape& g) { return g.c * g.r * g.s % 4 == 0; }
+
+// (which instance a call takes depends on its pointers: all that the layer can take)
 template <int TP>
-cudaError_t prepare_all() {
-  const int smem = int(conv_fp32_wide_smem_bytes(TP));
+cudaError_t prepare(const Fp32Shape& g) {
   cudaError_t e = cudaSuccess;
-  for (auto kernel : {conv_fp32_wide_kernel<TP, true, true>, conv_fp32_wide_kernel<TP, true, false>, conv_fp32_wide_kernel<TP, false, true>,
-                      conv_fp32_wide_kernel<TP, false, false>})
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  auto set = [&](bool reached, auto kernel) {
+    if (reached && e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(conv_fp32_wide_smem_bytes(TP)));
+  };
+  set(copies_x(g) && copies_w(g), conv_fp32_wide_kernel<TP, true, true>);
+  set(copies_x(g), conv_fp32_wide_kernel<TP, true, false>);
+  set(copies_w(g), conv_fp32_wide_kernel<TP, false, true>);
+  set(true, conv_fp32_wide_kernel<TP, false, false>);
   return e;
 }
 
@@ -352,8 +362,7 @@ cudaError_t go(const Fp32WideArgs& a, dim3 grid, cudaStream_t st) {
 
 }  // namespace
 
-// (which instance a call takes depends on its pointers: all of the tile width)
-cudaError_t conv_fp32_wide_prepare(int tile_p) { return tile_p == 128 ? prepare_all<128>() : prepare_all<64>(); }
+cudaError_t conv_fp32_wide_prepare(const Fp32Choice& ch, const Fp32Shape& g) { return ch.tile_p == 128 ? prepare<128>(g) : prepare<64>(g); }
 
 cudaError_t conv_fp32_wide_launch(const Fp32Choice& ch, const Fp32Shape& g, const void* x, const void* w, const void* bias, void* y, int relu,
                                   cudaStream_t stream) {
@@ -375,9 +384,8 @@ cudaError_t conv_fp32_wide_launch(const Fp32Choice& ch, const Fp32Shape& g, cons
   a.fd_pq = FastDiv::make(a.pq);
   a.fd_out_w = FastDiv::make(g.out_w);
   a.fd_slices = FastDiv::make(a.slices);
-  const bool xvec = g.r == 1 && g.s == 1 && g.stride_h == 1 && g.stride_w == 1 && g.pad_h == 0 && g.pad_w == 0 && a.pq % 4 == 0 &&
-                    (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
-  const bool w16 = a.k % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15u) == 0;
+  const bool xvec = copies_x(g) && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+  const bool w16 = copies_w(g) && (reinterpret_cast<uintptr_t>(w) & 15u) == 0;
   const dim3 grid(unsigned((int64_t(a.pixels) + ch.tile_p - 1) / ch.tile_p * ch.slices), unsigned((g.o + kTO - 1) / kTO));
   auto pick = [&](auto tp) {
     constexpr int TP = decltype(tp)::value;

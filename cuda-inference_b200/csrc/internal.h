@@ -297,7 +297,7 @@ struct Fp32Choice {
 Fp32Choice conv_fp32_choose(const Fp32Shape& g);
 size_t conv_fp32_smem_bytes(const Fp32Choice& ch, const Fp32Shape& g);  // dynamic, for tensors on 16-byte boundaries
 size_t conv_fp32_wide_smem_bytes(int tile_p);
-cudaError_t conv_fp32_wide_prepare(int tile_p);
+cudaError_t conv_fp32_wide_prepare(const Fp32Choice& ch, const Fp32Shape& g);
 cudaError_t conv_fp32_launch(const Fp32Choice& ch, const Fp32Shape& g, const void* x, const void* w, const void* bias, void* y, int relu,
                              cudaStream_t stream);
 cudaError_t conv_fp32_wide_launch(const Fp32Choice& ch, const Fp32Shape& g, const void* x, const void* w, const void* bias, void* y, int relu,
