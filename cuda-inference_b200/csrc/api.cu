@@ -502,7 +502,8 @@ bool resolve_image(const gieb_conv_desc& d, const Geometry& g, Resolved* r) {
       const size_t smem = conv_image_smem_bytes(d.kernel_h, r->gp_t, stage, staging);
       if (smem > (ctas == 2 ? kSmSmem / 2 - 1024 : kMaxDynamicSmem)) break;
       // cycles: instructions of a run of 32 positions and of a tile on an SM that two CTAs share; a group's loads take at least a
-      // round trip per 32 runs
+      // round trip per 32 runs.  (Not fitted: on 27 layers timed with 12 numbers of rows each the choice takes 1.11 of the fastest's
+      // time on average, 1.47 at most.  Waves x (1250 per tile + 150 per run), which comes to 1.02 on those, lost up to 13 % on others.)
       const int64_t groups = int64_t(d.batch) * ceil_div(g.out_h, rows);
       const double waves = double(ceil_div(groups * tiles_n, kNumSms * ctas)), runs = double(in_rows) * ceil_div(pitch, 32);
       const double busy = ctas * (12.0 * runs + 500.0 * tiles), load = 900.0 * std::ceil(runs / 32.0);
