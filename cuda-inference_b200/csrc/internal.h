@@ -256,6 +256,26 @@ cudaError_t splitk_reduce_launch(const float* partial, int splits, int64_t total
                                  const void* bias, int bias_fp32, int relu, int out_type, const void* residual, int out_nhwc,
                                  void* y, cudaStream_t stream);  // out_type: 0 fp16, 1 bf16, 2 fp32
 
+#if defined(__CUDACC__)
+// Launches blocks of 256 threads with shared memory nobody uses (beyond `fixed` declared bytes and `dynamic` needed ones), so that an SM
+// takes no more of them than an even share.  Programmatic launches begin while the kernel ahead still holds most SMs: blocks that need
+// next to nothing all pile up on the few it leaves idle, eight at a time, and are still at it there when the others are free.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl_spread(void (*kernel)(KArgs...), unsigned blocks, size_t fixed, size_t dynamic, cudaStream_t stream, Args&&... args) {
+  const size_t share = (blocks + kNumSms - 1) / kNumSms, total = 233472 / (share + 1) + 128;  // of an SM's 228 KiB; a block takes 1 KiB besides
+  size_t smem = dynamic;
+  if (share < 8 && total > 1024 + fixed + dynamic) smem = (total - 1024 - fixed) / 128 * 128;
+  if (fixed + smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kCtaSmemLimit - fixed));
+    if (e != cudaSuccess) return e;
+  }
+  return launch_pdl(kernel, dim3(blocks), dim3(256), smem, stream, static_cast<Args&&>(args)...);
+}
+#endif
+// The two repacks of repack_pair_launch where both are small (repack_direct.cu); false: not for these.  Either source may be null;
+// the second is filters of 9 taps or 1.
+bool repack_direct_launch(const void* src_a, void* dst_a, int batch_a, int ch_a, int hw_a, int cp_a, const void* src_b, void* dst_b, int batch_b,
+                          int ch_b, int hw_b, int cp_b, cudaStream_t stream, cudaError_t* status);
 // 16-bit [B][C][HW] -> [B][HW][Cp] (zero-filled channel padding).
 cudaError_t repack_launch(const void* src, void* dst, int batch, int channels, int hw, int c_padded, cudaStream_t stream);
 // FP32, two tensors in one launch: [batch][channels][hw] -> [batch][hw][c_padded], every value rounded to TF32 (ties away);

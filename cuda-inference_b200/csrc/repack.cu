@@ -219,14 +219,15 @@ __device__ __forceinline__ void repack_tile_sub(uint32_t* tile, const RepackJob&
   }
 }
 
-// Up to two jobs in one launch (activations + weights): block indices [0, a.blocks) belong to job a, the rest to job b.
+// Up to two jobs in one launch (activations + weights): block indices [0, b.blocks) belong to job b, the weights, whose blocks take
+// longest, the rest to job a (32 x 512 -> 512 at 14 x 14, 3x3: 34.05 us the other way round, 33.8 so).
 template <int RESIDENT>  // blocks per SM that the registers are cut for; 0: as they come
 __global__ void __launch_bounds__(256, RESIDENT) repack_jobs_kernel(const RepackJob a, const RepackJob b) {
   __shared__ __align__(16) uint32_t smem[kTile * kLdWords];
   static_assert(kTile * kLdWords * 4 >= kTile * kSmallHwMax * 2, "the slab must fit");
-  const bool first = blockIdx.x < a.blocks;
-  const RepackJob& j = first ? a : b;
-  const int id = int(first ? blockIdx.x : blockIdx.x - a.blocks);
+  const bool second = blockIdx.x < b.blocks;
+  const RepackJob& j = second ? b : a;
+  const int id = int(second ? blockIdx.x : blockIdx.x - b.blocks);
   const int row = j.fd_hw_tiles.div(id);
   const int hw_tile = id - row * j.hw_tiles;
   const int bi = j.fd_c_tiles.div(row);
@@ -428,16 +429,23 @@ cudaError_t launch_jobs(RepackJob a, int64_t tiles_a, RepackJob b, int64_t tiles
   b.set_tiles(tiles_b);
   // More than one wave: eight blocks per SM (46 x 430 x 57 x 57: 52.6 us, 60.1 with six).  A small job does not want them: its blocks
   // begin on the SMs that the kernel before it leaves idle, and the more those take the longer they are at it when all the others
-  // have finished (32 x 256 x 14 x 14 and its weights under a 100-block convolution: 0.6 us a pass).
+  // have finished (32 x 256 x 14 x 14 and its weights under a 100-block convolution: 0.6 us a pass).  Less than eight blocks per SM
+  // are spread evenly (launch_pdl_spread): 4 x 1024 x 14 x 14 ahead of its convolution 8.5 and 8.3 us, 16 x 256 x 30 x 31 14.6 and 14.4.
   // (A strided selection keeps sixteen loads in flight per thread, which 32 registers do not hold.)
   const auto kernel = a.blocks + b.blocks > unsigned(kNumSms) * 8 && a.mode != 4 ? repack_jobs_kernel<8> : repack_jobs_kernel<0>;
-  return launch_pdl(kernel, dim3(a.blocks + b.blocks), dim3(256), 0, stream, a, b);
+  return launch_pdl_spread(kernel, a.blocks + b.blocks, kTile * kLdWords * 4, 0, stream, a, b);
 }
 
 }  // namespace
 
 cudaError_t repack_pair_launch(const void* src_a, void* dst_a, int batch_a, int ch_a, int hw_a, int cp_a, const void* src_b,
                                void* dst_b, int batch_b, int ch_b, int hw_b, int cp_b, cudaStream_t stream) {
+  // (a plane of 9 pixels or 1 is turned as a filter is)
+  const bool alone = src_b == nullptr && (hw_a == 9 || hw_a == 1);
+  cudaError_t direct = cudaSuccess;
+  if (alone ? repack_direct_launch(nullptr, nullptr, 0, 0, 0, 0, src_a, dst_a, batch_a, ch_a, hw_a, cp_a, stream, &direct)
+            : repack_direct_launch(src_a, dst_a, batch_a, ch_a, hw_a, cp_a, src_b, dst_b, batch_b, ch_b, hw_b, cp_b, stream, &direct))
+    return direct;
   RepackJob a = make_job(src_a, dst_a, batch_a, ch_a, hw_a, cp_a);
   RepackJob b = a;
   const int64_t na = int64_t(a.hw_tiles) * a.c_tiles * batch_a;
@@ -628,9 +636,9 @@ __device__ __forceinline__ float to_tf32(float v) {
 __global__ void __launch_bounds__(256) repack_tf32_kernel(const Tf32Job a, const Tf32Job b, int prefetch) {
   __shared__ __align__(16) float tile[kTf32Slab];
   static_assert(32 * kTf32Pitch <= kTf32Slab, "the 32 x 64 tile must fit the slab buffer");
-  const bool first = blockIdx.x < a.blocks;
-  const Tf32Job& j = first ? a : b;
-  unsigned id = first ? blockIdx.x : blockIdx.x - a.blocks;
+  const bool second = blockIdx.x < b.blocks;  // (the weights first, as in repack_jobs_kernel: 16 x 96 -> 192 at 27 x 27, 5x5, 34.1 and 32.4 us)
+  const Tf32Job& j = second ? b : a;
+  unsigned id = second ? blockIdx.x : blockIdx.x - b.blocks;
   const int hw_tile = int(id % unsigned(j.hw_tiles));
   id /= unsigned(j.hw_tiles);
   const int c_tile = int(id % unsigned(j.c_tiles));
@@ -879,7 +887,9 @@ cudaError_t repack_bytes_pair_launch(const void* src_a, void* dst_a, int batch_a
   const bool wide = int64_t((hw_a + 127) / 128) * ((cp_a + 63) / 64) * batch_a > kNumSms * 8;
   const ByteJob a = make_byte_job(src_a, dst_a, batch_a, ch_a, hw_a, cp_a, wide ? 128 : 64);
   const ByteJob b = make_byte_job(src_b, dst_b, batch_b, ch_b, hw_b, cp_b, wide ? 128 : 64);
-  // (shared memory nobody uses keeps a small job at six blocks per SM: see launch_jobs)
+  // (shared memory nobody uses keeps a small job at six blocks per SM: see launch_jobs.  Fewer, or the weights first, do not pay here:
+  // 8 x 256 -> 256 at 14 x 14 8.9 and 8.6 us, but 2 x 512 -> 512 at 7 x 7 9.4 and 10.2, 3 x 200 -> 130 at 33 x 33, 1x1, 6.7 and 7.1,
+  // where the convolution's CTAs are small enough to lie beside the repack's.)
   const cudaError_t e = launch_pdl(wide ? repack_bytes_kernel<128> : repack_bytes_kernel<64>, dim3(a.blocks + b.blocks), dim3(256),
                                    wide ? 0 : 28 * 1024, stream, a, b, prefetch_enabled() ? 1 : 0);
   if (e != cudaSuccess) return e;
@@ -892,7 +902,7 @@ cudaError_t repack_tf32_pair_launch(const void* src_a, void* dst_a, int batch_a,
     return cudaErrorInvalidValue;
   const Tf32Job a = make_tf32_job(src_a, dst_a, batch_a, ch_a, hw_a, cp_a);
   const Tf32Job b = make_tf32_job(src_b, dst_b, batch_b, ch_b, hw_b, cp_b);
-  const cudaError_t e = launch_pdl(repack_tf32_kernel, dim3(a.blocks + b.blocks), dim3(256), 0, stream, a, b, prefetch_enabled() ? 1 : 0);
+  const cudaError_t e = launch_pdl_spread(repack_tf32_kernel, a.blocks + b.blocks, kTf32Slab * sizeof(float), 0, stream, a, b, prefetch_enabled() ? 1 : 0);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();
 }
