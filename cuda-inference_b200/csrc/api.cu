@@ -188,6 +188,11 @@ size_t smem_floor(int cols, bool waits_for_peers) {
   return cols > 256 ? kSmSmem / 2 : 0;
 }
 
+// Clusters of `split` CTAs that the machine holds with one CTA per SM (cudaOccupancyMaxActiveClusters), and the shared memory at which an
+// SM takes one CTA.
+int lone_clusters(int split) { return split >= 8 ? 15 : (split >= 4 ? 33 : 74); }
+constexpr size_t kLoneSmem = kSmSmem / 2;
+
 int resident_ctas(int tile_m, int tile_n, size_t smem) {
   int by_smem = int(kMaxDynamicSmem / (smem + 1024));
   int by_tmem = 512 / tmem_cols_of(tile_m, tile_n);
@@ -212,10 +217,10 @@ int pick_stages(int tile_m, int tile_n, int tile_k, int kb_per_split, int64_t ct
   return stages;
 }
 
-// Whether the split-K slices of one tile may be summed inside a cluster (distributed shared memory).
-bool cluster_reduce_ok(int tile_m, int tile_n, int tile_k, int stages, int split) {
-  const int chunks = tile_n / 32;
-  return tile_m == kTileM && (split == 2 || split == 4 || split == 8) && chunks % split == 0 &&
+// Whether the split-K slices of one tile may be summed inside a cluster (distributed shared memory).  A CTA finishes tile_n / split
+// columns: 8 or more, of tiles and splits that are asked for whole chunks of 32.
+bool cluster_reduce_ok(int tile_m, int tile_n, int tile_k, int stages, int split, bool asked) {
+  return tile_m == kTileM && (split == 2 || split == 4 || split == 8) && tile_n / split >= (asked ? 32 : 8) &&
          size_t(split - 1) * (tile_n / split) * kTileM * 4 <= size_t(stages) * stage_bytes_of(tile_m, tile_n, tile_k);
 }
 
@@ -254,8 +259,9 @@ double estimate_cycles(const gieb_conv_desc& d, const Geometry& g, int tile_m, i
   const bool overlapped = sharing >= 2.0 || (mh * tile_n <= 256 && tiles_per_sm >= 2.0);
   double total = 4500.0 + tiles_per_sm * kb_per_split * slab + (overlapped ? epilogue : tiles_per_sm * epilogue);
   if (real_split > 1) {
-    if (reduce == 2)  // two cluster barriers + pushing all but the own share of the FP32 tile at ~16 B/clk
-      total += 2000.0 + double(real_split - 1) / real_split * (double(kTileM) * tile_n * 4.0) / 16.0;
+    // two cluster barriers + pushing all but the own share of the FP32 tile at ~16 B/clk
+    if (reduce == 2)
+      total += (d.precision == GIEB_FP8_E4M3 || d.precision == GIEB_TF32 ? 2000.0 : 1000.0) + double(real_split - 1) / real_split * (double(kTileM) * tile_n * 4.0) / 16.0;
     else total += 6000.0 + 2.0 * real_split * double(g.y_elems) * 4.0 / 1500.0;      // extra launch + partial traffic
   }
   return total;
@@ -451,7 +457,9 @@ bool resolve_halo(const gieb_conv_desc& d, const Geometry& g, const gieb_conv_cf
   // channels the slab model is too short (co-resident CTAs do not double the issue rate there), except for FP8; TF32 layers
   // rarely gain (13 of the 15 between 0.85 and 1.05 lose).
   double margin = best_load >= 2 ? 0.85 : (b.pair ? 0.90 : 0.945);
-  if (b.split_k > 1) margin = 1.0;
+  // (FP8: two layers that went to slabs in clusters at par lost 5 and 8 %, 6 x 448 -> 64 at 8 x 22 8.05 and 8.7 us)
+  // (16-bit: of thirty layers whose two estimates lie within 8 % those up to 3 % apart are 2 % slower as slabs, the others 1.5 % faster)
+  if (b.split_k > 1) margin = d.precision == GIEB_FP8_E4M3 ? 1.15 : 1.03;
   if (best_load >= 3) margin = (b.tile_n <= 64 && ph * pw == 1 && d.precision != GIEB_FP8_E4M3) ? 1.2 : 1.0;
   if (d.precision == GIEB_TF32) margin = 0.85;
   if (best >= 1e299 || (!asked && best >= margin * slab)) return false;
@@ -693,6 +701,8 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
     swap_ok = swap_ok && e[0] != '0';
     swap_forced = e[0] == '2';
   }
+  // (outputs of less than 16 pixels keep the slices of up to a sixteenth that they sum through the workspace)
+  const bool asked_split = (!complete && (c.tile_n || c.split_k || c.reduce)) || g.pixels < 16;
   // search (tile_m, tile_n, split_k, pair) unless fixed
   double best = 1e300;
   int best_m = 0, best_n = 0, best_s = 0, best_mode = 0, best_pair = 0, best_swap = 0;
@@ -767,9 +777,14 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
           if (mode == 1 && size_t(s) * size_t(g.y_elems) * 4 > (size_t(1) << 31)) continue;
           if (mode == 2) {
             const int st = c.stages ? c.stages : pick_stages(tm, tn, r->tile_k, kbs, ctas);
-            if (!even || !cluster_reduce_ok(tm, tn, r->tile_k, st, s)) continue;
-            // unasked, clusters are used only when the whole grid is one wave of one CTA per SM
-            if (c.reduce == 0 && ctas > kNumSms) continue;
+            if (!even || !cluster_reduce_ok(tm, tn, r->tile_k, st, s, asked_split)) continue;
+            // unasked, clusters are used only when the whole grid is one wave of one CTA per SM (16 clusters of eight, of which 15 fit:
+            // 4 x 512 -> 512 at 14 x 14, 3x3/2, channel-contiguous 13.2 us, 8.1 as 32 of four)
+            // A tile in pieces of less than 32 columns is not for long slices of TF32, whose slabs take longer than the model has them:
+            // 8 x 640 -> 128 at 14 x 14, 5x5, eleven slices through the workspace 26.4 us, eight in clusters 28.3; up to 23 slabs per
+            // slice 19 of 21 such layers gain.
+            if (!asked_split && !complete && d.precision == GIEB_TF32 && tn / s < 32 && kbs > 24) continue;
+            if (c.reduce == 0 && (ctas > kNumSms || (!asked_split && !complete && ctas > int64_t(lone_clusters(s)) * s))) continue;
           }
           // tiles of 128 or 256 channels that a CTA finishes alone may keep the accumulator transposed: both forms compete
           const bool can_swap = swap_ok && s == 1 && tn >= 128;
@@ -869,10 +884,14 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
   // how the split-K slices are summed
   if (c.reduce < 0 || c.reduce > 2) return no("reduce must be 0 (auto), 1 (workspace) or 2 (cluster)");
   r->reduce = r->split_k > 1 ? best_mode : 0;
-  if (r->reduce == 2 && !cluster_reduce_ok(r->tile_m, r->tile_n, r->tile_k, stages, r->split_k))
+  if (r->reduce == 2 && !cluster_reduce_ok(r->tile_m, r->tile_n, r->tile_k, stages, r->split_k, asked_split))
     return no("cluster reduction needs tile_m 128, split_k 2, 4 or 8 dividing tile_n / 32, and a ring that holds the received slices");
   const size_t floor = smem_floor(r->pair ? tmem_cols_of(kTileM, r->tile_n) : tmem_cols_of(r->tile_m, r->tile_n), r->pair || r->reduce == 2);
   if (r->smem < floor) r->smem = floor;
+  // Clusters that fit the machine with one CTA per SM keep to that: two of a launch's CTAs on one SM while others have none share its
+  // operand feed (28 clusters of four, 4 x 1024 -> 256 at 14 x 14, channel-contiguous, four slabs per slice: 7.7 us, 5.9 with this; 16 of
+  // four, one image 5.8 and 5.1).
+  if (r->reduce == 2 && r->smem < kLoneSmem && int64_t(r->tiles_m) * r->tiles_n <= lone_clusters(r->split_k)) r->smem = kLoneSmem;
   r->ws_part = r->split_k > 1 && r->reduce == 1 ? align256(size_t(r->split_k) * size_t((g.y_elems + 3) & ~int64_t(3)) * 4) : 0;
   r->ws_total = r->ws_x + r->ws_w + r->ws_part;
   if (r->ws_total > (size_t(180) << 30) / 4) return no("workspace exceeds a quarter of device memory");

@@ -1,0 +1,74 @@
+"""Split-K inside clusters where a CTA finishes 8 or 16 columns of a tile instead of whole chunks of 32: every pair of tile and split,
+channel tails inside a unit of eight, both layouts with and without a residual, outputs off their alignment."""
+import numpy as np
+import pytest
+
+import gpu_util as gu
+
+pytestmark = pytest.mark.gpu
+
+# tile_n, split: units of 8 columns that a CTA finishes: 1, 2, 1, 2, 4
+POINTS = [(32, 4), (32, 2), (64, 8), (64, 4), (128, 4)]
+
+
+def _cfg(pkg, p, tile_n, split, flags=0):
+    """The point with every field set, as a query reports it (left to the library, narrow shares are its own choice)."""
+    auto = pkg.query(gu.pkg_problem(pkg, p, flags)).cfg
+    return pkg.make_cfg(tile_m=128, tile_n=tile_n, tile_k=auto.tile_k, stages=4, split_k=split, variant=1, reduce=2, cta_pair=1)
+
+
+@pytest.mark.parametrize("tile_n,split", POINTS)
+@pytest.mark.parametrize("filters,off", [(64, 0), (70, 0), (61, 1), (129, 3)])
+@pytest.mark.parametrize("prec_name", ["fp16", "bf16", "tf32"])
+def test_nchw(pkg, orc, oracle, tile_n, split, filters, off, prec_name):
+    prec = {"fp16": orc.FP16, "bf16": orc.BF16, "tf32": orc.TF32}[prec_name]
+    p = orc.Problem.P(2, 256, 9, 7, filters, 3, 3, 1, 1, 1, 1, precision=prec, bias=filters != 70, relu=filters % 2 == 0)
+    x, w, b = oracle.make_conv_data(p, 40 + tile_n + split, filters % 4)
+    ref, scale = oracle.conv2d(p, x, w, b if p.has_bias else None)
+    got, plan, out = gu.run_conv(pkg, oracle, p, x, w, b if p.has_bias else None, cfg=_cfg(pkg, p, tile_n, split), offsets=(0, 0, off))
+    c = plan.info.cfg
+    assert (c.tile_n, c.split_k, c.reduce) == (tile_n, split, 2)
+    m = oracle.compare(p, got, ref, scale)   # the reference's policy: rounding of sums of this length
+    assert m.passed(), m.summary()
+    again, _, out2 = gu.run_conv(pkg, oracle, p, x, w, b if p.has_bias else None, plan=plan, offsets=(0, 0, off))
+    assert np.array_equal(out.raw_bits(), out2.raw_bits())
+
+
+@pytest.mark.parametrize("tile_n,split", POINTS)
+@pytest.mark.parametrize("filters,off", [(64, 0), (72, 0), (72, 1), (61, 0)])
+@pytest.mark.parametrize("with_res", [False, True])
+@pytest.mark.parametrize("nhwc", [False, True])
+def test_layouts_and_residual(pkg, orc, oracle, tile_n, split, filters, off, with_res, nhwc):
+    import torch
+    prec = orc.FP16 if (tile_n + split) % 8 else orc.BF16
+    args = (3, 208, 6, 11, filters, 3, 3, 1, 1, 1, 1)
+    p_lin = orc.Problem.P(*args, precision=prec, bias=True, relu=False)
+    p = orc.Problem.P(*args, precision=prec, bias=True, relu=True)
+    x, w, b = oracle.make_conv_data(p, 90 + tile_n, split % 4)
+    lin, scale = oracle.conv2d(p_lin, x, w, b)
+    res = oracle.quantize(prec, oracle.rng(71).uniform(-1, 1, lin.size)).reshape(lin.shape) if with_res else np.zeros_like(lin)
+    ref = np.maximum(lin.astype(np.float64) + res, 0.0).astype(np.float32)
+    scale = (scale.astype(np.float64) + np.abs(res)).astype(np.float32)
+    swap = (lambda a: np.ascontiguousarray(a.transpose(0, 2, 3, 1))) if nhwc else (lambda a: a)
+    flags = (pkg.FLAG_INPUT_NHWC | pkg.FLAG_OUTPUT_NHWC if nhwc else 0) | (pkg.FLAG_RESIDUAL if with_res else 0)
+    plan = pkg.ConvPlan(gu.pkg_problem(pkg, p, flags), _cfg(pkg, p, tile_n, split, flags))
+    assert (plan.info.cfg.tile_n, plan.info.cfg.split_k, plan.info.cfg.reduce) == (tile_n, split, 2)
+    stream = torch.cuda.current_stream().cuda_stream
+    tx, px = gu.to_device_storage(oracle, prec, swap(x))
+    tw, pw = gu.to_device_storage(oracle, prec, w)
+    tb, pb = gu.to_device_storage(oracle, prec, b)
+    tr, pr = gu.to_device_storage(oracle, prec, swap(res), off)
+    ws = gu.Workspace(plan.workspace_bytes)
+    out = gu.OutBuf(prec, int(np.prod(p.y_shape)), off)
+    if with_res:
+        plan.launch_fused(px, pw, pb, pr, out.ptr, ws.ptr, plan.workspace_bytes, stream)
+    else:
+        plan.launch(px, pw, pb, out.ptr, ws.ptr, plan.workspace_bytes, stream)
+    torch.cuda.synchronize()
+    assert plan.device_status() == 0
+    ws.check_guard()
+    B, O, P, Q = p.y_shape
+    got = out.read(oracle)
+    got = np.ascontiguousarray(got.reshape(B, P, Q, O).transpose(0, 3, 1, 2)) if nhwc else got.reshape(p.y_shape)
+    m = oracle.compare(p, got, ref, scale)
+    assert m.passed(), m.summary()
