@@ -1386,6 +1386,7 @@ int launch_impl(const gieb_conv_plan* pl, const void* x, const void* w, const vo
   if (!(stage_mask & 2u)) {
   } else if (r.swap) GIEB_CUDA(conv_tc_swap_launch(r.tile_m, r.tile_n, r.tile_k, tm_act, tm_wgt, tm_out, p, grid, r.smem, st));
   else if (r.pair) GIEB_CUDA(conv_tc_pair_launch(r.tile_n, r.tile_k, tm_act, tm_wgt, tm_out, tm_res, p, grid, r.smem, st));
+  else if (r.reduce == 2) GIEB_CUDA(conv_tc_cluster_launch(r.tile_n, r.tile_k, r.epi_warps, tm_act, tm_wgt, p, grid, r.smem, st));
   else GIEB_CUDA(conv_tc_launch(r.tile_m, r.tile_n, r.tile_k, r.epi_warps, tm_act, tm_wgt, tm_out, tm_res, p, grid, r.smem, st));
   if (ev) GIEB_CUDA(cudaEventRecord(ev[2], st));
   if (r.reduce == 1 && (stage_mask & 4u))
@@ -1402,6 +1403,7 @@ cudaError_t prepare_kernels(const gieb_conv_desc& d, const Geometry& g, const Re
   if (r.halo) return conv_halo_prepare(r.tile_n, r.epi_warps, r.pair != 0, kMaxDynamicSmem);
   // The general kernel: a partial last slab, or rows that TMA cannot store (which tensors off their alignment are as well).
   const bool tail = r.tile_k == 64 && r.c_padded % 64 != 0;
+  if (r.reduce == 2) return conv_tc_cluster_prepare(r.tile_n, r.tile_k, r.epi_warps, tail, kMaxDynamicSmem);
   for (int general = 0; general < 2; ++general) {
     if (general ? !(tail || r.row_epilogue || r.tma_epilogue) : (tail || r.row_epilogue)) continue;
     const cudaError_t e = r.swap   ? conv_tc_swap_prepare(r.tile_m, r.tile_n, r.tile_k, general != 0, kMaxDynamicSmem)

@@ -349,7 +349,11 @@ __device__ __forceinline__ void with_output_type(const ConvTcParams& p, F&& f) {
 // GENERAL: with the slab loops over partial last slabs and the row-wise output.  Kernels without them are what a layer takes that
 // needs neither: carried along unused, the two cost every launch 0.2-0.4 us and odd NCHW planes 3-4 % (instruction fetch and
 // spilled registers: 64 -> 288 at 37 x 18, 3x3, 3 images 5.42 us, 5.23 without; 128 -> 284 at 35 x 35, 1x1, 45 images 21.3, 19.9).
-template <int BN, int BK, int MH, int EW, bool PAIR, bool SWAP, bool GENERAL>
+// CLUSTER: the split-K slices of a tile are the CTAs of a cluster and are summed inside it; one tile per CTA.  Kernels of their own for
+// the same reason: with this path in every kernel, 64 -> 16 at 12 x 34, 1x1, 17 images took 4.20 us, 4.03 without, FP8 64 -> 512 at 35 x
+// 35, 1x1, 6.44 and 5.98; and a cluster that need not carry the others' epilogues 640 -> 64 at 8 x 64, 1x1/2, 5 images 4.76 and 4.57, 512 -> 512
+// at 7 x 7, 3x3, repack included, 10.13 and 9.82.
+template <int BN, int BK, int MH, int EW, bool PAIR, bool SWAP, bool GENERAL, bool CLUSTER>
 __global__ void __launch_bounds__(32 * (kProducerWarps + 1 + EW), (EW == 16 || PAIR) ? 1 : 2)  // EW = 8: at most 80 registers, two CTAs per SM
 conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__ CUtensorMap tm_wgt,
                const __grid_constant__ CUtensorMap tm_out, const __grid_constant__ CUtensorMap tm_res, const ConvTcParams p) {
@@ -357,6 +361,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
   constexpr uint32_t A_HALF_BYTES = kTileM * ROW_BYTES;
   constexpr uint32_t A_BYTES = MH * A_HALF_BYTES;
   static_assert(!PAIR || (MH == 1 && BN >= 32), "a CTA pair computes one 256-pixel tile");
+  static_assert(!CLUSTER || (MH == 1 && !PAIR && !SWAP), "a cluster's tiles are 128 pixels of a CTA each");
   static_assert(!SWAP || (!PAIR && BN % 128 == 0), "the transposed accumulator takes 128 channels per instruction");
   constexpr int B_ROWS = PAIR ? BN / 2 : BN;                   // weight rows this CTA loads per slab
   constexpr uint32_t B_BYTES = B_ROWS * ROW_BYTES;
@@ -385,7 +390,6 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int stages = p.stages;
   const int tiles_mn = p.tiles_m * p.tiles_n;
-  const bool cluster = !PAIR && p.cluster_split > 1;
   const uint32_t pair_rank = PAIR ? ptx::cluster_ctarank() : 0u;  // 0 = leader (issues the MMAs), 1 = peer
   const bool leader = pair_rank == 0;
   // persistent walk over the tile list: by CTA, or by CTA pair
@@ -467,7 +471,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
     const uint32_t full0 = PAIR ? ptx::map_to_cta(ptx::smem_u32(&full_bar[0]), 0u) : 0u;
     for (int tile = tile_first; alive && tile < p.num_tiles; tile += tile_step) {
       int z, rest;
-      if (cluster) {  // slices of a tile sit side by side in one cluster
+      if constexpr (CLUSTER) {  // slices of a tile sit side by side in one cluster
         rest = p.fd_cluster.div(tile);
         z = tile - rest * p.cluster_split;
       } else {
@@ -552,7 +556,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
       skip = i - num_kb;  // how far this warp's next slab lies into the next tile
     }
     join_setup();  // warps without a slab of their own
-    if (cluster) {  // the two cluster barriers of the epilogue's reduction count every thread
+    if constexpr (CLUSTER) {  // the two cluster barriers of the epilogue's reduction count every thread
       ptx::cluster_sync_all();
       ptx::cluster_sync_all();
     }
@@ -567,7 +571,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
     bool alive = leader && !(p.debug_skip & 2u);  // the peer CTA of a pair issues nothing: the leader's instructions drive both tensor cores
     for (int tile = tile_first; alive && tile < p.num_tiles; tile += tile_step, ++tcount) {
       int z, rest;
-      if (cluster) {  // slices of a tile sit side by side in one cluster
+      if constexpr (CLUSTER) {  // slices of a tile sit side by side in one cluster
         rest = p.fd_cluster.div(tile);
         z = tile - rest * p.cluster_split;
       } else {
@@ -678,7 +682,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
       __syncwarp();
     }
     join_setup();  // the peer CTA's warp joins here (a no-op for a warp that had a tile)
-    if (cluster) {
+    if constexpr (CLUSTER) {
       ptx::cluster_sync_all();
       ptx::cluster_sync_all();
     }
@@ -726,7 +730,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
     const uint32_t acc_empty0 = PAIR ? ptx::map_to_cta(ptx::smem_u32(&acc_empty[0]), 0u) : 0u;  // the leader's barriers
     for (int tile = tile_first; tile < p.num_tiles; tile += tile_step, ++tcount) {
       int z, rest;
-      if (cluster) {  // slices of a tile sit side by side in one cluster
+      if constexpr (CLUSTER) {  // slices of a tile sit side by side in one cluster
         rest = p.fd_cluster.div(tile);
         z = tile - rest * p.cluster_split;
       } else {
@@ -756,7 +760,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
       // (before the accumulator is even complete) so that the load overlaps the main loop.
       auto stage_box = [&](int k) { return epi_base + size_t(we * p.epi_boxes + k) * 2048; };
       auto prefetch_residual = [&](int h) {
-        if (p.res_tma && lane == 0) {
+        if (!CLUSTER && p.res_tma && lane == 0) {
           ptx::bulk_wait_group_read0();  // earlier stores of this warp have left the boxes
           for (int k = 0; k < kEpiBufs; ++k) {
             const int chunk = par + EG * k;
@@ -804,19 +808,19 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
       __syncwarp();
       ptx::tc_fence_after_sync();
       if (!__all_sync(0xffffffffu, ok)) {
-        if (cluster) {  // keep the cluster's barriers balanced so that the peers can leave as well
+        if constexpr (CLUSTER) {  // keep the cluster's barriers balanced so that the peers can leave as well
           ptx::cluster_sync_all();
           ptx::cluster_sync_all();
         }
         break;
       }
-      if (!cluster && p.tiles_n > 1 && tile + tile_step < p.num_tiles) {
+      if (!CLUSTER && p.tiles_n > 1 && tile + tile_step < p.num_tiles) {
         const int next = tile + tile_step - p.fd_tiles_mn.div(tile + tile_step) * tiles_mn;
         const int next_n0 = (next - p.fd_tiles_n.div(next) * p.tiles_n) * BN;
         if (next_n0 != n0) bias_next = load_bias(next_n0);
       }
       const uint32_t acc = tmem_base + buf * ACC_COLS;
-      if (cluster) {
+      if constexpr (CLUSTER) {
         // Split-K inside a cluster (MH = 1, one tile per CTA).  CTA `rank` holds the partial sums of K-slice `rank` for the whole
         // tile and owns the columns [rank * cpo, (rank + 1) * cpo): every CTA pushes the columns it does not own into the owner's
         // (now idle) operand ring through distributed shared memory, then each owner adds the received slices to its own in a fixed
@@ -1109,16 +1113,16 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
 
 // One point of the family: its opt-in to large dynamic shared memory, and its launch.  Clusters are CTA pairs (blockIdx.x =
 // 2 * pair + rank) or the split-K slices of a tile.
-template <int BN, int BK, int MH, int EW, bool PAIR, bool SWAP, bool GENERAL>
+template <int BN, int BK, int MH, int EW, bool PAIR, bool SWAP, bool GENERAL, bool CLUSTER>
 cudaError_t prepare_point(size_t smem_bytes) {
-  return cudaFuncSetAttribute(conv_tc_kernel<BN, BK, MH, EW, PAIR, SWAP, GENERAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_bytes));
+  return cudaFuncSetAttribute(conv_tc_kernel<BN, BK, MH, EW, PAIR, SWAP, GENERAL, CLUSTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_bytes));
 }
 
-template <int BN, int BK, int MH, int EW, bool PAIR, bool SWAP, bool GENERAL>
+template <int BN, int BK, int MH, int EW, bool PAIR, bool SWAP, bool GENERAL, bool CLUSTER>
 cudaError_t launch_point(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& to, const CUtensorMap& tr, const ConvTcParams& p,
                          dim3 grid, size_t smem, cudaStream_t st) {
-  const unsigned cluster = PAIR ? 2u : unsigned(p.cluster_split > 1 ? p.cluster_split : 1);
-  const cudaError_t e = launch_pdl_cluster(conv_tc_kernel<BN, BK, MH, EW, PAIR, SWAP, GENERAL>, grid, dim3(32 * (kProducerWarps + 1 + EW)), smem,
+  const unsigned cluster = PAIR ? 2u : (CLUSTER ? unsigned(p.cluster_split) : 1u);
+  const cudaError_t e = launch_pdl_cluster(conv_tc_kernel<BN, BK, MH, EW, PAIR, SWAP, GENERAL, CLUSTER>, grid, dim3(32 * (kProducerWarps + 1 + EW)), smem,
                                            st, cluster, ta, tw, to, tr, p);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();
@@ -1126,7 +1130,7 @@ cudaError_t launch_point(const CUtensorMap& ta, const CUtensorMap& tw, const CUt
 
 // FN for the general or the lean kernel of a point, by the variable `general` of the caller.
 #define GIEB_TC_EITHER(FN, BN, BK, MH, EW, PAIR, SWAP, ...) \
-  return general ? FN<BN, BK, MH, EW, PAIR, SWAP, true>(__VA_ARGS__) : FN<BN, BK, MH, EW, PAIR, SWAP, false>(__VA_ARGS__)
+  return general ? FN<BN, BK, MH, EW, PAIR, SWAP, true, false>(__VA_ARGS__) : FN<BN, BK, MH, EW, PAIR, SWAP, false, false>(__VA_ARGS__)
 
 }  // namespace
 }  // namespace gieb

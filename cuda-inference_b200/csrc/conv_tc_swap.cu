@@ -8,16 +8,16 @@ namespace {
 
 #define GIEB_TC_SWAP_DISPATCH(FN, ...)                                                        \
   switch (tile_m / 128 * 100000 + tile_n * 100 + tile_k) {                                    \
-    case 1 * 100000 + 128 * 100 + 16: return FN<128, 16, 1, 8, false, true, false>(__VA_ARGS__); \
-    case 2 * 100000 + 128 * 100 + 16: return FN<128, 16, 2, 8, false, true, false>(__VA_ARGS__); \
-    case 1 * 100000 + 128 * 100 + 32: return FN<128, 32, 1, 8, false, true, false>(__VA_ARGS__); \
-    case 2 * 100000 + 128 * 100 + 32: return FN<128, 32, 2, 8, false, true, false>(__VA_ARGS__); \
+    case 1 * 100000 + 128 * 100 + 16: return FN<128, 16, 1, 8, false, true, false, false>(__VA_ARGS__); \
+    case 2 * 100000 + 128 * 100 + 16: return FN<128, 16, 2, 8, false, true, false, false>(__VA_ARGS__); \
+    case 1 * 100000 + 128 * 100 + 32: return FN<128, 32, 1, 8, false, true, false, false>(__VA_ARGS__); \
+    case 2 * 100000 + 128 * 100 + 32: return FN<128, 32, 2, 8, false, true, false, false>(__VA_ARGS__); \
     case 1 * 100000 + 128 * 100 + 64: GIEB_TC_EITHER(FN, 128, 64, 1, 8, false, true, __VA_ARGS__); \
     case 2 * 100000 + 128 * 100 + 64: GIEB_TC_EITHER(FN, 128, 64, 2, 8, false, true, __VA_ARGS__); \
-    case 1 * 100000 + 256 * 100 + 16: return FN<256, 16, 1, 8, false, true, false>(__VA_ARGS__); \
-    case 2 * 100000 + 256 * 100 + 16: return FN<256, 16, 2, 8, false, true, false>(__VA_ARGS__); \
-    case 1 * 100000 + 256 * 100 + 32: return FN<256, 32, 1, 8, false, true, false>(__VA_ARGS__); \
-    case 2 * 100000 + 256 * 100 + 32: return FN<256, 32, 2, 8, false, true, false>(__VA_ARGS__); \
+    case 1 * 100000 + 256 * 100 + 16: return FN<256, 16, 1, 8, false, true, false, false>(__VA_ARGS__); \
+    case 2 * 100000 + 256 * 100 + 16: return FN<256, 16, 2, 8, false, true, false, false>(__VA_ARGS__); \
+    case 1 * 100000 + 256 * 100 + 32: return FN<256, 32, 1, 8, false, true, false, false>(__VA_ARGS__); \
+    case 2 * 100000 + 256 * 100 + 32: return FN<256, 32, 2, 8, false, true, false, false>(__VA_ARGS__); \
     case 1 * 100000 + 256 * 100 + 64: GIEB_TC_EITHER(FN, 256, 64, 1, 8, false, true, __VA_ARGS__); \
     case 2 * 100000 + 256 * 100 + 64: GIEB_TC_EITHER(FN, 256, 64, 2, 8, false, true, __VA_ARGS__); \
     default: return cudaErrorInvalidValue;                                                    \

@@ -245,6 +245,11 @@ cudaError_t conv_tc_pair_prepare(int tile_n, int tile_k, bool general, size_t sm
 cudaError_t conv_tc_pair_launch(int tile_n, int tile_k, const CUtensorMap& tm_act, const CUtensorMap& tm_wgt, const CUtensorMap& tm_out,
                                 const CUtensorMap& tm_res, const ConvTcParams& p, dim3 grid, size_t smem_bytes, cudaStream_t stream);
 
+// Points whose split-K slices are summed inside a cluster: tile_m = 128, `grid` = tiles x p.cluster_split.  tail: partial last slabs.
+cudaError_t conv_tc_cluster_prepare(int tile_n, int tile_k, int epi_warps, bool tail, size_t smem_bytes);
+cudaError_t conv_tc_cluster_launch(int tile_n, int tile_k, int epi_warps, const CUtensorMap& tm_act, const CUtensorMap& tm_wgt, const ConvTcParams& p,
+                                   dim3 grid, size_t smem_bytes, cudaStream_t stream);
+
 // Transposed-accumulator points (lane = output channel): NCHW output through TMA stores; tile_n 128 or 256, 16-bit types, 8 epilogue warps.
 // tm_out: y as the 3-D tensor {P*Q, O, N} with a 32-pixel x 32-channel box and 64-byte swizzle (read when p.swap_tma).
 cudaError_t conv_tc_swap_prepare(int tile_m, int tile_n, int tile_k, bool general, size_t smem_bytes);

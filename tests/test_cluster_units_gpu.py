@@ -34,6 +34,22 @@ def test_nchw(pkg, orc, oracle, tile_n, split, filters, off, prec_name):
     assert np.array_equal(out.raw_bits(), out2.raw_bits())
 
 
+# channels 80 at tile_k 64: the last slab of a tap is partial (kernels of their own)
+@pytest.mark.parametrize("tile_k,channels,stages", [(16, 16, 8), (32, 32, 4), (64, 128, 4), (64, 80, 4)])
+@pytest.mark.parametrize("tile_n", [32, 64, 128, 256])
+@pytest.mark.parametrize("split", [2, 4])
+def test_every_kernel(pkg, orc, oracle, tile_k, channels, stages, tile_n, split):
+    p = orc.Problem.P(2, channels, 9, 8, 150, 4, 4, 1, 1, 0, 0, precision=orc.FP16, bias=True, relu=True)
+    x, w, b = oracle.make_conv_data(p, 7 + tile_n + split, 1)
+    ref, scale = oracle.conv2d(p, x, w, b)
+    cfg = pkg.make_cfg(tile_m=128, tile_n=tile_n, tile_k=tile_k, stages=stages, split_k=split, variant=1, reduce=2, cta_pair=1)
+    got, plan, _ = gu.run_conv(pkg, oracle, p, x, w, b, cfg=cfg)
+    c = plan.info.cfg
+    assert (c.tile_n, c.tile_k, c.split_k, c.reduce) == (tile_n, tile_k, split, 2)
+    m = oracle.compare(p, got, ref, scale)
+    assert m.passed(), m.summary()
+
+
 @pytest.mark.parametrize("tile_n,split", POINTS)
 @pytest.mark.parametrize("filters,off", [(64, 0), (72, 0), (72, 1), (61, 0)])
 @pytest.mark.parametrize("with_res", [False, True])
