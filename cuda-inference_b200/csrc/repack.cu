@@ -219,8 +219,10 @@ __device__ __forceinline__ void repack_tile_sub(uint32_t* tile, const RepackJob&
   }
 }
 
-// Up to two jobs in one launch (activations + weights): block indices [0, b.blocks) belong to job b, the weights, whose blocks take
-// longest, the rest to job a (32 x 512 -> 512 at 14 x 14, 3x3: 34.05 us the other way round, 33.8 so).
+// Up to two jobs in one launch (activations + weights): block indices [0, b.blocks) belong to job b, whose blocks take longest, the rest
+// to job a: the weights (32 x 512 -> 512 at 14 x 14, 3x3: 34.05 us the other way round, 33.8 so), but the activations where they are a
+// strided selection ahead of a 1x1 filter (64 -> 640 at 36 x 36, stride 2, 3 images: 6.9 us the other way round, 6.1 so; 24 such layers
+// 7.85 and 7.72 on average).
 template <int RESIDENT>  // blocks per SM that the registers are cut for; 0: as they come
 __global__ void __launch_bounds__(256, RESIDENT) repack_jobs_kernel(const RepackJob a, const RepackJob b) {
   __shared__ __align__(16) uint32_t smem[kTile * kLdWords];
@@ -433,7 +435,8 @@ cudaError_t launch_jobs(RepackJob a, int64_t tiles_a, RepackJob b, int64_t tiles
   // are spread evenly (launch_pdl_spread): 4 x 1024 x 14 x 14 ahead of its convolution 8.5 and 8.3 us, 16 x 256 x 30 x 31 14.6 and 14.4.
   // (A strided selection keeps sixteen loads in flight per thread, which 32 registers do not hold.)
   const auto kernel = a.blocks + b.blocks > unsigned(kNumSms) * 8 && a.mode != 4 ? repack_jobs_kernel<8> : repack_jobs_kernel<0>;
-  return launch_pdl_spread(kernel, a.blocks + b.blocks, kTile * kLdWords * 4, 0, stream, a, b);
+  const bool turned = a.mode == 4 && b.blocks > 0;
+  return launch_pdl_spread(kernel, a.blocks + b.blocks, kTile * kLdWords * 4, 0, stream, turned ? b : a, turned ? a : b);
 }
 
 }  // namespace
