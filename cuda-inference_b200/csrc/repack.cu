@@ -10,6 +10,7 @@
 
 #include "internal.h"
 #include "ptx.cuh"
+#include "repack_grid.h"
 
 namespace gieb {
 namespace {
@@ -407,18 +408,18 @@ RepackJob make_job(const void* src, void* dst, int batch, int channels, int hw, 
   j.src = static_cast<const uint16_t*>(src);
   j.dst = static_cast<uint16_t*>(dst);
   j.C = channels; j.HW = hw; j.Cp = c_padded; j.batch = batch;
-  j.c_tiles = (c_padded + kTile - 1) / kTile;
+  j.c_tiles = tiles_of(c_padded, kTile);
   j.span = kTile;
   if (hw < 32 && hw <= kSmallHwMax) {
     j.mode = 2;
     j.hw_tiles = 1;
     j.span = (kTile * kSmallHwMax / hw) / kTile * kTile;  // as many 64-channel groups as the slab holds
-    if (j.span > ((c_padded + kTile - 1) / kTile) * kTile) j.span = ((c_padded + kTile - 1) / kTile) * kTile;
-    j.c_tiles = (c_padded + j.span - 1) / j.span;
+    if (j.span / kTile > j.c_tiles) j.span = j.c_tiles * kTile;
+    j.c_tiles = tiles_of(c_padded, j.span);
   } else {
     j.mode = ((reinterpret_cast<uintptr_t>(src) & 15u) == 0 && (hw & 7) == 0) ? 1
              : (((reinterpret_cast<uintptr_t>(src) & 3u) == 0 && (hw & 1) == 0) ? 3 : 0);
-    j.hw_tiles = (hw + kTile - 1) / kTile;
+    j.hw_tiles = tiles_of(hw, kTile);
   }
   j.blocks = 0;
   j.prefetch = prefetch_enabled() ? 1 : 0;
@@ -465,8 +466,8 @@ cudaError_t repack_subsampled_launch(const void* x, void* xn, int batch, int cha
                                      int stride_w, int c_padded, const void* wsrc, void* wdst, int out_channels, cudaStream_t stream) {
   RepackJob a = make_job(x, xn, batch, channels, out_h * out_w, c_padded);
   a.mode = 4;
-  a.hw_tiles = (out_h * out_w + kTile - 1) / kTile;
-  a.c_tiles = (c_padded + kTile - 1) / kTile;
+  a.hw_tiles = tiles_of(out_h * out_w, kTile);
+  a.c_tiles = tiles_of(c_padded, kTile);
   a.span = kTile;
   a.src_hw = h * w; a.src_w = w; a.sub_ow = out_w; a.sub_sh = stride_h; a.sub_sw = stride_w;
   RepackJob b = a;

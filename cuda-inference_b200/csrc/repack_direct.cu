@@ -9,6 +9,7 @@
 
 #include "internal.h"
 #include "ptx.cuh"
+#include "repack_grid.h"
 
 namespace gieb {
 namespace {
@@ -137,15 +138,14 @@ bool repack_direct_launch(const void* src_a, void* dst_a, int batch_a, int ch_a,
   memset(&a, 0, sizeof(a));
   FilterJob b;
   memset(&b, 0, sizeof(b));
-  const uintptr_t at = reinterpret_cast<uintptr_t>(src_a);
-  int v = hw_a % 4 == 0 && at % 8 == 0 ? 4 : (hw_a % 2 == 0 && at % 4 == 0 ? 2 : 1);
+  int v = direct_pixels(hw_a, reinterpret_cast<uintptr_t>(src_a));
   if (src_a != nullptr) {
     a.src = static_cast<const uint16_t*>(src_a);
     a.dst = static_cast<uint16_t*>(dst_a);
     a.C = ch_a; a.HW = hw_a; a.Cp = cp_a;
-    a.hw_tiles = (hw_a + 32 * v - 1) / (32 * v);
-    a.c_tiles = (cp_a + 63) / 64;
-    const int64_t n = int64_t(a.hw_tiles) * a.c_tiles * batch_a;
+    a.hw_tiles = tiles_of(hw_a, 32 * v);
+    a.c_tiles = tiles_of(cp_a, 64);
+    const int64_t n = direct_blocks(v, hw_a, cp_a, batch_a);
     // Above these sizes repack.cu's wider rows count for more than its way is long (with the convolution, here and there): V 4 with
     // rows of whole vectors, 100 blocks 7.17 and 7.24 us, 192 13.8 and 13.6, 896 21.1 and 19.2; other rows of V 4, 256 blocks 13.6 and
     // 14.0, 512 21.3 and 21.0; V 2, 384 13.3 and 13.6, 960 15.6 and 14.4; V 1, 768 13.9 and 14.2, 1984 15.5 and 15.7, 3120 27.2 and
