@@ -858,6 +858,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant
         for (int u = par; u < cpo >> 3; u += EG) {
           const int col = rank * cpo + u * 8;
           if (n0 + col >= p.out_channels) break;
+          __syncwarp();  // lanes without a pixel come from the unit before ahead of the others; the load is for the whole warp
           uint32_t own[8];
           ptx::tmem_ld_32x32b_x8(acc_w + uint32_t(col), own);
           const uint8_t* src = stage_base + size_t(u * 2) * (kTileM * 16) + row * 16;

@@ -88,3 +88,46 @@ def test_layouts_and_residual(pkg, orc, oracle, tile_n, split, filters, off, wit
     got = np.ascontiguousarray(got.reshape(B, P, Q, O).transpose(0, 3, 1, 2)) if nhwc else got.reshape(p.y_shape)
     m = oracle.compare(p, got, ref, scale)
     assert m.passed(), m.summary()
+
+
+# Planes of 200 pixels in boxes of 64: the last box of an image has eight, so warps hold lanes with a pixel and lanes without one while
+# they go from unit to unit (tile_n / split / 8 units of the CTA, two or four warps of a lane quarter).
+@pytest.mark.parametrize("tile_n,split", [(64, 2), (64, 4), (128, 2), (128, 8), (256, 2), (256, 4), (256, 8)])
+@pytest.mark.parametrize("variant,nhwc_out", [(2, False), (2, True), (4, False)])
+@pytest.mark.parametrize("with_res", [False, True])
+def test_lanes_without_a_pixel(pkg, orc, oracle, tile_n, split, variant, nhwc_out, with_res):
+    import torch
+    prec = orc.BF16 if split == 4 else orc.FP16
+    args = (3, 1024, 10, 20, 139, 1, 1, 1, 1, 0, 0)
+    p_lin = orc.Problem.P(*args, precision=prec, bias=True, relu=False)
+    p = orc.Problem.P(*args, precision=prec, bias=True, relu=True)
+    x, w, b = oracle.make_conv_data(p, 17 + tile_n + split, variant % 4)
+    lin, scale = oracle.conv2d(p_lin, x, w, b)
+    res = oracle.quantize(prec, oracle.rng(5).uniform(-1, 1, lin.size)).reshape(lin.shape) if with_res else np.zeros_like(lin)
+    ref = np.maximum(lin.astype(np.float64) + res, 0.0).astype(np.float32)
+    scale = (scale.astype(np.float64) + np.abs(res)).astype(np.float32)
+    swap = (lambda a: np.ascontiguousarray(a.transpose(0, 2, 3, 1))) if nhwc_out else (lambda a: a)
+    flags = (pkg.FLAG_OUTPUT_NHWC if nhwc_out else 0) | (pkg.FLAG_RESIDUAL if with_res else 0)
+    cfg = pkg.make_cfg(tile_m=128, tile_n=tile_n, tile_k=64, stages=4, split_k=split, variant=variant, reduce=2, cta_pair=1)
+    plan = pkg.ConvPlan(gu.pkg_problem(pkg, p, flags), cfg)
+    c = plan.info.cfg
+    assert (c.variant, c.tile_n, c.split_k, c.reduce) == (variant, tile_n, split, 2)
+    stream = torch.cuda.current_stream().cuda_stream
+    tx, px = gu.to_device_storage(oracle, prec, x)
+    tw, pw = gu.to_device_storage(oracle, prec, w)
+    tb, pb = gu.to_device_storage(oracle, prec, b)
+    tr, pr = gu.to_device_storage(oracle, prec, swap(res))
+    ws = gu.Workspace(plan.workspace_bytes)
+    out = gu.OutBuf(prec, int(np.prod(p.y_shape)))
+    if with_res:
+        plan.launch_fused(px, pw, pb, pr, out.ptr, ws.ptr, plan.workspace_bytes, stream)
+    else:
+        plan.launch(px, pw, pb, out.ptr, ws.ptr, plan.workspace_bytes, stream)
+    torch.cuda.synchronize()
+    assert plan.device_status() == 0
+    ws.check_guard()
+    B, O, P, Q = p.y_shape
+    got = out.read(oracle)
+    got = np.ascontiguousarray(got.reshape(B, P, Q, O).transpose(0, 3, 1, 2)) if nhwc_out else got.reshape(p.y_shape)
+    m = oracle.compare(p, got, ref, scale)   # one rounding to the stored type of an FP32 sum of 1024 products, bias and residual
+    assert m.passed(), m.summary()
