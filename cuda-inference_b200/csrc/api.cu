@@ -644,10 +644,12 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
     r->tile_k = c.tile_k ? c.tile_k : pick_tile_k(d.in_channels);
   }
   if (r->tile_k != 16 && r->tile_k != 32 && r->tile_k != 64) return no("tile_k must be 16, 32 or 64");
-  // A slab width that was asked for pads to whole slabs.  A configuration with every field set that names the automatic width is
-  // one that gieb_conv_query reported, or as good as one: it stands for the automatic layout.
+  // A slab width that was asked for pads to whole slabs.  A configuration with every field set that names the automatic width (on the
+  // gather route that of a gathered row) is one that gieb_conv_query reported, or as good as one: it stands for the automatic layout.
   const int units = channel_units(d);
-  const bool complete = c.tile_m && c.tile_n && c.stages && c.split_k && c.variant && c.cta_pair && c.tile_k && r->tile_k == pick_tile_k(units);
+  const int gc2 = r->gather_pairs ? r->gp_t * 8 : gather_c2;
+  const int auto_tile_k = gather ? (gc2 % 64 == 0 ? 64 : (gc2 % 32 == 0 ? 32 : 16)) : pick_tile_k(units);
+  const bool complete = c.tile_m && c.tile_n && c.stages && c.split_k && c.variant && c.cta_pair && c.tile_k && r->tile_k == auto_tile_k;
   const bool asked = c.tile_k && !complete && !halo;
   // Channels of a copy are padded to whole slabs of 64 as well where that costs little: the general kernel with its partial last
   // slab takes longer than the steps it leaves out.  tile_k 64 asked for (whole slabs) against the partial slab: padding by up to
@@ -659,8 +661,7 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
   if (halo && c.tile_k && r->tile_k != 64) return no("variant 6 (halo tiles) takes rows of 128 bytes: tile_k 64 (32 for TF32, 128 for FP8)");
   if (in_nhwc && asked && d.in_channels % r->tile_k != 0) return no("tile_k must divide the channel count of a channel-contiguous input (it is read in place)");
   if (gather) {
-    const int gc2 = r->gather_pairs ? r->gp_t * 8 : gather_c2;
-    if (!c.tile_k) r->tile_k = gc2 % 64 == 0 ? 64 : (gc2 % 32 == 0 ? 32 : 16);
+    if (!c.tile_k) r->tile_k = auto_tile_k;
     if (gc2 % r->tile_k != 0) return no("tile_k must divide the gathered row length (padded kernel_w * channels)");
     r->c_padded = gc2;
   } else {

@@ -284,6 +284,30 @@ def test_reported_configuration_gives_the_same_plan(pkg):
         assert seen.get(kind, 0) >= 3, (kind, seen)
 
 
+def test_reported_configuration_of_gathered_rows(pkg):
+    """The same for layers of few channels and wide kernels, whose slab width is that of a gathered row: split and unsplit, with the
+    slices summed in clusters (shares of 8 columns and up) or in the workspace."""
+    import random
+    rng = random.Random(11)
+    seen = {}
+    for _ in range(2500):
+        k = rng.choice([5, 7, 9, 11, 13])
+        c, o = rng.randint(1, 7), rng.choice([8, 16, 24, 32, 48, 64, 96, 128, 200, 256])
+        h, w, s = rng.randint(5, 40), rng.randint(5, 40), rng.choice([1, 1, 2])
+        flags = rng.choice([0, pkg.FLAG_OUTPUT_NHWC]) | rng.choice([0, pkg.FLAG_RESIDUAL]) | rng.choice([0, pkg.FLAG_WEIGHTS_PREPACKED])
+        p = P(pkg, rng.choice([1, 1, 2, 3, 8]), c, h, w, o, k, k, s, s, k // 2, k // 2, precision=rng.choice([pkg.FP16, pkg.BF16]), has_bias=True, relu=True, flags=flags)
+        auto = pkg.query(p)
+        assert auto.supported
+        again = pkg.query(p, pkg.make_cfg(**{f: getattr(auto.cfg, f) for f, _ in auto.cfg._fields_}))
+        assert again.supported, (p, again.reason)
+        assert _reported(again) == _reported(auto), (p, _reported(auto), _reported(again))
+        kind = (auto.cfg.variant, auto.cfg.split_k > 1, auto.cfg.reduce)
+        seen[kind] = seen.get(kind, 0) + 1
+        if auto.cfg.variant == 5 and auto.cfg.reduce == 2 and auto.cfg.tile_n // auto.cfg.split_k < 32:
+            seen["narrow"] = seen.get("narrow", 0) + 1
+    assert all(seen.get(kind, 0) >= 50 for kind in [(5, False, 0), (5, True, 2), "narrow"]), seen
+
+
 def test_halo_variant_takes_and_refuses(pkg):
     """The halo-tile kernel by name: what it can run it runs with the fields given, what it cannot is refused with a reason."""
     p = P(pkg, 4, 144, 14, 14, 200, 3, 3, 1, 1, 1, 1, precision=pkg.FP16)
