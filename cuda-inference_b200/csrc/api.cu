@@ -549,7 +549,9 @@ int64_t image_ctas(const gieb_conv_desc& d, const Geometry& g, const Resolved& r
   return groups < ctas ? groups : ctas;
 }
 
-int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, char* why, size_t why_len) {
+// beyond_resident: slices that the workspace would sum may be clusters even where the machine does not hold all of them at once.  That is
+// slower (see the search), but takes no workspace.
+int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, char* why, size_t why_len, bool beyond_resident = false) {
   auto no = [&](const char* m) { snprintf(why, why_len, "%s", m); return GIEB_UNSUPPORTED; };
   memset(r, 0, sizeof(*r));
   const Geometry g = geometry(d);
@@ -785,7 +787,9 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
             // 8 x 640 -> 128 at 14 x 14, 5x5, eleven slices through the workspace 26.4 us, eight in clusters 28.3; up to 23 slabs per
             // slice 19 of 21 such layers gain.
             if (!asked_split && !complete && d.precision == GIEB_TF32 && tn / s < 32 && kbs > 24) continue;
-            if (c.reduce == 0 && (ctas > kNumSms || (!asked_split && !complete && ctas > int64_t(lone_clusters(s)) * s))) continue;
+            // Rounds of clusters lose to the workspace as well: 60 layers of 34 to 37 clusters of four or 16 to 18 of eight, the slices summed
+            // in the workspace instead: 0.71 of the time, 0.61 to 0.86 (6 x 696 -> 640 at 12 x 12, 5x5: 45.6 and 28.4 us).
+            if (c.reduce == 0 && (ctas > kNumSms || (!asked_split && !complete && !beyond_resident && ctas > int64_t(lone_clusters(s)) * s))) continue;
           }
           // tiles of 128 or 256 channels that a CTA finishes alone may keep the accumulator transposed: both forms compete
           const bool can_swap = swap_ok && s == 1 && tn >= 128;
@@ -1615,6 +1619,14 @@ int gieb_conv_forward_static(const gieb_conv_desc* desc, const gieb_conv_cfg* cf
   gieb_conv_plan pl;  // lives on the host stack for the duration of this call only
   char why[256] = "";
   if (resolve(*desc, cfg, &pl.r, why, sizeof(why)) != GIEB_OK) return fail(GIEB_UNSUPPORTED, "%.255s", why);
+  // Partial sums that the scratch does not hold: slices in clusters, more of them than fit the machine at once (6 x 624 -> 96 at 55 x 55,
+  // 5x5/2, channel-contiguous: 10.2 MB with partials, 3.0 MB without).
+  if (pl.r.ws_total > kStaticScratchBytes && pl.r.reduce == 1) {
+    Resolved rounds;
+    if (resolve(*desc, cfg, &rounds, why, sizeof(why), true) == GIEB_OK && rounds.ws_total <= kStaticScratchBytes &&
+        rounds.variant == pl.r.variant && rounds.c_padded == pl.r.c_padded)  // (converted weights are in the layout that a query reports)
+      pl.r = rounds;
+  }
   if (pl.r.ws_total > kStaticScratchBytes)
     return fail(GIEB_WORKSPACE_TOO_SMALL,
                 "this problem needs %zu bytes of scratch but the built-in scratch holds %zu bytes; "

@@ -199,6 +199,8 @@ GIEB_API int gieb_conv_launch_stages(const gieb_conv_plan* plan, unsigned stage_
  * call performs no cudaMalloc/cudaFree and calls no allocating routine.  Limits and rules:
  *   - problems whose scratch exceeds 8 MiB are refused with GIEB_WORKSPACE_TOO_SMALL (the message says how much is
  *     needed); use the plan API with your own workspace for those;
+ *     a layer whose slices a plan sums in the workspace, and whose partials alone are too much, has them summed in clusters
+ *     (reduce = 2) where a configuration does not say otherwise;
  *   - every GPU that loads the library carries the 8 MiB + 256 B until the process exits;
  *   - the first call on each device looks up the array's device address (with that device current); make that first
  *     call outside any stream capture;
@@ -208,7 +210,7 @@ GIEB_API int gieb_conv_launch_stages(const gieb_conv_plan* plan, unsigned stage_
  *   - a bounded device-side wait that runs out leaves y incomplete and is reported only through
  *     gieb_conv_static_status: call it (it waits for the stream) before using y;
  *   - there is no residual operand: GIEB_FLAG_RESIDUAL is refused, sm_100 devices only.
- * Results are bit-identical to gieb_conv_launch with the same configuration. */
+ * Results are bit-identical to gieb_conv_launch with the configuration that runs. */
 GIEB_API int gieb_conv_forward_static(const gieb_conv_desc* desc, const gieb_conv_cfg* cfg, const void* x, const void* w,
                                       const void* bias, void* y, void* stream);
 
