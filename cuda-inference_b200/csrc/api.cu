@@ -218,9 +218,9 @@ int pick_stages(int tile_m, int tile_n, int tile_k, int kb_per_split, int64_t ct
 }
 
 // Whether the split-K slices of one tile may be summed inside a cluster (distributed shared memory).  A CTA finishes tile_n / split
-// columns: 8 or more, of tiles and splits that are asked for whole chunks of 32.
-bool cluster_reduce_ok(int tile_m, int tile_n, int tile_k, int stages, int split, bool asked) {
-  return tile_m == kTileM && (split == 2 || split == 4 || split == 8) && tile_n / split >= (asked ? 32 : 8) &&
+// columns: 8 or more, or whole chunks of 32.
+bool cluster_reduce_ok(int tile_m, int tile_n, int tile_k, int stages, int split, bool whole_chunks) {
+  return tile_m == kTileM && (split == 2 || split == 4 || split == 8) && tile_n / split >= (whole_chunks ? 32 : 8) &&
          size_t(split - 1) * (tile_n / split) * kTileM * 4 <= size_t(stages) * stage_bytes_of(tile_m, tile_n, tile_k);
 }
 
@@ -235,8 +235,10 @@ bool cluster_reduce_ok(int tile_m, int tile_n, int tile_k, int stages, int split
 // reduce: 0 none, 1 FP32 partials in the workspace + reduction launch, 2 cluster.
 // swap: the accumulator is transposed (the instruction's M is 128 channels, its N the tile's pixels), so the issue cost
 // follows tile_m instead of tile_n, and the epilogue is short (one TMA store per 32 x 32 box).
+// asked: a tile, a split or a reduction is asked for; what is left open is chosen with the exchange at 2000 cycles for every type, the cost
+// of whole chunks of 32 columns that it is limited to.
 double estimate_cycles(const gieb_conv_desc& d, const Geometry& g, int tile_m, int tile_n, int tile_k, int split, int reduce, int total_kb,
-                       bool swap = false) {
+                       bool swap, bool asked) {
   const int kb_per_split = ceil_div(total_kb, split);
   const int real_split = ceil_div(total_kb, kb_per_split);
   const int64_t ctas = int64_t(ceil_div(g.pixels, tile_m)) * ceil_div(d.out_channels, tile_n) * real_split;
@@ -261,7 +263,7 @@ double estimate_cycles(const gieb_conv_desc& d, const Geometry& g, int tile_m, i
   if (real_split > 1) {
     // two cluster barriers + pushing all but the own share of the FP32 tile at ~16 B/clk
     if (reduce == 2)
-      total += (d.precision == GIEB_FP8_E4M3 || d.precision == GIEB_TF32 ? 2000.0 : 1000.0) + double(real_split - 1) / real_split * (double(kTileM) * tile_n * 4.0) / 16.0;
+      total += (asked || d.precision == GIEB_FP8_E4M3 || d.precision == GIEB_TF32 ? 2000.0 : 1000.0) + double(real_split - 1) / real_split * (double(kTileM) * tile_n * 4.0) / 16.0;
     else total += 6000.0 + 2.0 * real_split * double(g.y_elems) * 4.0 / 1500.0;      // extra launch + partial traffic
   }
   return total;
@@ -704,8 +706,9 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
     swap_ok = swap_ok && e[0] != '0';
     swap_forced = e[0] == '2';
   }
+  const bool asked_split = !complete && (c.tile_n || c.split_k || c.reduce);
   // (outputs of less than 16 pixels keep the slices of up to a sixteenth that they sum through the workspace)
-  const bool asked_split = (!complete && (c.tile_n || c.split_k || c.reduce)) || g.pixels < 16;
+  const bool whole_chunks = asked_split || g.pixels < 16;
   // search (tile_m, tile_n, split_k, pair) unless fixed
   double best = 1e300;
   int best_m = 0, best_n = 0, best_s = 0, best_mode = 0, best_pair = 0, best_swap = 0;
@@ -780,21 +783,21 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
           if (mode == 1 && size_t(s) * size_t(g.y_elems) * 4 > (size_t(1) << 31)) continue;
           if (mode == 2) {
             const int st = c.stages ? c.stages : pick_stages(tm, tn, r->tile_k, kbs, ctas);
-            if (!even || !cluster_reduce_ok(tm, tn, r->tile_k, st, s, asked_split)) continue;
+            if (!even || !cluster_reduce_ok(tm, tn, r->tile_k, st, s, whole_chunks)) continue;
             // unasked, clusters are used only when the whole grid is one wave of one CTA per SM (16 clusters of eight, of which 15 fit:
             // 4 x 512 -> 512 at 14 x 14, 3x3/2, channel-contiguous 13.2 us, 8.1 as 32 of four)
             // A tile in pieces of less than 32 columns is not for long slices of TF32, whose slabs take longer than the model has them:
             // 8 x 640 -> 128 at 14 x 14, 5x5, eleven slices through the workspace 26.4 us, eight in clusters 28.3; up to 23 slabs per
             // slice 19 of 21 such layers gain.
-            if (!asked_split && !complete && d.precision == GIEB_TF32 && tn / s < 32 && kbs > 24) continue;
+            if (!whole_chunks && !complete && d.precision == GIEB_TF32 && tn / s < 32 && kbs > 24) continue;
             // Rounds of clusters lose to the workspace as well: 60 layers of 34 to 37 clusters of four or 16 to 18 of eight, the slices summed
             // in the workspace instead: 0.71 of the time, 0.61 to 0.86 (6 x 696 -> 640 at 12 x 12, 5x5: 45.6 and 28.4 us).
-            if (c.reduce == 0 && (ctas > kNumSms || (!asked_split && !complete && !beyond_resident && ctas > int64_t(lone_clusters(s)) * s))) continue;
+            if (c.reduce == 0 && (ctas > kNumSms || (!whole_chunks && !complete && !beyond_resident && ctas > int64_t(lone_clusters(s)) * s))) continue;
           }
           // tiles of 128 or 256 channels that a CTA finishes alone may keep the accumulator transposed: both forms compete
           const bool can_swap = swap_ok && s == 1 && tn >= 128;
           for (int sw = (can_swap && swap_forced ? 1 : 0); sw <= (can_swap ? 1 : 0); ++sw) {
-            const double t = estimate_cycles(d, g, tm, tn, r->tile_k, s, mode, r->total_kb, sw != 0) +
+            const double t = estimate_cycles(d, g, tm, tn, r->tile_k, s, mode, r->total_kb, sw != 0, asked_split) +
                              (r->variant == 2 && !direct_n && tn < d.out_channels && tn < 256 ? 1e6 : 0.0);
             if (t < best) { best = t; best_m = tm; best_n = tn; best_s = s; best_mode = mode; best_pair = 0; best_swap = sw; }
           }
@@ -889,7 +892,7 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
   // how the split-K slices are summed
   if (c.reduce < 0 || c.reduce > 2) return no("reduce must be 0 (auto), 1 (workspace) or 2 (cluster)");
   r->reduce = r->split_k > 1 ? best_mode : 0;
-  if (r->reduce == 2 && !cluster_reduce_ok(r->tile_m, r->tile_n, r->tile_k, stages, r->split_k, asked_split))
+  if (r->reduce == 2 && !cluster_reduce_ok(r->tile_m, r->tile_n, r->tile_k, stages, r->split_k, whole_chunks))
     return no("cluster reduction needs tile_m 128, split_k 2, 4 or 8 dividing tile_n / 32, and a ring that holds the received slices");
   const size_t floor = smem_floor(r->pair ? tmem_cols_of(kTileM, r->tile_n) : tmem_cols_of(r->tile_m, r->tile_n), r->pair || r->reduce == 2);
   if (r->smem < floor) r->smem = floor;

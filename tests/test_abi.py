@@ -308,6 +308,29 @@ def test_reported_configuration_of_gathered_rows(pkg):
     assert all(seen.get(kind, 0) >= 50 for kind in [(5, False, 0), (5, True, 2), "narrow"]), seen
 
 
+def test_tiles_and_splits_asked_for_leave_the_rest_as_it_was(pkg):
+    """What is left open beside a tile, a split or a reduction that is asked for does not follow the choices for layers that ask for
+    nothing: shares of 32 columns and up, and their cost.  (route, tile_n, split_k, reduce) of layers where it makes a difference."""
+    for args, prec, flags, kw, want in [
+            ((11, 64, 85, 85, 232, 5, 5, 1, 1, 2, 2), pkg.FP16, 12, dict(reduce=2), (1, 256, 1, 0)),
+            ((22, 1024, 53, 53, 80, 1, 1, 1, 1, 0, 0), pkg.BF16, 2, dict(reduce=2), (4, 128, 1, 0)),
+            ((5, 835, 18, 18, 288, 1, 1, 2, 2, 0, 0), pkg.BF16, 16, dict(reduce=2), (4, 32, 1, 0)),
+            ((2, 576, 5, 4, 399, 5, 5, 2, 2, 2, 2), pkg.BF16, 12, dict(split_k=4), (1, 32, 4, 1)),
+            ((1, 1024, 17, 17, 128, 3, 3, 2, 2, 1, 1), pkg.BF16, 12, dict(split_k=4), (1, 32, 4, 1)),
+            ((9, 768, 6, 6, 400, 3, 3, 1, 1, 1, 1), pkg.FP16, 0, dict(split_k=8), (1, 128, 8, 1)),
+            ((2, 112, 33, 33, 32, 5, 5, 1, 1, 2, 2), pkg.FP16, 0, dict(tile_n=64), (1, 64, 8, 1)),
+            ((4, 704, 18, 12, 192, 1, 1, 1, 1, 0, 0), pkg.BF16, 14, dict(tile_n=64), (4, 64, 1, 0)),
+            ((2, 384, 31, 4, 192, 3, 3, 2, 2, 1, 1), pkg.BF16, 2, dict(tile_n=128), (1, 128, 14, 1)),
+            ((13, 64, 19, 19, 864, 5, 5, 1, 1, 2, 2), pkg.FP16, 12, dict(tile_n=64, reduce=2), (1, 64, 1, 0))]:
+        i = pkg.query(P(pkg, *args, precision=prec, has_bias=True, relu=True, flags=flags), pkg.make_cfg(**kw))
+        assert i.supported and (i.cfg.variant, i.cfg.tile_n, i.cfg.split_k, i.cfg.reduce) == want, (args, kw)
+    # shares of less than 32 columns: in a configuration whose fields are all set, not otherwise
+    p = P(pkg, 2, 256, 9, 7, 64, 3, 3, 1, 1, 1, 1, precision=pkg.FP16)
+    narrow = dict(tile_n=64, split_k=4, reduce=2)
+    assert not pkg.query(p, pkg.make_cfg(**narrow)).supported
+    assert pkg.query(p, pkg.make_cfg(tile_m=128, tile_k=64, stages=4, variant=1, cta_pair=1, **narrow)).supported
+
+
 def test_halo_variant_takes_and_refuses(pkg):
     """The halo-tile kernel by name: what it can run it runs with the fields given, what it cannot is refused with a reason."""
     p = P(pkg, 4, 144, 14, 14, 200, 3, 3, 1, 1, 1, 1, precision=pkg.FP16)
