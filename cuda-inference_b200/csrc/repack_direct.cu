@@ -20,6 +20,7 @@ struct DirectJob {
   int C, HW, Cp, hw_tiles, c_tiles;
   FastDiv fd_hw_tiles, fd_c_tiles;
   unsigned blocks;
+  int prefetch;  // L2 prefetch of the source lines before the dependency wait
 };
 struct FilterJob {
   const uint4* src;
@@ -27,6 +28,7 @@ struct FilterJob {
   int src_groups, groups, units;  // vectors of eight channels per filter before and after padding, units in all
   FastDiv fd_groups;
   unsigned blocks;
+  int prefetch;
 };
 
 // A block takes 64 channels by 128, 64 or 32 pixels (V = 4, 2, 1).  A warp covers 8 channel groups x 4 runs of V pixels, so that a store
@@ -44,7 +46,7 @@ __device__ __forceinline__ void direct_tile(const DirectJob& j, unsigned id) {
   const uint16_t* s = j.src + (size_t(bi) * j.C + c0) * j.HW + px;
   uint16_t* d = j.dst + (size_t(bi) * j.HW + px) * j.Cp + c0;
   // (an L2 fill, legal before the wait: see repack_jobs_kernel; one lane for each row of a warp)
-  if (ok && (V == 1 ? (lane >> 1) == 0 : (lane >> 3) == 0))
+  if (j.prefetch && ok && (V == 1 ? (lane >> 1) == 0 : (lane >> 3) == 0))
 #pragma unroll
     for (int k = 0; k < 8; ++k)
       if (c0 + k < j.C) ptx::prefetch_l2(s + size_t(k) * j.HW);
@@ -86,7 +88,8 @@ __device__ __forceinline__ void filter_units(uint4* slab, const FilterJob& j, un
   if (TAPS > 1 && j.src_groups == j.groups) {
     const uint4* s = j.src + size_t(id) * 256 * TAPS;
     const int n = min(256, j.units - int(id) * 256) * TAPS;
-    for (int i = t * 8; i < n; i += 256 * 8) ptx::prefetch_l2(s + i);
+    if (j.prefetch)
+      for (int i = t * 8; i < n; i += 256 * 8) ptx::prefetch_l2(s + i);
     ptx::grid_dep_wait();
     ptx::grid_dep_launch();
 #pragma unroll
@@ -138,6 +141,7 @@ bool repack_direct_launch(const void* src_a, void* dst_a, int batch_a, int ch_a,
   memset(&a, 0, sizeof(a));
   FilterJob b;
   memset(&b, 0, sizeof(b));
+  a.prefetch = b.prefetch = prefetch_enabled() ? 1 : 0;
   int v = direct_pixels(hw_a, reinterpret_cast<uintptr_t>(src_a));
   if (src_a != nullptr) {
     a.src = static_cast<const uint16_t*>(src_a);

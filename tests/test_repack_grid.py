@@ -39,3 +39,13 @@ def test_tiles_of_the_largest_planes(tmp_path):
     subprocess.check_call(["g++", "-std=c++17", "-Wall", "-Werror", "-ftrapv", "-I" + os.path.join(ROOT, "cuda-inference_b200", "csrc"), str(src), "-o", str(exe)])
     r = subprocess.run([str(exe)], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout
+
+
+def test_every_repack_asks_whether_to_prefetch():
+    """GIEB_DISABLE_PREFETCH switches the fills ahead of the dependency wait off in every file that issues them there."""
+    csrc = os.path.join(ROOT, "cuda-inference_b200", "csrc")
+    texts = {f: open(os.path.join(csrc, f)).read() for f in sorted(os.listdir(csrc)) if f.startswith("repack") and f.endswith(".cu")}
+    issuing = [f for f, t in texts.items() if "prefetch_l2(" in t]
+    assert len(issuing) == 2
+    for f in issuing:
+        assert "prefetch_enabled()" in texts[f], f

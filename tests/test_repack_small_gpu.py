@@ -79,3 +79,13 @@ def test_both_tensors_of_a_layer(pkg, shape, xoff, woff):
     assert torch.equal(got_w[:, :, :c], wt.view(o, c, rs).transpose(1, 2)) and not got_w[:, :, c:].any()
     assert torch.all(ws[nx:at_w] == 0x5a5a) and torch.all(ws[at_w + nw:] == 0x5a5a)
     plan.close()
+
+
+def test_without_prefetch():
+    """The same with the prefetches switched off (an environment variable that a process reads once)."""
+    import os
+    import subprocess
+    import sys
+    r = subprocess.run([sys.executable, "-m", "pytest", "-q", "-x", "-m", "gpu", "-k", "test_both_tensors_of_a_layer", os.path.abspath(__file__)],
+                       env=dict(os.environ, GIEB_DISABLE_PREFETCH="1"), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
