@@ -26,6 +26,7 @@ struct FilterJob {
   const uint4* src;
   uint4* dst;
   int src_groups, groups, units;  // vectors of eight channels per filter before and after padding, units in all
+  int per;                        // units of a block
   FastDiv fd_groups;
   unsigned blocks;
   int prefetch;
@@ -81,13 +82,14 @@ __device__ __forceinline__ void direct_tile(const DirectJob& j, unsigned id) {
 // to thread: no bank conflicts); where channels are padded, filters do not follow each other and each thread fetches its own.
 template <int TAPS>
 __device__ __forceinline__ void filter_units(uint4* slab, const FilterJob& j, unsigned id) {
-  const int t = threadIdx.x, unit = int(id) * 256 + t;
+  const int t = threadIdx.x, unit = int(id) * j.per + t;
+  const bool mine = t < j.per && unit < j.units;
   const int o = j.fd_groups.div(unit), g = unit - o * j.groups;
   uint4* d = j.dst + size_t(o) * TAPS * j.groups + g;
   uint4 v[TAPS];
   if (TAPS > 1 && j.src_groups == j.groups) {
-    const uint4* s = j.src + size_t(id) * 256 * TAPS;
-    const int n = min(256, j.units - int(id) * 256) * TAPS;
+    const uint4* s = j.src + size_t(id) * j.per * TAPS;
+    const int n = min(j.per, j.units - int(id) * j.per) * TAPS;
     if (j.prefetch)
       for (int i = t * 8; i < n; i += 256 * 8) ptx::prefetch_l2(s + i);
     ptx::grid_dep_wait();
@@ -99,16 +101,17 @@ __device__ __forceinline__ void filter_units(uint4* slab, const FilterJob& j, un
     for (int k = 0; k < TAPS; ++k)
       if (t + k * 256 < n) slab[t + k * 256] = v[k];
     __syncthreads();
+    if (mine)
 #pragma unroll
-    for (int k = 0; k < TAPS; ++k) v[k] = slab[t * TAPS + k];
+      for (int k = 0; k < TAPS; ++k) v[k] = slab[t * TAPS + k];
   } else {
     ptx::grid_dep_wait();
     ptx::grid_dep_launch();
 #pragma unroll
     for (int k = 0; k < TAPS; ++k)
-      v[k] = unit < j.units && g < j.src_groups ? j.src[(size_t(o) * j.src_groups + g) * TAPS + k] : make_uint4(0, 0, 0, 0);
+      v[k] = mine && g < j.src_groups ? j.src[(size_t(o) * j.src_groups + g) * TAPS + k] : make_uint4(0, 0, 0, 0);
   }
-  if (unit >= j.units) return;
+  if (!mine) return;
   uint32_t w[4 * TAPS];  // element (channel k, tap t) at TAPS * k + t
 #pragma unroll
   for (int k = 0; k < TAPS; ++k) {
@@ -130,7 +133,7 @@ __global__ void __launch_bounds__(256) repack_direct_kernel(const __grid_constan
 
 template <int V, int TAPS>
 cudaError_t direct_launch(const DirectJob& a, const FilterJob& b, cudaStream_t stream) {
-  return launch_pdl_spread(repack_direct_kernel<V, TAPS>, a.blocks + b.blocks, 0, TAPS > 1 ? 256 * TAPS * sizeof(uint4) : 0, stream, a, b);
+  return launch_pdl_spread(repack_direct_kernel<V, TAPS>, a.blocks + b.blocks, 0, TAPS > 1 ? size_t(b.per) * TAPS * sizeof(uint4) : 0, stream, a, b);
 }
 
 }  // namespace
@@ -169,7 +172,13 @@ bool repack_direct_launch(const void* src_a, void* dst_a, int batch_a, int ch_a,
     b.groups = cp_b / 8;
     b.units = int(units);
     b.fd_groups = FastDiv::make(b.groups);
-    b.blocks = unsigned((units + 255) / 256);
+    // Few filters of nine taps in blocks of 64 units, whose loads all threads share: as one block or a few of 256 they take one or a few
+    // SMs for 36 KB each (64 -> 64 at 56 x 56 7.14 and 6.92 us, 256 -> 16 at 10 x 10, 4 images 7.98 and 7.48, 160 -> 17 at 17 x 17, 6
+    // images 7.99 and 7.20, 128 -> 256 at 28 x 28 8.14 and 7.90).  From 8192 units on 256 are as fast or faster (256 -> 256 at 14 x 14,
+    // 32 images 14.55 and 14.82, 1024 -> 512 at 7 x 7 18.1 and 18.5; 320 -> 320 at 15 x 15, 12800 units, 9.61 and 9.30).  One tap: 512 ->
+    // 2048 at 7 x 7 7.95 and 9.59.
+    b.per = hw_b == 9 && units <= 4096 ? 64 : 256;
+    b.blocks = unsigned((units + b.per - 1) / b.per);
   }
   const int taps = src_b == nullptr ? 0 : hw_b;
   if (src_a == nullptr) v = 0;

@@ -38,7 +38,8 @@ def test_small_planes(pkg, shape, off):
 
 
 # filters, channels, taps, padded channels: shares of a block, exactly one, one more; padding; channels that are no whole groups
-FILTERS = [(31, 64, 9, 64), (32, 64, 9, 64), (33, 64, 9, 64), (257, 8, 9, 8), (70, 48, 9, 64), (3, 144, 9, 192), (5, 20, 9, 32), (512, 512, 9, 512),
+FILTERS = [(8, 64, 9, 64), (9, 56, 9, 64), (512, 64, 9, 64), (513, 64, 9, 64), (4097, 8, 9, 8),   # blocks of 64 units, and the first of 256
+           (31, 64, 9, 64), (32, 64, 9, 64), (33, 64, 9, 64), (257, 8, 9, 8), (70, 48, 9, 64), (3, 144, 9, 192), (5, 20, 9, 32), (512, 512, 9, 512),
            (31, 64, 1, 64), (257, 8, 1, 8), (70, 48, 1, 64), (1, 8, 1, 8), (9, 12, 1, 16)]
 
 
