@@ -221,9 +221,10 @@ __device__ __forceinline__ void repack_tile_sub(uint32_t* tile, const RepackJob&
 }
 
 // Up to two jobs in one launch (activations + weights): block indices [0, b.blocks) belong to job b, whose blocks take longest, the rest
-// to job a: the weights (32 x 512 -> 512 at 14 x 14, 3x3: 34.05 us the other way round, 33.8 so), but the activations where they are a
-// strided selection ahead of a 1x1 filter (64 -> 640 at 36 x 36, stride 2, 3 images: 6.9 us the other way round, 6.1 so; 24 such layers
-// 7.85 and 7.72 on average).
+// to job a: the weights (32 x 512 -> 512 at 14 x 14, 3x3: 34.05 us the other way round, 33.8 so; 24 x 339 -> 32 at 18 x 21, 3x3/2 11.65 and
+// 10.8), but the activations ahead of filters of one tap, whose block has no more than one filter's channels (12 x 77 -> 752 at 9 x 9:
+// 8.6 us the other way round, 7.1 so; 6 x 122 -> 768 at 13 x 13 8.0 and 6.5; 36 such layers 2.3 % on average, three 1.5 to 3.5 % slower; as a
+// strided selection, 64 -> 640 at 36 x 36, stride 2, 3 images, 6.9 and 6.1).
 template <int RESIDENT>  // blocks per SM that the registers are cut for; 0: as they come
 __global__ void __launch_bounds__(256, RESIDENT) repack_jobs_kernel(const RepackJob a, const RepackJob b) {
   __shared__ __align__(16) uint32_t smem[kTile * kLdWords];
@@ -436,7 +437,7 @@ cudaError_t launch_jobs(RepackJob a, int64_t tiles_a, RepackJob b, int64_t tiles
   // are spread evenly (launch_pdl_spread): 4 x 1024 x 14 x 14 ahead of its convolution 8.5 and 8.3 us, 16 x 256 x 30 x 31 14.6 and 14.4.
   // (A strided selection keeps sixteen loads in flight per thread, which 32 registers do not hold.)
   const auto kernel = a.blocks + b.blocks > unsigned(kNumSms) * 8 && a.mode != 4 ? repack_jobs_kernel<8> : repack_jobs_kernel<0>;
-  const bool turned = a.mode == 4 && b.blocks > 0;
+  const bool turned = b.blocks > 0 && b.HW == 1;
   return launch_pdl_spread(kernel, a.blocks + b.blocks, kTile * kLdWords * 4, 0, stream, turned ? b : a, turned ? a : b);
 }
 
