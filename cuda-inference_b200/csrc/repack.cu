@@ -8,6 +8,8 @@
 // always written with 128-bit stores (Cp % 8 == 0, 16-byte aligned base).
 #include <stdint.h>
 
+#include <utility>
+
 #include "internal.h"
 #include "ptx.cuh"
 #include "repack_grid.h"
@@ -224,7 +226,7 @@ __device__ __forceinline__ void repack_tile_sub(uint32_t* tile, const RepackJob&
 // to job a: the weights (32 x 512 -> 512 at 14 x 14, 3x3: 34.05 us the other way round, 33.8 so; 24 x 339 -> 32 at 18 x 21, 3x3/2 11.65 and
 // 10.8), but the activations ahead of filters of one tap, whose block has no more than one filter's channels (12 x 77 -> 752 at 9 x 9:
 // 8.6 us the other way round, 7.1 so; 6 x 122 -> 768 at 13 x 13 8.0 and 6.5; 36 such layers 2.3 % on average, three 1.5 to 3.5 % slower; as a
-// strided selection, 64 -> 640 at 36 x 36, stride 2, 3 images, 6.9 and 6.1).
+// strided selection, 64 -> 640 at 36 x 36, stride 2, 3 images, 6.9 and 6.1), and where they are few (activations_first()).
 template <int RESIDENT>  // blocks per SM that the registers are cut for; 0: as they come
 __global__ void __launch_bounds__(256, RESIDENT) repack_jobs_kernel(const RepackJob a, const RepackJob b) {
   __shared__ __align__(16) uint32_t smem[kTile * kLdWords];
@@ -437,7 +439,7 @@ cudaError_t launch_jobs(RepackJob a, int64_t tiles_a, RepackJob b, int64_t tiles
   // are spread evenly (launch_pdl_spread): 4 x 1024 x 14 x 14 ahead of its convolution 8.5 and 8.3 us, 16 x 256 x 30 x 31 14.6 and 14.4.
   // (A strided selection keeps sixteen loads in flight per thread, which 32 registers do not hold.)
   const auto kernel = a.blocks + b.blocks > unsigned(kNumSms) * 8 && a.mode != 4 ? repack_jobs_kernel<8> : repack_jobs_kernel<0>;
-  const bool turned = b.blocks > 0 && b.HW == 1;
+  const bool turned = b.blocks > 0 && (b.HW == 1 || activations_first(a.blocks, b.blocks));
   return launch_pdl_spread(kernel, a.blocks + b.blocks, kTile * kLdWords * 4, 0, stream, turned ? b : a, turned ? a : b);
 }
 
@@ -641,7 +643,7 @@ __device__ __forceinline__ float to_tf32(float v) {
 __global__ void __launch_bounds__(256) repack_tf32_kernel(const Tf32Job a, const Tf32Job b, int prefetch) {
   __shared__ __align__(16) float tile[kTf32Slab];
   static_assert(32 * kTf32Pitch <= kTf32Slab, "the 32 x 64 tile must fit the slab buffer");
-  const bool second = blockIdx.x < b.blocks;  // (the weights first, as in repack_jobs_kernel: 16 x 96 -> 192 at 27 x 27, 5x5, 34.1 and 32.4 us)
+  const bool second = blockIdx.x < b.blocks;  // (b first, mostly the weights, as in repack_jobs_kernel: 16 x 96 -> 192 at 27 x 27, 5x5, 34.1 and 32.4 us)
   const Tf32Job& j = second ? b : a;
   unsigned id = second ? blockIdx.x : blockIdx.x - b.blocks;
   const int hw_tile = int(id % unsigned(j.hw_tiles));
@@ -905,8 +907,9 @@ cudaError_t repack_tf32_pair_launch(const void* src_a, void* dst_a, int batch_a,
                                     void* dst_b, int batch_b, int ch_b, int hw_b, int cp_b, cudaStream_t stream) {
   if (int64_t((hw_a + 63) / 64) * ((cp_a + 31) / 32) * batch_a + int64_t((hw_b + 63) / 64) * ((cp_b + 31) / 32) * batch_b > 2147483647LL)
     return cudaErrorInvalidValue;
-  const Tf32Job a = make_tf32_job(src_a, dst_a, batch_a, ch_a, hw_a, cp_a);
-  const Tf32Job b = make_tf32_job(src_b, dst_b, batch_b, ch_b, hw_b, cp_b);
+  Tf32Job a = make_tf32_job(src_a, dst_a, batch_a, ch_a, hw_a, cp_a);
+  Tf32Job b = make_tf32_job(src_b, dst_b, batch_b, ch_b, hw_b, cp_b);
+  if (activations_first(a.blocks, b.blocks)) std::swap(a, b);
   const cudaError_t e = launch_pdl_spread(repack_tf32_kernel, a.blocks + b.blocks, kTf32Slab * sizeof(float), 0, stream, a, b, prefetch_enabled() ? 1 : 0);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();

@@ -60,7 +60,7 @@ def test_filters(pkg, shape, off):
 
 @pytest.mark.parametrize("xoff,woff", [(0, 0), (1, 0), (2, 8), (0, 1)])
 @pytest.mark.parametrize("shape", [(2, 64, 14, 14, 70, 3), (3, 128, 7, 7, 33, 3), (2, 72, 10, 9, 64, 3), (2, 144, 9, 11, 40, 3), (5, 64, 7, 7, 96, 1), (2, 96, 10, 5, 65, 1),
-                                   (2, 64, 9, 9, 40, 5), (3, 20, 7, 7, 24, 3)])
+                                   (2, 64, 9, 9, 40, 5), (3, 20, 7, 7, 24, 3), (12, 77, 9, 9, 752, 1), (1, 20, 6, 6, 300, 3)])  # the last two: activations first
 def test_both_tensors_of_a_layer(pkg, shape, xoff, woff):
     """One launch for the activations and the weights, as a forward call leaves them in the workspace."""
     import torch
@@ -79,6 +79,29 @@ def test_both_tensors_of_a_layer(pkg, shape, xoff, woff):
     assert torch.equal(got_x[:, :, :c], x.view(b, c, hw).transpose(1, 2)) and not got_x[:, :, c:].any()
     assert torch.equal(got_w[:, :, :c], wt.view(o, c, rs).transpose(1, 2)) and not got_w[:, :, c:].any()
     assert torch.all(ws[nx:at_w] == 0x5a5a) and torch.all(ws[at_w + nw:] == 0x5a5a)
+    plan.close()
+
+
+@pytest.mark.parametrize("shape", [(2, 64, 9, 9, 40, 3), (3, 20, 7, 7, 24, 5), (1, 64, 5, 5, 400, 3), (1, 40, 11, 13, 64, 1)])  # weights first, and few activations first
+def test_both_tensors_of_a_tf32_layer(pkg, shape):
+    """Values that TF32 holds exactly (13 low bits zero), so a permutation once more."""
+    import torch
+    b, c, h, w, o, k = shape
+    plan = pkg.ConvPlan(pkg.ConvProblem(b, c, h, w, o, k, k, 1, 1, k // 2, k // 2, precision=pkg.TF32, has_bias=False, relu=True))
+    cp, hw, rs = plan.info.padded_channels, h * w, k * k
+    g = torch.Generator(device="cuda")
+    g.manual_seed(c)
+    x, wt = [torch.randint(-1000, 1000, (n,), device="cuda", generator=g).float() for n in (b * c * hw, o * c * rs)]
+    y = torch.empty(b * o * hw, device="cuda")
+    ws = torch.full((plan.workspace_bytes // 4 + 64,), 0.5, device="cuda")
+    plan.launch_stages(1, x.data_ptr(), wt.data_ptr(), None, y.data_ptr(), ws.data_ptr(), plan.workspace_bytes, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    nx, nw = b * hw * cp, o * rs * cp
+    at_w = (4 * nx + 255) // 256 * 64
+    got_x, got_w = ws[:nx].view(b, hw, cp), ws[at_w:at_w + nw].view(o, rs, cp)
+    assert torch.equal(got_x[:, :, :c], x.view(b, c, hw).transpose(1, 2)) and not got_x[:, :, c:].any()
+    assert torch.equal(got_w[:, :, :c], wt.view(o, c, rs).transpose(1, 2)) and not got_w[:, :, c:].any()
+    assert torch.all(ws[nx:at_w] == 0.5) and torch.all(ws[at_w + nw:] == 0.5)
     plan.close()
 
 
