@@ -265,6 +265,11 @@ cudaError_t splitk_reduce_launch(const float* partial, int splits, int64_t total
 // Launches blocks of 256 threads with shared memory nobody uses (beyond `fixed` declared bytes and `dynamic` needed ones), so that an SM
 // takes no more of them than an even share.  Programmatic launches begin while the kernel ahead still holds most SMs: blocks that need
 // next to nothing all pile up on the few it leaves idle, eight at a time, and are still at it there when the others are free.
+// It is for one stream: 12 layers take 0.92 of the time without it.  Where another stream's kernel holds the machine, blocks that need not
+// wait for one of their own stream could all run on its idle SMs at once, and now wait for a place each: the same layer in two streams
+// takes 1.08 times as long, in three 1.10 (8 x 512 -> 512 at 14 x 14, 3x3, 25.6 and 30.0 us, 7 x 7 of one image 13.3 and 15.4), while 66
+// pairs of different layers take 0.995, 16 of them over 3 % longer.  Blocks kept apart by threads and registers that idle, which leave
+// shared memory to the other stream, cost two streams as much (30.0 and 29.9 us); two to an SM, 25.7, take most of the gain away.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl_spread(void (*kernel)(KArgs...), unsigned blocks, size_t fixed, size_t dynamic, cudaStream_t stream, Args&&... args) {
   const size_t share = (blocks + kNumSms - 1) / kNumSms, total = 233472 / (share + 1) + 128;  // of an SM's 228 KiB; a block takes 1 KiB besides

@@ -156,7 +156,9 @@ bool repack_direct_launch(const void* src_a, void* dst_a, int batch_a, int ch_a,
     // Above these sizes repack.cu's wider rows count for more than its way is long (with the convolution, here and there): V 4 with
     // rows of whole vectors, 100 blocks 7.17 and 7.24 us, 192 13.8 and 13.6, 896 21.1 and 19.2; other rows of V 4, 256 blocks 13.6 and
     // 14.0, 512 21.3 and 21.0; V 2, 384 13.3 and 13.6, 960 15.6 and 14.4; V 1, 768 13.9 and 14.2, 1984 15.5 and 15.7, 3120 27.2 and
-    // 26.9, beside filters of nine taps 768 14.2 and 14.6, 2048 23.9 and 23.4.
+    // 26.9, beside filters of nine taps 768 14.2 and 14.6, 2048 23.9 and 23.4.  140 layers of 40 to 2800 blocks: below these sizes 0.93 of
+    // the time (0.79 to 1.02), above them, to twice the size, 1.01 (0.92 to 1.11; V 1 with one tap, 0.965 up to 2800 blocks, and other rows
+    // of V 4, 0.99 up to 520, would bear a little more).
     if (n > (v == 4 ? (hw_a % 8 == 0 ? kNumSms : 2 * kNumSms) : (v == 2 ? 3 * kNumSms : (src_b != nullptr && hw_b == 9 ? 1024 : 2048)))) return false;
     a.fd_hw_tiles = FastDiv::make(a.hw_tiles);
     a.fd_c_tiles = FastDiv::make(a.c_tiles);
