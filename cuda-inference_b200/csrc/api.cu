@@ -712,6 +712,10 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
   // 1 x 59 -> 1663 at 4 x 3, 3x3/2: 6.7 and 7.5), but sum eight slices at most, each twice as long, and the error of that has not been
   // measured.)
   const bool whole_chunks = asked_split || g.pixels < 16;
+  const char* const cluster_needs =
+      whole_chunks ? "cluster reduction needs tile_m 128, split_k 2, 4 or 8 dividing tile_n / 32 (tile_n / 8 where every field is set and the output has "
+                     "16 pixels or more), no empty slice, and a ring that holds the received slices"
+                   : "cluster reduction needs tile_m 128, split_k 2, 4 or 8 dividing tile_n / 8, no empty slice, and a ring that holds the received slices";
   // search (tile_m, tile_n, split_k, pair) unless fixed
   double best = 1e300;
   int best_m = 0, best_n = 0, best_s = 0, best_mode = 0, best_pair = 0, best_swap = 0;
@@ -811,7 +815,7 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
   const bool untouched = c.tile_n == 0 && c.tile_k == 0 && c.stages == 0 && c.split_k == 0 && c.variant == 0 && c.tile_m == 0 && c.reduce == 0 && c.cta_pair == 0;
   if (untouched && resolve_halo(d, g, c, best, r)) return GIEB_OK;
   if (best_n == 0) {
-    if (c.reduce == 2) return no("cluster reduction needs tile_m 128, split_k 2, 4 or 8 dividing tile_n / 32 with no empty slice, and a ring that holds the received slices");
+    if (c.reduce == 2) return no(cluster_needs);
     if (c.split_k > 1) return no("reduction too short for this split-K factor");
     return no("no feasible tile configuration");
   }
@@ -896,7 +900,7 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
   if (c.reduce < 0 || c.reduce > 2) return no("reduce must be 0 (auto), 1 (workspace) or 2 (cluster)");
   r->reduce = r->split_k > 1 ? best_mode : 0;
   if (r->reduce == 2 && !cluster_reduce_ok(r->tile_m, r->tile_n, r->tile_k, stages, r->split_k, whole_chunks))
-    return no("cluster reduction needs tile_m 128, split_k 2, 4 or 8 dividing tile_n / 32, and a ring that holds the received slices");
+    return no(cluster_needs);
   const size_t floor = smem_floor(r->pair ? tmem_cols_of(kTileM, r->tile_n) : tmem_cols_of(r->tile_m, r->tile_n), r->pair || r->reduce == 2);
   if (r->smem < floor) r->smem = floor;
   // Clusters that fit the machine with one CTA per SM keep to that: two of a launch's CTAs on one SM while others have none share its

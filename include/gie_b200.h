@@ -107,8 +107,10 @@ typedef struct gieb_conv_cfg {
   int32_t tile_m;   /* output pixels per CTA tile: 128 or 256 (two accumulators share each weight tile); 0 = auto */
   int32_t reduce;   /* how split-K slices are summed: 0 = auto; 1 = FP32 partials in the workspace + a reduction launch;
                        2 = inside the convolution kernel: the slices of a tile form a thread-block cluster and are
-                           summed through distributed shared memory (split_k 2, 4 or 8 dividing tile_n / 32,
-                           tile_m 128); no partials in the workspace, no extra launch                       */
+                           summed through distributed shared memory (split_k 2, 4 or 8, tile_m 128); no partials in the
+                           workspace, no extra launch.  A CTA finishes tile_n / split_k columns: at least 8 in a
+                           configuration whose fields are all set as gieb_conv_query reports them, at least 32 (split_k
+                           divides tile_n / 32) beside fields left to the library and for outputs of less than 16 pixels */
   int32_t cta_pair; /* 0 = auto; 1 = every tile is computed by one CTA; 2 = 256-pixel tiles computed by pairs of CTAs (clusters
                        of two, tcgen05.mma.cta_group::2): each CTA stages its own 128 pixels and half of the weight tile, so
                        the weight traffic per SM is halved.  FP16 / BF16, tile_n 64, 128 or 256, tile_m 0 or 256, split-K

@@ -331,6 +331,21 @@ def test_tiles_and_splits_asked_for_leave_the_rest_as_it_was(pkg):
     assert pkg.query(p, pkg.make_cfg(tile_m=128, tile_k=64, stages=4, variant=1, cta_pair=1, **narrow)).supported
 
 
+def test_shares_of_a_cluster_are_named_in_the_refusal(pkg):
+    """Which columns per CTA a cluster reduction takes depends on what else is set and on the output's size; a refusal says so, in full."""
+    full = dict(tile_m=128, tile_k=64, stages=4, variant=1, cta_pair=1, reduce=2)
+    large, small = [P(pkg, 1, 512, s, s, 256, 3, 3, 1, 1, 1, 1, precision=pkg.FP16) for s in (4, 3)]   # 16 output pixels, and nine
+    for p, kw, takes, says in [(large, dict(full, tile_n=32, split_k=4), True, None), (large, dict(full, tile_n=128, split_k=8), True, None),
+                               (large, dict(full, tile_n=32, split_k=8), False, "dividing tile_n / 8,"), (large, dict(tile_n=32, split_k=4, reduce=2), False, "(tile_n / 8 where"),
+                               (large, dict(tile_n=128, split_k=4, reduce=2), True, None), (small, dict(full, tile_n=32, split_k=4), False, "16 pixels or more"),
+                               (small, dict(full, tile_n=128, split_k=4), True, None)]:
+        i = pkg.query(p, pkg.make_cfg(**kw))
+        assert bool(i.supported) == takes, (kw, i.reason)
+        if not takes:
+            reason = i.reason.decode() if isinstance(i.reason, bytes) else i.reason
+            assert says in reason and reason.endswith("received slices"), reason
+
+
 def test_halo_variant_takes_and_refuses(pkg):
     """The halo-tile kernel by name: what it can run it runs with the fields given, what it cannot is refused with a reason."""
     p = P(pkg, 4, 144, 14, 14, 200, 3, 3, 1, 1, 1, 1, precision=pkg.FP16)
