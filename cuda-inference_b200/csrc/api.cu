@@ -706,7 +706,8 @@ int resolve(const gieb_conv_desc& d, const gieb_conv_cfg* user, Resolved* r, cha
     swap_ok = swap_ok && e[0] != '0';
     swap_forced = e[0] == '2';
   }
-  const bool asked_split = !complete && (c.tile_n || c.split_k || c.reduce);
+  // (A split beside a reduction that is left open is asked for as well: a query reports both.)
+  const bool asked_split = (!complete || (c.split_k > 1 && c.reduce == 0)) && (c.tile_n || c.split_k || c.reduce);
   // (Outputs of less than 16 pixels keep whole chunks, and with them the slices of up to a sixteenth that they sum through the workspace.
   // Narrow shares would take 0.87 of the time, 60 layers, five of them 2 to 12 % slower (1 x 448 -> 1119 at 3 x 1, 3x3: 13.7 and 11.4 us;
   // 1 x 59 -> 1663 at 4 x 3, 3x3/2: 6.7 and 7.5), but sum eight slices at most, each twice as long, and the error of that has not been

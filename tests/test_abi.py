@@ -331,6 +331,21 @@ def test_tiles_and_splits_asked_for_leave_the_rest_as_it_was(pkg):
     assert pkg.query(p, pkg.make_cfg(tile_m=128, tile_k=64, stages=4, variant=1, cta_pair=1, **narrow)).supported
 
 
+def test_split_asked_for_with_its_reduction_left_open(pkg):
+    """A split with every field set but the reduction: no query reports that (it names the reduction of its slices), so how they are summed
+    is chosen as for any split that is asked for.  (tile_n, split_k) of layers where shares of less than 32 columns would be narrow ones."""
+    for args, prec, flags, tile_n, split, tile_k, want in [
+            ((1, 512, 26, 33, 83, 1, 1, 1, 1, 0, 0), pkg.FP16, 0, 64, 4, 64, 2103040), ((1, 512, 47, 37, 32, 5, 5, 1, 1, 2, 2), pkg.FP16, 12, 32, 4, 64, 1709568),
+            ((16, 32, 14, 24, 32, 5, 5, 2, 2, 2, 2), pkg.TF32, 0, 64, 4, 32, 1478656), ((2, 1024, 23, 23, 32, 1, 1, 1, 1, 0, 0), pkg.FP16, 14, 128, 8, 64, 1083392),
+            ((16, 768, 14, 14, 32, 1, 1, 1, 1, 0, 0), pkg.FP16, 28, 64, 4, 64, 1654784), ((2, 144, 51, 51, 64, 3, 3, 2, 2, 1, 1), pkg.FP8_E4M3, 0, 64, 4, 128, 2309120)]:
+        variant = 4 if args[5] == 1 else 1
+        cfg = dict(tile_m=128, tile_n=tile_n, tile_k=tile_k, stages=4, split_k=split, variant=variant, cta_pair=1)
+        p = P(pkg, *args, precision=prec, has_bias=True, relu=True, flags=flags)
+        i = pkg.query(p, pkg.make_cfg(**cfg))
+        assert i.supported and (i.cfg.reduce, i.workspace_bytes) == (1, want), (args, i.cfg.reduce, i.workspace_bytes)
+        assert pkg.query(p, pkg.make_cfg(reduce=2, **cfg)).supported
+
+
 def test_shares_of_a_cluster_are_named_in_the_refusal(pkg):
     """Which columns per CTA a cluster reduction takes depends on what else is set and on the output's size; a refusal says so, in full."""
     full = dict(tile_m=128, tile_k=64, stages=4, variant=1, cta_pair=1, reduce=2)
