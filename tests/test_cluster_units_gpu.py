@@ -131,3 +131,56 @@ def test_lanes_without_a_pixel(pkg, orc, oracle, tile_n, split, variant, nhwc_ou
     got = np.ascontiguousarray(got.reshape(B, P, Q, O).transpose(0, 3, 1, 2)) if nhwc_out else got.reshape(p.y_shape)
     m = oracle.compare(p, got, ref, scale)   # one rounding to the stored type of an FP32 sum of 1024 products, bias and residual
     assert m.passed(), m.summary()
+
+
+@pytest.mark.parametrize("tile_n,split", [(32, 4), (64, 4), (64, 8), (128, 8)])   # what plans of FP8 layers take by themselves
+@pytest.mark.parametrize("kernel", [3, 1])
+@pytest.mark.parametrize("filters", [64, 77])
+def test_fp8(pkg, orc, oracle, tile_n, split, kernel, filters):
+    import torch
+    from oracle import oracle as orc_mod
+    args = (2, 2048 if kernel == 1 else 512, 9, 7, filters, kernel, kernel, 1, 1, kernel // 2, kernel // 2)
+    p = orc.Problem.P(*args, precision=orc.FP16, bias=True, relu=True)   # every E4M3 value is an FP16 value
+    x, w, b = oracle.make_conv_data(p, 60 + tile_n + split, kernel)
+    x, w = orc_mod.e4m3_quantize(x), orc_mod.e4m3_quantize(w)
+    ref, scale = oracle.conv2d(p, x, w, b)
+    cfg = pkg.make_cfg(tile_m=128, tile_n=tile_n, tile_k=128, stages=4, split_k=split, variant=4 if kernel == 1 else 1, reduce=2, cta_pair=1)
+    plan = pkg.ConvPlan(pkg.ConvProblem(*args, precision=pkg.FP8_E4M3, has_bias=True, relu=True), cfg)
+    c = plan.info.cfg
+    assert (c.tile_n, c.split_k, c.reduce) == (tile_n, split, 2)
+    tx, tw, tb = [torch.from_numpy(a).cuda() for a in (orc_mod.e4m3_bits(x).ravel(), orc_mod.e4m3_bits(w).ravel(), np.ascontiguousarray(b, np.float32))]
+    ws = gu.Workspace(plan.workspace_bytes)
+    out = gu.OutBuf(orc.FP16, int(np.prod(p.y_shape)))
+    plan.launch(tx.data_ptr(), tw.data_ptr(), tb.data_ptr(), out.ptr, ws.ptr, plan.workspace_bytes, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert plan.device_status() == 0
+    ws.check_guard()
+    m = oracle.compare(p, out.read(oracle).reshape(p.y_shape), ref, scale)
+    assert m.passed(), m.summary()
+
+
+@pytest.mark.parametrize("relu", [False, True])
+@pytest.mark.parametrize("nhwc", [False, True])
+@pytest.mark.parametrize("prec_name", ["fp16", "bf16"])
+def test_infinities_and_nan(pkg, orc, oracle, relu, nhwc, prec_name):
+    """NaN, both infinities and infinities that meet, in different slices of the reduction: the classes of the outputs follow from the
+    inputs alone, whatever the order of the sums.  The ReLU of a NaN is zero here, as in every kernel of the library."""
+    import torch
+    prec = {"fp16": orc.FP16, "bf16": orc.BF16}[prec_name]
+    p = orc.Problem.P(1, 256, 9, 7, 72, 3, 3, 1, 1, 1, 1, precision=prec, bias=True, relu=relu)
+    x, w, b = oracle.make_conv_data(p, 3, 1)
+    x, w, b = x.reshape(1, 256, 9, 7).copy(), w.reshape(72, 256, 3, 3), b.reshape(72)
+    x[0, 5, 0, 0], x[0, 70, 4, 0], x[0, 130, 8, 6], x[0, 200, 8, 5], x[0, 255, 0, 6] = np.nan, np.inf, np.inf, -np.inf, -np.inf
+    want = torch.nn.functional.conv2d(torch.from_numpy(x).double(), torch.from_numpy(w).double(), torch.from_numpy(b).double(), padding=1).numpy()
+    if relu:
+        want = np.where(want > 0, want, 0.0)
+    flags = pkg.FLAG_OUTPUT_NHWC if nhwc else 0
+    got, plan, _ = gu.run_conv(pkg, oracle, p, x, w, b, cfg=_cfg(pkg, p, 64, 4, flags), flags=flags)
+    assert (plan.info.cfg.tile_n, plan.info.cfg.split_k, plan.info.cfg.reduce) == (64, 4, 2)
+    got = got.reshape(9, 7, 72).transpose(2, 0, 1)[None] if nhwc else got
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isposinf(got), np.isposinf(want)) and np.array_equal(np.isneginf(got), np.isneginf(want))
+    fin = np.isfinite(want)
+    # one rounding to the stored type (2^-11 or 2^-8 of the value), and the FP32 rounding of 2304 terms near zero
+    tol = {"fp16": 2.0 ** -11, "bf16": 2.0 ** -8}[prec_name] * np.abs(want[fin]) * 1.01 + 2304 * 2.0 ** -23 * np.abs(want[fin]).max()
+    assert np.all(np.abs(got[fin] - want[fin]) <= tol)
+    assert fin.sum() > 0.5 * fin.size and (relu or np.isnan(want).sum() >= 72)
