@@ -226,7 +226,8 @@ __device__ __forceinline__ void repack_tile_sub(uint32_t* tile, const RepackJob&
 // to job a: the weights (32 x 512 -> 512 at 14 x 14, 3x3: 34.05 us the other way round, 33.8 so; 24 x 339 -> 32 at 18 x 21, 3x3/2 11.65 and
 // 10.8), but the activations ahead of filters of one tap, whose block has no more than one filter's channels (12 x 77 -> 752 at 9 x 9:
 // 8.6 us the other way round, 7.1 so; 6 x 122 -> 768 at 13 x 13 8.0 and 6.5; 36 such layers 2.3 % on average, three 1.5 to 3.5 % slower; as a
-// strided selection, 64 -> 640 at 36 x 36, stride 2, 3 images, 6.9 and 6.1), and where they are few (activations_first()).
+// strided selection, 64 -> 640 at 36 x 36, stride 2, 3 images, 6.9 and 6.1), where they are few (activations_first()), and
+// where they are odd planes and not few (launch_jobs()).
 template <int RESIDENT>  // blocks per SM that the registers are cut for; 0: as they come
 __global__ void __launch_bounds__(256, RESIDENT) repack_jobs_kernel(const RepackJob a, const RepackJob b) {
   __shared__ __align__(16) uint32_t smem[kTile * kLdWords];
@@ -439,7 +440,11 @@ cudaError_t launch_jobs(RepackJob a, int64_t tiles_a, RepackJob b, int64_t tiles
   // are spread evenly (launch_pdl_spread): 4 x 1024 x 14 x 14 ahead of its convolution 8.5 and 8.3 us, 16 x 256 x 30 x 31 14.6 and 14.4.
   // (A strided selection keeps sixteen loads in flight per thread, which 32 registers do not hold.)
   const auto kernel = a.blocks + b.blocks > unsigned(kNumSms) * 8 && a.mode != 4 ? repack_jobs_kernel<8> : repack_jobs_kernel<0>;
-  const bool turned = b.blocks > 0 && (b.HW == 1 || activations_first(a.blocks, b.blocks));
+  // Activations of odd planes (nine vectors to a row, the longest tiles) come first as well where they are five blocks per SM or more: 30 x
+  // 64 -> 256 at 43 x 43, 3x3/2 15.35 us weights first, 14.6 so; 41 x 437 -> 64 at 39 x 39, 5x5/2 69.8 and 67.3.  70 such layers 0.992 of the
+  // time, 27 faster and six slower by over 1 %; four of 500 to 740 blocks 1.006, and even planes (94 layers of 600 blocks and more) 1.008.
+  const bool odd = a.mode == 0 && a.blocks >= unsigned(kNumSms) * 5;
+  const bool turned = b.blocks > 0 && (b.HW == 1 || odd || activations_first(a.blocks, b.blocks));
   return launch_pdl_spread(kernel, a.blocks + b.blocks, kTile * kLdWords * 4, 0, stream, turned ? b : a, turned ? a : b);
 }
 

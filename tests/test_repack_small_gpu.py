@@ -60,7 +60,8 @@ def test_filters(pkg, shape, off):
 
 @pytest.mark.parametrize("xoff,woff", [(0, 0), (1, 0), (2, 8), (0, 1)])
 @pytest.mark.parametrize("shape", [(2, 64, 14, 14, 70, 3), (3, 128, 7, 7, 33, 3), (2, 72, 10, 9, 64, 3), (2, 144, 9, 11, 40, 3), (5, 64, 7, 7, 96, 1), (2, 96, 10, 5, 65, 1),
-                                   (2, 64, 9, 9, 40, 5), (3, 20, 7, 7, 24, 3), (12, 77, 9, 9, 752, 1), (1, 20, 6, 6, 300, 3)])  # the last two: activations first
+                                   (2, 64, 9, 9, 40, 5), (3, 20, 7, 7, 24, 3), (12, 77, 9, 9, 752, 1), (1, 20, 6, 6, 300, 3),
+                                   (41, 130, 19, 21, 40, 3), (43, 130, 19, 21, 40, 5)])  # the last four: activations first (odd planes: from 740 blocks)
 def test_both_tensors_of_a_layer(pkg, shape, xoff, woff):
     """One launch for the activations and the weights, as a forward call leaves them in the workspace."""
     import torch
